@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "kernels.h"
+#include "panel_fp64.cuh"
 #include "../../include/wbem.h"
 
 namespace wbem {
@@ -291,64 +292,63 @@ cudaError_t launch_tile_fp64(int N, int q1, const double* X, const int* dnset, i
 // Vertex-singular panels: for row i, every panel holding a node of its
 // double-node set; the singular vertex is the first local vertex in the set
 // (source/bem_problem.cc:223-230), the rule is the polar vertex rule for that
-// vertex (:478-522). One thread per row, panels in ascending order.
-__global__ void k_singular_fp64(int N, const double* __restrict__ X, const int* __restrict__ dnset,
-                                const int* __restrict__ sptr, const int* __restrict__ scell,
-                                const int4* __restrict__ cell_dofs, double* __restrict__ Nm,
-                                double* __restrict__ Dm, DevErr* err) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= N) return;
-  const double xi = X[3 * (size_t)row], yi = X[3 * (size_t)row + 1], zi = X[3 * (size_t)row + 2];
+// vertex (:478-522). One CTA per row: its four warps take every fourth panel
+// with the rule's points over the lanes, then eight threads add the entries
+// (panels share vertices) in ascending panel order. Bound by the latency of
+// one panel's FP64 chain, not by throughput, at the sizes of the plain form:
+// one thread per row (panel after panel, 50 points each) took 0.57 ms at any
+// N up to 16,000; this takes 0.078 ms at N = 2,000.
+constexpr int kSingWarps = 4, kSingBatch = 32;  // panels whose sums are held at a time
+
+__global__ void __launch_bounds__(kSingWarps * 32)
+    k_singular_fp64(int N, const double* __restrict__ X, const int* __restrict__ dnset,
+                    const int* __restrict__ sptr, const int* __restrict__ scell,
+                    const int4* __restrict__ cell_dofs, double* __restrict__ Nm,
+                    double* __restrict__ Dm, DevErr* err) {
+  __shared__ double sums[kSingBatch][8];
+  __shared__ int ids[kSingBatch][4];
+  const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double x[3] = {X[3 * (size_t)row], X[3 * (size_t)row + 1], X[3 * (size_t)row + 2]};
   int set[kMaxSet];
 #pragma unroll
   for (int k = 0; k < kMaxSet; ++k) set[k] = dnset[(size_t)row * kMaxSet + k];
-  const int nsp = c_q.nsp;
-  for (int e = sptr[row]; e < sptr[row + 1]; ++e) {
-    const int cell = scell[e];
-    const int4 d = cell_dofs[cell];
-    const int id[4] = {d.x, d.y, d.z, d.w};
-    int v = -1;
-    for (int j = 0; j < 4 && v < 0; ++j)
-      if (in_set(set, id[j])) v = j;
-    if (v < 0) {
-      dev_fail(err, WBEM_ERR_ARG, 21, row, cell);
-      continue;
-    }
-    double P[4][3];
+  const int e1 = sptr[row + 1];
+  for (int e0 = sptr[row]; e0 < e1; e0 += kSingBatch) {
+    const int n = min(kSingBatch, e1 - e0);
+    for (int e = warp; e < n; e += kSingWarps) {
+      const int4 d = cell_dofs[scell[e0 + e]];
+      const int id[4] = {d.x, d.y, d.z, d.w};
+      int v = -1;
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+      for (int j = 3; j >= 0; --j)
+        if (in_set(set, id[j])) v = j;
+      double val = 0.0;
+      if (v < 0) {
+        if (lane == 0) dev_fail(err, WBEM_ERR_ARG, 21, row, scell[e0 + e]);
+      } else {
+        double P[4][3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) P[k][c] = X[3 * (size_t)id[k] + c];
-    double ln[4] = {0, 0, 0, 0}, ld[4] = {0, 0, 0, 0};
-    for (int q = 0; q < nsp; ++q) {
-      const double s = c_q.sp[v][q][0], t = c_q.sp[v][q][1], w = c_q.sp[v][q][2] * kInv4Pi;
-      double x[3], cr[3];
-      q1_geometry(P, s, t, x, cr);
-      const double det = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
-      const double Rx = x[0] - xi, Ry = x[1] - yi, Rz = x[2] - zi;
-      const double ri = rsqrt(fma(Rx, Rx, fma(Ry, Ry, Rz * Rz)));
-      const double sq = ri * det * w;
-      const double dq = -(Rx * cr[0] + Ry * cr[1] + Rz * cr[2]) * (ri * ri * ri) * w;
-      const double ph[4] = {(1 - s) * (1 - t), s * (1 - t), (1 - s) * t, s * t};
+        for (int k = 0; k < 4; ++k)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        ln[j] = fma(dq, ph[j], ln[j]);
-        ld[j] = fma(sq, ph[j], ld[j]);
+          for (int c = 0; c < 3; ++c) P[k][c] = X[3 * (size_t)id[k] + c];
+        val = singular_panel(P, x, c_q.sp[v], c_q.nsp, lane);
       }
+      if ((lane & 17) == 0) sums[e][(lane >> 1) & 7] = val;
+      if (lane < 4) ids[e][lane] = id[lane];
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      Nm[(size_t)row * N + id[j]] += ln[j];
-      Dm[(size_t)row * N + id[j]] += ld[j];
+    __syncthreads();
+    if (tid < 8) {
+      double* M = (tid < 4 ? Nm : Dm) + (size_t)row * N;
+      for (int e = 0; e < n; ++e) M[ids[e][tid & 3]] += sums[e][tid];
     }
+    __syncthreads();
   }
 }
 
 cudaError_t launch_singular_fp64(int N, const double* X, const int* dnset, const int* sptr,
                                  const int* scell, const int4* cell_dofs, double* Nm, double* Dm,
                                  DevErr* err, cudaStream_t s) {
-  const int bs = 64;
-  k_singular_fp64<<<(N + bs - 1) / bs, bs, 0, s>>>(N, X, dnset, sptr, scell, cell_dofs, Nm, Dm, err);
+  k_singular_fp64<<<N, kSingWarps * 32, 0, s>>>(N, X, dnset, sptr, scell, cell_dofs, Nm, Dm, err);
   return cudaGetLastError();
 }
 

@@ -19,6 +19,7 @@
 #include "context.h"
 #include "host_util.h"
 #include "kernels.h"
+#include "panel_fp64.cuh"
 
 namespace wbem {
 
@@ -73,91 +74,129 @@ struct SysOut {
   const uint8_t* sel;        // column selection of A2 / B2
 };
 
-// One thread per panel: FP64 geometry -> mixed record + near-test data.
-__global__ void k_cell_records_mixed(int C, const double* __restrict__ X,
-                                     const int4* __restrict__ cell_dofs, float* __restrict__ rec,
-                                     float4* __restrict__ cellgeo, float ratio) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
+// FP64 geometry -> mixed record + near-test data, a quadrature point per lane;
+// the panel sums (normal and moments) run over the points in ascending order
+// on seven lanes. HALF: two panels per warp (rules of at most 16 points).
+// Latency-bound at small N and FP64-bound at large: a thread per panel took
+// 0.128 ms at N = 600 as at N = 12,000, now 0.012 and 0.092 ms (a
+// whole warp per 16-point panel left half the FP64 lanes idle: 0.267 ms).
+constexpr int kRecWarps = 4;
+constexpr int kRecPoints = 36;  // most points of the mixed form's rule (order 6)
+
+template <bool HALF>
+__global__ void __launch_bounds__(kRecWarps * 32)
+    k_cell_records_mixed(int C, const double* __restrict__ X, const int4* __restrict__ cell_dofs,
+                         float* __restrict__ rec, float4* __restrict__ cellgeo, float ratio) {
+  constexpr int W = HALF ? 16 : 32, kPts = HALF ? 16 : kRecPoints;
+  // per panel and point: offset from the centre, cross product, its norm
+  __shared__ double s_pt[kRecWarps * (32 / W)][7][kPts];
+  const int slot = threadIdx.x / W, lane = threadIdx.x & (W - 1);
+  const int c0 = blockIdx.x * (kRecWarps * 32 / W) + slot;
+  const int c = min(c0, C - 1);  // past the last panel: its work again, not written
+  double(*pt)[kPts] = s_pt[slot];
   const int nq = c_qm.q1 * c_qm.q1;
   const int RF = mixed_rec_floats(nq);
   const int4 d = cell_dofs[c];
   const int id[4] = {d.x, d.y, d.z, d.w};
   double P[4][3];
+#pragma unroll
   for (int k = 0; k < 4; ++k)
+#pragma unroll
     for (int e = 0; e < 3; ++e) P[k][e] = X[3 * (size_t)id[k] + e];
-  double cen[3], nu[3] = {0, 0, 0};
+  double cen[3];
+#pragma unroll
   for (int e = 0; e < 3; ++e) cen[e] = 0.25 * (P[0][e] + P[1][e] + P[2][e] + P[3][e]);
-  double M[4] = {0, 0, 0, 0};
-  for (int q = 0; q < nq; ++q) {
+  for (int q = lane; q < nq; q += W) {
     double x[3], cr[3];
     q1_geo(P, c_qm.gp[q][0], c_qm.gp[q][1], x, cr);
-    const double w = c_qm.gp[q][2];
-    for (int e = 0; e < 3; ++e) nu[e] += cr[e] * w;
-    const double jw = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]) * w * kInv4PiM;
-    for (int j = 0; j < 4; ++j) M[j] += c_qm.phi[q][j] * jw;
-  }
-  const double nl = sqrt(nu[0] * nu[0] + nu[1] * nu[1] + nu[2] * nu[2]);
-  for (int e = 0; e < 3; ++e) nu[e] /= nl;
-  float* r = rec + (size_t)c * RF;
-  for (int q = 0; q < nq; ++q) {
-    double x[3], cr[3];
-    q1_geo(P, c_qm.gp[q][0], c_qm.gp[q][1], x, cr);
-    const double det = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
-    double del[3], n[3];
+#pragma unroll
     for (int e = 0; e < 3; ++e) {
-      del[e] = x[e] - cen[e];
-      n[e] = cr[e] / det;
+      pt[e][q] = x[e] - cen[e];
+      pt[3 + e][q] = cr[e];
     }
-    r[4 * q + 0] = (float)del[0];
-    r[4 * q + 1] = (float)del[1];
-    r[4 * q + 2] = (float)del[2];
-    r[4 * q + 3] = (float)(del[0] * del[0] + del[1] * del[1] + del[2] * del[2]);
-    r[4 * nq + 4 * q + 0] = (float)(n[0] - nu[0]);
-    r[4 * nq + 4 * q + 1] = (float)(n[1] - nu[1]);
-    r[4 * nq + 4 * q + 2] = (float)(n[2] - nu[2]);
-    r[4 * nq + 4 * q + 3] = (float)(del[0] * n[0] + del[1] * n[1] + del[2] * n[2]);
+    pt[6][q] = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+  }
+  __syncwarp();
+  // lanes 0..2: normal; lanes 3..6: moments
+  double sum = 0.0;
+  if (lane < 7) {
+    const double* a = lane < 3 ? pt[3 + lane] : pt[6];
+    for (int q = 0; q < nq; ++q) {
+      const double w = c_qm.gp[q][2];
+      sum += lane < 3 ? a[q] * w : c_qm.phi[q][max(lane - 3, 0)] * (a[q] * w * kInv4PiM);
+    }
+  }
+  double nu[3], M[4];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) nu[e] = __shfl_sync(0xffffffffu, sum, e, W);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) M[j] = __shfl_sync(0xffffffffu, sum, 3 + j, W);
+  const bool on = c0 < C;
+  const double nl = 1.0 / sqrt(nu[0] * nu[0] + nu[1] * nu[1] + nu[2] * nu[2]);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) nu[e] *= nl;
+  float* r = rec + (size_t)c * RF;
+  for (int q = lane; on && q < nq; q += W) {
+    const double det = pt[6][q], rdet = 1.0 / det;
+    double del[3], n[3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      del[e] = pt[e][q];
+      n[e] = pt[3 + e][q] * rdet;
+    }
+    reinterpret_cast<float4*>(r)[q] =
+        make_float4((float)del[0], (float)del[1], (float)del[2],
+                    (float)(del[0] * del[0] + del[1] * del[1] + del[2] * del[2]));
+    reinterpret_cast<float4*>(r)[nq + q] =
+        make_float4((float)(n[0] - nu[0]), (float)(n[1] - nu[1]), (float)(n[2] - nu[2]),
+                    (float)(del[0] * n[0] + del[1] * n[1] + del[2] * n[2]));
     r[8 * nq + q] = (float)(det * c_qm.gp[q][2] * kInv4PiM);
   }
+  // panel data: lane e splits one of centre, normal, moments, moment sum
   float* cd = r + 9 * nq;
-  for (int e = 0; e < 3; ++e) {
-    const df a = df_from_double(cen[e]);
-    cd[e] = a.hi;
-    cd[3 + e] = a.lo;
-    const df b = df_from_double(nu[e]);
-    cd[6 + e] = b.hi;
-    cd[9 + e] = b.lo;
+  if (on && lane < 11) {
+    const double v = lane < 3   ? (lane == 0 ? cen[0] : lane == 1 ? cen[1] : cen[2])
+                     : lane < 6 ? (lane == 3 ? nu[0] : lane == 4 ? nu[1] : nu[2])
+                     : lane < 8 ? (lane == 6 ? M[0] : M[1])
+                     : lane < 10 ? (lane == 8 ? M[2] : M[3])
+                                 : ((M[0] + M[1]) + M[2]) + M[3];
+    const df a = df_from_double(v);
+    // hi at 0..2, 6..8, 12..15, 20; lo at 3..5, 9..11, 16..19, 21
+    const int hi = lane < 3 ? lane : lane < 6 ? 3 + lane : lane < 10 ? 6 + lane : 20;
+    const int lo = lane < 6 ? 3 + hi : lane < 10 ? 4 + hi : 21;
+    cd[hi] = a.hi;
+    cd[lo] = a.lo;
+  } else if (on && lane == 11) {
+    cd[22] = 0.f;
+    cd[23] = 0.f;
+    for (int k = 9 * nq + 24; k < RF; ++k) r[k] = 0.f;
   }
-  double Mt = 0;
-  for (int j = 0; j < 4; ++j) {
-    const df a = df_from_double(M[j]);
-    cd[12 + j] = a.hi;
-    cd[16 + j] = a.lo;
-    Mt += M[j];
-  }
-  const df t = df_from_double(Mt);
-  cd[20] = t.hi;
-  cd[21] = t.lo;
-  cd[22] = 0.f;
-  cd[23] = 0.f;
-  for (int k = 9 * nq + 24; k < RF; ++k) r[k] = 0.f;
   // near test: centre (float) and (ratio * largest diagonal)^2, at least
   // 1.01 x the farthest vertex, so that every panel with the collocation
   // point (or a double-node partner of it) as a vertex tests near: the
-  // regular far-field kernel then needs no singular test of its own
-  double d1 = 0, d2 = 0, dv = 0;
-  for (int e = 0; e < 3; ++e) {
-    d1 += (P[3][e] - P[0][e]) * (P[3][e] - P[0][e]);
-    d2 += (P[2][e] - P[1][e]) * (P[2][e] - P[1][e]);
+  // regular far-field kernel then needs no singular test of its own.
+  // Lanes 0, 1: squared diagonals; lanes 2..5: squared vertex distances.
+  double d2 = 0.0;
+  if (lane < 6) {
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const double a = lane == 0   ? P[3][e]
+                       : lane == 1 ? P[2][e]
+                       : lane == 2 ? P[0][e]
+                       : lane == 3 ? P[1][e]
+                       : lane == 4 ? P[2][e]
+                                   : P[3][e];
+      const double b = lane == 0 ? P[0][e] : lane == 1 ? P[1][e] : cen[e];
+      d2 += (a - b) * (a - b);
+    }
   }
-  for (int k = 0; k < 4; ++k) {
-    double v = 0;
-    for (int e = 0; e < 3; ++e) v += (P[k][e] - cen[e]) * (P[k][e] - cen[e]);
-    dv = v > dv ? v : dv;
+  const double diag = fmax(__shfl_sync(0xffffffffu, d2, 0, W), __shfl_sync(0xffffffffu, d2, 1, W));
+  const double vert = fmax(fmax(__shfl_sync(0xffffffffu, d2, 2, W), __shfl_sync(0xffffffffu, d2, 3, W)),
+                           fmax(__shfl_sync(0xffffffffu, d2, 4, W), __shfl_sync(0xffffffffu, d2, 5, W)));
+  if (on && lane == 0) {
+    const double rad = fmax((double)ratio * sqrt(diag), 1.01 * sqrt(vert));
+    cellgeo[c] = make_float4((float)cen[0], (float)cen[1], (float)cen[2], (float)(rad * rad));
   }
-  const double diam = sqrt(d1 > d2 ? d1 : d2);
-  const double rad = fmax((double)ratio * diam, 1.01 * sqrt(dv));
-  cellgeo[c] = make_float4((float)cen[0], (float)cen[1], (float)cen[2], (float)(rad * rad));
 }
 
 constexpr int kChunkM = 8;
@@ -448,21 +487,50 @@ __device__ __forceinline__ void add_entry(float2* A2, float2* B2, SysOut so, int
   B2[o] = make_float2(h, __double2float_rn(s - (double)h));
 }
 
-// One thread per row: near items, then singular items, in order.
-__global__ void k_merge_items(int N, const int* __restrict__ cnt, const int* __restrict__ dof,
-                              const double2* __restrict__ val, float2* __restrict__ A2,
-                              float2* __restrict__ B2, SysOut so) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= N) return;
+// Adds a row's items to its entries, one warp per row. Each lane takes an
+// item; the lane with the first item of a column sums that column's items in
+// ascending order (near items, then singular ones) in FP64 and updates the
+// entry once, so the updates of a row run side by side. Latency-bound: one
+// thread per row (a read-modify-write after the other, about 140 per row) took
+// 0.28 ms from N = 600 to 12,000, now 0.037 and 0.115 ms.
+constexpr int kMergeWarps = 4;
+
+__global__ void __launch_bounds__(kMergeWarps * 32)
+    k_merge_items(int N, const int* __restrict__ cnt, const int* __restrict__ dof,
+                  const double2* __restrict__ val, float2* __restrict__ A2,
+                  float2* __restrict__ B2, SysOut so) {
+  __shared__ int s_col[kMergeWarps][kItemCap];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = blockIdx.x * kMergeWarps + warp;
+  if (row >= N) return;  // whole warps
   const size_t base = (size_t)row * kItemCap;
   const int nn = min(cnt[2 * row], kNearItems), ns = min(cnt[2 * row + 1], kSingItems);
-  for (int k = 0; k < nn; ++k) {
-    const double2 v = val[base + k];
-    add_entry(A2, B2, so, N, row, dof[base + k], v.x, v.y);
-  }
-  for (int k = 0; k < ns; ++k) {
-    const double2 v = val[base + kNearItems + k];
-    add_entry(A2, B2, so, N, row, dof[base + kNearItems + k], v.x, v.y);
+  const int n = nn + ns;
+  int* col = s_col[warp];
+  // item k of the row sits at base + k (near) or in the singular part
+  for (int k = lane; k < n; k += 32) col[k] = dof[base + (k < nn ? k : kNearItems + k - nn)];
+  __syncwarp();
+  for (int p0 = 0; p0 < n; p0 += 32) {
+    const int k = p0 + lane;
+    const int c = k < n ? col[k] : -1;
+    bool first = k < n;
+    double sn = 0.0, sd = 0.0;
+    for (int q0 = 0; q0 < n; q0 += 32) {
+      unsigned m = 0;
+      const int qn = min(32, n - q0);
+      for (int b = 0; b < qn; ++b) m |= (unsigned)(col[q0 + b] == c) << b;
+      // an earlier item of the column: its lane has the column
+      if (m && q0 + __ffs(m) - 1 < k) first = false;
+      if (!first) m = 0;
+      while (m) {
+        const int e = q0 + __ffs(m) - 1;
+        m &= m - 1;
+        const double2 v = val[base + (e < nn ? e : kNearItems + e - nn)];
+        sn += v.x;
+        sd += v.y;
+      }
+    }
+    if (first) add_entry(A2, B2, so, N, row, c, sn, sd);
   }
 }
 
@@ -537,8 +605,14 @@ __global__ void __launch_bounds__(256)
 // FP64 near field: one warp per row. The lanes test 32 candidate panels at a
 // time against the near criterion (same test as the tile kernel); each near,
 // non-singular panel is then integrated with the regular rule in FP64, one
-// quadrature point per lane, and lane 0 appends its four contributions to the
-// row's items in ascending panel order.
+// quadrature point per lane, and its four contributions go to the row's items
+// in ascending panel order. Bound by the FP64 pipe (and by latency at small
+// N). Rules of up to 16 points take two panels at a time, one per half warp,
+// and the eight sums of a panel are reduce-scattered: half the lanes no longer
+// idle and the reduction's additions fall from 40 to 8 per lane. N = 12,000:
+// 1.51 ms -> 0.54, N = 600: 0.205 ms -> 0.063 (kernel times).
+// HALF: two panels per step (rules of at most 16 points).
+template <bool HALF>
 __global__ void __launch_bounds__(256)
     k_near_mixed(int N, int C, const double* __restrict__ X, const int* __restrict__ dnset,
                  const int4* __restrict__ cell_dofs, const float4* __restrict__ cellgeo,
@@ -555,8 +629,19 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int k = 0; k < kMaxSet; ++k) set[k] = dnset[(size_t)row * kMaxSet + k];
   const int nq = c_qm.q1 * c_qm.q1;
+  constexpr int W = HALF ? 16 : 32;
+  const int q0 = lane & (W - 1), half = HALF ? lane >> 4 : 0;
+  // the lane that holds component j of a panel's sums writes it once
+  const int j = (lane >> 1) & 7;
+  const bool writer = HALF ? (lane & 1) == 0 : (lane & 17) == 0;
+  double ph[4] = {0, 0, 0, 0};
+  if (HALF && q0 < nq)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ph[k] = c_qm.phi[q0][k];
   double asum = 0.0;
   int nitem = 0;
+  double* vals = reinterpret_cast<double*>(item_val + (size_t)row * kItemCap);
+  int* dofs = item_dof + (size_t)row * kItemCap;
   // candidates of this row's block (ascending panel order), else every panel
   const int nc = ncnt[row / kNearBlock];
   const int* cl = nlist + (size_t)(row / kNearBlock) * kNearCap;
@@ -570,44 +655,51 @@ __global__ void __launch_bounds__(256)
     }
     unsigned m = __ballot_sync(0xffffffffu, nr);
     while (m) {
-      const int b = __ffs(m) - 1;
+      const int b0 = __ffs(m) - 1;
       m &= m - 1;
-      const int cell = __shfl_sync(0xffffffffu, c, b);
-      const double* r = rec64 + (size_t)cell * nq * 8;
-      double ln[4] = {0, 0, 0, 0}, ld[4] = {0, 0, 0, 0};
-      for (int q = lane; q < nq; q += 32) {
-        const double Rx = r[8 * q] - xi, Ry = r[8 * q + 1] - yi, Rz = r[8 * q + 2] - zi;
+      int b1 = -1;  // the second half warp's panel, if there is one more
+      if (HALF && m) {
+        b1 = __ffs(m) - 1;
+        m &= m - 1;
+      }
+      const int cell = __shfl_sync(0xffffffffu, c, half ? max(b1, 0) : b0);
+      const bool on = !half || b1 >= 0;
+      double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      const double2* r = reinterpret_cast<const double2*>(rec64 + (size_t)cell * nq * 8);
+      for (int q = q0; on && q < nq; q += W) {
+        const double2 p01 = r[4 * q], p23 = r[4 * q + 1], p45 = r[4 * q + 2], p67 = r[4 * q + 3];
+        const double Rx = p01.x - xi, Ry = p01.y - yi, Rz = p23.x - zi;
         const double ri = rsqrt(fma(Rx, Rx, fma(Ry, Ry, Rz * Rz)));
-        const double sq = ri * r[8 * q + 3];
-        const double dq = -fma(Rx, r[8 * q + 4], fma(Ry, r[8 * q + 5], Rz * r[8 * q + 6])) * (ri * ri * ri);
+        const double sq = ri * p23.y;
+        const double dq = -fma(Rx, p45.x, fma(Ry, p45.y, Rz * p67.x)) * (ri * ri * ri);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          ln[j] = fma(dq, c_qm.phi[q][j], ln[j]);
-          ld[j] = fma(sq, c_qm.phi[q][j], ld[j]);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          ln[j] += __shfl_xor_sync(0xffffffffu, ln[j], o);
-          ld[j] += __shfl_xor_sync(0xffffffffu, ld[j], o);
-        }
-      if (lane == 0) {
-        const int4 d = cell_dofs[cell];
-        const int id[4] = {d.x, d.y, d.z, d.w};
-        for (int j = 0; j < 4; ++j) {
-          if (nitem < kNearItems) {
-            const size_t o = (size_t)row * kItemCap + nitem;
-            item_dof[o] = id[j];
-            item_val[o] = make_double2(ln[j], ld[j]);
+        for (int k = 0; k < 4; ++k) {
+          if (HALF) {  // one point per lane
+            v[k] = dq * ph[k];
+            v[4 + k] = sq * ph[k];
+          } else {
+            v[k] = fma(dq, c_qm.phi[q][k], v[k]);
+            v[4 + k] = fma(sq, c_qm.phi[q][k], v[4 + k]);
           }
-          ++nitem;
-          asum += ln[j];
         }
       }
+      const double s = panel_reduce8<!HALF>(v, lane);
+      if (writer && on) {
+        const int it = nitem + 4 * half + (j & 3);
+        if (it < kNearItems) {
+          if (j < 4) {
+            const int4 d = cell_dofs[cell];
+            dofs[it] = j < 2 ? (j == 0 ? d.x : d.y) : (j == 2 ? d.z : d.w);
+          }
+          vals[2 * it + (j >> 2)] = s;
+        }
+        if (j < 4) asum += s;
+      }
+      nitem += b1 >= 0 ? 8 : 4;
     }
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) asum += __shfl_xor_sync(0xffffffffu, asum, o);
   if (lane == 0) {
     alpha_near[row] = asum;
     item_cnt[2 * row] = nitem;
@@ -615,74 +707,88 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// FP64 vertex-singular panels (one thread per row), appended to the row's
-// singular items.
-__global__ void k_singular_mixed(int N, const double* __restrict__ X, const int* __restrict__ dnset,
-                                 const int* __restrict__ sptr, const int* __restrict__ scell,
-                                 const int4* __restrict__ cell_dofs, int* __restrict__ item_cnt,
-                                 int* __restrict__ item_dof, double2* __restrict__ item_val,
-                                 double* __restrict__ alpha_sing, DevErr* err) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= N) return;
-  const double xi = X[3 * (size_t)row], yi = X[3 * (size_t)row + 1], zi = X[3 * (size_t)row + 2];
+// FP64 vertex-singular panels, appended to the row's singular items in
+// ascending panel order: one CTA per row, its four warps take every fourth
+// panel with the rule's points over the lanes. Bound by the FP64 pipe at large
+// N, by the latency of one panel's chain at small N; one thread per row took
+// 0.55 ms at N = 600 and 0.60 ms at 12,000, now 0.034 and 0.59 ms.
+constexpr int kSingWarpsM = 4;
+
+__global__ void __launch_bounds__(kSingWarpsM * 32)
+    k_singular_mixed(int N, const double* __restrict__ X, const int* __restrict__ dnset,
+                     const int* __restrict__ sptr, const int* __restrict__ scell,
+                     const int4* __restrict__ cell_dofs, int* __restrict__ item_cnt,
+                     int* __restrict__ item_dof, double2* __restrict__ item_val,
+                     double* __restrict__ alpha_sing, DevErr* err) {
+  __shared__ double s_alpha[kSingWarpsM];
+  const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double x[3] = {X[3 * (size_t)row], X[3 * (size_t)row + 1], X[3 * (size_t)row + 2]};
   int set[kMaxSet];
 #pragma unroll
   for (int k = 0; k < kMaxSet; ++k) set[k] = dnset[(size_t)row * kMaxSet + k];
-  const int nsp = c_qm.nsp;
+  const int j = (lane >> 1) & 7;
+  double* vals = reinterpret_cast<double*>(item_val + (size_t)row * kItemCap + kNearItems);
+  int* dofs = item_dof + (size_t)row * kItemCap + kNearItems;
+  const int e0 = sptr[row], n = sptr[row + 1] - e0;
   double asum = 0.0;
-  int nitem = 0;
-  for (int e = sptr[row]; e < sptr[row + 1]; ++e) {
-    const int cell = scell[e];
-    const int4 d = cell_dofs[cell];
+  for (int e = warp; e < n; e += kSingWarpsM) {
+    const int4 d = cell_dofs[scell[e0 + e]];
     const int id[4] = {d.x, d.y, d.z, d.w};
     int v = -1;
-    for (int j = 0; j < 4 && v < 0; ++j)
-      if (in_set_m(set, id[j])) v = j;
+#pragma unroll
+    for (int k = 3; k >= 0; --k)
+      if (in_set_m(set, id[k])) v = k;
+    double s = 0.0;
     if (v < 0) {
-      dev_fail(err, WBEM_ERR_ARG, 42, row, cell);
-      continue;
+      if (lane == 0) dev_fail(err, WBEM_ERR_ARG, 42, row, scell[e0 + e]);
+    } else {
+      double P[4][3];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) P[k][c] = X[3 * (size_t)id[k] + c];
+      s = singular_panel(P, x, c_qm.sp[v], c_qm.nsp, lane);
     }
-    double P[4][3];
-    for (int k = 0; k < 4; ++k)
-      for (int c = 0; c < 3; ++c) P[k][c] = X[3 * (size_t)id[k] + c];
-    double ln[4] = {0, 0, 0, 0}, ld[4] = {0, 0, 0, 0};
-    for (int q = 0; q < nsp; ++q) {
-      const double s = c_qm.sp[v][q][0], t = c_qm.sp[v][q][1], w = c_qm.sp[v][q][2] * kInv4PiM;
-      double x[3], cr[3];
-      q1_geo(P, s, t, x, cr);
-      const double det = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
-      const double Rx = x[0] - xi, Ry = x[1] - yi, Rz = x[2] - zi;
-      const double ri = rsqrt(fma(Rx, Rx, fma(Ry, Ry, Rz * Rz)));
-      const double sq = ri * det * w;
-      const double dq = -(Rx * cr[0] + Ry * cr[1] + Rz * cr[2]) * (ri * ri * ri) * w;
-      const double ph[4] = {(1 - s) * (1 - t), s * (1 - t), (1 - s) * t, s * t};
-      for (int j = 0; j < 4; ++j) {
-        ln[j] = fma(dq, ph[j], ln[j]);
-        ld[j] = fma(sq, ph[j], ld[j]);
+    if ((lane & 17) == 0) {
+      const int it = 4 * e + (j & 3);
+      if (it < kSingItems) {
+        if (j < 4) dofs[it] = j < 2 ? (j == 0 ? d.x : d.y) : (j == 2 ? d.z : d.w);
+        vals[2 * it + (j >> 2)] = s;
       }
-    }
-    for (int j = 0; j < 4; ++j) {
-      if (nitem < kSingItems) {
-        const size_t o = (size_t)row * kItemCap + kNearItems + nitem;
-        item_dof[o] = id[j];
-        item_val[o] = make_double2(ln[j], ld[j]);
-      }
-      ++nitem;
-      asum += ln[j];
+      if (j < 4) asum += s;
     }
   }
-  alpha_sing[row] = asum;
-  item_cnt[2 * row + 1] = nitem;
-  if (nitem > kSingItems) dev_fail(err, WBEM_ERR_NOMEM, 44, row, nitem);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) asum += __shfl_xor_sync(0xffffffffu, asum, o);
+  if (lane == 0) s_alpha[warp] = asum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < kSingWarpsM; ++w) s += s_alpha[w];
+    alpha_sing[row] = s;
+    item_cnt[2 * row + 1] = 4 * n;
+    if (4 * n > kSingItems) dev_fail(err, WBEM_ERR_NOMEM, 44, row, 4 * n);
+  }
 }
 
-__global__ void k_alpha_mixed(int N, int n_tiles, const double* __restrict__ part,
-                              const double* __restrict__ an, const double* __restrict__ as,
-                              double* __restrict__ alpha) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
+// alpha = -(far-field partial sums of every tile + near + singular): a CTA
+// takes 32 rows, its 8 warps every eighth tile (a thread per row took
+// 0.23 ms at N = 32,768 for want of loads in flight).
+__global__ void __launch_bounds__(256)
+    k_alpha_mixed(int N, int n_tiles, const double* __restrict__ part,
+                  const double* __restrict__ an, const double* __restrict__ as,
+                  double* __restrict__ alpha) {
+  __shared__ double red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
   double s = 0;
-  for (int t = 0; t < n_tiles; ++t) s += part[(size_t)t * N + i];
+  if (i < N)
+#pragma unroll 4
+    for (int t = warp; t < n_tiles; t += 8) s += part[(size_t)t * N + i];
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp || i >= N) return;
+  for (int w = 1; w < 8; ++w) s += red[w][lane];
   alpha[i] = -(s + an[i] + as[i]);
 }
 
@@ -731,9 +837,13 @@ int assemble_mixed(wbem_context* h) {
   h->rec_cells = (size_t)C * nq;
   EvTimer tm(h->stream);
   CUM(launch_cell_records_fp64(C, h->d_X, h->d_cell_dofs, h->d_rec, q1, h->stream));
-  k_cell_records_mixed<<<(C + 127) / 128, 128, 0, h->stream>>>(
-      C, h->d_X, h->d_cell_dofs, h->d_rec32, reinterpret_cast<float4*>(h->d_cellgeo),
-      (float)o.near_field_ratio);
+  float4* geo_w = reinterpret_cast<float4*>(h->d_cellgeo);
+  if (nq <= 16)
+    k_cell_records_mixed<true><<<(C + 2 * kRecWarps - 1) / (2 * kRecWarps), kRecWarps * 32, 0, h->stream>>>(
+        C, h->d_X, h->d_cell_dofs, h->d_rec32, geo_w, (float)o.near_field_ratio);
+  else
+    k_cell_records_mixed<false><<<(C + kRecWarps - 1) / kRecWarps, kRecWarps * 32, 0, h->stream>>>(
+        C, h->d_X, h->d_cell_dofs, h->d_rec32, geo_w, (float)o.near_field_ratio);
   CUM(cudaGetLastError());
   h->stats.t_geometry_ms = tm.ms();
   const float4* geo = reinterpret_cast<const float4*>(h->d_cellgeo);
@@ -781,13 +891,20 @@ int assemble_mixed(wbem_context* h) {
     CUM(cudaStreamWaitEvent(ax, h->ev_aux_fork, 0));
     k_near_candidates<<<nblk, 256, 0, ax>>>(N, C, h->d_X, geo, h->d_near_cnt, h->d_near_cells);
     CUM(cudaGetLastError());
-    k_near_mixed<<<(unsigned)(((size_t)N * 32 + 255) / 256), 256, 0, ax>>>(
-        N, C, h->d_X, h->d_dnset, h->d_cell_dofs, geo, h->d_rec, h->d_item_cnt, h->d_item_dof,
-        h->d_item_val, h->d_alpha_near, h->d_near_cnt, h->d_near_cells, h->d_err);
+    const unsigned nwb = (unsigned)(((size_t)N * 32 + 255) / 256);
+    if (nq <= 16)
+      k_near_mixed<true><<<nwb, 256, 0, ax>>>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, geo, h->d_rec,
+                                              h->d_item_cnt, h->d_item_dof, h->d_item_val,
+                                              h->d_alpha_near, h->d_near_cnt, h->d_near_cells, h->d_err);
+    else
+      k_near_mixed<false><<<nwb, 256, 0, ax>>>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, geo, h->d_rec,
+                                               h->d_item_cnt, h->d_item_dof, h->d_item_val,
+                                               h->d_alpha_near, h->d_near_cnt, h->d_near_cells,
+                                               h->d_err);
     CUM(cudaGetLastError());
-    k_singular_mixed<<<(N + 63) / 64, 64, 0, ax>>>(N, h->d_X, h->d_dnset, h->d_sptr, h->d_scell,
-                                                    h->d_cell_dofs, h->d_item_cnt, h->d_item_dof,
-                                                    h->d_item_val, h->d_alpha_sing, h->d_err);
+    k_singular_mixed<<<N, kSingWarpsM * 32, 0, ax>>>(N, h->d_X, h->d_dnset, h->d_sptr, h->d_scell,
+                                                     h->d_cell_dofs, h->d_item_cnt, h->d_item_dof,
+                                                     h->d_item_val, h->d_alpha_sing, h->d_err);
     CUM(cudaGetLastError());
     CUM(cudaEventRecord(h->ev_aux_join, ax));
   }
@@ -803,11 +920,12 @@ int assemble_mixed(wbem_context* h) {
   h->stats.t_assemble_ms = tm.ms();
   // join the near / singular work and add it to the far-field entries
   CUM(cudaStreamWaitEvent(h->stream, h->ev_aux_join, 0));
-  k_merge_items<<<(N + 127) / 128, 128, 0, h->stream>>>(N, h->d_item_cnt, h->d_item_dof,
+  k_merge_items<<<(N + kMergeWarps - 1) / kMergeWarps, kMergeWarps * 32, 0, h->stream>>>(
+      N, h->d_item_cnt, h->d_item_dof,
                                                          h->d_item_val, h->d_A2, h->d_B2, so);
   CUM(cudaGetLastError());
   h->stats.t_singular_ms = tm.ms();
-  k_alpha_mixed<<<(N + 255) / 256, 256, 0, h->stream>>>(N, h->n_tiles, h->d_alpha_part,
+  k_alpha_mixed<<<(N + 31) / 32, 256, 0, h->stream>>>(N, h->n_tiles, h->d_alpha_part,
                                                          h->d_alpha_near, h->d_alpha_sing,
                                                          h->d_alpha);
   CUM(cudaGetLastError());

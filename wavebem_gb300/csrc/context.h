@@ -165,6 +165,9 @@ struct wbem_context {
   double* d_vec[kNumVec] = {};  // N-vectors: [0..2] GMRES, [7] transposed operator, [8..9] refinement
   double* d_part = nullptr;
   double* d_small = nullptr;
+  double* d_opart = nullptr;   // k_ortho: the CTAs' partial sums
+  unsigned* d_octr = nullptr;  // and its grid barrier's counter
+  int sms = 0;                 // SMs of the device
   float* d_lu = nullptr;   // mixed: FP32 system matrix, then its LU factors
   // state of d_lu: 0 = neither, 1 = system entries from the assembly (free
   // term and constraint rows pending), 2 = complete system matrix

@@ -106,8 +106,16 @@ cudaError_t launch_bj_apply(int N, const double* binv, const double* x, double* 
                             cudaStream_t s);
 
 // Krylov helpers (FP64)
-cudaError_t launch_multidot(int N, int k, const double* V, const double* w, double* part,
-                            double* out, cudaStream_t s);
+// One Arnoldi step: w orthogonalised against the k vectors of V (classical
+// Gram-Schmidt, twice), v = w / |w|; out[0..k) the coefficients, out[k] the
+// norm. part: ortho_part_size(n_ctas) doubles; ctr: a device counter, zero when
+// *epoch was last set to zero; n_ctas = ortho_ctas(N, SMs, ordered). ordered:
+// the sums in a fixed order that does not depend on N or the GPU (FMA method).
+cudaError_t launch_ortho(int N, int k, const double* V, double* w, double* v, double* part,
+                         double* out, unsigned* ctr, unsigned* epoch, int n_ctas, bool ordered,
+                         DevErr* err, cudaStream_t s);
+size_t ortho_part_size(int n_ctas);
+int ortho_ctas(int N, int sms, bool ordered);
 cudaError_t launch_axpy_basis(int N, int k, const double* V, const double* h, double* w,
                               double sign, cudaStream_t s);
 cudaError_t launch_scale(int N, const double* x, double a, double* y, cudaStream_t s);

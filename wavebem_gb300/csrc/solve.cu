@@ -504,40 +504,207 @@ cudaError_t launch_bj_apply(int N, const double* binv, const double* x, double* 
 // ------------------------------------------------------------ Krylov helpers
 constexpr int kRedBlocks = 120;
 
-__global__ void k_multidot(int N, int k, const double* __restrict__ V, const double* __restrict__ w,
-                           double* __restrict__ part) {
-  __shared__ double red[256];
-  const int per = (N + gridDim.x - 1) / gridDim.x;
-  const int i0 = blockIdx.x * per, i1 = min(N, i0 + per);
-  for (int j = 0; j < k; ++j) {
-    double s = 0;
-    const double* v = V + (size_t)j * N;
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) s = fma(v[i], w[i], s);
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-      __syncthreads();
+// One Arnoldi step: classical Gram-Schmidt of w against the k basis vectors of
+// V, once more, the norm, and the next basis vector v = w / |w|. out[0..k) =
+// the summed coefficients, out[k] = the norm. A cooperative launch: CTA b owns
+// the rows of chunk b (of w, V and v), the dot products and the norm meet in
+// grid barriers (bounded waits on a counter), and every CTA adds the partial
+// sums of all CTAs itself, in the same order.
+// Bound by latency: the work is 4 k N FP64 operations on a basis that sits in
+// L2. As nine launches (dots, a serial sum of the CTAs' parts, update, twice,
+// then norm and scaling) a step took 110 us at N = 2,000 (mean over the 34
+// steps of a solve), now 25 us.
+// ORDERED: every sum in the order that those launches used (kRedBlocks chunks,
+// trees of 256 threads, serial sums of the chunks and over the vectors). The
+// FMA product is linear to FP32 round-off only, so that an FMA solve repeats
+// to 1e-8 if any sum changes in its last bit; with these orders it repeats
+// exactly: 94 us at N = 32,768 (mean over 55 steps), as launches 178 us.
+constexpr int kOrthoThreads = 256;
+constexpr int kOrthoRows = 64;   // fewest rows per CTA
+constexpr int kOrthoMaxK = 256;  // basis vectors (restart <= 250)
+
+__device__ __forceinline__ void ortho_barrier(unsigned* ctr, unsigned target, DevErr* err) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(ctr, 1u);
+    uint32_t it = 0;
+    while ((int)(*((volatile unsigned*)ctr) - target) < 0) {
+      if (++it > (1u << 26)) {
+        dev_fail(err, WBEM_ERR_TIMEOUT, 61, blockIdx.x, (int)target);
+        break;
+      }
     }
-    if (threadIdx.x == 0) part[(size_t)j * gridDim.x + blockIdx.x] = red[0];
-    __syncthreads();
+    __threadfence();
   }
+  __syncthreads();
 }
 
-__global__ void k_multidot_finish(int k, int nb, const double* __restrict__ part,
-                                  double* __restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= k) return;
-  double s = 0;
-  for (int b = 0; b < nb; ++b) s += part[(size_t)j * nb + b];
-  out[j] = s;
+// Sum over rows first, first + 256, ... < end of a[i] * c[i] for "threads"
+// t = 0..255 (row first + t + 256 m), then their tree sum, all by one warp:
+// lane l stands for threads l, l + 32, ..., l + 224. The total is on lane 0.
+__device__ __forceinline__ double tree256_dot(const double* a, const double* c, int first, int end,
+                                              int stride, int lane) {
+  double t[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    double s = 0.0;
+    for (int i = first + lane + 32 * m; i < end; i += stride) s = fma(__ldcg(a + i), __ldcg(c + i), s);
+    t[m] = s;
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+      if (m < o) t[m] += t[m + o];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t[0] += __shfl_down_sync(0xffffffffu, t[0], o);
+  return t[0];
 }
 
-cudaError_t launch_multidot(int N, int k, const double* V, const double* w, double* part,
-                            double* out, cudaStream_t s) {
-  k_multidot<<<kRedBlocks, 256, 0, s>>>(N, k, V, w, part);
-  k_multidot_finish<<<(k + 127) / 128, 128, 0, s>>>(k, kRedBlocks, part, out);
-  return cudaGetLastError();
+// Sum of p[0..n) by one warp, in every lane. ORDERED: one after the other.
+template <bool ORDERED>
+__device__ __forceinline__ double warp_total(const double* p, int n, int lane) {
+  double s = 0.0;
+  if (ORDERED) {
+    for (int g0 = 0; g0 < n; g0 += 32) {
+      const double x = g0 + lane < n ? __ldcg(p + g0 + lane) : 0.0;
+      const int m = min(32, n - g0);
+      for (int u = 0; u < m; ++u) s += __shfl_sync(0xffffffffu, x, u);
+    }
+  } else {
+    for (int g = lane; g < n; g += 32) s += __ldcg(p + g);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  }
+  return s;
+}
+
+template <bool ORDERED>
+__global__ void __launch_bounds__(kOrthoThreads)
+    k_ortho(int N, int k, const double* __restrict__ V, double* w, double* __restrict__ v,
+            double* part, double* __restrict__ out, unsigned* ctr, unsigned base, DevErr* err) {
+  __shared__ double hs[kOrthoMaxK];
+  __shared__ double red[4][kOrthoRows];
+  __shared__ double wsum[kOrthoThreads / 32];
+  constexpr int kWarps = kOrthoThreads / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = gridDim.x, b = blockIdx.x;
+  const int per = (N + G - 1) / G;
+  const int i0 = min(N, b * per), i1 = min(N, i0 + per);
+  double nrm = 0.0;
+  for (int pass = 0; pass < 2; ++pass) {
+    double* pp = part + (size_t)pass * kOrthoMaxK * G;
+    // this CTA's part of every dot product: a warp per basis vector
+    for (int j = warp; j < k; j += kWarps) {
+      const double* vj = V + (size_t)j * N;
+      double s = 0.0;
+      if (ORDERED) {
+        s = tree256_dot(vj, w, i0, i1, 256, lane);
+      } else {
+#pragma unroll 4
+        for (int i = i0 + lane; i < i1; i += 32) s = fma(vj[i], w[i], s);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      }
+      if (lane == 0) pp[(size_t)j * G + b] = s;
+    }
+    ortho_barrier(ctr, base + (unsigned)(pass + 1) * G, err);
+    if (ORDERED) {
+      // a thread per vector adds the CTAs' parts in ascending order
+      for (int j = tid; j < k; j += kOrthoThreads) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int g = 0; g < G; ++g) s += __ldcg(pp + (size_t)j * G + g);
+        hs[j] = s;
+        if (b == 0) out[j] = pass == 0 ? s : out[j] + s;
+      }
+    } else {
+      for (int j = warp; j < k; j += kWarps) {
+        const double s = warp_total<false>(pp + (size_t)j * G, G, lane);
+        if (lane == 0) {
+          hs[j] = s;
+          if (b == 0) out[j] = pass == 0 ? s : out[j] + s;
+        }
+      }
+    }
+    __syncthreads();
+    // w -= V h on this CTA's rows
+    if (ORDERED) {
+      for (int i = i0 + tid; i < i1; i += kOrthoThreads) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int j = 0; j < k; ++j) s = fma(hs[j], V[(size_t)j * N + i], s);
+        w[i] -= s;
+      }
+      __syncthreads();
+    } else {
+      // 64 rows at a time, the vectors over 4 groups
+      const int r = tid & (kOrthoRows - 1), q = tid / kOrthoRows;
+      for (int c0 = i0; c0 < i1; c0 += kOrthoRows) {
+        const int i = c0 + r;
+        double s = 0.0;
+        if (i < i1)
+#pragma unroll 8
+          for (int j = q; j < k; j += 4) s = fma(hs[j], V[(size_t)j * N + i], s);
+        red[q][r] = s;
+        __syncthreads();
+        if (q == 0 && i < i1) {
+          const double x = w[i] - ((red[0][r] + red[1][r]) + (red[2][r] + red[3][r]));
+          w[i] = x;
+          if (pass == 1) nrm = fma(x, x, nrm);
+        }
+        __syncthreads();
+      }
+    }
+  }
+  double* pn = part + (size_t)2 * kOrthoMaxK * G;
+  unsigned target = base + 3u * G;
+  if (ORDERED) {
+    // the norm's rows: 256 b + t + 256 G m, of other CTAs' chunks too
+    ortho_barrier(ctr, target, err);
+    target += G;
+    if (warp == 0) {
+      const double s = tree256_dot(w, w, 256 * b, N, 256 * G, lane);
+      if (lane == 0) pn[b] = s;
+    }
+  } else {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+    if (lane == 0) wsum[warp] = nrm;
+    __syncthreads();
+    if (tid == 0) {
+      double s = 0.0;
+      for (int u = 0; u < kWarps; ++u) s += wsum[u];
+      pn[b] = s;
+    }
+  }
+  ortho_barrier(ctr, target, err);
+  const double hn = sqrt(warp_total<ORDERED>(pn, G, lane));
+  if (b == 0 && tid == 0) out[k] = hn;
+  const double inv = 1.0 / hn;
+  if (hn > 0.0)
+    for (int i = i0 + tid; i < i1; i += kOrthoThreads) v[i] = inv * w[i];
+}
+
+size_t ortho_part_size(int n_ctas) { return (size_t)(2 * kOrthoMaxK + 1) * n_ctas; }
+
+// CTAs of k_ortho for N rows: at most one per SM (co-resident), and no more
+// than give each kOrthoRows rows (fewer arrivals per barrier at small N).
+// The ordered form always has kRedBlocks chunks.
+int ortho_ctas(int N, int sms, bool ordered) {
+  return ordered ? kRedBlocks : std::max(1, std::min(sms, N / kOrthoRows));
+}
+
+cudaError_t launch_ortho(int N, int k, const double* V, double* w, double* v, double* part,
+                         double* out, unsigned* ctr, unsigned* epoch, int n_ctas, bool ordered,
+                         DevErr* err, cudaStream_t s) {
+  unsigned base = *epoch;
+  *epoch += (ordered ? 4u : 3u) * (unsigned)n_ctas;
+  void* args[] = {(void*)&N, (void*)&k, (void*)&V, (void*)&w, (void*)&v, (void*)&part,
+                  (void*)&out, (void*)&ctr, (void*)&base, (void*)&err};
+  const void* f = ordered ? (const void*)k_ortho<true> : (const void*)k_ortho<false>;
+  return cudaLaunchCooperativeKernel(f, dim3(n_ctas), dim3(kOrthoThreads), args, 0, s);
 }
 
 __global__ void k_axpy_basis(int N, int k, const double* __restrict__ V, const double* __restrict__ h,
@@ -545,6 +712,7 @@ __global__ void k_axpy_basis(int N, int k, const double* __restrict__ V, const d
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   double s = 0;
+#pragma unroll 8
   for (int j = 0; j < k; ++j) s = fma(h[j], V[(size_t)j * N + i], s);
   w[i] = fma(sign, s, w[i]);
 }
@@ -587,12 +755,10 @@ __global__ void k_nrm2_part(int N, const double* __restrict__ x, double* __restr
   }
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
+// one warp; the parts added in ascending order
 __global__ void k_nrm2_finish(int nb, const double* __restrict__ part, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0;
-    for (int b = 0; b < nb; ++b) s += part[b];
-    out[0] = sqrt(s);
-  }
+  const double s = warp_total<true>(part, nb, threadIdx.x);
+  if (threadIdx.x == 0) out[0] = sqrt(s);
 }
 cudaError_t launch_nrm2(int N, const double* x, double* part, double* out, cudaStream_t s) {
   k_nrm2_part<<<kRedBlocks, 256, 0, s>>>(N, x, part);

@@ -400,6 +400,13 @@ int ensure_vectors(wbem_context* h, int restart) {
     if (!h->d_vec[k]) CHK(dev_alloc(h, &h->d_vec[k], (size_t)N));
   if (!h->d_part) CHK(dev_alloc(h, &h->d_part, (size_t)256 * 128 + (size_t)40 * N));
   if (!h->d_small) CHK(dev_alloc(h, &h->d_small, (size_t)512));
+  if (!h->d_opart) {
+    int sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    h->sms = sms;
+    CHK(dev_alloc(h, &h->d_opart, ortho_part_size(std::max(ortho_ctas(N, sms, true), ortho_ctas(N, sms, false)))));
+    CHK(dev_alloc(h, &h->d_octr, (size_t)1));
+  }
   if (!h->d_sol) CHK(dev_alloc(h, &h->d_sol, (size_t)N));
   if (!h->d_rhs) CHK(dev_alloc(h, &h->d_rhs, (size_t)N));
   if (!h->d_b) CHK(dev_alloc(h, &h->d_b, (size_t)N));
@@ -474,30 +481,31 @@ int gmres(wbem_context* h, const double* rhs, double* x, int restart, int max_st
   double* r = h->d_vec[0];
   double* w = h->d_vec[1];
   double* Z = h->d_V + (size_t)h->V_cap * N;  // restart vectors
-  double* hbuf = h->d_small;  // [0..restart+1] h, [256..] h2
+  double* hbuf = h->d_small;  // [0..restart) coefficients of a step, then its norm
   double* part = h->d_part;
   double bnorm;
   CU(launch_nrm2(N, rhs, part, hbuf, h->stream));
   CHK(read_scalar(h, hbuf, &bnorm));
   const double target = std::max(tol, 1e-14 * bnorm);
   CU(cudaMemsetAsync(x, 0, sizeof(double) * N, h->stream));
+  CU(cudaMemsetAsync(h->d_octr, 0, sizeof(unsigned), h->stream));
+  unsigned epoch = 0;
+  const bool ordered = h->assembled_prec == kAssembledFma;
+  const int n_ctas = ortho_ctas(N, h->sms, ordered);
   int it = 0;
   double res = bnorm;
   std::vector<double> H((size_t)(restart + 1) * restart), cs(restart), sn(restart), g(restart + 1),
-      hv(restart + 2), hv2(restart + 2), y(restart);
+      hv(restart + 2), y(restart);
   bool first = true;
   while (true) {
-    // r = rhs - A x
-    if (first) {
-      CU(cudaMemcpyAsync(r, rhs, sizeof(double) * N, cudaMemcpyDeviceToDevice, h->stream));
-      first = false;
-    } else {
+    // r = rhs - A x (x = 0 at first)
+    double beta = bnorm;
+    if (!first) {
       CHK(op(x, r));
       CU(launch_axpby(N, 1.0, rhs, -1.0, r, h->stream));
+      CU(launch_nrm2(N, r, part, hbuf, h->stream));
+      CHK(read_scalar(h, hbuf, &beta));
     }
-    CU(launch_nrm2(N, r, part, hbuf, h->stream));
-    double beta;
-    CHK(read_scalar(h, hbuf, &beta));
     res = beta;
     if (!std::isfinite(beta)) return fail(h, WBEM_ERR_NONFINITE, "GMRES: non-finite residual");
     if (beta <= target) break;
@@ -506,7 +514,8 @@ int gmres(wbem_context* h, const double* rhs, double* x, int restart, int max_st
       if (resid) *resid = res;
       return fail(h, WBEM_ERR_NOCONV, "GMRES: no convergence within max_steps");
     }
-    CU(launch_scale(N, r, 1.0 / beta, h->d_V, h->stream));
+    CU(launch_scale(N, first ? rhs : r, 1.0 / beta, h->d_V, h->stream));
+    first = false;
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int k = 0;
@@ -516,21 +525,15 @@ int gmres(wbem_context* h, const double* rhs, double* x, int restart, int max_st
       double* z = Z + (size_t)k * N;
       CHK(prec(vk, z));
       CHK(op(z, w));
-      CU(launch_multidot(N, k + 1, h->d_V, w, part, hbuf, h->stream));
-      CU(launch_axpy_basis(N, k + 1, h->d_V, hbuf, w, -1.0, h->stream));
-      CU(launch_multidot(N, k + 1, h->d_V, w, part, hbuf + 256, h->stream));
-      CU(launch_axpy_basis(N, k + 1, h->d_V, hbuf + 256, w, -1.0, h->stream));
-      CU(launch_nrm2(N, w, part, hbuf + 255, h->stream));
-      CU(cudaMemcpyAsync(hv.data(), hbuf, sizeof(double) * (k + 1), cudaMemcpyDeviceToHost, h->stream));
-      CU(cudaMemcpyAsync(hv2.data(), hbuf + 256, sizeof(double) * (k + 1), cudaMemcpyDeviceToHost, h->stream));
-      double hn;
-      CU(cudaMemcpyAsync(&hn, hbuf + 255, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+      CU(launch_ortho(N, k + 1, h->d_V, w, vk1, h->d_opart, hbuf, h->d_octr, &epoch, n_ctas, ordered,
+                      h->d_err, h->stream));
+      CU(cudaMemcpyAsync(hv.data(), hbuf, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, h->stream));
       CU(cudaStreamSynchronize(h->stream));
-      h->launches += 9;
+      h->launches += 1;
       ++it;
-      for (int j = 0; j <= k; ++j) H[(size_t)j * restart + k] = hv[j] + hv2[j];
+      for (int j = 0; j <= k; ++j) H[(size_t)j * restart + k] = hv[j];
+      const double hn = hv[k + 1];
       H[(size_t)(k + 1) * restart + k] = hn;
-      if (hn > 0) CU(launch_scale(N, w, 1.0 / hn, vk1, h->stream));
       for (int j = 0; j < k; ++j) {
         double a = H[(size_t)j * restart + k], b = H[(size_t)(j + 1) * restart + k];
         H[(size_t)j * restart + k] = cs[j] * a + sn[j] * b;
@@ -839,7 +842,8 @@ static void release_mesh_buffers(wbem_context* h) {
                    (void**)&h->d_ccol, (void**)&h->d_cval, (void**)&h->d_cinh, (void**)&h->d_cflag,
                    (void**)&h->d_cptr_full, (void**)&h->d_ccol_full, (void**)&h->d_cval_full,
                    (void**)&h->d_tptr, (void**)&h->d_tsrc, (void**)&h->d_tval, (void**)&h->d_binv,
-                   (void**)&h->d_V, (void**)&h->d_part, (void**)&h->d_small, (void**)&h->d_lu,
+                   (void**)&h->d_V, (void**)&h->d_part, (void**)&h->d_small, (void**)&h->d_opart,
+                   (void**)&h->d_octr, (void**)&h->d_lu,
                    (void**)&h->d_split, (void**)&h->d_lutmp, (void**)&h->d_info, (void**)&h->d_sol,
                    (void**)&h->d_rhs, (void**)&h->d_b};
   for (void** p : ptrs)

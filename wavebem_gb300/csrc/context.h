@@ -167,6 +167,9 @@ struct wbem_context {
   double* d_small = nullptr;
   double* d_opart = nullptr;   // k_ortho: the CTAs' partial sums
   unsigned* d_octr = nullptr;  // and its grid barrier's counter
+  // mixed mat-vecs: x as float pairs, the second half for the right-hand
+  // side's product, which may run on rhs_stream beside the handle's stream
+  float2* d_xs = nullptr;
   int sms = 0;                 // SMs of the device
   float* d_lu = nullptr;   // mixed: FP32 system matrix, then its LU factors
   // state of d_lu: 0 = neither, 1 = system entries from the assembly (free

@@ -68,9 +68,11 @@ cudaError_t launch_reselect_pairs(int N, int nflip, const int* flips, float2* A2
 cudaError_t launch_matvec_fp64(int N, int mode, const double* Nm, const double* Dm,
                                const uint8_t* mask, const double* alpha, const double* x,
                                double* y, cudaStream_t s);
-// mixed form: P = A2 (mode 0) or B2 (mode 1), the selection already applied
+// mixed form: P = A2 (mode 0) or B2 (mode 1), the selection already applied;
+// xs: N float pairs of scratch that no other stream uses meanwhile
 cudaError_t launch_matvec_mixed(int N, int mode, const float2* P, const uint8_t* mask,
-                                const double* alpha, const double* x, double* y, cudaStream_t s);
+                                const double* alpha, const double* x, float2* xs, double* y,
+                                cudaStream_t s);
 // transposed system operator: y_j = sum_i sel(i,j) x_i (+ diagonal)
 cudaError_t launch_matvec_t_fp64(int N, const double* Nm, const double* Dm, const uint8_t* mask,
                                  const double* alpha, const double* x, double* y, double* part,

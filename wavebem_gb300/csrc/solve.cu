@@ -15,100 +15,71 @@
 
 namespace wbem {
 
-constexpr int kMvChunk = 2048;  // columns staged per chunk
-constexpr int kMvWarps = 8;     // rows per block (one warp each)
+constexpr int kMvThreads = 256;
+constexpr int kMvWarps = kMvThreads / 32;
 
-// y_i = sum_j sel(i,j) x_j + diag. FP64 matrices.
-__global__ void __launch_bounds__(kMvWarps * 32)
+// Sums v[0..R) over the threads of the CTA; thread r < R returns row r's
+// total. Reduce-scatter inside the warps (FP64 additions issue at 1/64 of the
+// FP32 rate), then the warps' sums in order.
+template <int R>
+__device__ __forceinline__ double cta_rows_sum(double v[R]) {
+  static_assert(R == 4 || R == 8, "rows per CTA");
+  __shared__ double red[kMvWarps][R];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int o = 16, n = R / 2; n > 0; o >>= 1, n >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < R / 2; ++i)
+      if (i < n) {
+        const double keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+  }
+  constexpr int G = 32 / R;  // lanes that hold the same row now
+  double s = v[0];
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane % G == 0) red[warp][lane / G] = s;
+  __syncthreads();
+  s = 0.0;
+  if (tid < R)
+    for (int w = 0; w < kMvWarps; ++w) s += red[w][tid];
+  return s;
+}
+
+// y_i = sum_j sel(i,j) x_j + diag. FP64 matrices. A CTA takes 4 rows, its
+// threads the columns: x_j and the column's matrix are read once for the 4
+// rows, whose loads are independent. Bound by the FP64 pipe (one DFMA per 8
+// bytes: 4.6 TB/s at most). With a warp per row and x staged in shared memory
+// it took 46 us at N = 2,000 and 1.10 ms at N = 16,226, now 20 us and
+// 0.61 ms (3.4 TB/s).
+constexpr int kMvRows64 = 4;
+
+__global__ void __launch_bounds__(kMvThreads)
     k_matvec_fp64(int N, int mode, const double* __restrict__ Nm, const double* __restrict__ Dm,
                   const uint8_t* __restrict__ mask, const double* __restrict__ alpha,
                   const double* __restrict__ x, double* __restrict__ y) {
-  __shared__ double xs[kMvChunk];
-  __shared__ uint8_t ms[kMvChunk];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * kMvWarps + warp;
-  const bool active = row < N;
+  constexpr int R = kMvRows64;
+  const int row0 = blockIdx.x * R, tid = threadIdx.x;
   // mode 0: mask ? -D : N ; mode 1: mask ? -N : D
   const double* A0 = (mode == 0) ? Nm : Dm;  // used where mask == 0
   const double* A1 = (mode == 0) ? Dm : Nm;  // used (negated) where mask == 1
-  const double* r0 = A0 + (size_t)(active ? row : 0) * N;
-  const double* r1 = A1 + (size_t)(active ? row : 0) * N;
-  double acc = 0.0;
-  for (int c0 = 0; c0 < N; c0 += kMvChunk) {
-    const int cn = min(kMvChunk, N - c0);
-    __syncthreads();
-    for (int k = threadIdx.x; k < cn; k += blockDim.x) {
-      xs[k] = x[c0 + k];
-      ms[k] = mask[c0 + k];
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll 8
-      for (int k = lane; k < cn; k += 32) {
-        const int j = c0 + k;
-        const double v = ms[k] ? -__ldcs(r1 + j) : __ldcs(r0 + j);
-        acc = fma(v, xs[k], acc);
-      }
-    }
-  }
+  size_t off[R];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (active && lane == 0) {
-    const double xi = x[row];
-    if (mode == 0) {
-      if (!mask[row]) acc = fma(alpha[row], xi, acc);
-    } else {
-      if (mask[row]) acc = fma(-alpha[row], xi, acc);
-    }
-    y[row] = acc;
-  }
-}
-
-cudaError_t launch_matvec_fp64(int N, int mode, const double* Nm, const double* Dm,
-                               const uint8_t* mask, const double* alpha, const double* x,
-                               double* y, cudaStream_t s) {
-  k_matvec_fp64<<<(N + kMvWarps - 1) / kMvWarps, kMvWarps * 32, 0, s>>>(N, mode, Nm, Dm, mask,
-                                                                         alpha, x, y);
-  return cudaGetLastError();
-}
-
-// Same operator with (hi, lo) float pairs whose boundary-condition selection
-// was applied at assembly (P = A2 for mode 0, B2 for mode 1): one contiguous
-// matrix per apply. entry = hi + lo; products and sums in double-float on
-// FP32 units, x given in FP64 and split on the fly.
-__global__ void __launch_bounds__(kMvWarps * 32)
-    k_matvec_mixed(int N, int mode, const float2* __restrict__ P, const uint8_t* __restrict__ mask,
-                   const double* __restrict__ alpha, const double* __restrict__ x,
-                   double* __restrict__ y) {
-  __shared__ float2 xs[kMvChunk];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * kMvWarps + warp;
-  const bool active = row < N;
-  const float2* r0 = P + (size_t)(active ? row : 0) * N;
-  df acc = {0.f, 0.f};
-  for (int c0 = 0; c0 < N; c0 += kMvChunk) {
-    const int cn = min(kMvChunk, N - c0);
-    __syncthreads();
-    for (int k = threadIdx.x; k < cn; k += blockDim.x) {
-      const df v = df_from_double(x[c0 + k]);
-      xs[k] = make_float2(v.hi, v.lo);
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll 8
-      for (int k = lane; k < cn; k += 32) {
-        const float2 a = __ldcs(r0 + c0 + k);
-        const float2 xv = xs[k];
-        df p = two_prod(a.x, xv.x);
-        p.lo = __fmaf_rn(a.x, xv.y, __fmaf_rn(a.y, xv.x, p.lo));
-        acc = df_add(acc, p);
-      }
-    }
-  }
-  double s = df_to_double(acc);
+  for (int r = 0; r < R; ++r) off[r] = (size_t)min(row0 + r, N - 1) * N;
+  double acc[R] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int j = tid; j < N; j += kMvThreads) {
+    const bool m = mask[j] != 0;
+    const double* A = (m ? A1 : A0) + j;
+    const double xj = m ? -x[j] : x[j];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (active && lane == 0) {
+    for (int r = 0; r < R; ++r) acc[r] = fma(__ldcs(A + off[r]), xj, acc[r]);
+  }
+  double s = cta_rows_sum<R>(acc);
+  const int row = row0 + tid;
+  if (tid < R && row < N) {
     const double xi = x[row];
     if (mode == 0) {
       if (!mask[row]) s = fma(alpha[row], xi, s);
@@ -119,58 +90,170 @@ __global__ void __launch_bounds__(kMvWarps * 32)
   }
 }
 
+cudaError_t launch_matvec_fp64(int N, int mode, const double* Nm, const double* Dm,
+                               const uint8_t* mask, const double* alpha, const double* x,
+                               double* y, cudaStream_t s) {
+  k_matvec_fp64<<<(N + kMvRows64 - 1) / kMvRows64, kMvThreads, 0, s>>>(N, mode, Nm, Dm, mask, alpha,
+                                                                       x, y);
+  return cudaGetLastError();
+}
+
+// Same operator with (hi, lo) float pairs whose boundary-condition selection
+// was applied at assembly (P = A2 for mode 0, B2 for mode 1): one contiguous
+// matrix per apply. entry = hi + lo; products and sums in double-float on
+// FP32 units, x given in FP64 and split into float pairs (k_split_x) first: a
+// split per CTA and column would cost three FP64-rate instructions for every
+// 4 entries. A CTA takes 4 rows, a thread two columns (16 bytes of each row)
+// per step where N is even. HBM-bound: 285 us (4.0 TB/s) at N = 12,000 with a
+// warp per row, now 182 us (6.3 TB/s); 1.55 ms at N = 32,768, now 1.21 ms.
+constexpr int kMvRowsM = 4;
+
+__global__ void k_split_x(int N, const double* __restrict__ x, float2* __restrict__ xs) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const df v = df_from_double(x[i]);
+  xs[i] = make_float2(v.hi, v.lo);
+}
+
+__device__ __forceinline__ void pair_fma(df& acc, float ah, float al, float xh, float xl) {
+  df p = two_prod(ah, xh);
+  p.lo = __fmaf_rn(ah, xl, __fmaf_rn(al, xh, p.lo));
+  acc = df_add(acc, p);
+}
+
+template <bool EVEN>
+__global__ void __launch_bounds__(kMvThreads)
+    k_matvec_mixed(int N, int mode, const float2* __restrict__ P, const uint8_t* __restrict__ mask,
+                   const double* __restrict__ alpha, const float2* __restrict__ xs,
+                   const double* __restrict__ x, double* __restrict__ y) {
+  constexpr int R = kMvRowsM;
+  const int row0 = blockIdx.x * R, tid = threadIdx.x;
+  const float2* row[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) row[r] = P + (size_t)min(row0 + r, N - 1) * N;
+  df acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] = {0.f, 0.f};
+  if (EVEN) {
+#pragma unroll 2
+    for (int j = 2 * tid; j < N; j += 2 * kMvThreads) {
+      float4 a[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[r] = __ldcs(reinterpret_cast<const float4*>(row[r] + j));
+      const float4 xv = *reinterpret_cast<const float4*>(xs + j);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        pair_fma(acc[r], a[r].x, a[r].y, xv.x, xv.y);
+        pair_fma(acc[r], a[r].z, a[r].w, xv.z, xv.w);
+      }
+    }
+  } else {
+#pragma unroll 4
+    for (int j = tid; j < N; j += kMvThreads) {
+      float2 a[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[r] = __ldcs(row[r] + j);
+      const float2 xv = xs[j];
+#pragma unroll
+      for (int r = 0; r < R; ++r) pair_fma(acc[r], a[r].x, a[r].y, xv.x, xv.y);
+    }
+  }
+  double v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = df_to_double(acc[r]);
+  double s = cta_rows_sum<R>(v);
+  const int i = row0 + tid;
+  if (tid < R && i < N) {
+    const double xi = x[i];
+    if (mode == 0) {
+      if (!mask[i]) s = fma(alpha[i], xi, s);
+    } else {
+      if (mask[i]) s = fma(-alpha[i], xi, s);
+    }
+    y[i] = s;
+  }
+}
+
 cudaError_t launch_matvec_mixed(int N, int mode, const float2* P, const uint8_t* mask,
-                                const double* alpha, const double* x, double* y, cudaStream_t s) {
-  k_matvec_mixed<<<(N + kMvWarps - 1) / kMvWarps, kMvWarps * 32, 0, s>>>(N, mode, P, mask, alpha,
-                                                                          x, y);
+                                const double* alpha, const double* x, float2* xs, double* y,
+                                cudaStream_t s) {
+  k_split_x<<<(N + 255) / 256, 256, 0, s>>>(N, x, xs);
+  const int g = (N + kMvRowsM - 1) / kMvRowsM;
+  if (N & 1)
+    k_matvec_mixed<false><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, xs, x, y);
+  else
+    k_matvec_mixed<true><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, xs, x, y);
   return cudaGetLastError();
 }
 
 // y = S x for the FP32 system matrix S (row-major, leading dimension ld, the
 // constrained operator with alpha on its diagonal): the inner operator of the
-// refinement solver. One warp per row, each lane streams float4 quads of the
-// row; products and sums in FP32 with the lane sums moved into FP64 after
-// every chunk of kMvChunk columns (64 terms per FP32 partial sum), so the
+// refinement solver. A CTA takes 8 rows, a thread four columns (16 bytes) of
+// each per step; products and sums in FP32, at most kMvFlush terms per FP32
+// partial sum (as pairs of floats beyond, FP64 across the threads), so the
 // operator is S to about 1e-6 relative, at 4 bytes of HBM traffic per entry.
-__global__ void __launch_bounds__(kMvWarps * 32)
+// HBM-bound: 317 us (5.1 TB/s) at N = 20,011 with a warp per row, now 271 us.
+constexpr int kMvRows32 = 8;
+constexpr int kMvFlush = 64;
+
+__global__ void __launch_bounds__(kMvThreads, 2)
     k_matvec_s32(int N, int ld, const float* __restrict__ S, const double* __restrict__ x,
                  double* __restrict__ y) {
-  __shared__ __align__(16) float xs[kMvChunk];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * kMvWarps + warp;
-  const bool active = row < N;
-  const float* sr = S + (size_t)(active ? row : 0) * ld;
-  double acc = 0.0;
-  for (int c0 = 0; c0 < N; c0 += kMvChunk) {
-    const int cn = min(kMvChunk, N - c0);
-    __syncthreads();
-    for (int k = threadIdx.x; k < kMvChunk; k += blockDim.x)
-      xs[k] = (k < cn) ? (float)x[c0 + k] : 0.f;
-    __syncthreads();
-    if (active) {
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-      const int cq = cn & ~3;  // whole quads (row starts are 16-byte aligned)
-#pragma unroll 4
-      for (int k = 4 * lane; k < cq; k += 128) {
-        const float4 v = __ldcs(reinterpret_cast<const float4*>(sr + c0 + k));
-        const float4 xv = *reinterpret_cast<const float4*>(xs + k);
-        a0 = __fmaf_rn(v.x, xv.x, a0);
-        a1 = __fmaf_rn(v.y, xv.y, a1);
-        a2 = __fmaf_rn(v.z, xv.z, a2);
-        a3 = __fmaf_rn(v.w, xv.w, a3);
-      }
-      for (int k = cq + lane; k < cn; k += 32) a0 = __fmaf_rn(sr[c0 + k], xs[k], a0);
-      acc += ((double)a0 + (double)a1) + ((double)a2 + (double)a3);
+  constexpr int R = kMvRows32;
+  const int row0 = blockIdx.x * R, tid = threadIdx.x;
+  const float* row[R];
+  df acc[R];
+  float a[R][4];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    row[r] = S + (size_t)min(row0 + r, N - 1) * ld;
+    acc[r] = {0.f, 0.f};
+    a[r][0] = a[r][1] = a[r][2] = a[r][3] = 0.f;
+  }
+  auto flush = [&]() {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const df u = two_sum(a[r][0], a[r][1]), w = two_sum(a[r][2], a[r][3]);
+      acc[r] = df_add(acc[r], df_add(u, w));
+      a[r][0] = a[r][1] = a[r][2] = a[r][3] = 0.f;
+    }
+  };
+  const int nq = N & ~3;  // whole quads (row starts are 16-byte aligned)
+  int n = 0;
+  for (int j = 4 * tid; j < nq; j += 4 * kMvThreads) {
+    float4 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = __ldcs(reinterpret_cast<const float4*>(row[r] + j));
+    // x may be a basis vector of odd length N: 8-byte aligned only
+    const float f0 = (float)x[j], f1 = (float)x[j + 1], f2 = (float)x[j + 2], f3 = (float)x[j + 3];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      a[r][0] = __fmaf_rn(v[r].x, f0, a[r][0]);
+      a[r][1] = __fmaf_rn(v[r].y, f1, a[r][1]);
+      a[r][2] = __fmaf_rn(v[r].z, f2, a[r][2]);
+      a[r][3] = __fmaf_rn(v[r].w, f3, a[r][3]);
+    }
+    if (++n == kMvFlush) {
+      flush();
+      n = 0;
     }
   }
+  flush();
+  if (nq + tid < N) {  // the last one to three columns
+    const float f = (float)x[nq + tid];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (active && lane == 0) y[row] = acc;
+    for (int r = 0; r < R; ++r) acc[r] = df_add(acc[r], two_prod(row[r][nq + tid], f));
+  }
+  double v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = df_to_double(acc[r]);
+  const double s = cta_rows_sum<R>(v);
+  if (tid < R && row0 + tid < N) y[row0 + tid] = s;
 }
 
 cudaError_t launch_matvec_s32(int N, int ld, const float* S, const double* x, double* y,
                               cudaStream_t s) {
-  k_matvec_s32<<<(N + kMvWarps - 1) / kMvWarps, kMvWarps * 32, 0, s>>>(N, ld, S, x, y);
+  k_matvec_s32<<<(N + kMvRows32 - 1) / kMvRows32, kMvThreads, 0, s>>>(N, ld, S, x, y);
   return cudaGetLastError();
 }
 

@@ -400,6 +400,7 @@ int ensure_vectors(wbem_context* h, int restart) {
     if (!h->d_vec[k]) CHK(dev_alloc(h, &h->d_vec[k], (size_t)N));
   if (!h->d_part) CHK(dev_alloc(h, &h->d_part, (size_t)256 * 128 + (size_t)40 * N));
   if (!h->d_small) CHK(dev_alloc(h, &h->d_small, (size_t)512));
+  if (!h->d_xs) CHK(dev_alloc(h, &h->d_xs, (size_t)2 * N));
   if (!h->d_opart) {
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
@@ -426,7 +427,7 @@ int apply_system(wbem_context* h, const double* x, double* y) {
     CU(launch_matvec_fp64(h->N, 0, h->d_N, h->d_D, h->d_mask, h->d_alpha, x, y, h->stream));
   else {
     if (h->profiling) h->prof_matvec.begin(h->stream);
-    CU(launch_matvec_mixed(h->N, 0, h->d_A2, h->d_mask, h->d_alpha, x, y, h->stream));
+    CU(launch_matvec_mixed(h->N, 0, h->d_A2, h->d_mask, h->d_alpha, x, h->d_xs, y, h->stream));
     if (h->profiling) h->prof_matvec.end(h->stream, 8.0 * (double)h->N * h->N);
   }
   CU(launch_constraint_rows(h->n_crows, h->d_crow, h->d_cptr, h->d_ccol, h->d_cval, x, y, h->stream));
@@ -843,7 +844,7 @@ static void release_mesh_buffers(wbem_context* h) {
                    (void**)&h->d_cptr_full, (void**)&h->d_ccol_full, (void**)&h->d_cval_full,
                    (void**)&h->d_tptr, (void**)&h->d_tsrc, (void**)&h->d_tval, (void**)&h->d_binv,
                    (void**)&h->d_V, (void**)&h->d_part, (void**)&h->d_small, (void**)&h->d_opart,
-                   (void**)&h->d_octr, (void**)&h->d_lu,
+                   (void**)&h->d_octr, (void**)&h->d_xs, (void**)&h->d_lu,
                    (void**)&h->d_split, (void**)&h->d_lutmp, (void**)&h->d_info, (void**)&h->d_sol,
                    (void**)&h->d_rhs, (void**)&h->d_b};
   for (void** p : ptrs)
@@ -1118,7 +1119,7 @@ static int prepare_rhs(wbem_handle h, const double* tmp_rhs, bool beside = false
   } else if (h->assembled_prec == WBEM_PREC_FP64)
     CU(launch_matvec_fp64(N, 1, h->d_N, h->d_D, h->d_mask, h->d_alpha, h->d_b, h->d_rhs, rs));
   else
-    CU(launch_matvec_mixed(N, 1, h->d_B2, h->d_mask, h->d_alpha, h->d_b, h->d_rhs, rs));
+    CU(launch_matvec_mixed(N, 1, h->d_B2, h->d_mask, h->d_alpha, h->d_b, h->d_xs + N, h->d_rhs, rs));
   CU(launch_set_rows(h->n_crows, h->d_crow, h->d_cinh, h->d_rhs, rs));
   h->launches += 2;
   if (rs != h->stream) {
@@ -1235,7 +1236,7 @@ static int op_caller(wbem_handle h, int mode, const double* src, double* dst) {
     CU(launch_matvec_fp64(N, mode, h->d_N, h->d_D, h->d_mask, h->d_alpha, h->d_vec[3], h->d_vec[4], h->stream));
   else
     CU(launch_matvec_mixed(N, mode, mode == 0 ? h->d_A2 : h->d_B2, h->d_mask, h->d_alpha, h->d_vec[3],
-                           h->d_vec[4], h->stream));
+                           h->d_xs, h->d_vec[4], h->stream));
   CU(copy_sync(h, yi.data(), h->d_vec[4], sizeof(double) * N, cudaMemcpyDeviceToHost));
   for (int i = 0; i < N; ++i) dst[h->perm[i]] = yi[i];
   if (mode == 0) {

@@ -60,12 +60,44 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait on an mbarrier phase. Returns false after `limit` polls.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
-                                                  uint32_t limit = (1u << 24)) {
-  for (uint32_t it = 0; it < limit; ++it)
-    if (mbar_try_wait(bar, parity)) return true;
+// Waits on other CTAs or on the copy engine give up after this long.
+constexpr unsigned long long kWaitNs = 2000000000ull;
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Bounded wait on an mbarrier phase. Returns false after kWaitNs (a poll may
+// itself be suspended for a while, so a count of polls would not bound it).
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = global_ns();
+  do {
+    for (int it = 0; it < 16; ++it)
+      if (mbar_try_wait(bar, parity)) return true;
+  } while (global_ns() - t0 < kWaitNs);
   return false;
+}
+
+// Bounded wait until *flag == value, or (AT_LEAST) until it has reached value
+// (as a counter that may wrap around). Returns false after kWaitNs, or at once
+// if a wait has already given up somewhere (code set in the error word), so
+// that a queue of dependent launches ends soon.
+template <bool AT_LEAST>
+__device__ __forceinline__ bool flag_wait_bounded(const unsigned* flag, unsigned value, const DevErr* err) {
+  auto done = [&]() {
+    const unsigned v = *((const volatile unsigned*)flag);
+    return AT_LEAST ? (int)(v - value) >= 0 : v == value;
+  };
+  if (done()) return true;
+  const unsigned long long t0 = global_ns();
+  do {
+    for (int it = 0; it < 64; ++it)
+      if (done()) return true;
+  } while (*((const volatile int*)&err->code) == 0 && global_ns() - t0 < kWaitNs);
+  return done();
 }
 
 // 1-D bulk copy global -> shared (TMA engine), completion counted on `bar`.

@@ -12,13 +12,12 @@
 // non-finite -> WBEM_ERR_SINGULAR).
 //
 // Step k (block size kNB = 128), inside outer panels of kNB2 = 512 columns:
-//   1. k_diag_block: LU of A_kk (one CTA, registers + shared memory), plus
-//      the inverses of its unit-lower and upper factors;
-//   2. k_panel_small: L_ik = A_ik inv(U_kk) and U_kj = inv(L_kk) A_kj (FP32
-//      SIMT); then the panel's own trailing update A_ij -= L_ik U_kj (FP32,
-//      K = 128). Both run first for the next block's 128 rows (the strip the
-//      next diagonal block needs) and then, on a second stream, for the rows
-//      below.
+//   1. k_diag_block: LU of A_kk (one CTA, shared memory), plus the inverses of
+//      its unit-lower and upper factors;
+//   2. L_ik = A_ik inv(U_kk) and U_kj = inv(L_kk) A_kj (FP32 SIMT), then the
+//      panel's own trailing update A_ij -= L_ik U_kj (FP32, K = 128): for the
+//      next block's 128 rows (the strip the next diagonal block needs) by
+//      k_strip, on a second stream for the rows below by k_panel_small.
 // Per outer panel P: U12 = inv(L11) A12 for the rest of its rows (FP32, with
 // the earlier blocks' updates first; block row k as soon as A_kk is factored,
 // on its own stream, writing an FP32 copy of U12^T), then the bulk trailing
@@ -30,8 +29,8 @@
 // vector instead of 5e-6) for one more GMRES iteration, and takes 8% off the
 // update, which streams the same operand bytes per K step either way.
 // The update is split between the next panel's columns (high-priority
-// stream) and the remainder (low-priority stream). The panel kernels have a
-// 13 KB footprint, so the next panel's chain runs beside the remainder's CTAs
+// stream) and the remainder (low-priority stream). The panel kernels have 13
+// and 16 KB footprints, so the next panel's chain runs beside the remainder's CTAs
 // on every SM (look-ahead); a few SMs stay free for the 200 KB diagonal
 // blocks.
 #include <cuda.h>
@@ -110,29 +109,30 @@ __global__ void k_lu_constraint_entries(int nrows, const int* __restrict__ crow,
 
 // ------------------------------------------------------------ diagonal block
 // LU (no pivoting) of the kNB x kNB block at (k0, k0) and the inverses of its
-// unit-lower and upper factors; writes the factors back to A, the inverses
-// row-major (linv, uinv) and column-major (linvT, uinvT). One CTA, a
-// register-resident unblocked elimination with one CTA barrier per pivot and
-// every thread busy at every pivot. 1024 threads:
-// thread (r, q) holds 16 entries of row r (columns 16q .. 16q+15) in
-// registers:
-//   * while r > k (row below the pivot) the combined row of the LU: the
-//     working matrix right of the pivot, the row of inv(L) left of it (both
-//     obey w_r -= l_rk * w_k), the pivot slot turning from a_rk into -l_rk;
-//   * from r = k on, the row of Z = inv(U1), U = D U1 (D = diag(U)): the
-//     column operations z_rj -= (u_kj / u_kk) z_rk, j > k, that take U to D.
-// Each finished row is published to a row history in shared memory (U and
-// inv(L) are read from it at the end), each column of Z to the upper
-// triangle of the L array when it is final (later steps may leave garbage in
-// register slots j <= k of a Z row, none of which is read again), and
-// inv(U) = Z D^-1. The pivot loop is unrolled by 16 so every register slot is
-// a compile-time index. Warp w takes column block q = w / 4 and row group g
-// with g + q = w (mod 4): each scheduler (w mod 4) holds two warps of every
-// row group and one of the four warps that own a pivot column.
-constexpr int kDLD = kNB + 1;     // padded shared rows
-constexpr int kDiagThreads = 1024;
-constexpr int kDRowLD = 132;      // row history: 16-byte rows
-constexpr size_t kDiagSmemBytes = ((size_t)kNB * kDLD + (size_t)kNB * kDRowLD + 2 * kNB + kNB) * sizeof(float);
+// unit-lower and upper factors; writes the factors back to A and the inverses
+// that the panels read (inv(L) column-major, inv(U) row-major; the other
+// orientations follow in k_transpose_inverses). One CTA, everything
+// in shared memory: S (the block, then L and U), IL and IU (the inverses).
+// Eight steps of 16 columns, two CTA barriers each:
+//   A  warp 0 factors the 16 x 16 diagonal block in registers, a row per lane;
+//      lanes 16..31 carry the rows of the identity along, which become the
+//      inverse of its L. The registers rotate by one column per pivot, so one
+//      short loop body serves all 16 pivots;
+//   B  a thread per row solves x U = a for L21, two threads per column apply
+//      the inverse of L for U12;
+//   C  warps 1..14 update the trailing block in 4 x 4 tiles, except its leading
+//      16 x 16, which warp 0 updates and factors meanwhile (look-ahead); warp
+//      15 inverts the 16 x 16 block of U.
+// Then the inverses by doubling: from two inverted blocks of size b (16, 32,
+// 64), X21 = -L22^-1 (L21 L11^-1) and X12 = -(U11^-1 U12) U22^-1, two barriers
+// each; the inner products T sit in the blocks of the other inverse that are
+// zero, which are cleared again afterwards.
+// Bound by the latency of A (16 pivots in a row, eight times). Unblocked, with
+// a CTA barrier per pivot, the block took 51.5 us; now 34.6 us.
+constexpr int kDThreads = 512;
+constexpr int kDB = 16;     // columns per step
+constexpr int kDLD = 132;   // shared rows: 16-byte aligned, rows r and r + 8 share banks
+constexpr size_t kDiagSmemBytes = ((size_t)3 * kNB * kDLD + kDB * kDLD + kNB) * sizeof(float);
 
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
@@ -140,113 +140,336 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-__global__ void __launch_bounds__(kDiagThreads, 1)
-    k_diag_block(int ld, int k0, int nb, float* __restrict__ A, float* __restrict__ linv,
-                  float* __restrict__ uinv, float* __restrict__ linvT, float* __restrict__ uinvT,
-                  DevErr* err) {
-  extern __shared__ __align__(16) float dsm[];
-  float* sLZ = dsm;                       // [128][129]: input; then L (strict lower), Z (upper)
-  float* sRows = sLZ + kNB * kDLD;        // [128][132]: row history (inv(L) | U)
-  float* sCol = sRows + kNB * kDRowLD;    // [2][128] pivot column of the rows below
-  float* sInv = sCol + 2 * kNB;           // [128] 1 / u_kk
-  __shared__ int bad;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int q = warp >> 2, g = ((warp & 3) - q) & 3;
-  const int r = 32 * g + lane, c0 = 16 * q;
-  for (int idx = tid; idx < kNB * kNB; idx += kDiagThreads) {
-    const int rr = idx >> 7, cc = idx & 127;
-    float* dst = sLZ + rr * kDLD + cc;
-    if (rr < nb && cc < nb)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                   "l"(A + (size_t)(k0 + rr) * ld + k0 + cc));
-    else
-      *dst = rr == cc ? 1.f : 0.f;
-  }
-  asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
-  if (tid == 0) bad = 0;
-  __syncthreads();
-  float w[16];
+// O (4 x 4) = sign * sum over k0 <= k < k1 of Lp(i, k) Rp(k, j), all with rows
+// of kDLD floats; the tile's rows are rs apart
+__device__ __forceinline__ void diag_tile(const float* Lp, const float* Rp, float* Op, int rs, int k0,
+                                          int k1, float sign) {
+  float acc[4][4];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) w[i] = sLZ[r * kDLD + c0 + i];  // lanes are rows: distinct banks
-  __syncthreads();
-  // publish row 0 and column 0; row 0 continues as a Z row
-  if (r == 0) {
+  for (int u = 0; u < 4; ++u)
 #pragma unroll
-    for (int i = 0; i < 16; i += 4)
-      *reinterpret_cast<float4*>(sRows + c0 + i) = make_float4(w[i], w[i + 1], w[i + 2], w[i + 3]);
-    if (q == 0) {
-      const float p = w[0];
-      if (!(fabsf(p) > 0.f && isfinite(p))) bad = 1;
-      sInv[0] = rcp_approx(p);
-      sLZ[0] = 1.f;
+    for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
+  const int ls = rs * kDLD;
+#pragma unroll 1
+  for (int k = k0; k < k1; k += 4) {  // k0 and k1 are multiples of 4
+    float4 l[4], r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      l[u] = *reinterpret_cast<const float4*>(Lp + u * ls + k);
+      r[u] = *reinterpret_cast<const float4*>(Rp + (k + u) * kDLD);
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) w[i] = 0.f;
+    for (int u = 0; u < 4; ++u) {
+      const float lu[4] = {l[u].x, l[u].y, l[u].z, l[u].w};
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        acc[u][0] = __fmaf_rn(lu[w], r[w].x, acc[u][0]);
+        acc[u][1] = __fmaf_rn(lu[w], r[w].y, acc[u][1]);
+        acc[u][2] = __fmaf_rn(lu[w], r[w].z, acc[u][2]);
+        acc[u][3] = __fmaf_rn(lu[w], r[w].w, acc[u][3]);
+      }
+    }
   }
-  if (q == 0 && r > 0) sCol[r] = w[0];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    *reinterpret_cast<float4*>(Op + u * ls) =
+        make_float4(sign * acc[u][0], sign * acc[u][1], sign * acc[u][2], sign * acc[u][3]);
+}
+
+__global__ void __launch_bounds__(kDThreads, 1)
+    k_diag_block(int ld, int k0, int nb, float* __restrict__ A, float* __restrict__ uinv,
+                 float* __restrict__ linvT, DevErr* err) {
+  extern __shared__ __align__(16) float dsm[];
+  float* S = dsm;                  // [128][132]
+  float* IL = S + kNB * kDLD;      // inverse of L (unit diagonal stored)
+  float* IU = IL + kNB * kDLD;     // inverse of U
+  float* LT = IU + kNB * kDLD;     // [16][132]: L21 of the step, transposed
+  float* dinv = LT + kDB * kDLD;   // [128] 1 / u_kk
+  __shared__ __align__(16) float t16[kDB][kDB];  // the step's 16 x 16 inverse of L, transposed
+  __shared__ __align__(16) float prow[2][2 * kDB];  // the pivot row of step A
+  __shared__ int bad;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int idx = tid; idx < kNB * kNB / 4; idx += kDThreads) {
+    const int r = idx >> 5, c = (idx & 31) * 4;
+    float* dst = S + r * kDLD + c;
+    if (r < nb && c + 3 < nb) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                   "l"(A + (size_t)(k0 + r) * ld + k0 + c));
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        dst[u] = r < nb && c + u < nb ? A[(size_t)(k0 + r) * ld + k0 + c + u] : (r == c + u ? 1.f : 0.f);
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int idx = tid; idx < 2 * kNB * kDLD / 4; idx += kDThreads)
+    reinterpret_cast<float4*>(IL)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid == 0) bad = 0;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+  const int r = lane & 15;
 #pragma unroll 1
-  for (int kb = 0; kb < 8; ++kb) {
+  for (int j0 = 0; j0 < kNB; j0 += kDB) {
+    if (warp == 0) {
+      float* D = S + (j0 + r) * kDLD + j0;
+      if (j0 > 0) {  // the diagonal block's share of the previous step's update
+        const int h = lane >> 4;
+        float4 c0 = *reinterpret_cast<float4*>(D + 8 * h), c1 = *reinterpret_cast<float4*>(D + 8 * h + 4);
 #pragma unroll
-    for (int s = 0; s < 16; ++s) {
-      if (s == 15 && kb == 7) break;  // the last pivot has nothing below it
-      const int k = 16 * kb + s, k1 = k + 1;
-      const int s1 = (s + 1) & 15, kb1 = kb + (s == 15 ? 1 : 0);
-      const float* row = sRows + k * kDRowLD;
-      const float* srcp = r > k ? sCol + (s & 1) * kNB + r : sLZ + r * kDLD + k;
-      const float m = *srcp * sInv[k];
-      // a warp whose rows are all Z rows and whose columns are all left of
-      // the pivot holds only slots that are never read again: skip it
-      if (32 * g + 31 > k || c0 + 15 > k) {
+        for (int k = 0; k < kDB; ++k) {
+          const float l = LT[k * kDLD + j0 + r];
+          const float* u = S + (j0 - kDB + k) * kDLD + j0 + 8 * h;
+          const float4 u0 = *reinterpret_cast<const float4*>(u), u1 = *reinterpret_cast<const float4*>(u + 4);
+          c0.x = __fmaf_rn(-l, u0.x, c0.x);
+          c0.y = __fmaf_rn(-l, u0.y, c0.y);
+          c0.z = __fmaf_rn(-l, u0.z, c0.z);
+          c0.w = __fmaf_rn(-l, u0.w, c0.w);
+          c1.x = __fmaf_rn(-l, u1.x, c1.x);
+          c1.y = __fmaf_rn(-l, u1.y, c1.y);
+          c1.z = __fmaf_rn(-l, u1.z, c1.z);
+          c1.w = __fmaf_rn(-l, u1.w, c1.w);
+        }
+        *reinterpret_cast<float4*>(D + 8 * h) = c0;
+        *reinterpret_cast<float4*>(D + 8 * h + 4) = c1;
+        __syncwarp();
+      }
+      // ---- A: [block | identity], a row per lane
+      float a[kDB];
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(row + c0 + i);  // broadcast
-          w[i] = __fmaf_rn(-m, v.x, w[i]);
-          w[i + 1] = __fmaf_rn(-m, v.y, w[i + 1]);
-          w[i + 2] = __fmaf_rn(-m, v.z, w[i + 2]);
-          w[i + 3] = __fmaf_rn(-m, v.w, w[i + 3]);
+      for (int j = 0; j < kDB; ++j) a[j] = lane < 16 ? D[j] : (j == r ? 1.f : 0.f);
+      float mypiv = 0.f, myinv = 0.f;
+      const int half = lane & 16;
+#pragma unroll 1
+      for (int k = 0; k < kDB; ++k) {
+        // the pivot row (and its row of the identity part) through shared memory
+        if (r == k) {
+#pragma unroll
+          for (int j = 0; j < kDB; j += 4)
+            *reinterpret_cast<float4*>(&prow[k & 1][half + j]) = make_float4(a[j], a[j + 1], a[j + 2], a[j + 3]);
+        }
+        const float c = __shfl_sync(0xffffffffu, a[0], r);
+        __syncwarp();
+        const float p = prow[k & 1][0];
+        float v[kDB];
+#pragma unroll
+        for (int j = 0; j < kDB; j += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(&prow[k & 1][half + j]);
+          v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
+        }
+        const float pi = rcp_approx(p);
+        const float m = r > k ? c * pi : 0.f;
+        mypiv = lane == k ? p : mypiv;
+        myinv = lane == k ? pi : myinv;
+        if (lane < 16 && r > k) D[k] = m;
+        const float last = __fmaf_rn(-m, v[0], a[0]);
+#pragma unroll
+        for (int j = 0; j + 1 < kDB; ++j) a[j] = __fmaf_rn(-m, v[j + 1], a[j + 1]);
+        a[kDB - 1] = last;
+      }
+      if (lane < 16) {
+        dinv[j0 + r] = myinv;
+        if (!(fabsf(mypiv) > 0.f && isfinite(mypiv))) bad = 1;
+#pragma unroll
+        for (int j = 0; j < kDB; ++j)
+          if (j >= r) D[j] = a[j];
+      } else {
+        float* out = IL + (j0 + r) * kDLD + j0;
+#pragma unroll
+        for (int j = 0; j < kDB; ++j) {
+          out[j] = a[j];
+          t16[j][r] = a[j];
         }
       }
-      if (q == kb && r > k) {  // pivot slot of a row below: -l_rk; L keeps l_rk
-        w[s] = -m;
-        sLZ[r * kDLD + k] = m;
-      }
-      if (__any_sync(0xffffffffu, r == k1)) {  // warp-uniform: the warp holding row k+1
-        if (r == k1) {  // row k+1 is final: publish it, continue as a Z row
-          float* nrow = sRows + k1 * kDRowLD;
+    }
+    __syncthreads();
+    const int j1 = j0 + kDB;
+    if (j1 < kNB) {
+      // ---- B
+      if (tid < kNB) {
+        const int row = j1 + tid;
+        if (row < kNB) {
+          float* p = S + row * kDLD + j0;
+          float x[kDB];
 #pragma unroll
-          for (int i = 0; i < 16; i += 4)
-            *reinterpret_cast<float4*>(nrow + c0 + i) = make_float4(w[i], w[i + 1], w[i + 2], w[i + 3]);
-          if (q == kb1) {
-            const float p = w[s1];
-            if (!(fabsf(p) > 0.f && isfinite(p))) bad = 1;
-            sInv[k1] = rcp_approx(p);
-            sLZ[k1 * kDLD + k1] = 1.f;  // z_kk
+          for (int q = 0; q < kDB; q += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(p + q);
+            x[q] = t.x; x[q + 1] = t.y; x[q + 2] = t.z; x[q + 3] = t.w;
           }
 #pragma unroll
-          for (int i = 0; i < 16; ++i) w[i] = 0.f;
+          for (int i = 0; i < kDB; ++i) {
+            x[i] *= dinv[j0 + i];
+            const float* u = S + (j0 + i) * kDLD + j0;
+#pragma unroll
+            for (int q = (i + 1) & ~3; q < kDB; q += 4) {
+              const float4 t = *reinterpret_cast<const float4*>(u + q);
+              const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+              for (int w = 0; w < 4; ++w)
+                if (q + w > i) x[q + w] = __fmaf_rn(-x[i], tv[w], x[q + w]);
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < kDB; q += 4)
+            *reinterpret_cast<float4*>(p + q) = make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]);
+#pragma unroll
+          for (int j = 0; j < kDB; ++j) LT[j * kDLD + row] = x[j];
         }
-      }
-      if (q == kb1 && r != k1) {  // column k+1: multipliers below, final Z column above
-        float* dst = r > k1 ? sCol + ((s + 1) & 1) * kNB + r : sLZ + r * kDLD + k1;
-        *dst = w[s1];
+      } else if (tid < 3 * kNB) {
+        // two threads per column, eight of the sixteen rows each
+        const int q = tid - kNB, col = j1 + (q & (kNB - 1)), h = 8 * (q >> 7);
+        float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (col < kNB) {
+#pragma unroll
+          for (int k = 0; k < kDB; ++k) {
+            const float x = S[(j0 + k) * kDLD + col];
+            const float4 t0 = *reinterpret_cast<const float4*>(&t16[k][h]);
+            const float4 t1 = *reinterpret_cast<const float4*>(&t16[k][h + 4]);
+            y[0] = __fmaf_rn(t0.x, x, y[0]);
+            y[1] = __fmaf_rn(t0.y, x, y[1]);
+            y[2] = __fmaf_rn(t0.z, x, y[2]);
+            y[3] = __fmaf_rn(t0.w, x, y[3]);
+            y[4] = __fmaf_rn(t1.x, x, y[4]);
+            y[5] = __fmaf_rn(t1.y, x, y[5]);
+            y[6] = __fmaf_rn(t1.z, x, y[6]);
+            y[7] = __fmaf_rn(t1.w, x, y[7]);
+          }
+        }
+        asm volatile("barrier.sync 1, 256;" ::: "memory");  // both halves have read the column
+        if (col < kNB)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) S[(j0 + h + i) * kDLD + col] = y[i];
       }
       __syncthreads();
     }
+    // ---- C
+    if (warp == 15) {
+      // column `lane` of the inverse of the 16 x 16 block of U, from the last row up
+      const float* U = S + j0 * kDLD + j0;
+      float x[kDB];
+#pragma unroll
+      for (int i = kDB - 1; i >= 0; --i) {
+        float t0 = i == r ? 1.f : 0.f, t1 = 0.f;
+#pragma unroll
+        for (int q = i & ~3; q < kDB; q += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(U + i * kDLD + q);
+          if (q > i) t0 = __fmaf_rn(-t.x, x[q], t0);
+          if (q + 1 > i) t1 = __fmaf_rn(-t.y, x[q + 1], t1);
+          if (q + 2 > i) t0 = __fmaf_rn(-t.z, x[q + 2], t0);
+          if (q + 3 > i) t1 = __fmaf_rn(-t.w, x[q + 3], t1);
+        }
+        x[i] = (t0 + t1) * dinv[j0 + i];
+      }
+      if (lane < 16)
+#pragma unroll
+        for (int i = 0; i < kDB; ++i) IU[(j0 + i) * kDLD + j0 + r] = x[i];
+    } else if (warp >= 1 && j1 < kNB) {
+      const int nt = (kNB - j1) / 4;
+      for (int q = tid - 32; q < nt * nt; q += kDThreads - 64) {
+        const int ti = q / nt, tj = q - ti * nt;
+        if (ti < kDB / 4 && tj < kDB / 4) continue;  // warp 0's
+        const int i = j1 + 4 * ti, j = j1 + 4 * tj;
+        float* c = S + i * kDLD + j;
+        float4 o[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) o[u] = *reinterpret_cast<float4*>(c + u * kDLD);
+#pragma unroll 4
+        for (int k = 0; k < kDB; ++k) {
+          const float4 l = *reinterpret_cast<const float4*>(LT + k * kDLD + i);
+          const float4 t = *reinterpret_cast<const float4*>(S + (j0 + k) * kDLD + j);
+          const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            o[u].x = __fmaf_rn(-lv[u], t.x, o[u].x);
+            o[u].y = __fmaf_rn(-lv[u], t.y, o[u].y);
+            o[u].z = __fmaf_rn(-lv[u], t.z, o[u].z);
+            o[u].w = __fmaf_rn(-lv[u], t.w, o[u].w);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(c + u * kDLD) = o[u];
+      }
+    }
   }
+  __syncthreads();
   if (bad) {
     if (tid == 0) dev_fail(err, WBEM_ERR_SINGULAR, 51, k0, 0);
     return;  // uniform
   }
-  for (int idx = tid; idx < kNB * kNB; idx += kDiagThreads) {
-    const int rr = idx >> 7, cc = idx & 127;
-    const float rowv = sRows[rr * kDRowLD + cc];
-    if (rr < nb && cc < nb) A[(size_t)(k0 + rr) * ld + k0 + cc] = cc < rr ? sLZ[rr * kDLD + cc] : rowv;
-    linv[idx] = cc < rr ? rowv : (cc == rr ? 1.f : 0.f);
-    linvT[idx] = rr < cc ? sRows[cc * kDRowLD + rr] : (cc == rr ? 1.f : 0.f);
-    uinv[idx] = rr <= cc ? sLZ[rr * kDLD + cc] * sInv[cc] : 0.f;
-    uinvT[idx] = cc <= rr ? sLZ[cc * kDLD + rr] * sInv[rr] : 0.f;
+  // ---- inverses by doubling; tiles of 4 x 4, half of the threads on L, half on
+  // U. The triangular factor of a product bounds its k by the tile's column
+  // or row: a warp takes tiles with the same bound fc, the factor U in the
+  // opposite order, so that short and long warps share a scheduler. Bounded by
+  // the column: columns fc .., rows fr + b / 4 u (consecutive lanes, consecutive
+  // rows); by the row: rows fc .., columns 4 fr ...
+#pragma unroll 1
+  for (int b = kDB; b < kNB; b *= 2) {
+    const int sd = b / 4, per = sd * sd, n = per * (kNB / (2 * b));  // tiles per block, per factor
+    const int w = tid < n ? 0 : 1, q = w == 0 ? tid : 2 * n - 1 - tid;
+    const bool on = q >= 0;
+    const int o = on ? 2 * b * (q / per) : 0;
+    const int fr = (on ? q % per : 0) % sd, fc = 4 * ((on ? q % per : 0) / sd);
+    // T_L = L21 IL11 in IU's lower block, T_U = IU11 U12 in IL's upper block
+    if (on) {
+      if (w == 0)
+        diag_tile(S + (o + b + fr) * kDLD + o, IL + o * kDLD + o + fc, IU + (o + b + fr) * kDLD + o + fc, sd,
+                  fc, b, 1.f);
+      else
+        diag_tile(IU + (o + fc) * kDLD + o, S + o * kDLD + o + b + 4 * fr, IL + (o + fc) * kDLD + o + b + 4 * fr,
+                  1, fc, b, 1.f);
+    }
+    __syncthreads();
+    if (on) {
+      if (w == 0)
+        diag_tile(IL + (o + b + fc) * kDLD + o + b, IU + (o + b) * kDLD + o + 4 * fr,
+                  IL + (o + b + fc) * kDLD + o + 4 * fr, 1, 0, fc + 4, -1.f);
+      else
+        diag_tile(IL + (o + fr) * kDLD + o + b, IU + (o + b) * kDLD + o + b + fc,
+                  IU + (o + fr) * kDLD + o + b + fc, sd, 0, fc + 4, -1.f);
+    }
+    __syncthreads();
+    if (2 * b == kNB) break;  // the last products are masked on the way out
+    if (on) {
+      float* t = w == 0 ? IU + (o + b + fc) * kDLD + o + 4 * fr : IL + (o + fc) * kDLD + o + b + 4 * fr;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(t + u * kDLD) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
   }
+  for (int idx = tid; idx < kNB * kNB / 4; idx += kDThreads) {
+    const int rr = idx >> 5, cc = (idx & 31) * 4;
+    const float4 v = *reinterpret_cast<const float4*>(S + rr * kDLD + cc);
+    float* ap = A + (size_t)(k0 + rr) * ld + k0 + cc;
+    if (rr < nb) {
+      if (cc + 3 < nb) {
+        *reinterpret_cast<float4*>(ap) = v;
+      } else {
+        const float e[4] = {v.x, v.y, v.z, v.w};
+        for (int u = 0; cc + u < nb; ++u) ap[u] = e[u];
+      }
+    }
+    float4 x = *reinterpret_cast<const float4*>(IU + rr * kDLD + cc);
+    if (cc + 3 < rr) x = make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<float4*>(uinv)[idx] = x;
+  }
+  // transposed: consecutive lanes read consecutive rows (4 of them share a bank)
+  for (int idx = tid; idx < kNB * kNB; idx += kDThreads)
+    linvT[idx] = (idx & (kNB - 1)) >= (idx >> 7) ? IL[(idx & (kNB - 1)) * kDLD + (idx >> 7)] : 0.f;
+}
+
+// The inverses the chain does not read, once per factorisation: linv from
+// linvT and uinvT from uinv, one 32 x 32 tile per CTA.
+__global__ void __launch_bounds__(256)
+    k_transpose_inverses(const float* __restrict__ linvT, const float* __restrict__ uinv,
+                         float* __restrict__ linv, float* __restrict__ uinvT) {
+  __shared__ float t[32][33];
+  const size_t o = (size_t)blockIdx.x * kNB * kNB;
+  const float* src = (blockIdx.z ? uinv : linvT) + o;
+  float* dst = (blockIdx.z ? uinvT : linv) + o;
+  const int r0 = (blockIdx.y >> 2) * 32, c0 = (blockIdx.y & 3) * 32;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int i = w; i < 32; i += 8) t[i][lane] = src[(r0 + i) * kNB + c0 + lane];
+  __syncthreads();
+  for (int i = w; i < 32; i += 8) dst[(c0 + i) * kNB + r0 + lane] = t[lane][i];
 }
 
 // ------------------------------------------------------------- panel GEMM
@@ -500,6 +723,153 @@ static cudaError_t run_panel_small(const PanelArgs& pa, const SplitOut& s1, cons
                                    cudaStream_t s) {
   dim3 g((pa.rows + TM - 1) / TM, (pa.cols + TN - 1) / TN);
   k_panel_small<TM, TN, ATRANS><<<g, 256, 0, s>>>(pa, s1, s2);
+  return cudaGetLastError();
+}
+
+// Products of the chain from one diagonal block to the next: 128 x 128 blocks
+// at K = 128, where a launch's latency counts. X (8 x 128) = Y (8 x K) Z (K x
+// 128) per CTA, or subtracted from X; up to two products share a launch. X and
+// Y are given by the strides of their (y, z) and (y, k) elements, so a row
+// panel is computed transposed, and X may overlie Y: a CTA reads its Y first,
+// and no other CTA reads it. 16 CTAs per 128 x 128 block; each of four warps
+// takes a quarter of K (its rows of Z come straight into registers, 16 at a
+// time, so the loads' latency is paid once or twice), the partial sums meet in
+// shared memory (16 KB: fits beside a trailing-update CTA). One launch takes
+// 5.2 us; the 64 x 128 tiles of k_panel_small put such a block on two CTAs
+// and took 13.9 to 15.5 us.
+struct StripProd {
+  const float* Y;
+  const float* Z;  // Z(k, z) = Z[k * ldz + z]
+  float* X;
+  int yy, yk;      // Y(y, k) = Y[y * yy + k * yk]; one of the two is 1
+  int xy, xz;      // X(y, z) = X[y * xy + z * xz]; one of the two is 1
+  int ldz;
+  int ny, nz;      // valid y and z
+  int sub;         // 1: X -= product, 0: X = product
+};
+constexpr int kStripY = 8, kStripZ = 128, kStripThreads = 128, kStripWarps = kStripThreads / 32;
+constexpr int kStripB = 16;  // rows of Z in registers at a time
+
+__host__ __device__ inline int strip_ctas(const StripProd& p) {
+  return ((p.ny + kStripY - 1) / kStripY) * ((p.nz + kStripZ - 1) / kStripZ);
+}
+
+// n0: CTAs of product p0; the others take p1
+__global__ void __launch_bounds__(kStripThreads) k_strip(StripProd p0, StripProd p1, int n0) {
+  __shared__ __align__(16) float Ys[kNB][kStripY];  // then the last warp's partial sums
+  __shared__ __align__(16) float red[kStripWarps - 1][kStripY][kStripZ];
+  static_assert(kNB * kStripY == kStripY * kStripZ, "the partial sums fit in Ys");
+  const bool first = (int)blockIdx.x < n0;
+  const StripProd p = first ? p0 : p1;
+  const int t = first ? blockIdx.x : blockIdx.x - n0;
+  const int nty = (p.ny + kStripY - 1) / kStripY;
+  const int y0 = (t % nty) * kStripY, z0 = (t / nty) * kStripZ;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int z = z0 + 4 * lane, kw = warp * (kNB / kStripWarps);
+  const bool zfull = z + 3 < p.nz;
+  float4 zr[kStripB];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int k = 0; k < kStripB; ++k) {
+      const float* src = p.Z + (size_t)(k0 + k) * p.ldz + z;
+      if (zfull) {
+        zr[k] = __ldcg(reinterpret_cast<const float4*>(src));
+      } else {
+        zr[k].x = z < p.nz ? src[0] : 0.f;
+        zr[k].y = z + 1 < p.nz ? src[1] : 0.f;
+        zr[k].z = z + 2 < p.nz ? src[2] : 0.f;
+        zr[k].w = 0.f;
+      }
+    }
+  };
+  load(kw);
+  if (p.yk == 1) {  // rows of K floats
+#pragma unroll
+    for (int u = 0; u < kStripY * kNB / 4 / kStripThreads; ++u) {
+      const int q = tid + kStripThreads * u, y = q >> 5, k = (q & 31) * 4;
+      const float4 v = y0 + y < p.ny
+                           ? __ldcg(reinterpret_cast<const float4*>(p.Y + (size_t)(y0 + y) * p.yy + k))
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+      Ys[k][y] = v.x;
+      Ys[k + 1][y] = v.y;
+      Ys[k + 2][y] = v.z;
+      Ys[k + 3][y] = v.w;
+    }
+  } else {  // a row of 8 floats per k
+    const float* src = p.Y + (size_t)tid * p.yk + y0;
+    if (y0 + kStripY <= p.ny) {
+      *reinterpret_cast<float4*>(&Ys[tid][0]) = __ldcg(reinterpret_cast<const float4*>(src));
+      *reinterpret_cast<float4*>(&Ys[tid][4]) = __ldcg(reinterpret_cast<const float4*>(src) + 1);
+    } else {
+#pragma unroll
+      for (int y = 0; y < kStripY; ++y) Ys[tid][y] = y0 + y < p.ny ? src[y] : 0.f;
+    }
+  }
+  __syncthreads();
+  float acc[kStripY][4];
+#pragma unroll
+  for (int y = 0; y < kStripY; ++y)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) acc[y][v] = 0.f;
+#pragma unroll
+  for (int kb = 0; kb < kNB / kStripWarps; kb += kStripB) {
+#pragma unroll
+    for (int k = 0; k < kStripB; ++k) {
+      const float4 a = *reinterpret_cast<const float4*>(&Ys[kw + kb + k][0]);
+      const float4 b = *reinterpret_cast<const float4*>(&Ys[kw + kb + k][4]);
+      const float4 w = zr[k];
+      const float ya[kStripY] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int y = 0; y < kStripY; ++y) {
+        acc[y][0] = __fmaf_rn(ya[y], w.x, acc[y][0]);
+        acc[y][1] = __fmaf_rn(ya[y], w.y, acc[y][1]);
+        acc[y][2] = __fmaf_rn(ya[y], w.z, acc[y][2]);
+        acc[y][3] = __fmaf_rn(ya[y], w.w, acc[y][3]);
+      }
+      // the next batch's row as soon as this one is used
+      if (kb + kStripB < kNB / kStripWarps) {
+        const float* src = p.Z + (size_t)(kw + kb + kStripB + k) * p.ldz + z;
+        if (zfull) {
+          zr[k] = __ldcg(reinterpret_cast<const float4*>(src));
+        } else {
+          zr[k].x = z < p.nz ? src[0] : 0.f;
+          zr[k].y = z + 1 < p.nz ? src[1] : 0.f;
+          zr[k].z = z + 2 < p.nz ? src[2] : 0.f;
+          zr[k].w = 0.f;
+        }
+      }
+    }
+  }
+  __syncthreads();  // Ys is read
+  float(*mine)[kStripZ] = warp + 1 < kStripWarps ? red[warp] : reinterpret_cast<float(*)[kStripZ]>(&Ys[0][0]);
+#pragma unroll
+  for (int y = 0; y < kStripY; ++y)
+    *reinterpret_cast<float4*>(&mine[y][4 * lane]) = make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
+  __syncthreads();
+  const float(*last)[kStripZ] = reinterpret_cast<const float(*)[kStripZ]>(&Ys[0][0]);
+#pragma unroll
+  for (int u = 0; u < kStripY / kStripWarps; ++u) {
+    const int yl = warp * (kStripY / kStripWarps) + u, y = y0 + yl;
+    if (y >= p.ny) continue;
+    const float4 s0 = *reinterpret_cast<const float4*>(&red[0][yl][4 * lane]);
+    const float4 s1 = *reinterpret_cast<const float4*>(&red[1][yl][4 * lane]);
+    const float4 s2 = *reinterpret_cast<const float4*>(&red[2][yl][4 * lane]);
+    const float4 s3 = *reinterpret_cast<const float4*>(&last[yl][4 * lane]);
+    const float sum[4] = {(s0.x + s1.x) + (s2.x + s3.x), (s0.y + s1.y) + (s2.y + s3.y),
+                          (s0.z + s1.z) + (s2.z + s3.z), (s0.w + s1.w) + (s2.w + s3.w)};
+    float* x = p.X + (size_t)y * p.xy + (size_t)z * p.xz;
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (z + v < p.nz) {
+        float* o = x + (size_t)v * p.xz;
+        *o = p.sub ? *o - sum[v] : sum[v];
+      }
+  }
+}
+
+static cudaError_t run_strip(const StripProd& p0, const StripProd* p1, cudaStream_t s) {
+  const int n0 = strip_ctas(p0), n1 = p1 ? strip_ctas(*p1) : 0;
+  k_strip<<<n0 + n1, kStripThreads, 0, s>>>(p0, p1 ? *p1 : p0, n0);
   return cudaGetLastError();
 }
 
@@ -1032,13 +1402,9 @@ __global__ void __launch_bounds__(kTriThreads)
     for (int j = jbeg; j != jend; j += jstep) {
       const int j0 = j * kNB, jn = min(kNB, N - j0);
       if (tid == 0 && !bad) {
-        uint32_t it = 0;
-        while (*((volatile unsigned*)&flags[j]) != epoch) {
-          if (++it > (1u << 26)) {
-            bad = 1;
-            dev_fail(err, WBEM_ERR_TIMEOUT, 71, k, j);
-            break;
-          }
+        if (!flag_wait_bounded<false>(&flags[j], epoch, err)) {
+          bad = 1;
+          dev_fail(err, WBEM_ERR_TIMEOUT, 71, k, j);
         }
         __threadfence();
       }
@@ -1129,13 +1495,12 @@ struct LuState {
   // second one, the rest of the trailing update on a low-priority stream
   cudaStream_t s_panel = nullptr;
   cudaStream_t s_row = nullptr;
-  cudaStream_t s_inrow = nullptr;      // in-panel row panel, beside the column panel
   cudaStream_t s_col2 = nullptr;       // column panel and in-panel update below the next block
   cudaStream_t s_trail = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_row = nullptr, ev_trail = nullptr, ev_join = nullptr;
   cudaEvent_t ev_next_rows = nullptr;  // bulk update of the next panel's rows done
   cudaEvent_t ev_blk = nullptr;        // diagonal block ready for its row panel
-  cudaEvent_t ev_inrow = nullptr;      // in-panel row panel done
+  cudaEvent_t ev_inrow = nullptr;      // strip and in-panel row panel of the block done
   cudaEvent_t ev_u12 = nullptr;        // row panel of the outer panel done
   cudaEvent_t ev_col2[2] = {nullptr, nullptr};  // s_col2 work of block k done (k % 2)
   float* w = nullptr;         // 2 x N ping-pong vectors
@@ -1163,7 +1528,6 @@ void free_lu(wbem_context* h) {
   if (L.s_panel) cudaStreamDestroy(L.s_panel);
   if (L.s_trail) cudaStreamDestroy(L.s_trail);
   if (L.s_row) cudaStreamDestroy(L.s_row);
-  if (L.s_inrow) cudaStreamDestroy(L.s_inrow);
   if (L.s_col2) cudaStreamDestroy(L.s_col2);
   for (cudaEvent_t e : {L.ev_fork, L.ev_row, L.ev_trail, L.ev_join, L.ev_next_rows, L.ev_blk, L.ev_u12,
                         L.ev_inrow, L.ev_col2[0], L.ev_col2[1]})
@@ -1320,7 +1684,6 @@ int factor_mixed(wbem_context* h) {
     WB_CU(cudaStreamCreateWithPriority(&L.s_panel, cudaStreamNonBlocking, hi));
     WB_CU(cudaStreamCreateWithPriority(&L.s_trail, cudaStreamNonBlocking, lo));
     WB_CU(cudaStreamCreateWithPriority(&L.s_row, cudaStreamNonBlocking, hi < lo ? hi + 1 : hi));
-    WB_CU(cudaStreamCreateWithPriority(&L.s_inrow, cudaStreamNonBlocking, hi));
     WB_CU(cudaStreamCreateWithPriority(&L.s_col2, cudaStreamNonBlocking, hi));
     for (cudaEvent_t* e : {&L.ev_fork, &L.ev_row, &L.ev_trail, &L.ev_join, &L.ev_next_rows, &L.ev_blk,
                            &L.ev_u12, &L.ev_inrow, &L.ev_col2[0], &L.ev_col2[1]})
@@ -1345,8 +1708,6 @@ int factor_mixed(wbem_context* h) {
   //   s_panel: the column work of P (diagonal blocks, column panels, inner
   //     updates; columns [p0, p1) only), then the trailing update of the next
   //     panel's columns [p1, p2).
-  //   s_inrow: the in-panel row panel of block k (U_kj for the panel's
-  //     columns right of the block), beside the column panel of block k.
   //   s_col2: the column panel and the in-panel update of block k for the
   //     rows below block k + 1, beside the diagonal block k + 1; s_panel
   //     does them for the rows of block k + 1 only (the strip the next
@@ -1367,7 +1728,6 @@ int factor_mixed(wbem_context* h) {
   const bool prof = h->profiling;
   cudaStream_t sp = prof ? h->stream : L.s_panel, st = prof ? h->stream : L.s_trail;
   cudaStream_t su = prof ? h->stream : L.s_row;
-  cudaStream_t sr = prof ? h->stream : L.s_inrow;
   cudaStream_t sc = prof ? h->stream : L.s_col2;
   if (prof) {
     h->prof_gemm.reset();
@@ -1387,7 +1747,6 @@ int factor_mixed(wbem_context* h) {
   WB_CU(cudaStreamWaitEvent(sp, L.ev_fork, 0));
   WB_CU(cudaStreamWaitEvent(st, L.ev_fork, 0));
   WB_CU(cudaStreamWaitEvent(su, L.ev_fork, 0));
-  WB_CU(cudaStreamWaitEvent(sr, L.ev_fork, 0));
   WB_CU(cudaStreamWaitEvent(sc, L.ev_fork, 0));
   for (int e = 0; e < 2; ++e) WB_CU(cudaEventRecord(L.ev_col2[e], sc));
   bool trail_pending = false;  // a trailing update was queued on s_trail
@@ -1401,23 +1760,10 @@ int factor_mixed(wbem_context* h) {
       const size_t bo = (size_t)k * kNB * kNB;
       WB_CU(cudaStreamWaitEvent(sp, L.ev_col2[k & 1], 0));  // s_col2 work of block k - 2
       pb(h->prof_diag, sp);
-      k_diag_block<<<1, kDiagThreads, kDiagSmem, sp>>>(ld, k0, nb, A, L.linv + bo, L.uinv + bo,
-                                                        L.linvT + bo, L.uinvT + bo, h->d_err);
+      k_diag_block<<<1, kDThreads, kDiagSmem, sp>>>(ld, k0, nb, A, L.uinv + bo, L.linvT + bo, h->d_err);
       pe(h->prof_diag, sp, 0.0);
       h->launches++;
       WB_CU(cudaEventRecord(L.ev_blk, sp));
-      if (k1 < p1) {
-        // U_kj = inv(L_kk) A_kj for the panel's remaining columns, in place,
-        // beside the column panel
-        WB_CU(cudaStreamWaitEvent(sr, L.ev_blk, 0));
-        const PanelArgs pr{L.linvT + bo, kNB, A + (size_t)k0 * ld + k1, ld, A + (size_t)k0 * ld + k1,
-                           ld, kNB, p1 - k1, kNB, k0, k1, 0, 1};
-        pb(h->prof_panel, sr);
-        WB_CU((run_panel_small<128, 64, true>(pr, none, none, sr)));
-        pe(h->prof_panel, sr, 0.0);
-        WB_CU(cudaEventRecord(L.ev_inrow, sr));
-        h->launches++;
-      }
       if (p1 < N) {
         // ---- row panel block row k: A_kj -= L_k,[p0,k0) U_[p0,k0),j, then
         // U_kj = inv(L_kk) A_kj, for the columns right of the panel. L_k,[p0,k0)
@@ -1443,14 +1789,18 @@ int factor_mixed(wbem_context* h) {
       const int sh = std::min(kNB, m);  // the strip: rows of block k + 1
       const SplitOut l21 = none;  // the trailing update reads L21 in place
       // column panel L_ik = A_ik inv(U_kk), in place: the strip on s_panel
-      // (after the s_col2 work of block k - 1, which updated these rows),
-      // the rows below on s_col2
+      // (after the s_col2 work of block k - 1, which updated these rows) with
+      // the in-panel row panel U_kj = inv(L_kk) A_kj, the rows below on s_col2
       WB_CU(cudaStreamWaitEvent(sp, L.ev_col2[(k + 1) & 1], 0));
-      const PanelArgs pc{A + (size_t)k1 * ld + k0, ld, L.uinv + bo, kNB, A + (size_t)k1 * ld + k0,
-                         ld, sh, kNB, kNB, k1, k0, 0, 0};
+      const int w = p1 - k1;  // the panel's columns right of the block
+      float* Akj = A + (size_t)k0 * ld + k1;
+      float* Aik = A + (size_t)k1 * ld + k0;
+      const StripProd lik{Aik, L.uinv + bo, Aik, ld, 1, ld, 1, kNB, sh, kNB, 0};
+      const StripProd ukj{Akj, L.linvT + bo, Akj, 1, ld, 1, ld, kNB, w, kNB, 0};
       pb(h->prof_panel, sp);
-      WB_CU((run_panel_small<64, 128, false>(pc, none, l21, sp)));
+      WB_CU(run_strip(lik, w > 0 ? &ukj : nullptr, sp));
       pe(h->prof_panel, sp, 0.0);
+      WB_CU(cudaEventRecord(L.ev_inrow, sp));
       h->launches++;
       if (m > sh) {
         WB_CU(cudaStreamWaitEvent(sc, L.ev_blk, 0));
@@ -1462,16 +1812,13 @@ int factor_mixed(wbem_context* h) {
         pe(h->prof_panel, sc, 0.0);
         h->launches++;
       }
-      if (k1 < p1) {
-        const int w = p1 - k1;
+      if (w > 0) {
         // in-panel update A[k1:, k1:p1] -= L_ik U_kj in FP32 (small footprint,
         // so it runs beside the previous outer panel's bulk update): the strip
         // on s_panel, the rows below on s_col2
-        WB_CU(cudaStreamWaitEvent(sp, L.ev_inrow, 0));
-        const PanelArgs pi{A + (size_t)k1 * ld + k0, ld, A + (size_t)k0 * ld + k1, ld,
-                           A + (size_t)k1 * ld + k1, ld, sh, w, kNB, k1, k1, 1, 0};
+        const StripProd upd{Aik, Akj, A + (size_t)k1 * ld + k1, ld, 1, ld, 1, ld, sh, w, 1};
         pb(h->prof_panel, sp);
-        WB_CU((run_panel_small<64, 128, false>(pi, none, none, sp)));
+        WB_CU(run_strip(upd, nullptr, sp));
         pe(h->prof_panel, sp, 0.0);
         h->launches++;
         if (m > sh) {
@@ -1505,7 +1852,7 @@ int factor_mixed(wbem_context* h) {
       WB_CU(cudaEventRecord(L.ev_row, sp));
       WB_CU(cudaStreamWaitEvent(st, L.ev_row, 0));
       // a few SMs stay free for the next panel's diagonal blocks (one
-      // 200 KB CTA each); its panel kernels (13 KB CTAs) run beside this
+      // 200 KB CTA each); its panel kernels (13 and 16 KB CTAs) run beside this
       // update's CTAs on every SM. The next panel's rows [p1, p2) go first,
       // so that its row panel can start while the rows below are updated.
       const int spare = prof ? 0 : kLookaheadSMs;
@@ -1524,8 +1871,6 @@ int factor_mixed(wbem_context* h) {
     }
   }
   // join the streams back into the handle's stream
-  WB_CU(cudaEventRecord(L.ev_join, sr));
-  WB_CU(cudaStreamWaitEvent(h->stream, L.ev_join, 0));
   WB_CU(cudaEventRecord(L.ev_join, sc));
   WB_CU(cudaStreamWaitEvent(h->stream, L.ev_join, 0));
   WB_CU(cudaEventRecord(L.ev_join, su));
@@ -1534,6 +1879,9 @@ int factor_mixed(wbem_context* h) {
   WB_CU(cudaStreamWaitEvent(h->stream, L.ev_join, 0));
   WB_CU(cudaEventRecord(L.ev_join, st));
   WB_CU(cudaStreamWaitEvent(h->stream, L.ev_join, 0));
+  k_transpose_inverses<<<dim3(nblk, 16, 2), 256, 0, h->stream>>>(L.linvT, L.uinv, L.linv, L.uinvT);
+  WB_CU(cudaGetLastError());
+  h->launches++;
   WB_CHK(check_device_error(h, "LU factorisation"));
   h->stats.t_factor_ms = tm.ms();
   return WBEM_OK;

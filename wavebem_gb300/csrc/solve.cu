@@ -684,13 +684,8 @@ __device__ __forceinline__ void ortho_barrier(unsigned* ctr, unsigned target, De
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(ctr, 1u);
-    uint32_t it = 0;
-    while ((int)(*((volatile unsigned*)ctr) - target) < 0) {
-      if (++it > (1u << 26)) {
-        dev_fail(err, WBEM_ERR_TIMEOUT, 61, blockIdx.x, (int)target);
-        break;
-      }
-    }
+    if (!flag_wait_bounded<true>(ctr, target, err))
+      dev_fail(err, WBEM_ERR_TIMEOUT, 61, blockIdx.x, (int)target);
     __threadfence();
   }
   __syncthreads();

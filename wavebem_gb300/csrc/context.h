@@ -95,6 +95,8 @@ struct wbem_context {
   double* d_cellc = nullptr;    // mixed: panel centre / normal / moments (double-float source)
   float* d_cellgeo = nullptr;   // mixed: centre (float), radius^2 for the near test
   size_t rec_cells = 0;
+  unsigned char* d_far = nullptr;  // FP64 form: scale and far-field panel records
+  size_t far_size = 0;
 
   // ---- matrices (internal order)
   double* d_N = nullptr;

@@ -45,9 +45,10 @@ cudaError_t upload_quadrature(const QuadTables& t);
 // ---- assembly (FP64 plain form)
 cudaError_t launch_cell_records_fp64(int C, const double* X, const int4* cell_dofs, double* rec,
                                      int q1, cudaStream_t s);
-cudaError_t launch_tile_fp64(int N, int q1, const double* X, const int* dnset, int n_tiles,
+size_t far_bytes(int q1, int C);  // scratch of launch_tile_fp64 (may be 0)
+cudaError_t launch_tile_fp64(int N, int C, int q1, const double* X, const int* dnset, int n_tiles,
                              const int* tile_ptr, const int2* tile_ent, const int4* cell_dofs,
-                             const double* rec, double* Nm, double* Dm, DevErr* err,
+                             const double* rec, void* far, double* Nm, double* Dm, DevErr* err,
                              cudaStream_t s);
 cudaError_t launch_singular_fp64(int N, const double* X, const int* dnset, const int* sptr,
                                  const int* scell, const int4* cell_dofs, double* Nm, double* Dm,

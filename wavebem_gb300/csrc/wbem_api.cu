@@ -329,6 +329,38 @@ static int build_topology(wbem_context* h) {
   if (tstart64.back() != N) tstart64.push_back(N);
   h->n_tiles64 = (int)tstart64.size() - 1;
   tile_lists(tstart64, tptr64, tent64);
+  // order of an FP64 tile's panels: groups of four that share no column where
+  // that can be had (k_tile_far adds such a group's entries at once). The
+  // members are looked for a quarter of the list apart.
+  std::vector<int2> in;
+  std::vector<char> used;
+  for (int t = 0; t < h->n_tiles64; ++t) {
+    in.assign(tent64.begin() + tptr64[t], tent64.begin() + tptr64[t + 1]);
+    const int n = (int)in.size(), quarter = (n + 3) / 4;
+    used.assign(n, 0);
+    int taken[256];  // the group that last used a column
+    std::fill(taken, taken + 256, -1);
+    for (int k = 0; k < n; ++k) {
+      int pick = -1, any = -1, i = (k % 4 * quarter + k / 4) % n;
+      for (int tries = 0; tries < n && pick < 0; ++tries, i = i + 1 < n ? i + 1 : 0) {
+        if (used[i]) continue;
+        any = i;
+        bool free = true;
+        for (int v = 0; v < 4; ++v) {
+          const int sl = ((uint32_t)in[i].y >> (8 * v)) & 255u;
+          free &= sl == 255 || taken[sl] != k / 4;
+        }
+        if (free) pick = i;
+      }
+      if (pick < 0) pick = any;
+      used[pick] = 1;
+      tent64[tptr64[t] + k] = in[pick];
+      for (int v = 0; v < 4; ++v) {
+        const int sl = ((uint32_t)in[pick].y >> (8 * v)) & 255u;
+        if (sl != 255) taken[sl] = k / 4;
+      }
+    }
+  }
   // double-node sets (internal)
   std::vector<int> dnset((size_t)N * kMaxSet, -1);
   for (int p = 0; p < N; ++p) {
@@ -846,7 +878,7 @@ static void release_mesh_buffers(wbem_context* h) {
                    (void**)&h->d_cptr_full, (void**)&h->d_ccol_full, (void**)&h->d_cval_full,
                    (void**)&h->d_tptr, (void**)&h->d_tsrc, (void**)&h->d_tval, (void**)&h->d_binv,
                    (void**)&h->d_V, (void**)&h->d_part, (void**)&h->d_small, (void**)&h->d_opart,
-                   (void**)&h->d_octr, (void**)&h->d_xs, (void**)&h->d_hull, (void**)&h->d_hull_part,
+                   (void**)&h->d_octr, (void**)&h->d_xs, (void**)&h->d_hull, (void**)&h->d_hull_part, (void**)&h->d_far,
                    (void**)&h->d_lu,
                    (void**)&h->d_split, (void**)&h->d_lutmp, (void**)&h->d_info, (void**)&h->d_sol,
                    (void**)&h->d_rhs, (void**)&h->d_b};
@@ -865,6 +897,7 @@ static void release_mesh_buffers(wbem_context* h) {
   h->item_rows = 0;
   h->near_cap = 0;
   h->hull_cap = 0;
+  h->far_size = 0;
   h->V_cap = 0;
   h->lu_elems = 0;
   h->flips_cap = 0;
@@ -1074,15 +1107,22 @@ int wbem_assemble(wbem_handle h, const wbem_options* opt) {
     }
     CU(launch_cell_records_fp64(h->C, h->d_X, h->d_cell_dofs, h->d_rec, o.quadrature_order, h->stream));
     h->stats.t_geometry_ms = tm.ms();
-    CU(launch_tile_fp64(N, o.quadrature_order, h->d_X, h->d_dnset, h->n_tiles64, h->d_tile_ptr64,
-                        h->d_tile_ent64, h->d_cell_dofs, h->d_rec, h->d_N, h->d_D, h->d_err, h->stream));
+    const size_t fb = far_bytes(o.quadrature_order, h->C);
+    if (fb > h->far_size) {
+      h->far_size = 0;
+      CHK(dev_alloc(h, &h->d_far, fb));
+      h->far_size = fb;
+    }
+    CU(launch_tile_fp64(N, h->C, o.quadrature_order, h->d_X, h->d_dnset, h->n_tiles64,
+                        h->d_tile_ptr64, h->d_tile_ent64, h->d_cell_dofs, h->d_rec, h->d_far,
+                        h->d_N, h->d_D, h->d_err, h->stream));
     h->stats.t_assemble_ms = tm.ms();
     CU(launch_singular_fp64(N, h->d_X, h->d_dnset, h->d_sptr, h->d_scell, h->d_cell_dofs, h->d_N,
                             h->d_D, h->d_err, h->stream));
     h->stats.t_singular_ms = tm.ms();
     CU(launch_alpha_rowsum(N, h->d_N, h->d_alpha, h->stream));
     h->stats.t_alpha_ms = tm.ms();
-    h->launches += 4;
+    h->launches += fb ? 6 : 4;
     CHK(check_device_error(h, "wbem_assemble"));
     h->assembled_prec = WBEM_PREC_FP64;
   } else {

@@ -142,128 +142,35 @@ __device__ __forceinline__ void adj_point(const double* __restrict__ X, int4 d, 
   p[11] = w * fn;
 }
 
-// FP64 terms of one (row, regular point) pair: row part into grow, the 4
-// panel-vertex parts into g (vertex v, component e at 3 v + e).
-__device__ __forceinline__ void adj_point_terms(const double* p, int q, const double xi[3],
-                                                double li, double phii, double g[12],
-                                                double grow[3]) {
-  const double R[3] = {p[0] - xi[0], p[1] - xi[1], p[2] - xi[2]};
-  const double c[3] = {p[4] * p[8] - p[5] * p[7], p[5] * p[6] - p[3] * p[8],
-                       p[3] * p[7] - p[4] * p[6]};
-  const double w = c_qa.gp[q][2] * kI4P;
-  const double s1 = li * (p[10] - w * phii), s2 = li * p[11];
-  double aR[3], ac[3];
-  point_grad<double>(R, c, p[9], s1, s2, aR, ac);
-  const double s = c_qa.gp[q][0], u = c_qa.gp[q][1];
-  const double Ns[4] = {-(1 - u), (1 - u), -u, u};
-  const double Nt[4] = {-(1 - s), -s, (1 - s), s};
-  const double gjx[3] = {p[7] * ac[2] - p[8] * ac[1], p[8] * ac[0] - p[6] * ac[2],
-                         p[6] * ac[1] - p[7] * ac[0]};
-  const double gje[3] = {ac[1] * p[5] - ac[2] * p[4], ac[2] * p[3] - ac[0] * p[5],
-                         ac[0] * p[4] - ac[1] * p[3]};
-  for (int e = 0; e < 3; ++e) grow[e] -= aR[e];
-  for (int v = 0; v < 4; ++v)
-    for (int e = 0; e < 3; ++e)
-      g[3 * v + e] += c_qa.phi[q][v] * aR[e] + Ns[v] * gjx[e] + Nt[v] * gje[e];
-}
-
-// FP64 terms of one near (row, regular point) pair of the mixed form, in the
-// moment form of the far field (B_v += N4_v aR, D_v += N4_v ac, row part into
-// grow). p: x (3), c = jx x je (3), w'phi(q), w'dn(q) |c|, w'dn(q) / |c|;
-// lpw = lambda_i phi_i / (4 pi).
-__device__ __forceinline__ void adj_near_moments(const double* __restrict__ p, int q,
-                                                 const double xi[3], double li, double lpw,
-                                                 double B[12], double D[12], double grow[3]) {
+// FP64 terms of one near (row, regular point) pair of the mixed form: aR and
+// ac are added over the rows, g over the points (minus the row part).
+// p: x (3), c = jx x je (3), w'phi(q), w'dn(q) |c|, w'dn(q) / |c|; w the
+// point's weight, lpw = lambda_i phi_i / (4 pi).
+__device__ __forceinline__ void adj_near_point(const double p[9], double w, const double xi[3],
+                                               double li, double lpw, double aR[3], double ac[3],
+                                               double g[3]) {
   const double R[3] = {p[0] - xi[0], p[1] - xi[1], p[2] - xi[2]};
   const double c[3] = {p[3], p[4], p[5]};
   const double r2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
   const double ri = rsqrt(r2), ri2 = ri * ri, ri3 = ri2 * ri;
   const double u = R[0] * c[0] + R[1] * c[1] + R[2] * c[2];
-  const double s1 = li * p[6] - lpw * c_qa.gp[q][2];
-  const double a = s1 * ri3;
-  const double kr = 3.0 * s1 * u * ri3 * ri2 + li * p[7] * ri3;
+  const double a = fma(li, p[6], -lpw * w) * ri3;
+  const double kr = fma(a * u, 3.0 * ri2, li * p[7] * ri3);
   const double kc = li * p[8] * ri;
-  double aR[3], ac[3];
   for (int e = 0; e < 3; ++e) {
-    aR[e] = kr * R[e] - a * c[e];
-    ac[e] = -a * R[e] - kc * c[e];
-    grow[e] -= aR[e];
-  }
-  for (int v = 0; v < 4; ++v) {
-    const double nv = c_qa.phi[q][v];
-    for (int e = 0; e < 3; ++e) {
-      B[3 * v + e] += nv * aR[e];
-      D[3 * v + e] += nv * ac[e];
-    }
+    const double t = fma(kr, R[e], -a * c[e]);
+    aR[e] += t;
+    g[e] += t;
+    ac[e] = fma(-a, R[e], fma(-kc, c[e], ac[e]));
   }
 }
 
-// Plain form. One CTA: 128 rows x a range of panels, FP64 throughout.
-template <int Q1>
-__global__ void __launch_bounds__(128)
-    k_adj_tile(int N, int C, const double* __restrict__ X, const int* __restrict__ dnset,
-               const int4* __restrict__ cell_dofs, const double* __restrict__ lam,
-               const double* __restrict__ phi, const double* __restrict__ dn,
-               double* __restrict__ grow_part, double* __restrict__ gcell_part,
-               int cells_per_block) {
-  constexpr int NQ = Q1 * Q1;
-  __shared__ double pt[kAdjChunk][NQ][kPt];
-  __shared__ double wred[4][kAdjChunk][12];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = blockIdx.y * 128 + tid;
-  const bool active = row < N;
-  double xi[3] = {0, 0, 0}, li = 0, phii = 0;
-  int set[kMaxSet];
-  for (int k = 0; k < kMaxSet; ++k) set[k] = -2;
-  if (active) {
-    for (int d = 0; d < 3; ++d) xi[d] = X[3 * (size_t)row + d];
-    li = lam[row];
-    phii = phi[row];
-    for (int k = 0; k < kMaxSet; ++k) set[k] = dnset[(size_t)row * kMaxSet + k];
-  }
-  double grow[3] = {0, 0, 0};
-  const int c_begin = blockIdx.x * cells_per_block;
-  const int c_end = min(C, c_begin + cells_per_block);
-  for (int cb = c_begin; cb < c_end; cb += kAdjChunk) {
-    const int cnt = min(kAdjChunk, c_end - cb);
-    __syncthreads();
-    for (int t = tid; t < cnt * NQ; t += 128) {
-      const int k = t / NQ, q = t % NQ;
-      adj_point(X, cell_dofs[cb + k], q, phi, dn, pt[k][q]);
-    }
-    __syncthreads();
-    for (int k = 0; k < cnt; ++k) {
-      const int4 d = cell_dofs[cb + k];
-      bool sing = false;
-      for (int s = 0; s < kMaxSet; ++s)
-        sing |= (set[s] == d.x) | (set[s] == d.y) | (set[s] == d.z) | (set[s] == d.w);
-      double g[12];
-      for (int t = 0; t < 12; ++t) g[t] = 0;
-      if (active && !sing && li != 0.0)
-        for (int q = 0; q < NQ; ++q) adj_point_terms(pt[k][q], q, xi, li, phii, g, grow);
-      // sum the 12 panel-vertex terms over the 32 rows of the warp
-      for (int t = 0; t < 12; ++t) {
-        double v = g[t];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) wred[warp][k][t] = v;
-      }
-    }
-    __syncthreads();
-    for (int t = tid; t < cnt * 12; t += 128) {
-      const int k = t / 12, e = t % 12;
-      const double v = wred[0][k][e] + wred[1][k][e] + wred[2][k][e] + wred[3][k][e];
-      gcell_part[((size_t)blockIdx.y * C + cb + k) * 12 + e] = v;
-    }
-  }
-  if (active)
-    for (int e = 0; e < 3; ++e) grow_part[((size_t)blockIdx.x * N + row) * 3 + e] = grow[e];
-}
-
-// ---------------------------------------------------- mixed form (K7 mixed)
-// Far pairs (panels that fail the assembly's near test) run in FP32, near
-// pairs in FP64, singular pairs in k_adj_singular.
+// ---------------------------------------------------------- moments (K7)
+// The plain form runs in FP64 throughout; in the mixed form far pairs (panels
+// that fail the assembly's near test) run in FP32 and near pairs in FP64.
+// Singular pairs: k_adj_singular.
 //
-// The far-field sum over the regular points q of one panel is kept in the
+// The sum over the regular points q of one panel is kept in the
 // bilinear basis N4_v(q) of the panel:
 //     B_v = sum_q N4_v aR_q,   D_v = sum_q N4_v ac_q      (v = 0..3)
 // with aR, ac the derivatives with respect to the point offset R and the
@@ -283,9 +190,9 @@ static_assert(kMaxSet % 4 == 0, "double-node sets are read as int4");
 static_assert(kAdjRpt * kAdjChunk <= 32, "near mask of a chunk in one word");
 
 // Per (panel, regular point), once per adjoint call:
-//   recd (12 doubles): x, c = jx x je, w'phi, w'dn |c|, w'dn / |c| (near pairs);
-//   recf (3 float4):   (x_hi, c.x), (x_lo, c.y), (c.z, w'phi, w'dn |c|, w'dn / |c|)
-//                      with x = x_hi + x_lo and c = jx x je;
+//   recd (12 doubles): x, c = jx x je, w'phi, w'dn |c|, w'dn / |c| (FP64 pairs);
+//   recf (3 float4, mixed form): (x_hi, c.x), (x_lo, c.y), (c.z, w'phi, w'dn |c|,
+//                      w'dn / |c|) with x = x_hi + x_lo and c = jx x je;
 // per panel pgeo (12 doubles): E0, E1, F0, F1.
 template <int Q1>
 __global__ void k_adj_points(int C, const double* __restrict__ X,
@@ -304,15 +211,17 @@ __global__ void k_adj_points(int C, const double* __restrict__ X,
   const double rd[kPt] = {p[0], p[1], p[2], c0, c1, c2, p[10], p[11] * p[9], p[11] / p[9], 0.0, 0.0, 0.0};
   double* pd = recd + (size_t)t * kPt;
   for (int e = 0; e < kPt; ++e) pd[e] = rd[e];
-  float hi[3], lo[3];
-  for (int e = 0; e < 3; ++e) {
-    hi[e] = (float)p[e];
-    lo[e] = (float)(p[e] - (double)hi[e]);
+  if (recf) {
+    float hi[3], lo[3];
+    for (int e = 0; e < 3; ++e) {
+      hi[e] = (float)p[e];
+      lo[e] = (float)(p[e] - (double)hi[e]);
+    }
+    recf[3 * (size_t)t + 0] = make_float4(hi[0], hi[1], hi[2], (float)c0);
+    recf[3 * (size_t)t + 1] = make_float4(lo[0], lo[1], lo[2], (float)c1);
+    recf[3 * (size_t)t + 2] =
+        make_float4((float)c2, (float)p[10], (float)(p[11] * p[9]), (float)(p[11] / p[9]));
   }
-  recf[3 * (size_t)t + 0] = make_float4(hi[0], hi[1], hi[2], (float)c0);
-  recf[3 * (size_t)t + 1] = make_float4(lo[0], lo[1], lo[2], (float)c1);
-  recf[3 * (size_t)t + 2] =
-      make_float4((float)c2, (float)p[10], (float)(p[11] * p[9]), (float)(p[11] / p[9]));
   if (q == 0) {
     const int id[4] = {d.x, d.y, d.z, d.w};
     double P[4][3];
@@ -351,6 +260,164 @@ __device__ __forceinline__ void warp_sum24(const T v[24], int lane, T out[3]) {
     y += __shfl_xor_sync(0xffffffffu, y, 2);
     y += __shfl_xor_sync(0xffffffffu, y, 1);
     out[i] = y;
+  }
+}
+
+// Vertex gradient o = 3 v + e of a panel from its moments m (B, D) and edges G
+// (E0, E1, F0, F1).
+__device__ __forceinline__ double adj_vertex_grad(const double* m, const double* __restrict__ G,
+                                                  int o) {
+  const int w = o / 3, e = o - 3 * w;
+  const int e1 = e == 2 ? 0 : e + 1, e2 = e == 0 ? 2 : e - 1;
+  const double* D = m + 12;  // D_i at D[3 i]
+  // X-part: E0 x D_i + E1 x D_{i+1}, i = 0 (vertices 0, 1) or 2 (vertices 2, 3)
+  const int ix = w < 2 ? 0 : 2;
+  const double xs = G[e1] * D[3 * ix + e2] - G[e2] * D[3 * ix + e1] +
+                    G[3 + e1] * D[3 * ix + 3 + e2] - G[3 + e2] * D[3 * ix + 3 + e1];
+  // Y-part: D_i x F0 + D_{i+2} x F1, i = 0 (vertices 0, 2) or 1 (vertices 1, 3)
+  const int iy = w & 1;
+  const double ys = D[3 * iy + e1] * G[6 + e2] - D[3 * iy + e2] * G[6 + e1] +
+                    D[3 * iy + 6 + e1] * G[9 + e2] - D[3 * iy + 6 + e2] * G[9 + e1];
+  return m[o] + ((w & 1) ? xs : -xs) + (w >= 2 ? ys : -ys);
+}
+
+__device__ __forceinline__ bool adj_singular_pair(const int4* __restrict__ set4, int4 d) {
+  bool sing = false;
+  for (int h = 0; h < kMaxSet / 4; ++h) {
+    const int4 s = set4[h];
+    const int m[4] = {s.x, s.y, s.z, s.w};
+    for (int i = 0; i < 4; ++i)
+      sing |= (m[i] == d.x) | (m[i] == d.y) | (m[i] == d.z) | (m[i] == d.w);
+  }
+  return sing;
+}
+
+// Plain form, FP64 throughout and bound by the FP64 pipe. One CTA:
+// kAdjRowsCta rows (kAdjRpt per thread) x a range of panels, in chunks of
+// kAdjChunk panels whose point records sit in shared memory. The moments are
+// linear in the rows, so a thread adds aR and ac over its rows before it
+// spreads a point over the 24 moments: 38 FP64 instructions per row and point
+// plus 30 per point, against 140 when each row formed the derivatives with
+// respect to jx and je, their cross products and the 12 vertex terms: 31.7 ->
+// 12.2 ms at 3,001 dofs.
+template <int Q1>
+__global__ void __launch_bounds__(128)
+    k_adj_tile(int N, int C, const double* __restrict__ X, const int* __restrict__ dnset,
+               const int4* __restrict__ cell_dofs, const double* __restrict__ recd,
+               const double* __restrict__ pgeo, const double* __restrict__ lam,
+               const double* __restrict__ phi, double* __restrict__ grow_part,
+               double* __restrict__ gcell_part, int cells_per_block) {
+  constexpr int NQ = Q1 * Q1, kRec = 10;  // record: x, c, w'phi, w'dn |c|, w'dn / |c|
+  __shared__ __align__(16) double sp[kAdjChunk][NQ][kRec];
+  __shared__ double wmom[4][kAdjChunk][24];
+  __shared__ double smom[kAdjChunk][24];
+  __shared__ int4 sdofs[kAdjChunk];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r0 = blockIdx.y * kAdjRowsCta;
+  double x[kAdjRpt][3], l[kAdjRpt], lp[kAdjRpt], grow[kAdjRpt][3];
+#pragma unroll
+  for (int j = 0; j < kAdjRpt; ++j) {
+    const int row = min(r0 + 128 * j + tid, N - 1);
+    for (int e = 0; e < 3; ++e) {
+      x[j][e] = X[3 * (size_t)row + e];
+      grow[j][e] = 0.0;
+    }
+    l[j] = r0 + 128 * j + tid < N ? lam[row] : 0.0;
+    lp[j] = l[j] * phi[row] * kI4P;
+  }
+  const int c_begin = blockIdx.x * cells_per_block;
+  const int c_end = min(C, c_begin + cells_per_block);
+  for (int cb = c_begin; cb < c_end; cb += kAdjChunk) {
+    const int cnt = min(kAdjChunk, c_end - cb);
+    __syncthreads();
+    for (int t = tid; t < cnt * NQ * kRec; t += 128) {
+      const int pt = t / kRec, i = t - kRec * pt;
+      (&sp[0][0][0])[t] = recd[((size_t)cb * NQ + pt) * kPt + i];
+    }
+    if (tid < cnt) sdofs[tid] = cell_dofs[cb + tid];
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < cnt; ++k) {
+      const int4 d = sdofs[k];
+      unsigned use = 0;
+      double lk[kAdjRpt], lpk[kAdjRpt];
+#pragma unroll
+      for (int j = 0; j < kAdjRpt; ++j) {
+        const int row = min(r0 + 128 * j + tid, N - 1);
+        const bool u =
+            l[j] != 0.0 &&
+            !adj_singular_pair(reinterpret_cast<const int4*>(dnset + (size_t)row * kMaxSet), d);
+        use |= u ? 1u << j : 0u;
+        lk[j] = u ? l[j] : 0.0;
+        lpk[j] = u ? lp[j] : 0.0;
+      }
+      double v[24];
+#pragma unroll
+      for (int i = 0; i < 24; ++i) v[i] = 0.0;
+#pragma unroll 1
+      for (int q = 0; q < NQ; ++q) {
+        const double2* p2 = reinterpret_cast<const double2*>(sp[k][q]);
+        const double2 A = p2[0], B = p2[1], Cc = p2[2], E = p2[3];
+        const double wnoj = sp[k][q][8];
+        const double c[3] = {B.y, Cc.x, Cc.y};
+        const double gw = c_qa.gp[q][2];
+        double aR[3] = {0, 0, 0}, ac[3] = {0, 0, 0}, Ks = 0, Kc = 0;
+#pragma unroll
+        for (int j = 0; j < kAdjRpt; ++j) {
+          const double R[3] = {A.x - x[j][0], A.y - x[j][1], B.x - x[j][2]};
+          double r2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
+          r2 = (use >> j) & 1u ? r2 : 1.0;
+          const double ri = rsqrt(r2), ri2 = ri * ri, ri3 = ri * ri2;
+          const double u = R[0] * c[0] + R[1] * c[1] + R[2] * c[2];
+          const double a = fma(lk[j], E.x, -lpk[j] * gw) * ri3;
+          const double kr = fma(a * u, 3.0 * ri2, lk[j] * E.y * ri3);
+          Ks += a;
+          Kc = fma(lk[j], ri, Kc);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            aR[e] = fma(kr, R[e], aR[e]);
+            ac[e] = fma(-a, R[e], ac[e]);
+            grow[j][e] = fma(-kr, R[e], fma(a, c[e], grow[j][e]));
+          }
+        }
+        Kc *= wnoj;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          aR[e] = fma(-Ks, c[e], aR[e]);
+          ac[e] = fma(-Kc, c[e], ac[e]);
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const double nv = c_qa.phi[q][w];
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            v[3 * w + e] = fma(nv, aR[e], v[3 * w + e]);
+            v[12 + 3 * w + e] = fma(nv, ac[e], v[12 + 3 * w + e]);
+          }
+        }
+      }
+      double o3[3];
+      warp_sum24<double>(v, lane, o3);
+      if ((lane & 3) == 0)
+        for (int i = 0; i < 3; ++i) wmom[warp][k][3 * (lane >> 2) + i] = o3[i];
+    }
+    __syncthreads();
+    for (int t = tid; t < cnt * 24; t += 128) {
+      const int k = t / 24, m = t - 24 * k;
+      smom[k][m] = (wmom[0][k][m] + wmom[1][k][m]) + (wmom[2][k][m] + wmom[3][k][m]);
+    }
+    __syncthreads();
+    for (int t = tid; t < cnt * 12; t += 128) {
+      const int k = t / 12, o = t - 12 * k;
+      gcell_part[((size_t)blockIdx.y * C + cb + k) * 12 + o] =
+          adj_vertex_grad(smom[k], pgeo + (size_t)(cb + k) * 12, o);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kAdjRpt; ++j) {
+    const int row = r0 + 128 * j + tid;
+    if (row < N)
+      for (int e = 0; e < 3; ++e) grow_part[((size_t)blockIdx.x * N + row) * 3 + e] = grow[j][e];
   }
 }
 
@@ -504,41 +571,91 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll
     for (int j = 0; j < kAdjRpt; ++j)
       for (int e = 0; e < 3; ++e) sgrow[j][e][tid] -= (double)gr[j][e];
-    // near pairs of the chunk: FP64 terms, unless the pair is singular
+    // near pairs of the chunk, FP64, unless the pair is singular: two rows at
+    // a time, the panel's points over the lanes of a half warp. A lane adds aR
+    // and ac over the rows at its points; the moments are formed once per warp
+    // and panel. (A row per lane ran all points of the panel for every warp that
+    // had one near row, with a few lanes on: 8.6 -> 3.65 ms at 8,192 dofs.)
+    constexpr int NPT = (NQ + 15) / 16;  // points per lane
+    __syncwarp();  // sgrow is written by other lanes below
     for (int k = 0; k < cnt; ++k) {
-      unsigned nm = (nmask >> (kAdjRpt * k)) & ((1u << kAdjRpt) - 1u);
-      if (__any_sync(0xffffffffu, nm != 0u)) {
-        double m64[24];
-        for (int t = 0; t < 24; ++t) m64[t] = 0.0;
-        const int4 d = sdofs[k];
-        const double* pc = recd + (size_t)(cb + k) * NQ * kPt;
-        while (nm) {
-          const int j = __ffs(nm) - 1;
-          nm &= nm - 1u;
-          const int row = r0 + 128 * j + tid;
-          const int4* s4 = reinterpret_cast<const int4*>(dnset + (size_t)row * kMaxSet);
-          bool sing = false;
-          for (int h = 0; h < kMaxSet / 4; ++h) {
-            const int4 s = s4[h];
-            const int m[4] = {s.x, s.y, s.z, s.w};
-            for (int i = 0; i < 4; ++i)
-              sing |= (m[i] == d.x) | (m[i] == d.y) | (m[i] == d.z) | (m[i] == d.w);
-          }
-          if (sing) continue;
-          const double xi[3] = {X[3 * (size_t)row], X[3 * (size_t)row + 1], X[3 * (size_t)row + 2]};
-          const double li = lam[row], lpw = li * phi[row] * kI4P;
-          double grow[3] = {0.0, 0.0, 0.0};
-          for (int q = 0; q < NQ; ++q)
-            adj_near_moments(pc + q * kPt, q, xi, li, lpw, m64, m64 + 12, grow);
-          for (int e = 0; e < 3; ++e) sgrow[j][e][tid] += grow[e];
-        }
-        double n3[3];
-        warp_sum24<double>(m64, lane, n3);
-        if ((lane & 3) == 0)
-          for (int i = 0; i < 3; ++i) wnmom[warp][k][3 * (lane >> 2) + i] = n3[i];
-      } else if (lane < 24) {
-        wnmom[warp][k][lane] = 0.0;
+      unsigned todo[kAdjRpt], any = 0;
+#pragma unroll
+      for (int j = 0; j < kAdjRpt; ++j) {
+        bool nt = (nmask >> (kAdjRpt * k + j)) & 1u;
+        if (nt)
+          nt = !adj_singular_pair(
+              reinterpret_cast<const int4*>(dnset + (size_t)(r0 + 128 * j + tid) * kMaxSet), sdofs[k]);
+        todo[j] = __ballot_sync(0xffffffffu, nt);
+        any |= todo[j];
       }
+      if (any == 0) {
+        if (lane < 24) wnmom[warp][k][lane] = 0.0;
+        continue;
+      }
+      double p[NPT][9], aR[NPT][3], ac[NPT][3];
+#pragma unroll
+      for (int i = 0; i < NPT; ++i) {
+        const int q = (lane & 15) + 16 * i;
+        const double* pc = recd + ((size_t)(cb + k) * NQ + min(q, NQ - 1)) * kPt;
+        for (int e = 0; e < 9; ++e) p[i][e] = pc[e];
+        for (int e = 0; e < 3; ++e) aR[i][e] = ac[i][e] = 0.0;
+      }
+#pragma unroll 1
+      for (int j = 0; j < kAdjRpt; ++j) {
+        unsigned m = todo[0];
+#pragma unroll
+        for (int i = 1; i < kAdjRpt; ++i) m = i == j ? todo[i] : m;
+        while (m) {
+          const int l0 = __ffs(m) - 1;
+          m &= m - 1u;
+          const int l1 = m ? __ffs(m) - 1 : -1;
+          if (m) m &= m - 1u;
+          const int src = lane < 16 ? l0 : l1;
+          const int col = 32 * warp + max(src, 0), row = r0 + 128 * j + col;
+          double g[4] = {0.0, 0.0, 0.0, 0.0};
+          if (src >= 0) {
+            const double xi[3] = {X[3 * (size_t)row], X[3 * (size_t)row + 1], X[3 * (size_t)row + 2]};
+            const double li = lam[row], lpw = li * phi[row] * kI4P;
+#pragma unroll
+            for (int i = 0; i < NPT; ++i)
+              if (NQ % 16 == 0 || (lane & 15) + 16 * i < NQ)
+                adj_near_point(p[i], c_qa.gp[(lane & 15) + 16 * i][2], xi, li, lpw, aR[i], ac[i], g);
+          }
+          // g over the 16 points: component (lane >> 2) & 3 ends on lane & 15 = 0, 4, 8
+          const bool h1 = lane & 8, h2 = lane & 4;
+          const double k0 = h1 ? g[2] : g[0], k1 = h1 ? g[3] : g[1];
+          const double s0 = h1 ? g[0] : g[2], s1 = h1 ? g[1] : g[3];
+          const double y0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 8);
+          const double y1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 8);
+          const double keep = h2 ? y1 : y0, send = h2 ? y0 : y1;
+          double z = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+          z += __shfl_xor_sync(0xffffffffu, z, 2);
+          z += __shfl_xor_sync(0xffffffffu, z, 1);
+          const int e = (lane >> 2) & 3;
+          if (src >= 0 && (lane & 3) == 0 && e < 3) sgrow[j][e][col] -= z;
+          __syncwarp();
+        }
+      }
+      double m64[24];
+#pragma unroll
+      for (int t = 0; t < 24; ++t) m64[t] = 0.0;
+#pragma unroll
+      for (int i = 0; i < NPT; ++i) {
+        const int q = (lane & 15) + 16 * i;
+        if (NQ % 16 == 0 || q < NQ)
+#pragma unroll
+          for (int w = 0; w < 4; ++w)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+              m64[3 * w + e] = fma(c_qa.phi[q][w], aR[i][e], m64[3 * w + e]);
+              m64[12 + 3 * w + e] = fma(c_qa.phi[q][w], ac[i][e], m64[12 + 3 * w + e]);
+            }
+      }
+      double n3[3];
+      warp_sum24<double>(m64, lane, n3);
+      if ((lane & 3) == 0)
+        for (int i = 0; i < 3; ++i) wnmom[warp][k][3 * (lane >> 2) + i] = n3[i];
     }
     __syncthreads();
     for (int t = tid; t < cnt * 24; t += 128) {
@@ -549,23 +666,12 @@ __global__ void __launch_bounds__(128, 4)
     }
     __syncthreads();
     for (int t = tid; t < cnt * 12; t += 128) {
-      const int k = t / 12, o = t - 12 * k, w = o / 3, e = o - 3 * w;
-      const int e1 = e == 2 ? 0 : e + 1, e2 = e == 0 ? 2 : e - 1;
-      const double* G = pgeo + (size_t)(cb + k) * 12;  // E0, E1, F0, F1
-      const double* D = &smom[k][12];                  // D_i at D[3 i]
-      // X-part: E0 x D_i + E1 x D_{i+1}, i = 0 (vertices 0, 1) or 2 (vertices 2, 3)
-      const int ix = w < 2 ? 0 : 2;
-      const double xs = G[e1] * D[3 * ix + e2] - G[e2] * D[3 * ix + e1] +
-                        G[3 + e1] * D[3 * ix + 3 + e2] - G[3 + e2] * D[3 * ix + 3 + e1];
-      // Y-part: D_i x F0 + D_{i+2} x F1, i = 0 (vertices 0, 2) or 1 (vertices 1, 3)
-      const int iy = w & 1;
-      const double ys = D[3 * iy + e1] * G[6 + e2] - D[3 * iy + e2] * G[6 + e1] +
-                        D[3 * iy + 6 + e1] * G[9 + e2] - D[3 * iy + 6 + e2] * G[9 + e1];
-      const double val = smom[k][o] + ((w & 1) ? xs : -xs) + (w >= 2 ? ys : -ys);
+      const int k = t / 12, o = t - 12 * k;
+      const double val = adj_vertex_grad(smom[k], pgeo + (size_t)(cb + k) * 12, o);
       gcell_part[((size_t)blockIdx.y * C + cb + k) * 12 + o] = val;
     }
   }
-  // each thread reads back only the entries of sgrow it wrote itself
+  __syncthreads();
 #pragma unroll
   for (int j = 0; j < kAdjRpt; ++j) {
     const int row = r0 + 128 * j + tid;
@@ -722,11 +828,14 @@ __global__ void k_gb(int N, const uint8_t* __restrict__ mask, const double* __re
 template <int Q1>
 static cudaError_t launch_adj_tile_t(int N, int C, const double* X, const int* dnset,
                                      const int4* cd, const double* lam, const double* phi,
-                                     const double* dn, double* grow_part, double* gcell_part,
-                                     int cpb, cudaStream_t s) {
-  dim3 grid((C + cpb - 1) / cpb, (N + 127) / 128);
-  k_adj_tile<Q1><<<grid, 128, 0, s>>>(N, C, X, dnset, cd, lam, phi, dn, grow_part, gcell_part,
-                                      cpb);
+                                     const double* dn, double* recd, double* pgeo,
+                                     double* grow_part, double* gcell_part, int cpb,
+                                     cudaStream_t s) {
+  constexpr int NQ = Q1 * Q1;
+  k_adj_points<Q1><<<(C * NQ + 255) / 256, 256, 0, s>>>(C, X, cd, phi, dn, recd, nullptr, pgeo);
+  dim3 grid((C + cpb - 1) / cpb, (N + kAdjRowsCta - 1) / kAdjRowsCta);
+  k_adj_tile<Q1><<<grid, 128, 0, s>>>(N, C, X, dnset, cd, recd, pgeo, lam, phi, grow_part,
+                                      gcell_part, cpb);
   return cudaGetLastError();
 }
 
@@ -784,9 +893,11 @@ static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const
   std::vector<int> hoc(C, -1);
   for (int k = 0; k < n_hull; ++k) hoc[hull_ids[k]] = k;
   // panels per CTA column and rows per CTA of the tile kernel
-  const int cpb = mixed ? 128 : 64;
-  const int rows_cta = mixed ? kAdjRowsCta : 128;
-  const int n_cb = (C + cpb - 1) / cpb, n_rb = (N + rows_cta - 1) / rows_cta;
+  // (plain form: eight to 64 panels, a thousand CTAs where the mesh has them)
+  const int n_rb = (N + kAdjRowsCta - 1) / kAdjRowsCta;
+  const int cpb = mixed ? 128
+                        : kAdjChunk * std::min(8, std::max(1, (int)((size_t)C * n_rb / (1000 * kAdjChunk))));
+  const int n_cb = (C + cpb - 1) / cpb;
   const size_t npts = (size_t)C * q1 * q1;
   int st = WBEM_OK;
   // cell -> singular pair index lists (inverse of the per-row singular lists)
@@ -817,11 +928,9 @@ static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const
     if ((st = dev_alloc(h, &gpair, (size_t)std::max<size_t>(1, scell.size()) * 12)) != WBEM_OK) break;
     if ((st = dev_alloc(h, &d_out, (size_t)N * 3)) != WBEM_OK) break;
     if ((st = dev_alloc(h, &d_nph, (size_t)N * 2)) != WBEM_OK) break;
-    if (mixed) {
-      if ((st = dev_alloc(h, &recd, npts * kPt)) != WBEM_OK) break;
-      if ((st = dev_alloc(h, &recf, npts * 3)) != WBEM_OK) break;
-      if ((st = dev_alloc(h, &pgeo, (size_t)C * 12)) != WBEM_OK) break;
-    }
+    if ((st = dev_alloc(h, &recd, npts * kPt)) != WBEM_OK) break;
+    if ((st = dev_alloc(h, &pgeo, (size_t)C * 12)) != WBEM_OK) break;
+    if (mixed && (st = dev_alloc(h, &recf, npts * 3)) != WBEM_OK) break;
     double* phi = h->d_vec[3];
     double* dn = h->d_vec[4];
     double* gx = h->d_vec[5];
@@ -869,11 +978,11 @@ static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const
       }
     } else {
       switch (q1) {
-        case 2: e = launch_adj_tile_t<2>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, grow_part, gcell_part, cpb, h->stream); break;
-        case 3: e = launch_adj_tile_t<3>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, grow_part, gcell_part, cpb, h->stream); break;
-        case 4: e = launch_adj_tile_t<4>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, grow_part, gcell_part, cpb, h->stream); break;
-        case 5: e = launch_adj_tile_t<5>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, grow_part, gcell_part, cpb, h->stream); break;
-        default: e = launch_adj_tile_t<6>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, grow_part, gcell_part, cpb, h->stream); break;
+        case 2: e = launch_adj_tile_t<2>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
+        case 3: e = launch_adj_tile_t<3>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
+        case 4: e = launch_adj_tile_t<4>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
+        case 5: e = launch_adj_tile_t<5>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
+        default: e = launch_adj_tile_t<6>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
       }
     }
     WB_CU(e);
@@ -893,7 +1002,7 @@ static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const
     double* gb = h->d_vec[0];
     k_gb<<<nb, bs, 0, h->stream>>>(N, h->d_mask, nph, npn, bt, h->d_alpha, lamu, gb);
     WB_CU(cudaGetLastError());
-    h->launches += (mixed ? 13 : 12) - (hull_cells ? 0 : 2);
+    h->launches += 13 - (hull_cells ? 0 : 2);
     WB_CHK(check_device_error(h, "adjoint"));
     // back to the caller's order; constraint inhomogeneities tied to b
     std::vector<double> gXi(3 * (size_t)N), gbi(N), li(N);

@@ -141,11 +141,12 @@ __global__ void k_fma_panel_geo(int C, const double* __restrict__ X,
 }
 
 // Close pairs of each row, in the order of the row's neighbour leaves and
-// their panels; one thread per row, the rows taken in leaf order (tidx) so
-// that a warp walks the same neighbour panels. Count pass (ptr == nullptr):
-// cnt[i] = (pairs, singular pairs). List pass: the pairs as (row, panel) from ptr[i]
-// on, and their indices in the correction list, the regular pairs from
-// lptr[i].x on and the singular ones from lptr[i].y on.
+// their panels; one warp per row, its lanes on consecutive panels, the pairs
+// placed by ballot (a thread per row took 1.50 ms a pass at 32,768 dofs, this
+// takes 0.74: the FP64 of the distance). Count pass (ptr == nullptr): cnt[i] =
+// (pairs, singular pairs). List pass: the pairs as (row, panel) from ptr[i] on,
+// and their indices in the correction list, the regular pairs from lptr[i].x on
+// and the singular ones from lptr[i].y on.
 __global__ void k_fma_close(int N, const int* __restrict__ tidx, const int* __restrict__ tgt_leaf,
                             const int* __restrict__ nb_ptr,
                             const int* __restrict__ nb, const int* __restrict__ leaf_pptr,
@@ -155,7 +156,7 @@ __global__ void k_fma_close(int N, const int* __restrict__ tidx, const int* __re
                             const int2* __restrict__ lptr, int2* __restrict__ cnt,
                             int* __restrict__ prow, int* __restrict__ ppan,
                             int* __restrict__ plist) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (j >= N) return;
   const int i = tidx[j];
   const double xi = X[3 * (size_t)i], yi = X[3 * (size_t)i + 1], zi = X[3 * (size_t)i + 2];
@@ -170,30 +171,36 @@ __global__ void k_fma_close(int N, const int* __restrict__ tidx, const int* __re
   int c = 0, ns = 0;
   for (int e = nb_ptr[t]; e < nb_ptr[t + 1]; ++e) {
     const int s = nb[e];
-    for (int k = leaf_pptr[s]; k < leaf_pptr[s + 1]; ++k) {
-      const int cell = leaf_pan[k];
-      const double* g = geo + 4 * (size_t)cell;
-      const double dx = g[0] - xi, dy = g[1] - yi, dz = g[2] - zi;
-      bool sing = false;  // a double-node partner of the row is a vertex of the panel
-      if (nsr <= 16) {
+    const int k1 = leaf_pptr[s + 1];
+    for (int k0 = leaf_pptr[s]; k0 < k1; k0 += 32) {
+      const bool on = k0 + lane < k1;
+      const int cell = on ? leaf_pan[k0 + lane] : -2;
+      bool sing = false, close = false;  // sing: a double-node partner of the row is a vertex of the panel
+      if (on) {
+        const double* g = geo + 4 * (size_t)cell;
+        const double dx = g[0] - xi, dy = g[1] - yi, dz = g[2] - zi;
+        if (nsr <= 16) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) sing |= sc[q] == cell;
-      } else {
-        for (int m = s0; m < s0 + nsr && !sing; ++m) sing = scell[m] == cell;
+          for (int q = 0; q < 16; ++q) sing |= sc[q] == cell;
+        } else {
+          for (int m = s0; m < s0 + nsr && !sing; ++m) sing = scell[m] == cell;
+        }
+        close = sing || dx * dx + dy * dy + dz * dz < 12.0 * g[3] * g[3];
       }
-      const bool close = sing || dx * dx + dy * dy + dz * dz < 12.0 * g[3] * g[3];
-      if (!close) continue;
-      if (ptr) {
-        prow[base + c] = i;
-        ppan[base + c] = cell;
-        if (sing) plist[lp.y + ns] = base + c;
-        else plist[lp.x + c - ns] = base + c;
+      const unsigned mc = __ballot_sync(0xffffffffu, close), ms = __ballot_sync(0xffffffffu, sing);
+      if (ptr && close) {
+        const unsigned before = (1u << lane) - 1u;
+        const int ci = c + __popc(mc & before), si = ns + __popc(ms & before);
+        prow[base + ci] = i;
+        ppan[base + ci] = cell;
+        if (sing) plist[lp.y + si] = base + ci;
+        else plist[lp.x + ci - si] = base + ci;
       }
-      ns += sing ? 1 : 0;
-      ++c;
+      c += __popc(mc);
+      ns += __popc(ms);
     }
   }
-  if (!ptr) cnt[i] = make_int2(c, ns);
+  if (!ptr && lane == 0) cnt[i] = make_int2(c, ns);
 }
 
 // The FP32 value the product computes for one (row, panel) pair, as the 4 N
@@ -307,48 +314,111 @@ __global__ void k_fma_close_val(long long npairs, const int* __restrict__ plist,
 // (sel_j ? -D_ij : N_ij, plus alpha on Neumann diagonals), for the
 // block-Jacobi preconditioner of the FMA solve: the FP32 values of the
 // neighbour panels with a vertex in the row's block plus the close-pair
-// corrections. One thread per row writes its own block row (blocks zeroed
-// before).
-__global__ void k_fma_near_blocks(int N, const int* __restrict__ tgt_leaf,
+// corrections. One warp per row: the panels with such a vertex are collected
+// in order, 32 at a time, a lane computes one panel's values, and four lanes
+// add the panels' entries one panel after the other, in the order of the
+// lists. (A thread per row took 4.0 ms at 32,768 dofs, this takes 1.6.)
+constexpr int kNbWarps = 4;
+__global__ void __launch_bounds__(32 * kNbWarps)
+    k_fma_near_blocks(int N, const int* __restrict__ tgt_leaf,
                                   const int* __restrict__ nb_ptr, const int* __restrict__ nb,
                                   const int* __restrict__ leaf_pptr, const int* __restrict__ leaf_pan,
+                                  const int* __restrict__ pos_leaf,
                                   const double* __restrict__ cen, const float4* __restrict__ xloc,
                                   const float4* __restrict__ ppos, const double* __restrict__ rec,
                                   const int* __restrict__ close_ptr, const int* __restrict__ pair_pan,
                                   const double* __restrict__ val, const int4* __restrict__ cell_dofs,
                                   const uint8_t* __restrict__ mask, const double* __restrict__ alpha,
                                   double* __restrict__ blocks, const __grid_constant__ FmaConst c_fma) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double sacc[kNbWarps][kBJ], sval[kNbWarps][32][4];
+  __shared__ int scol[kNbWarps][32][4], shit[kNbWarps][64];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kNbWarps + w;
   if (i >= N) return;
   const int b = i / kBJ, r = i % kBJ, t = tgt_leaf[i], nq = c_fma.nq;
   const float4 xl = xloc[i];
-  double* row = blocks + ((size_t)b * kBJ + r) * kBJ;
-  for (int e = nb_ptr[t]; e < nb_ptr[t + 1]; ++e) {
-    const int s = nb[e];
-    const float cx = (float)(cen[3 * s] - cen[3 * t]) - xl.x;
-    const float cy = (float)(cen[3 * s + 1] - cen[3 * t + 1]) - xl.y;
-    const float cz = (float)(cen[3 * s + 2] - cen[3 * t + 2]) - xl.z;
-    for (int k = leaf_pptr[s]; k < leaf_pptr[s + 1]; ++k) {
-      const int cell = leaf_pan[k];
+  double* acc = sacc[w];
+  for (int c = lane; c < kBJ; c += 32) acc[c] = 0.0;
+  // adds the staged entries of n panels in order
+  auto add = [&](int n) {
+    __syncwarp();
+    if (lane < 4)
+      for (int l = 0; l < n; ++l) {
+        const int c = scol[w][l][lane];
+        // a panel with a vertex twice: its entries one after the other
+        const int c0 = scol[w][l][0], c1 = scol[w][l][1], c2 = scol[w][l][2], c3 = scol[w][l][3];
+        const bool dup = (c1 >= 0 && c1 == c0) || (c2 >= 0 && (c2 == c0 || c2 == c1)) ||
+                         (c3 >= 0 && (c3 == c0 || c3 == c1 || c3 == c2));
+        if (!dup) {
+          if (c >= 0) acc[c] += sval[w][l][lane];
+        } else if (lane == 0) {
+          for (int j = 0; j < 4; ++j)
+            if (scol[w][l][j] >= 0) acc[scol[w][l][j]] += sval[w][l][j];
+        }
+        __syncwarp(0xfu);
+      }
+    __syncwarp();
+  };
+  int nh = 0;  // panels collected: position in the leaf lists
+  auto flush = [&](int n) {
+    __syncwarp();
+    if (lane < n) {
+      const int k = shit[w][lane], s = pos_leaf[k], cell = leaf_pan[k];
       const int4 d = cell_dofs[cell];
       const int id[4] = {d.x, d.y, d.z, d.w};
-      if (id[0] / kBJ != b && id[1] / kBJ != b && id[2] / kBJ != b && id[3] / kBJ != b) continue;
+      const float cx = (float)(cen[3 * s] - cen[3 * t]) - xl.x;
+      const float cy = (float)(cen[3 * s + 1] - cen[3 * t + 1]) - xl.y;
+      const float cz = (float)(cen[3 * s + 2] - cen[3 * t + 2]) - xl.z;
       float lnf[4], ldf[4];
       fma_pair_approx(ppos + (size_t)k * nq, rec + (size_t)cell * nq * 8, cx, cy, cz, c_fma, lnf, ldf);
-      for (int j = 0; j < 4; ++j)
-        if (id[j] / kBJ == b) row[id[j] % kBJ] += mask[id[j]] ? -(double)ldf[j] : (double)lnf[j];
+      for (int j = 0; j < 4; ++j) {
+        scol[w][lane][j] = id[j] / kBJ == b ? id[j] % kBJ : -1;
+        sval[w][lane][j] = mask[id[j]] ? -(double)ldf[j] : (double)lnf[j];
+      }
+    }
+    add(n);
+  };
+  for (int e = nb_ptr[t]; e < nb_ptr[t + 1]; ++e) {
+    const int s = nb[e], k1 = leaf_pptr[s + 1];
+    for (int k0 = leaf_pptr[s]; k0 < k1; k0 += 32) {
+      const int k = k0 + lane;
+      bool hit = false;
+      if (k < k1) {
+        const int4 d = cell_dofs[leaf_pan[k]];
+        hit = d.x / kBJ == b || d.y / kBJ == b || d.z / kBJ == b || d.w / kBJ == b;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (hit) shit[w][nh + __popc(m & ((1u << lane) - 1u))] = k;
+      nh += __popc(m);
+      if (nh >= 32) {
+        flush(32);
+        const int keep = lane < nh - 32 ? shit[w][32 + lane] : 0;
+        __syncwarp();
+        if (lane < nh - 32) shit[w][lane] = keep;
+        nh -= 32;
+        __syncwarp();
+      }
     }
   }
-  for (int k = close_ptr[i]; k < close_ptr[i + 1]; ++k) {
-    const int4 d = cell_dofs[pair_pan[k]];
-    const int id[4] = {d.x, d.y, d.z, d.w};
-    for (int j = 0; j < 4; ++j) {
-      const int c = id[j];
-      if (c / kBJ != b) continue;
-      row[c % kBJ] += mask[c] ? -val[8 * (size_t)k + 4 + j] : val[8 * (size_t)k + j];
+  flush(nh);
+  for (int k0 = close_ptr[i]; k0 < close_ptr[i + 1]; k0 += 32) {
+    const int n = min(32, close_ptr[i + 1] - k0);
+    if (lane < n) {
+      const int k = k0 + lane;
+      const int4 d = cell_dofs[pair_pan[k]];
+      const int id[4] = {d.x, d.y, d.z, d.w};
+      for (int j = 0; j < 4; ++j) {
+        const int c = id[j];
+        scol[w][lane][j] = c / kBJ == b ? c % kBJ : -1;
+        sval[w][lane][j] = mask[c] ? -val[8 * (size_t)k + 4 + j] : val[8 * (size_t)k + j];
+      }
     }
+    add(n);
   }
-  if (!mask[i]) row[r] += alpha[i];
+  if (lane == 0 && !mask[i]) acc[r] += alpha[i];
+  __syncwarp();
+  double* row = blocks + ((size_t)b * kBJ + r) * kBJ;
+  for (int c = lane; c < kBJ; c += 32) row[c] = acc[c];
 }
 
 // ------------------------------------------------------------ far field
@@ -478,8 +548,10 @@ __global__ void k_fma_p2m_sum(const int* __restrict__ iptr, const float* __restr
 // S1[h][c][P] (the parent's weight of node P at child node c, h = the
 // child's half along the axis): the n^3 x n^3 translation is their tensor
 // product, applied as three passes of n^4 multiply-adds.
-// M2M: one CTA per parent box; W_P[P] = sum_children sum_c T[c][P] W_c[c],
-// for each of the kMpSets coefficient sets (stride kMpSets n^3 per box).
+// M2M: one CTA per parent box and coefficient set (stride kMpSets n^3 per box);
+// W_P[P] = sum_children sum_c T[c][P] W_c[c]. A chain of barriers over the
+// children, so the sets run beside one another: one CTA per box took 52 us per
+// level, this takes 17.
 __global__ void k_fma_m2m(const int* __restrict__ child_ptr, const int* __restrict__ child,
                           const int* __restrict__ child_oct, const float* __restrict__ Wc,
                           float* __restrict__ Wp, const __grid_constant__ FmaConst c_fma) {
@@ -487,7 +559,8 @@ __global__ void k_fma_m2m(const int* __restrict__ child_ptr, const int* __restri
   __shared__ float w[kFmaMaxOrder * kFmaMaxOrder * kFmaMaxOrder];
   __shared__ float t1[kFmaMaxOrder * kFmaMaxOrder * kFmaMaxOrder];
   const int i0 = tid / (n * n), i1 = (tid / n) % n, i2 = tid % n;
-  for (int set = 0; set < kMpSets; ++set) {
+  {
+    const int set = blockIdx.y;
     float acc = 0.f;
     for (int e = child_ptr[p]; e < child_ptr[p + 1]; ++e) {
       const int o = child_oct[e];
@@ -559,62 +632,106 @@ __global__ void k_fma_m2l_ops(int n, double e2, float* __restrict__ K) {
 }
 
 // items: (offset, first entry, entries, level); entries: source box and
-// output row (global over the levels); one CTA of 256 threads per item, each
-// thread an 8 x 4 block of C per pass of kM2LRows target nodes. The dipole
-// columns (m' >= n3) carry one more factor 1 / s, applied when staged.
+// output row (global over the levels). A CTA takes one item and blockDim.x / 2
+// target nodes (m2l_split: the nodes in equal shares of up to kM2LRows), each
+// thread an 8 x 4 block of C. The dipole columns (m' >= n3) carry one more
+// factor 1 / s, applied when staged. Staged values are stored at 16-byte block
+// (r / 4) ^ (c / 4 & 7) of their row c, which makes the transposing stores and
+// the reads free of bank conflicts; the next chunk is loaded into registers
+// meanwhile. One CTA per item with two passes of 128 nodes (216 exist at
+// order 6), 4-way store conflicts and no prefetch took 574 us at 32,768 dofs,
+// a third of it with SMs idle; this takes 360. Sums and their order are the
+// same.
+struct M2LSplit {
+  int parts, threads;
+};
+static M2LSplit m2l_split(int n3) {
+  const int groups = (n3 + 7) / 8, parts = (groups + kM2LRows / 8 - 1) / (kM2LRows / 8);
+  return {parts, 16 * ((groups + parts - 1) / parts)};
+}
+
 __global__ void __launch_bounds__(256)
 k_fma_m2l_gemm(const int4* __restrict__ items, const int* __restrict__ ent_src,
                const int* __restrict__ ent_out, const float* __restrict__ K,
                const float* __restrict__ Wall, const float* __restrict__ lvl_scale,
                float* __restrict__ part, int n3) {
-  __shared__ __align__(16) float Ks[kM2LK][kM2LRows + 4];
-  __shared__ __align__(16) float Ws[kM2LK][kM2LPairs + 4];
+  static_assert(kM2LRows == 128 && kM2LPairs == 64 && kM2LK == 32, "stage layout");
+  __shared__ __align__(16) float Ks[kM2LK][kM2LRows];
+  __shared__ __align__(16) float Ws[kM2LK][kM2LPairs];
   const int kd = kMpSets * n3;
   const int4 it = items[blockIdx.x];
   const int begin = it.y, cnt = it.z;
   const float sc = lvl_scale[it.w];
   const float* Ko = K + (size_t)it.x * n3 * kd;
+  const int nthr = blockDim.x, rows = nthr / 2, a0 = blockIdx.y * rows;
   const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
-  for (int a0 = 0; a0 < n3; a0 += kM2LRows) {
-    float acc[8][4];
+  constexpr int kKLoads = 4, kWLoads = 8;  // rows * 8 / nthr; 64 * 8 / nthr, at most (64 threads)
+  float4 kr[kKLoads], wr[kWLoads];
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto load = [&](int m0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    for (int m0 = 0; m0 < kd; m0 += kM2LK) {
-      __syncthreads();
-      for (int x = tid; x < kM2LRows * kM2LK; x += 256) {
-        const int r = x / kM2LK, c = x % kM2LK, a = a0 + r, m = m0 + c;
-        Ks[c][r] = (a < n3 && m < kd) ? Ko[(size_t)a * kd + m] : 0.f;
-      }
-      for (int x = tid; x < kM2LPairs * kM2LK; x += 256) {
-        const int p = x / kM2LK, c = x % kM2LK, m = m0 + c;
-        float w = (p < cnt && m < kd) ? Wall[(size_t)ent_src[begin + p] * kd + m] : 0.f;
-        Ws[c][p] = m >= n3 ? w * sc : w;
-      }
-      __syncthreads();
-#pragma unroll 8
-      for (int c = 0; c < kM2LK; ++c) {
-        const float4 k0 = *reinterpret_cast<const float4*>(&Ks[c][ty * 8]);
-        const float4 k1 = *reinterpret_cast<const float4*>(&Ks[c][ty * 8 + 4]);
-        const float4 w = *reinterpret_cast<const float4*>(&Ws[c][tx * 4]);
-        const float av[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-        const float wv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-      }
+    for (int u = 0; u < kKLoads; ++u) {
+      const int x = tid + u * nthr, r = x / 8, a = a0 + r, m = m0 + 4 * (x % 8);
+      kr[u] = (a < n3 && m < kd) ? *reinterpret_cast<const float4*>(Ko + (size_t)a * kd + m) : zero;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int a = a0 + ty * 8 + i;
-      if (a >= n3) continue;
+    for (int u = 0; u < kWLoads; ++u) {
+      const int x = tid + u * nthr, p = x / 8, m = m0 + 4 * (x % 8);
+      if (p < kM2LPairs)
+        wr[u] = (p < cnt && m < kd)
+                    ? *reinterpret_cast<const float4*>(Wall + (size_t)ent_src[begin + p] * kd + m)
+                    : zero;
+    }
+  };
+  float acc[8][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int p = tx * 4 + j;
-        if (p < cnt) part[(size_t)ent_out[begin + p] * n3 + a] = acc[i][j] * sc;
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  load(0);
+  for (int m0 = 0; m0 < kd; m0 += kM2LK) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kKLoads; ++u) {
+      const int x = tid + u * nthr, r = x / 8, c4 = x % 8;
+      const float v[4] = {kr[u].x, kr[u].y, kr[u].z, kr[u].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) Ks[4 * c4 + e][((r / 4) ^ c4) * 4 + r % 4] = v[e];
+    }
+#pragma unroll
+    for (int u = 0; u < kWLoads; ++u) {
+      const int x = tid + u * nthr, p = x / 8, c4 = x % 8, m = m0 + 4 * c4;
+      if (p < kM2LPairs) {
+        const float v[4] = {wr[u].x, wr[u].y, wr[u].z, wr[u].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          Ws[4 * c4 + e][((p / 4) ^ c4) * 4 + p % 4] = m + e >= n3 ? v[e] * sc : v[e];
       }
+    }
+    __syncthreads();
+    if (m0 + kM2LK < kd) load(m0 + kM2LK);
+#pragma unroll 8
+    for (int c = 0; c < kM2LK; ++c) {
+      const int sw = c / 4;
+      const float4 k0 = *reinterpret_cast<const float4*>(&Ks[c][((2 * ty) ^ sw) * 4]);
+      const float4 k1 = *reinterpret_cast<const float4*>(&Ks[c][((2 * ty + 1) ^ sw) * 4]);
+      const float4 w = *reinterpret_cast<const float4*>(&Ws[c][(tx ^ sw) * 4]);
+      const float av[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+      const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int a = a0 + ty * 8 + i;
+    if (a >= n3) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int p = tx * 4 + j;
+      if (p < cnt) part[(size_t)ent_out[begin + p] * n3 + a] = acc[i][j] * sc;
     }
   }
 }
@@ -664,22 +781,26 @@ __global__ void k_fma_l2l(const int* __restrict__ parent, const int* __restrict_
   }
 }
 
-// The product's evaluation at the collocation points, one CTA per chunk of
-// up to kEvalTargets rows of one leaf, each thread holding four rows (two
-// packed pairs) and kEvalLanes threads sharing a quad: the far field (L2P of
-// the leaf's local expansion), the near field evaluated on the fly over the
-// points of the neighbour leaves (FP32 in coordinates local to this leaf's
-// centre, two rows per packed FP32x2 instruction, points staged in shared
-// memory with each value duplicated for the packed operands and the next
-// chunk loaded into registers meanwhile; FP64 sum of FP32 partials) and the
-// close-pair corrections (FP64). The lanes of a quad split every sum the same
-// way on every call and are combined by shuffles: the product is
-// deterministic.
+// The product's evaluation at the collocation points, in blocks of up to
+// kEvalTargets rows of one leaf (items), each thread holding four rows (two
+// packed pairs) and kEvalLanes threads sharing a quad. k_fma_near: the near
+// field evaluated on the fly over the points of the neighbour leaves (FP32 in
+// coordinates local to this leaf's centre, two rows per packed FP32x2
+// instruction, points staged in shared memory with each value duplicated for
+// the packed operands and the next chunk loaded into registers meanwhile), one
+// CTA per item and segment of kEvalSegment chunks, whose FP32 sums it stores.
+// k_fma_eval: the far field (L2P of the leaf's local expansion), the segments'
+// sums in order and the close-pair corrections, in FP64. The lanes of a quad
+// split every sum the same way on every call and are combined by shuffles: the
+// product is deterministic. (All segments of an item in one CTA: 718 us at
+// 32,768 dofs, 683 CTAs of unequal length and 2.5 warps per scheduler; now 337
+// and 90, the sums and their order the same.)
 constexpr int kEvalTargets = 64;
 constexpr int kEvalLanes = 8;
 constexpr int kEvalRows = 4;  // rows per thread
 constexpr int kEvalThreads = kEvalTargets / kEvalRows * kEvalLanes;
 constexpr int kEvalChunk = 256;
+constexpr int kEvalSegment = 8;  // chunks per FP32 sum
 // Packed FP32x2 arithmetic on 64-bit registers (two rows per instruction).
 __device__ __forceinline__ unsigned long long pk2(float lo, float hi) {
   unsigned long long r;
@@ -705,24 +826,136 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+// segs: (leaf, first row in tidx, first chunk, -); one CTA per segment.
 __global__ void __launch_bounds__(kEvalThreads)
-k_fma_eval(const int2* __restrict__ items, const int* __restrict__ tptr, const int* __restrict__ tidx,
+k_fma_near(const int4* __restrict__ segs, const int* __restrict__ tptr, const int* __restrict__ tidx,
            const float4* __restrict__ xloc, const int* __restrict__ nb_ptr, const int* __restrict__ nb,
-           const int* __restrict__ leaf_pptr, const double* __restrict__ cen, double half,
-           const float* __restrict__ Lx, const float4* __restrict__ ppos,
-           const float4* __restrict__ pstr, const int* __restrict__ close_ptr,
-           const int* __restrict__ pair_pan, const double* __restrict__ val,
-           const int4* __restrict__ cell_dofs, const double* __restrict__ a,
-           const double* __restrict__ b, double* __restrict__ y,
-           const __grid_constant__ FmaConst c_fma) {
+           const int* __restrict__ leaf_pptr, const double* __restrict__ cen, int nq,
+           const float4* __restrict__ ppos, const float4* __restrict__ pstr,
+           float4* __restrict__ part) {
   // point k, each value duplicated for the packed operands:
   // sA = ((x, x), (y, y)), sB = ((z, z), (q, q)), sC = ((-mx, -mx), (-my, -my)), sD = (-mz, -mz)
   __shared__ ulonglong2 sA[kEvalChunk], sB[kEvalChunk], sC[kEvalChunk];
   __shared__ unsigned long long sD[kEvalChunk];
+  __shared__ int snp[28], sfirst[27];  // a neighbour's first point: in the sequence, of all points
+  __shared__ float soff[27][3];
+  const int4 sg = segs[blockIdx.x];
+  const int leaf = sg.x, t0 = sg.y;
+  const int nt = min(kEvalTargets, tptr[leaf + 1] - t0);
+  const int tid = threadIdx.x, qd = tid / kEvalLanes, lane = tid % kEvalLanes;
+  if (tid < 32) {
+    const int ne = nb_ptr[leaf + 1] - nb_ptr[leaf];
+    int np = 0;
+    if (tid < ne) {
+      const int sl = nb[nb_ptr[leaf] + tid];
+      sfirst[tid] = leaf_pptr[sl] * nq;
+      np = (leaf_pptr[sl + 1] - leaf_pptr[sl]) * nq;
+      for (int d = 0; d < 3; ++d) soff[tid][d] = (float)(cen[3 * sl + d] - cen[3 * leaf + d]);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, np, o);
+      if (tid >= o) np += u;
+    }
+    if (tid < ne) snp[tid + 1] = np;
+    if (tid == 0) snp[0] = 0;
+  }
+  float4 xr[kEvalRows];
+#pragma unroll
+  for (int h = 0; h < kEvalRows; ++h) {
+    const int r = kEvalRows * qd + h;
+    xr[h] = r < nt ? xloc[tidx[t0 + r]] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __syncthreads();
+  const int total = snp[nb_ptr[leaf + 1] - nb_ptr[leaf]];
+  const unsigned long long cx0 = pk2(-xr[0].x, -xr[1].x), cy0 = pk2(-xr[0].y, -xr[1].y),
+                           cz0 = pk2(-xr[0].z, -xr[1].z);
+  const unsigned long long cx1 = pk2(-xr[2].x, -xr[3].x), cy1 = pk2(-xr[2].y, -xr[3].y),
+                           cz1 = pk2(-xr[2].z, -xr[3].z);
+  const int first = sg.z * kEvalChunk, last = min(total, first + kEvalSegment * kEvalChunk);
+  // point g of the sequence: leaf-local position plus its leaf's offset (a
+  // thread's points come in ascending order)
+  int e = 0;
+  auto fetch = [&](int g, float4& P, float4& Q) {
+    while (g >= snp[e + 1]) ++e;
+    const int f = sfirst[e] + (g - snp[e]);
+    P = ppos[f];
+    Q = pstr[f];
+    P.x += soff[e][0];
+    P.y += soff[e][1];
+    P.z += soff[e][2];
+  };
+  constexpr int kPer = kEvalChunk / kEvalThreads;  // staged points per thread
+  float4 nP[kPer], nQ[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u)
+    if (first + u * kEvalThreads + tid < last) fetch(first + u * kEvalThreads + tid, nP[u], nQ[u]);
+  unsigned long long pa0 = 0ull, pa1 = 0ull;
+  const bool rows = (tid & ~31) / kEvalLanes * kEvalRows < nt;  // the warp has any
+  for (int base = first; base < last; base += kEvalChunk) {
+    const int cnt = min(kEvalChunk, last - base);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int j = u * kEvalThreads + tid;
+      if (j < cnt) {
+        const float4 P = nP[u], Q = nQ[u];
+        sA[j] = make_ulonglong2(pk2(P.x, P.x), pk2(P.y, P.y));
+        sB[j] = make_ulonglong2(pk2(P.z, P.z), pk2(Q.x, Q.x));
+        sC[j] = make_ulonglong2(pk2(-Q.y, -Q.y), pk2(-Q.z, -Q.z));
+        sD[j] = pk2(-Q.w, -Q.w);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int g = base + kEvalChunk + u * kEvalThreads + tid;
+      if (g < last) fetch(g, nP[u], nQ[u]);
+    }
+    // q / r - (R . m) / r^3 = (q - (R . m) / r^2) / r for two row pairs
+    auto term = [&](int k, unsigned long long& p0, unsigned long long& p1) {
+      const ulonglong2 A = sA[k], B = sB[k], C = sC[k];
+      const unsigned long long D = sD[k];
+      {
+        const unsigned long long rx = add2(A.x, cx0), ry = add2(A.y, cy0), rz = add2(B.x, cz0);
+        const unsigned long long r2 = fma2(rx, rx, fma2(ry, ry, mul2(rz, rz)));
+        float q0, q1;
+        upk2(r2, q0, q1);
+        const unsigned long long ri = pk2(rsqrt_approx(q0), rsqrt_approx(q1));
+        const unsigned long long dn = fma2(rx, C.x, fma2(ry, C.y, mul2(rz, D)));
+        p0 = fma2(fma2(dn, mul2(ri, ri), B.y), ri, p0);
+      }
+      {
+        const unsigned long long rx = add2(A.x, cx1), ry = add2(A.y, cy1), rz = add2(B.x, cz1);
+        const unsigned long long r2 = fma2(rx, rx, fma2(ry, ry, mul2(rz, rz)));
+        float q0, q1;
+        upk2(r2, q0, q1);
+        const unsigned long long ri = pk2(rsqrt_approx(q0), rsqrt_approx(q1));
+        const unsigned long long dn = fma2(rx, C.x, fma2(ry, C.y, mul2(rz, D)));
+        p1 = fma2(fma2(dn, mul2(ri, ri), B.y), ri, p1);
+      }
+    };
+    if (rows)
+      for (int k = lane; k < cnt; k += kEvalLanes) term(k, pa0, pa1);
+  }
+  float4 o;
+  upk2(pa0, o.x, o.y);
+  upk2(pa1, o.z, o.w);
+  part[(size_t)blockIdx.x * kEvalThreads + tid] = o;
+}
+
+// seg_ptr: an item's segments in part.
+__global__ void __launch_bounds__(kEvalThreads)
+k_fma_eval(const int2* __restrict__ items, const int* __restrict__ seg_ptr,
+           const float4* __restrict__ part, const int* __restrict__ tptr,
+           const int* __restrict__ tidx, const float4* __restrict__ xloc, double half,
+           const float* __restrict__ Lx, const int* __restrict__ close_ptr,
+           const int* __restrict__ pair_pan, const double* __restrict__ val,
+           const int4* __restrict__ cell_dofs, const double* __restrict__ a,
+           const double* __restrict__ b, double* __restrict__ y,
+           const __grid_constant__ FmaConst c_fma) {
   __shared__ float sL[kFmaMaxOrder * kFmaMaxOrder * kFmaMaxOrder];
   __shared__ float sw[kEvalTargets][3][kFmaMaxOrder];
-  __shared__ int snp[28];
-  __shared__ float soff[27][3];
   const int2 it = items[blockIdx.x];
   const int leaf = it.x, t0 = it.y;
   const int nt = min(kEvalTargets, tptr[leaf + 1] - t0);
@@ -735,7 +968,7 @@ k_fma_eval(const int2* __restrict__ items, const int* __restrict__ tptr, const i
     ix[h] = r < nt ? tidx[t0 + r] : -1;
     xr[h] = ix[h] >= 0 ? xloc[ix[h]] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  const int n = c_fma.n, n3 = c_fma.n3, nq = c_fma.nq;
+  const int n = c_fma.n, n3 = c_fma.n3;
   double acc[kEvalRows] = {0.0, 0.0, 0.0, 0.0};
   if (Lx) {
     for (int k = tid; k < n3; k += kEvalThreads) sL[k] = Lx[(size_t)leaf * n3 + k];
@@ -761,96 +994,13 @@ k_fma_eval(const int2* __restrict__ items, const int* __restrict__ tptr, const i
       acc[h] = (double)f;
     }
   }
-  const int ne = nb_ptr[leaf + 1] - nb_ptr[leaf];
-  if (tid == 0) {
-    int c = 0;
-    for (int e = 0; e < ne; ++e) {
-      const int sl = nb[nb_ptr[leaf] + e];
-      snp[e] = c;
-      c += (leaf_pptr[sl + 1] - leaf_pptr[sl]) * nq;
-      for (int d = 0; d < 3; ++d) soff[e][d] = (float)(cen[3 * sl + d] - cen[3 * leaf + d]);
-    }
-    snp[ne] = c;
-  }
-  __syncthreads();
-  const int total = snp[ne];
-  const unsigned long long cx0 = pk2(-xr[0].x, -xr[1].x), cy0 = pk2(-xr[0].y, -xr[1].y),
-                           cz0 = pk2(-xr[0].z, -xr[1].z);
-  const unsigned long long cx1 = pk2(-xr[2].x, -xr[3].x), cy1 = pk2(-xr[2].y, -xr[3].y),
-                           cz1 = pk2(-xr[2].z, -xr[3].z);
-  // point g of the sequence: leaf-local position plus its leaf's offset
-  auto fetch = [&](int g, float4& P, float4& Q) {
-    int e = 0;
-    while (g >= snp[e + 1]) ++e;
-    const int f = leaf_pptr[nb[nb_ptr[leaf] + e]] * nq + (g - snp[e]);
-    P = ppos[f];
-    Q = pstr[f];
-    P.x += soff[e][0];
-    P.y += soff[e][1];
-    P.z += soff[e][2];
-  };
-  constexpr int kPer = kEvalChunk / kEvalThreads;  // staged points per thread
-  float4 nP[kPer], nQ[kPer];
-#pragma unroll
-  for (int u = 0; u < kPer; ++u)
-    if (u * kEvalThreads + tid < total) fetch(u * kEvalThreads + tid, nP[u], nQ[u]);
-  unsigned long long pa0 = 0ull, pa1 = 0ull;
-  int nchunk = 0;
-  for (int base = 0; base < total; base += kEvalChunk) {
-    const int cnt = min(kEvalChunk, total - base);
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int j = u * kEvalThreads + tid;
-      if (j < cnt) {
-        const float4 P = nP[u], Q = nQ[u];
-        sA[j] = make_ulonglong2(pk2(P.x, P.x), pk2(P.y, P.y));
-        sB[j] = make_ulonglong2(pk2(P.z, P.z), pk2(Q.x, Q.x));
-        sC[j] = make_ulonglong2(pk2(-Q.y, -Q.y), pk2(-Q.z, -Q.z));
-        sD[j] = pk2(-Q.w, -Q.w);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int g = base + kEvalChunk + u * kEvalThreads + tid;
-      if (g < total) fetch(g, nP[u], nQ[u]);
-    }
-    // q / r - (R . m) / r^3 = (q - (R . m) / r^2) / r for two row pairs
-    auto term = [&](int k, unsigned long long& p0, unsigned long long& p1) {
-      const ulonglong2 A = sA[k], B = sB[k], C = sC[k];
-      const unsigned long long D = sD[k];
-      {
-        const unsigned long long rx = add2(A.x, cx0), ry = add2(A.y, cy0), rz = add2(B.x, cz0);
-        const unsigned long long r2 = fma2(rx, rx, fma2(ry, ry, mul2(rz, rz)));
-        float q0, q1;
-        upk2(r2, q0, q1);
-        const unsigned long long ri = pk2(rsqrt_approx(q0), rsqrt_approx(q1));
-        const unsigned long long dn = fma2(rx, C.x, fma2(ry, C.y, mul2(rz, D)));
-        p0 = fma2(fma2(dn, mul2(ri, ri), B.y), ri, p0);
-      }
-      {
-        const unsigned long long rx = add2(A.x, cx1), ry = add2(A.y, cy1), rz = add2(B.x, cz1);
-        const unsigned long long r2 = fma2(rx, rx, fma2(ry, ry, mul2(rz, rz)));
-        float q0, q1;
-        upk2(r2, q0, q1);
-        const unsigned long long ri = pk2(rsqrt_approx(q0), rsqrt_approx(q1));
-        const unsigned long long dn = fma2(rx, C.x, fma2(ry, C.y, mul2(rz, D)));
-        p1 = fma2(fma2(dn, mul2(ri, ri), B.y), ri, p1);
-      }
-    };
-    for (int k = lane; k < cnt; k += kEvalLanes) term(k, pa0, pa1);
-    // FP64 sum of FP32 partials every eight chunks
-    if ((++nchunk & 7) == 0 || base + kEvalChunk >= total) {
-      float l0, h0, l1, h1;
-      upk2(pa0, l0, h0);
-      upk2(pa1, l1, h1);
-      acc[0] += (double)l0;
-      acc[1] += (double)h0;
-      acc[2] += (double)l1;
-      acc[3] += (double)h1;
-      pa0 = pa1 = 0ull;
-    }
+#pragma unroll 4
+  for (int s = seg_ptr[blockIdx.x]; s < seg_ptr[blockIdx.x + 1]; ++s) {
+    const float4 p = part[(size_t)s * kEvalThreads + tid];
+    acc[0] += (double)p.x;
+    acc[1] += (double)p.y;
+    acc[2] += (double)p.z;
+    acc[3] += (double)p.w;
   }
 #pragma unroll
   for (int h = 0; h < kEvalRows; ++h) {
@@ -969,6 +1119,10 @@ struct FmaState {
   int* d_nb = nullptr;
   int2* d_items = nullptr;       // evaluation work items: (leaf, first row in tidx)
   int n_items = 0;
+  int4* d_segs = nullptr;        // near-field segments: (leaf, first row in tidx, first chunk, -)
+  int* d_seg_ptr = nullptr;      // segments per item (CSR)
+  float4* d_seg_part = nullptr;  // their sums
+  int n_segs = 0;
   int4* d_p2m_items = nullptr;   // P2M work items: (leaf, first and end panel position)
   int* d_p2m_iptr = nullptr;     // P2M items per leaf (CSR)
   float* d_Wpart = nullptr;      // partial expansions of the P2M items
@@ -1270,6 +1424,16 @@ static int fma_build(wbem_context* h, FmaState* F, const QuadTables& qt) {
   std::vector<int2> items;
   for (const auto& c : it_cost) items.push_back(c.second);
   F->n_items = (int)items.size();
+  std::vector<int4> segs;
+  std::vector<int> seg_ptr(1, 0);
+  for (const int2& i : items) {
+    long long np = 0;
+    for (int e = nbp[i.x]; e < nbp[i.x + 1]; ++e) np += pptr[nbl[e] + 1] - pptr[nbl[e]];
+    const int chunks = (int)((np * F->nq + kEvalChunk - 1) / kEvalChunk);
+    for (int c = 0; c < chunks; c += kEvalSegment) segs.push_back(make_int4(i.x, i.y, c, 0));
+    seg_ptr.push_back((int)segs.size());
+  }
+  F->n_segs = (int)segs.size();
   std::vector<int4> p2m_items;
   std::vector<int> p2m_iptr(LV.nbox + 1, 0);
   for (int b = 0; b < LV.nbox; ++b) {
@@ -1298,6 +1462,9 @@ static int fma_build(wbem_context* h, FmaState* F, const QuadTables& qt) {
   WB_CHK(fma_upload(h, F, &F->d_tptr, tptr));
   WB_CHK(fma_upload(h, F, &F->d_tidx, tidx));
   WB_CHK(fma_upload(h, F, &F->d_items, items));
+  WB_CHK(fma_upload(h, F, &F->d_segs, segs));
+  WB_CHK(fma_upload(h, F, &F->d_seg_ptr, seg_ptr));
+  WB_CHK(fma_alloc(h, F, &F->d_seg_part, (size_t)F->n_segs * kEvalThreads));
   WB_CHK(fma_upload(h, F, &F->d_nb_ptr, nbp));
   if (nbl.empty()) nbl.push_back(0);
   WB_CHK(fma_upload(h, F, &F->d_nb, nbl));
@@ -1313,7 +1480,7 @@ static int fma_build(wbem_context* h, FmaState* F, const QuadTables& qt) {
     int2 *d_cnt = nullptr, *d_lptr = nullptr;
     DeviceFreeGuard guard{{(void**)&d_cnt, (void**)&d_lptr}};
     WB_CHK(dev_alloc(h, &d_cnt, (size_t)N));
-    k_fma_close<<<(N + 127) / 128, 128, 0, h->stream>>>(
+    k_fma_close<<<(N + 3) / 4, 128, 0, h->stream>>>(
         N, F->d_tidx, F->d_tgt_leaf, F->d_nb_ptr, F->d_nb, F->d_leaf_pptr, F->d_leaf_pan, h->d_X, F->d_geo,
         h->d_sptr, h->d_scell, nullptr, nullptr, d_cnt, nullptr, nullptr, nullptr);
     std::vector<int2> cnt(N), lptr(N);
@@ -1342,7 +1509,7 @@ static int fma_build(wbem_context* h, FmaState* F, const QuadTables& qt) {
     WB_CHK(fma_alloc(h, F, &F->d_pair_pan, std::max<size_t>(1, F->npairs)));
     WB_CHK(fma_alloc(h, F, &F->d_close_val, 8 * std::max<size_t>(1, F->npairs)));
     WB_CHK(fma_alloc(h, F, &F->d_plist, std::max<size_t>(1, F->npairs)));
-    k_fma_close<<<(N + 127) / 128, 128, 0, h->stream>>>(
+    k_fma_close<<<(N + 3) / 4, 128, 0, h->stream>>>(
         N, F->d_tidx, F->d_tgt_leaf, F->d_nb_ptr, F->d_nb, F->d_leaf_pptr, F->d_leaf_pan, h->d_X, F->d_geo,
         h->d_sptr, h->d_scell, F->d_close_ptr, d_lptr, nullptr, F->d_pair_row, F->d_pair_pan,
         F->d_plist);
@@ -1417,22 +1584,28 @@ static int fma_product(wbem_context* h, const double* a, const double* b, double
   k_fma_p2m_sum<<<LV.nbox, 256, 0, s>>>(F->d_p2m_iptr, F->d_Wpart, LV.d_W, kMpSets * n3);
   for (int l = L; l > kFmaMinLevel; --l) {
     FmaLevel& P = F->lev[l - 1];
-    k_fma_m2m<<<P.nbox, nt, 0, s>>>(P.d_child_ptr, P.d_child, P.d_child_oct, F->lev[l].d_W, P.d_W,
+    k_fma_m2m<<<dim3(P.nbox, kMpSets), nt, 0, s>>>(P.d_child_ptr, P.d_child, P.d_child_oct, F->lev[l].d_W, P.d_W,
                                     F->cst);
   }
-  if (F->n_m2l_items > 0)
-    k_fma_m2l_gemm<<<F->n_m2l_items, 256, 0, s>>>(F->d_m2l_items, F->d_ent_src, F->d_ent_out, F->d_K,
-                                                  F->d_Wall, F->d_lvl_scale, F->d_part, n3);
+  if (F->n_m2l_items > 0) {
+    const M2LSplit sp = m2l_split(n3);
+    k_fma_m2l_gemm<<<dim3(F->n_m2l_items, sp.parts), sp.threads, 0, s>>>(
+        F->d_m2l_items, F->d_ent_src, F->d_ent_out, F->d_K, F->d_Wall, F->d_lvl_scale, F->d_part, n3);
+  }
   k_fma_m2l_sum<<<F->total_boxes, nt, 0, s>>>(F->d_gptr, F->d_part, F->d_Lall, n3);
   for (int l = kFmaMinLevel + 1; l <= L; ++l) {
     FmaLevel& V = F->lev[l];
     k_fma_l2l<<<V.nbox, nt, 0, s>>>(V.d_parent, V.d_oct, F->lev[l - 1].d_L, V.d_L, F->cst);
   }
+  if (F->n_segs > 0)
+    k_fma_near<<<F->n_segs, kEvalThreads, 0, s>>>(F->d_segs, F->d_tptr, F->d_tidx, F->d_xloc,
+                                                  F->d_nb_ptr, F->d_nb, F->d_leaf_pptr, LV.d_cen,
+                                                  F->nq, F->d_ppos, F->d_pstr, F->d_seg_part);
   k_fma_eval<<<F->n_items, kEvalThreads, 0, s>>>(
-      F->d_items, F->d_tptr, F->d_tidx, F->d_xloc, F->d_nb_ptr, F->d_nb, F->d_leaf_pptr, LV.d_cen,
-      LV.half, L >= kFmaMinLevel ? LV.d_L : nullptr, F->d_ppos, F->d_pstr, F->d_close_ptr,
-      F->d_pair_pan, F->d_close_val, h->d_cell_dofs, a, b, y, F->cst);
-  h->launches += 6 + 2 * (L - kFmaMinLevel);
+      F->d_items, F->d_seg_ptr, F->d_seg_part, F->d_tptr, F->d_tidx, F->d_xloc, LV.half,
+      L >= kFmaMinLevel ? LV.d_L : nullptr, F->d_close_ptr, F->d_pair_pan, F->d_close_val,
+      h->d_cell_dofs, a, b, y, F->cst);
+  h->launches += 7 + 2 * (L - kFmaMinLevel);
   WB_CU(cudaGetLastError());
   return WBEM_OK;
 }
@@ -1459,8 +1632,8 @@ int fma_near_blocks(wbem_context* h, double** blocks) {
   if (!F) return fail(h, WBEM_ERR_STATE, "FMA: not assembled");
   const int N = h->N, nb = (N + kBJ - 1) / kBJ;
   WB_CU(cudaMemsetAsync(F->d_blocks, 0, sizeof(double) * (size_t)nb * kBJ * kBJ, h->stream));
-  k_fma_near_blocks<<<(N + 127) / 128, 128, 0, h->stream>>>(
-      N, F->d_tgt_leaf, F->d_nb_ptr, F->d_nb, F->d_leaf_pptr, F->d_leaf_pan, F->lev[F->L].d_cen,
+  k_fma_near_blocks<<<(N + kNbWarps - 1) / kNbWarps, 32 * kNbWarps, 0, h->stream>>>(
+      N, F->d_tgt_leaf, F->d_nb_ptr, F->d_nb, F->d_leaf_pptr, F->d_leaf_pan, F->d_pos_leaf, F->lev[F->L].d_cen,
       F->d_xloc, F->d_ppos, h->d_rec, F->d_close_ptr, F->d_pair_pan, F->d_close_val,
       h->d_cell_dofs, h->d_mask, h->d_alpha, F->d_blocks, F->cst);
   WB_CU(cudaGetLastError());

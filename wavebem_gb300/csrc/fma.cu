@@ -41,6 +41,7 @@
 #include "context.h"
 #include "host_util.h"
 #include "fma_tree.h"
+#include "packed.cuh"
 #include "kernels.h"
 
 namespace wbem {
@@ -801,31 +802,6 @@ constexpr int kEvalRows = 4;  // rows per thread
 constexpr int kEvalThreads = kEvalTargets / kEvalRows * kEvalLanes;
 constexpr int kEvalChunk = 256;
 constexpr int kEvalSegment = 8;  // chunks per FP32 sum
-// Packed FP32x2 arithmetic on 64-bit registers (two rows per instruction).
-__device__ __forceinline__ unsigned long long pk2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void upk2(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
-                                                   unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 // segs: (leaf, first row in tidx, first chunk, -); one CTA per segment.
 __global__ void __launch_bounds__(kEvalThreads)
 k_fma_near(const int4* __restrict__ segs, const int* __restrict__ tptr, const int* __restrict__ tidx,

@@ -18,6 +18,7 @@
 #include <stdint.h>
 #include "context.h"
 #include "host_util.h"
+#include "packed.cuh"
 #include "kernels.h"
 #include "panel_fp64.cuh"
 
@@ -30,7 +31,13 @@ cudaError_t upload_quadrature_mixed(const QuadTables& t) {
 
 constexpr double kInv4PiM = 0.07957747154594766788;
 
-__host__ __device__ constexpr int mixed_rec_floats(int nq) { return ((9 * nq + 24 + 3) / 4) * 4; }
+// Panel record: 20 floats per pair of points (2 p, 2 p + 1), the nine values of
+// the two points side by side: offset from the centre (3), minus its square,
+// minus the normal's difference from nu (3), minus offset . normal, J weight /
+// (4 pi); then 24 floats of panel data.
+constexpr int kPairFloats = 20;
+__host__ __device__ constexpr int mixed_rec_panel(int nq) { return (nq + 1) / 2 * kPairFloats; }
+__host__ __device__ constexpr int mixed_rec_floats(int nq) { return mixed_rec_panel(nq) + 24; }
 
 // Same near test in every kernel (no contraction: explicit round-to-nearest ops).
 __device__ __forceinline__ bool near_test(float xi, float yi, float zi, float4 g) {
@@ -144,16 +151,25 @@ __global__ void __launch_bounds__(kRecWarps * 32)
       del[e] = pt[e][q];
       n[e] = pt[3 + e][q] * rdet;
     }
-    reinterpret_cast<float4*>(r)[q] =
-        make_float4((float)del[0], (float)del[1], (float)del[2],
-                    (float)(del[0] * del[0] + del[1] * del[1] + del[2] * del[2]));
-    reinterpret_cast<float4*>(r)[nq + q] =
-        make_float4((float)(n[0] - nu[0]), (float)(n[1] - nu[1]), (float)(n[2] - nu[2]),
-                    (float)(del[0] * n[0] + del[1] * n[1] + del[2] * n[2]));
-    r[8 * nq + q] = (float)(det * c_qm.gp[q][2] * kInv4PiM);
+    const float v[10] = {(float)del[0],
+                         (float)del[1],
+                         (float)del[2],
+                         -(float)(del[0] * del[0] + del[1] * del[1] + del[2] * del[2]),
+                         -(float)(n[0] - nu[0]),
+                         -(float)(n[1] - nu[1]),
+                         -(float)(n[2] - nu[2]),
+                         -(float)(del[0] * n[0] + del[1] * n[1] + del[2] * n[2]),
+                         (float)(det * c_qm.gp[q][2] * kInv4PiM),
+                         0.f};
+    float* rp = r + (q >> 1) * kPairFloats + (q & 1);
+#pragma unroll
+    for (int e = 0; e < 10; ++e) {
+      rp[2 * e] = v[e];
+      if (q == nq - 1 && !(q & 1)) rp[2 * e + 1] = v[e];  // a last point alone: paired with itself
+    }
   }
   // panel data: lane e splits one of centre, normal, moments, moment sum
-  float* cd = r + 9 * nq;
+  float* cd = r + mixed_rec_panel(nq);
   if (on && lane < 11) {
     const double v = lane < 3   ? (lane == 0 ? cen[0] : lane == 1 ? cen[1] : cen[2])
                      : lane < 6 ? (lane == 3 ? nu[0] : lane == 4 ? nu[1] : nu[2])
@@ -169,7 +185,6 @@ __global__ void __launch_bounds__(kRecWarps * 32)
   } else if (on && lane == 11) {
     cd[22] = 0.f;
     cd[23] = 0.f;
-    for (int k = 9 * nq + 24; k < RF; ++k) r[k] = 0.f;
   }
   // near test: centre (float) and (ratio * largest diagonal)^2, at least
   // 1.01 x the farthest vertex, so that every panel with the collocation
@@ -200,6 +215,19 @@ __global__ void __launch_bounds__(kRecWarps * 32)
 }
 
 constexpr int kChunkM = 8;
+
+// The approximate root and quotient without the steps for subnormal operands:
+// the same values (1 / r^3 overflows long before r^2 is subnormal).
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float div_ftz(float x, float y) {
+  float r;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+  return r;
+}
 
 template <int Q1>
 __global__ void __launch_bounds__(kRowsPerTile)
@@ -303,10 +331,7 @@ __global__ void __launch_bounds__(kRowsPerTile)
       // near (FP64 kernel) or singular (always near, see the cell records)
       if (!active || near_test(xf, yf, zf, mt.geo)) continue;
       const float* r = stage + (size_t)((c & 1) * kChunkM + k) * RF;
-      const float4* qa = reinterpret_cast<const float4*>(r);
-      const float4* qb = reinterpret_cast<const float4*>(r + 4 * NQ);
-      const float* qj = r + 8 * NQ;
-      const float* cd = r + 9 * NQ;
+      const float* cd = r + mixed_rec_panel(NQ);
       // ---- panel base term in double-float
       df R[3];
 #pragma unroll
@@ -345,7 +370,9 @@ __global__ void __launch_bounds__(kRowsPerTile)
       df gR = df_mul(Rn, ri3);
       gR.hi = -gR.hi;
       gR.lo = -gR.lo;
-      // ---- per-point differences in FP32
+      // ---- per-point differences in FP32, two points per packed instruction: the
+      // kernel is bound by issue slots (84% busy at 62% of the FP32 pipe with
+      // scalar ones; 6.08 -> 5.23 ms at 12,000 dofs, the same bits)
       // with num = rc^2 - rq^2 = -(2 R_c.delta + |delta|^2):
       //   rc - rq = num / (rc + rq),  1/rq - 1/rc = (rc - rq) / (rq rc),
       //   (R.n)(-1/r^3) - (R_c.nu)(-1/rc^3)
@@ -356,43 +383,57 @@ __global__ void __launch_bounds__(kRowsPerTile)
       const float rc = rc2 * rcinv;
       const float K1 = -Rn.hi * ri3.hi;
       float ls0 = 0.f, ls1 = 0.f, ls2 = 0.f, ls3 = 0.f, ln0 = 0.f, ln1 = 0.f, ln2 = 0.f, ln3 = 0.f;
+      const unsigned long long RX = pk2(Rcx, Rcx), RY = pk2(Rcy, Rcy), RZ = pk2(Rcz, Rcz);
+      const unsigned long long rc_2 = pk2(rc, rc), rc2_2 = pk2(rc2, rc2), K1_2 = pk2(K1, K1);
+      const unsigned long long m1 = pk2(-1.f, -1.f), m2 = pk2(-2.f, -2.f);
+      // tensor-product accumulation: row sums over xi, then the two eta weights
+      float st = 0.f, s1 = 0.f, nt = 0.f, n1 = 0.f;
 #pragma unroll
-      for (int bq = 0; bq < Q1; ++bq) {
-        // tensor-product accumulation: row sums over xi, then the two eta weights
-        float st = 0.f, s1 = 0.f, nt = 0.f, n1 = 0.f;
+      for (int p = 0; p < (NQ + 1) / 2; ++p) {
+        const ulonglong2* g = reinterpret_cast<const ulonglong2*>(r + p * kPairFloats);
+        const ulonglong2 g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3];
+        const unsigned long long J = *reinterpret_cast<const unsigned long long*>(g + 4);
+        const unsigned long long Rd = fma2(RX, g0.x, fma2(RY, g0.y, mul2(RZ, g1.x)));
+        const unsigned long long num = fma2(m2, Rd, g1.y);
+        const unsigned long long rq2 = fma2(num, m1, rc2_2);
+        float a0, a1, b0, b1;
+        upk2(rq2, a0, a1);
+        const unsigned long long rqinv = pk2(rsqrt_ftz(a0), rsqrt_ftz(a1));
+        const unsigned long long rq = mul2(rq2, rqinv);
+        upk2(num, a0, a1);
+        upk2(add2(rc_2, rq), b0, b1);
+        const unsigned long long dr = pk2(div_ftz(a0, b0), div_ftz(a1, b1));
+        const unsigned long long u = mul2(rqinv, J);
+        const unsigned long long fs2 = mul2(dr, u);  // times 1/rc after the point sums
+        const unsigned long long tsum = add2(fma2(rc_2, rq, rc2_2), rq2);
+        const unsigned long long t2 = fma2(RX, g2.x, fma2(RY, g2.y, fma2(RZ, g3.x, g3.y)));
+        const unsigned long long fn2 =
+            mul2(mul2(mul2(rqinv, rqinv), u), fma2(mul2(dr, tsum), K1_2, t2));
+        float fs[2], fn[2];
+        upk2(fs2, fs[0], fs[1]);
+        upk2(fn2, fn[0], fn[1]);
 #pragma unroll
-        for (int aq = 0; aq < Q1; ++aq) {
-          const int q = aq + Q1 * bq;
-          const float4 A = qa[q];
-          const float4 B = qb[q];
-          const float J = qj[q];
-          const float Rd = __fmaf_rn(Rcx, A.x, __fmaf_rn(Rcy, A.y, Rcz * A.z));
-          const float num = -__fmaf_rn(2.f, Rd, A.w);
-          const float rq2 = rc2 - num;
-          const float rqinv = rsqrtf(rq2);
-          const float rq = rq2 * rqinv;
-          const float dr = __fdividef(num, rc + rq);
-          const float u = rqinv * J;
-          const float fs = dr * u;  // times 1/rc after the point sums
-          const float tsum = __fmaf_rn(rc, rq, rc2) + rq2;
-          const float t2 = __fmaf_rn(Rcx, B.x, __fmaf_rn(Rcy, B.y, __fmaf_rn(Rcz, B.z, B.w)));
-          const float fn = (rqinv * rqinv) * u * __fmaf_rn(dr * tsum, K1, -t2);
+        for (int h = 0; h < 2; ++h) {
+          const int q = 2 * p + h;
+          if (q >= NQ) break;
           const float xa = c_qm.gpf[q][0];
-          st += fs;
-          s1 = __fmaf_rn(fs, xa, s1);
-          nt += fn;
-          n1 = __fmaf_rn(fn, xa, n1);
+          st = __fadd_rn(st, fs[h]);
+          s1 = __fmaf_rn(fs[h], xa, s1);
+          nt = __fadd_rn(nt, fn[h]);
+          n1 = __fmaf_rn(fn[h], xa, n1);
+          if ((q + 1) % Q1) continue;
+          const float eb = c_qm.gpf[q][1];
+          const float s0 = st - s1, n0 = nt - n1;
+          ls0 = __fmaf_rn(s0, 1.f - eb, ls0);
+          ls1 = __fmaf_rn(s1, 1.f - eb, ls1);
+          ls2 = __fmaf_rn(s0, eb, ls2);
+          ls3 = __fmaf_rn(s1, eb, ls3);
+          ln0 = __fmaf_rn(n0, 1.f - eb, ln0);
+          ln1 = __fmaf_rn(n1, 1.f - eb, ln1);
+          ln2 = __fmaf_rn(n0, eb, ln2);
+          ln3 = __fmaf_rn(n1, eb, ln3);
+          st = s1 = nt = n1 = 0.f;
         }
-        const float eb = c_qm.gpf[Q1 * bq][1];
-        const float s0 = st - s1, n0 = nt - n1;
-        ls0 = __fmaf_rn(s0, 1.f - eb, ls0);
-        ls1 = __fmaf_rn(s1, 1.f - eb, ls1);
-        ls2 = __fmaf_rn(s0, eb, ls2);
-        ls3 = __fmaf_rn(s1, eb, ls3);
-        ln0 = __fmaf_rn(n0, 1.f - eb, ln0);
-        ln1 = __fmaf_rn(n1, 1.f - eb, ln1);
-        ln2 = __fmaf_rn(n0, eb, ln2);
-        ln3 = __fmaf_rn(n1, eb, ln3);
       }
       const float fnsum = (ln0 + ln1) + (ln2 + ln3);
       const float lsv[4] = {ls0 * rcinv, ls1 * rcinv, ls2 * rcinv, ls3 * rcinv};

@@ -53,8 +53,8 @@ __device__ __forceinline__ double cta_rows_sum(double v[R]) {
 // threads the columns: x_j and the column's matrix are read once for the 4
 // rows, whose loads are independent. Bound by the FP64 pipe (one DFMA per 8
 // bytes: 4.6 TB/s at most). With a warp per row and x staged in shared memory
-// it took 46 us at N = 2,000 and 1.10 ms at N = 16,226, now 20 us and
-// 0.61 ms (3.4 TB/s).
+// it took 46 us at N = 2,000 and 1.10 ms at N = 16,226, now 16 us and
+// 0.47 ms (4.5 TB/s; 0.61 ms with the sign of x taken by an FP64 instruction).
 constexpr int kMvRows64 = 4;
 
 __global__ void __launch_bounds__(kMvThreads)
@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(kMvThreads)
   for (int j = tid; j < N; j += kMvThreads) {
     const bool m = mask[j] != 0;
     const double* A = (m ? A1 : A0) + j;
-    const double xj = m ? -x[j] : x[j];
+    const double xv = x[j];  // the sign by its bit: the FP64 pipe is the bound
+    const double xj = __hiloint2double(__double2hiint(xv) ^ (m ? 0x80000000 : 0), __double2loint(xv));
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[r] = fma(__ldcs(A + off[r]), xj, acc[r]);
   }

@@ -106,7 +106,7 @@ cudaError_t launch_bj_build(int N, const double* Nm, const double* Dm, const flo
                             const uint8_t* cflag, const int* cptr_full, const int* ccol_full,
                             const double* cval_full, double* binv, DevErr* err, cudaStream_t s);
 cudaError_t launch_bj_apply(int N, const double* binv, const double* x, double* y, int transpose,
-                            cudaStream_t s);
+                            bool ordered, cudaStream_t s);
 
 // Krylov helpers (FP64)
 // One Arnoldi step: w orthogonalised against the k vectors of V (classical

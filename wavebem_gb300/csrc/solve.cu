@@ -626,9 +626,39 @@ cudaError_t launch_bj_build(int N, const double* Nm, const double* Dm, const flo
   return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(kBJ)
+// z = inverse block * x. A CTA takes 32 rows of a block, its four warps a
+// quarter of the columns each: a row's 128 FP64 multiply-adds in one chain (a
+// CTA per block, a thread per row) take 8,192 cycles of each FP64 pipe, 14-15
+// us with the launch at 2,000 to 16,000 dofs; here 2,048, and 5.8 us.
+template <bool TRANS>
+__global__ void __launch_bounds__(128)
     k_bj_apply(int N, const double* __restrict__ binv, const double* __restrict__ x,
-               double* __restrict__ y, int transpose) {
+               double* __restrict__ y) {
+  __shared__ double part[4][32];
+  const int b = blockIdx.x / 4, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r = (blockIdx.x % 4) * 32 + lane, k0 = 32 * w, i0 = b * kBJ + k0;
+  const double* B = binv + (size_t)b * kBJ * kBJ + (TRANS ? (size_t)r * kBJ + k0 : (size_t)k0 * kBJ + r);
+  double v[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) v[k] = B[TRANS ? k : (size_t)k * kBJ];
+  const double xl = i0 + lane < N ? x[i0 + lane] : 0.0;
+  double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 32; k += 2) {
+    s0 = fma(v[k], __shfl_sync(0xffffffffu, xl, k), s0);
+    s1 = fma(v[k + 1], __shfl_sync(0xffffffffu, xl, k + 1), s1);
+  }
+  part[w][lane] = s0 + s1;
+  __syncthreads();
+  const int i = b * kBJ + r;
+  if (w == 0 && i < N) y[i] = (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
+}
+
+// A row's products in one chain: the order of sums that the FMA solve, which
+// repeats to 1e-8 if a last bit changes, has always had.
+__global__ void __launch_bounds__(kBJ)
+    k_bj_apply_ordered(int N, const double* __restrict__ binv, const double* __restrict__ x,
+               double* __restrict__ y) {
   __shared__ double xs[kBJ];
   const int b = blockIdx.x, r = threadIdx.x;
   const int i = b * kBJ + r;
@@ -636,25 +666,24 @@ __global__ void __launch_bounds__(kBJ)
   __syncthreads();
   const double* B = binv + (size_t)b * kBJ * kBJ;
   double s = 0;
-  if (!transpose) {
-    // 32 loads in flight ahead of the chain of additions
+  // 32 loads in flight ahead of the chain of additions
 #pragma unroll
-    for (int k0 = 0; k0 < kBJ; k0 += 32) {
-      double v[32];
+  for (int k0 = 0; k0 < kBJ; k0 += 32) {
+    double v[32];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) v[k] = B[(size_t)(k0 + k) * kBJ + r];
+    for (int k = 0; k < 32; ++k) v[k] = B[(size_t)(k0 + k) * kBJ + r];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) s = fma(v[k], xs[k0 + k], s);
-    }
-  } else {
-    for (int k = 0; k < kBJ; ++k) s = fma(B[(size_t)r * kBJ + k], xs[k], s);
+    for (int k = 0; k < 32; ++k) s = fma(v[k], xs[k0 + k], s);
   }
   if (i < N) y[i] = s;
 }
 
 cudaError_t launch_bj_apply(int N, const double* binv, const double* x, double* y, int transpose,
-                            cudaStream_t s) {
-  k_bj_apply<<<(N + kBJ - 1) / kBJ, kBJ, 0, s>>>(N, binv, x, y, transpose);
+                            bool ordered, cudaStream_t s) {
+  const int nb = (N + kBJ - 1) / kBJ;
+  if (transpose) k_bj_apply<true><<<4 * nb, 128, 0, s>>>(N, binv, x, y);
+  else if (ordered) k_bj_apply_ordered<<<nb, kBJ, 0, s>>>(N, binv, x, y);
+  else k_bj_apply<false><<<4 * nb, 128, 0, s>>>(N, binv, x, y);
   return cudaGetLastError();
 }
 

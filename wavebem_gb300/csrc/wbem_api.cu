@@ -612,7 +612,7 @@ int gmres_fp64(wbem_context* h, const double* rhs, double* x, int transpose) {
     return transpose ? apply_system_t(h, a, b) : apply_system(h, a, b);
   };
   auto prec = [&](const double* a, double* b) -> int {
-    CU(launch_bj_apply(h->N, h->d_binv, a, b, transpose, h->stream));
+    CU(launch_bj_apply(h->N, h->d_binv, a, b, transpose, h->assembled_prec == kAssembledFma, h->stream));
     return WBEM_OK;
   };
   int it = 0;
@@ -684,7 +684,7 @@ int gmres_ir(wbem_context* h, const double* rhs, double* x, int transpose) {
     return WBEM_OK;
   };
   auto prec = [&](const double* a, double* b) -> int {
-    CU(launch_bj_apply(N, h->d_binv, a, b, transpose, h->stream));
+    CU(launch_bj_apply(N, h->d_binv, a, b, transpose, false, h->stream));
     h->launches++;
     return WBEM_OK;
   };

@@ -635,13 +635,14 @@ __global__ void k_fma_m2l_ops(int n, double e2, float* __restrict__ K) {
 // items: (offset, first entry, entries, level); entries: source box and
 // output row (global over the levels). A CTA takes one item and blockDim.x / 2
 // target nodes (m2l_split: the nodes in equal shares of up to kM2LRows), each
-// thread an 8 x 4 block of C. The dipole columns (m' >= n3) carry one more
+// thread two 4 x 4 blocks of C; a warp's threads share a few columns, so that
+// the warps beyond a group's last pair only stage. The dipole columns (m' >= n3) carry one more
 // factor 1 / s, applied when staged. Staged values are stored at 16-byte block
 // (r / 4) ^ (c / 4 & 7) of their row c, which makes the transposing stores and
 // the reads free of bank conflicts; the next chunk is loaded into registers
 // meanwhile. One CTA per item with two passes of 128 nodes (216 exist at
 // order 6), 4-way store conflicts and no prefetch took 574 us at 32,768 dofs,
-// a third of it with SMs idle; this takes 360. Sums and their order are the
+// a third of it with SMs idle; this takes 301. Sums and their order are the
 // same.
 struct M2LSplit {
   int parts, threads;
@@ -665,7 +666,9 @@ k_fma_m2l_gemm(const int4* __restrict__ items, const int* __restrict__ ent_src,
   const float sc = lvl_scale[it.w];
   const float* Ko = K + (size_t)it.x * n3 * kd;
   const int nthr = blockDim.x, rows = nthr / 2, a0 = blockIdx.y * rows;
-  const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
+  // columns 4 tx .. + 3, rows 4 ty .. + 3 and 4 (ty + G) .. + 3
+  const int G = nthr / 16, tid = threadIdx.x, ty = tid % G, tx = tid / G;
+  const bool busy = 4 * ((tid & ~31) / G) < cnt;  // the warp has a column
   constexpr int kKLoads = 4, kWLoads = 8;  // rows * 8 / nthr; 64 * 8 / nthr, at most (64 threads)
   float4 kr[kKLoads], wr[kWLoads];
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -711,11 +714,12 @@ k_fma_m2l_gemm(const int4* __restrict__ items, const int* __restrict__ ent_src,
     }
     __syncthreads();
     if (m0 + kM2LK < kd) load(m0 + kM2LK);
+    if (!busy) continue;
 #pragma unroll 8
     for (int c = 0; c < kM2LK; ++c) {
       const int sw = c / 4;
-      const float4 k0 = *reinterpret_cast<const float4*>(&Ks[c][((2 * ty) ^ sw) * 4]);
-      const float4 k1 = *reinterpret_cast<const float4*>(&Ks[c][((2 * ty + 1) ^ sw) * 4]);
+      const float4 k0 = *reinterpret_cast<const float4*>(&Ks[c][(ty ^ sw) * 4]);
+      const float4 k1 = *reinterpret_cast<const float4*>(&Ks[c][((ty + G) ^ sw) * 4]);
       const float4 w = *reinterpret_cast<const float4*>(&Ws[c][(tx ^ sw) * 4]);
       const float av[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
       const float wv[4] = {w.x, w.y, w.z, w.w};
@@ -727,7 +731,7 @@ k_fma_m2l_gemm(const int4* __restrict__ items, const int* __restrict__ ent_src,
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int a = a0 + ty * 8 + i;
+    const int a = a0 + 4 * (i < 4 ? ty : ty + G) + i % 4;
     if (a >= n3) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

@@ -85,16 +85,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
-// Bounded wait until *flag == value, or (AT_LEAST) until it has reached value
-// (as a counter that may wrap around). Returns false after kWaitNs, or at once
-// if a wait has already given up somewhere (code set in the error word), so
-// that a queue of dependent launches ends soon.
-template <bool AT_LEAST>
+// Bounded wait until the counter *flag has reached value (it may wrap around).
+// Returns false after kWaitNs, or at once if a wait has already given up
+// somewhere (code set in the error word), so that a queue of dependent launches
+// ends soon.
 __device__ __forceinline__ bool flag_wait_bounded(const unsigned* flag, unsigned value, const DevErr* err) {
   auto done = [&]() {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-    return AT_LEAST ? (int)(v - value) >= 0 : v == value;
+    return (int)(v - value) >= 0;
   };
   // the clock is read only if the wait is a long one: reading it takes about
   // as long as the usual wait
@@ -119,7 +118,7 @@ __device__ __forceinline__ void grid_barrier(unsigned* ctr, unsigned target, int
     // release: this CTA's writes (ordered before by the CTA barrier) are seen
     // by whoever acquires the count
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
-    if (!flag_wait_bounded<true>(ctr, target, err)) dev_fail(err, WBEM_ERR_TIMEOUT, where, blockIdx.x, (int)target);
+    if (!flag_wait_bounded(ctr, target, err)) dev_fail(err, WBEM_ERR_TIMEOUT, where, blockIdx.x, (int)target);
   }
   __syncthreads();
 }

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
+#include <atomic>
 #include "kernels.h"
 #include "../../include/wbem.h"
 
@@ -856,6 +857,128 @@ __global__ void __launch_bounds__(kOrthoThreads)
     for (int i = i0 + tid; i < i1; i += kOrthoThreads) v[i] = inv * w[i];
 }
 
+// The same step for small N by one cluster of 16 CTAs: the parts meet in
+// distributed shared memory and hardware cluster barriers. Up to 200 rows per
+// CTA: beyond that sixteen FP64 pipes take longer than the barriers save. Whole
+// FP64 solves, ms, this form against k_ortho: 2,000 dofs 2.35 / 2.43, 3,001 3.17
+// / 3.27, 4,000 4.53 / 4.48.
+constexpr int kOrthoCluster = 16;
+constexpr int kOrthoClusterRows = 200;  // rows per CTA
+
+__global__ void __launch_bounds__(kOrthoThreads)
+    k_ortho_cluster(int N, int k, const double* __restrict__ V, double* __restrict__ w,
+                    double* __restrict__ v, double* __restrict__ out) {
+  __shared__ double dots[2][kOrthoMaxK], hs[kOrthoMaxK], ws[kOrthoClusterRows];
+  __shared__ double red[4][kOrthoRows], wsum[kOrthoThreads / 32], nsum;
+  constexpr int kWarps = kOrthoThreads / 32;
+  static_assert(kOrthoClusterRows <= kOrthoThreads, "a thread per row");
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = (int)cl.block_rank();
+  const int per = (N + kOrthoCluster - 1) / kOrthoCluster;
+  const int i0 = min(N, b * per), n = min(N, i0 + per) - i0;
+  if (tid < n) ws[tid] = w[i0 + tid];
+  __syncthreads();
+  double nrm = 0.0;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int j = warp; j < k; j += kWarps) {
+      const double* vj = V + (size_t)j * N + i0;
+      double s = 0.0;
+#pragma unroll 4
+      for (int i = lane; i < n; i += 32) s = fma(vj[i], ws[i], s);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) dots[pass][j] = s;
+    }
+    cl.sync();
+    // two vectors per warp and step: lane 16 h + r reads rank r's part
+    for (int j0 = 2 * warp; j0 < k; j0 += 2 * kWarps) {
+      const int j = j0 + (lane >> 4);
+      double s = j < k ? cl.map_shared_rank(dots[pass], lane & 15)[j] : 0.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((lane & 15) == 0 && j < k) {
+        hs[j] = s;
+        if (b == 0) out[j] = pass == 0 ? s : out[j] + s;
+      }
+    }
+    __syncthreads();
+    // 64 rows at a time, the vectors over 4 groups
+    const int r = tid & (kOrthoRows - 1), q = tid / kOrthoRows;
+    for (int c0 = 0; c0 < n; c0 += kOrthoRows) {
+      const int i = c0 + r;
+      double s = 0.0;
+      if (i < n)
+#pragma unroll 8
+        for (int j = q; j < k; j += 4) s = fma(hs[j], V[(size_t)j * N + i0 + i], s);
+      red[q][r] = s;
+      __syncthreads();
+      if (q == 0 && i < n) {
+        const double x = ws[i] - ((red[0][r] + red[1][r]) + (red[2][r] + red[3][r]));
+        ws[i] = x;
+        if (pass == 1) {
+          nrm = fma(x, x, nrm);
+          w[i0 + i] = x;
+        }
+      }
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+  if (lane == 0) wsum[warp] = nrm;
+  __syncthreads();
+  if (tid == 0) {
+    double s = 0.0;
+    for (int u = 0; u < kWarps; ++u) s += wsum[u];
+    nsum = s;
+  }
+  cl.sync();
+  double s = *cl.map_shared_rank(&nsum, lane & 15);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const double hn = sqrt(s);
+  if (b == 0 && tid == 0) out[k] = hn;
+  const double inv = 1.0 / hn;
+  if (hn > 0.0 && tid < n) v[i0 + tid] = inv * ws[tid];
+  cl.sync();  // no CTA leaves while another reads its shared memory
+}
+
+static cudaLaunchConfig_t ortho_cluster_config(cudaLaunchAttribute* attr, cudaStream_t s) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = kOrthoCluster;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(kOrthoCluster);
+  c.blockDim = dim3(kOrthoThreads);
+  c.stream = s;
+  c.attrs = attr;
+  c.numAttrs = 1;
+  return c;
+}
+
+// Whether this device takes a cluster of 16 CTAs (it is beyond the portable
+// size); asked once per device.
+static bool ortho_cluster_fits() {
+  static std::atomic<int> known[kMaxDev];  // 0: not asked, 1: yes, 2: no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDev) return false;
+  int r = known[dev].load(std::memory_order_acquire);
+  if (r == 0) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t c = ortho_cluster_config(&attr, nullptr);
+    int n = 0;
+    const bool ok = cudaFuncSetAttribute(k_ortho_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                         1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, k_ortho_cluster, &c) == cudaSuccess && n > 0;
+    if (!ok) cudaGetLastError();
+    r = ok ? 1 : 2;
+    known[dev].store(r, std::memory_order_release);
+  }
+  return r == 1;
+}
+
 size_t ortho_part_size(int n_ctas) { return (size_t)(2 * kOrthoMaxK + 1) * n_ctas; }
 
 // CTAs of k_ortho for N rows: at most one per SM (co-resident), and no more
@@ -868,6 +991,11 @@ int ortho_ctas(int N, int sms, bool ordered) {
 cudaError_t launch_ortho(int N, int k, const double* V, double* w, double* v, double* part,
                          double* out, unsigned* ctr, unsigned* epoch, int n_ctas, bool ordered,
                          DevErr* err, cudaStream_t s) {
+  if (!ordered && N <= kOrthoCluster * kOrthoClusterRows && ortho_cluster_fits()) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t c = ortho_cluster_config(&attr, s);
+    return cudaLaunchKernelEx(&c, k_ortho_cluster, N, k, V, w, v, out);
+  }
   unsigned base = *epoch;
   *epoch += (ordered ? 4u : 3u) * (unsigned)n_ctas;
   void* args[] = {(void*)&N, (void*)&k, (void*)&V, (void*)&w, (void*)&v, (void*)&part,

@@ -30,7 +30,7 @@
 // update, which streams the same operand bytes per K step either way.
 // The update is split between the next panel's columns (high-priority
 // stream) and the remainder (low-priority stream). The panel kernels have 13
-// and 16 KB footprints, so the next panel's chain runs beside the remainder's CTAs
+// and 4 KB footprints, so the next panel's chain runs beside the remainder's CTAs
 // on every SM (look-ahead); a few SMs stay free for the 200 KB diagonal
 // blocks.
 #include <cuda.h>
@@ -113,22 +113,28 @@ __global__ void k_lu_constraint_entries(int nrows, const int* __restrict__ crow,
 // that the panels read (inv(L) column-major, inv(U) row-major; the other
 // orientations follow in k_transpose_inverses). One CTA, everything
 // in shared memory: S (the block, then L and U), IL and IU (the inverses).
-// Eight steps of 16 columns, two CTA barriers each:
+// The elimination runs on the bordered matrix [[S, I], [I, 0]]: the rows of S
+// and of the right-hand identity become U and inv(L), the columns of the lower
+// identity inv(U). Eight steps of 16 columns, two CTA barriers each:
 //   A  warp 0 factors the 16 x 16 diagonal block in registers, a row per lane;
 //      lanes 16..31 carry the rows of the identity along, which become the
 //      inverse of its L. The registers rotate by one column per pivot, so one
 //      short loop body serves all 16 pivots;
-//   B  a thread per row solves x U = a for L21, two threads per column apply
-//      the inverse of L for U12;
-//   C  warps 1..14 update the trailing block in 4 x 4 tiles, except its leading
-//      16 x 16, which warp 0 updates and factors meanwhile (look-ahead); warp
-//      15 inverts the 16 x 16 block of U.
-// Then the inverses by doubling: from two inverted blocks of size b (16, 32,
-// 64), X21 = -L22^-1 (L21 L11^-1) and X12 = -(U11^-1 U12) U22^-1, two barriers
-// each; the inner products T sit in the blocks of the other inverse that are
-// zero, which are cleared again afterwards.
+//   B  a thread per row solves x U = a: L21 for the rows below the block,
+//      entries of inv(U) for those in it and above; a thread per column solves
+//      L y = a: U12 right of the block, entries of inv(L) left of it;
+//   C  warps 1..15 update everything beyond in 8 x 4 tiles, except the next
+//      16 x 16 diagonal block, which warp 0 updates and factors meanwhile
+//      (look-ahead).
+// The order of operations is part of the result: every entry takes its
+// multiply-subtracts one pivot after the other in ascending order, as an
+// unblocked elimination does, whatever the blocking. A refinement that stops at
+// its tolerance after two or three steps carries the rounding of these factors
+// into its answer (the multipliers of an adjoint at 1e-10 of their norm), so
+// another order gives other answers.
 // Bound by the latency of A (16 pivots in a row, eight times). Unblocked, with
-// a CTA barrier per pivot, the block took 51.5 us; now 34.6 us.
+// a CTA barrier per pivot, the block took 51.5 us; now 30.6 us (of which the
+// loads and stores are 4).
 constexpr int kDThreads = 512;
 constexpr int kDB = 16;     // columns per step
 constexpr int kDLD = 132;   // shared rows: 16-byte aligned, rows r and r + 8 share banks
@@ -140,42 +146,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-// O (4 x 4) = sign * sum over k0 <= k < k1 of Lp(i, k) Rp(k, j), all with rows
-// of kDLD floats; the tile's rows are rs apart
-__device__ __forceinline__ void diag_tile(const float* Lp, const float* Rp, float* Op, int rs, int k0,
-                                          int k1, float sign) {
-  float acc[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
-  const int ls = rs * kDLD;
-#pragma unroll 1
-  for (int k = k0; k < k1; k += 4) {  // k0 and k1 are multiples of 4
-    float4 l[4], r[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      l[u] = *reinterpret_cast<const float4*>(Lp + u * ls + k);
-      r[u] = *reinterpret_cast<const float4*>(Rp + (k + u) * kDLD);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float lu[4] = {l[u].x, l[u].y, l[u].z, l[u].w};
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        acc[u][0] = __fmaf_rn(lu[w], r[w].x, acc[u][0]);
-        acc[u][1] = __fmaf_rn(lu[w], r[w].y, acc[u][1]);
-        acc[u][2] = __fmaf_rn(lu[w], r[w].z, acc[u][2]);
-        acc[u][3] = __fmaf_rn(lu[w], r[w].w, acc[u][3]);
-      }
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-    *reinterpret_cast<float4*>(Op + u * ls) =
-        make_float4(sign * acc[u][0], sign * acc[u][1], sign * acc[u][2], sign * acc[u][3]);
-}
-
 __global__ void __launch_bounds__(kDThreads, 1)
     k_diag_block(int ld, int k0, int nb, float* __restrict__ A, float* __restrict__ uinv,
                  float* __restrict__ linvT, DevErr* err) {
@@ -183,9 +153,9 @@ __global__ void __launch_bounds__(kDThreads, 1)
   float* S = dsm;                  // [128][132]
   float* IL = S + kNB * kDLD;      // inverse of L (unit diagonal stored)
   float* IU = IL + kNB * kDLD;     // inverse of U
-  float* LT = IU + kNB * kDLD;     // [16][132]: L21 of the step, transposed
+  float* LT = IU + kNB * kDLD;     // [16][132]: the step's row solutions (L21, inv(U)), transposed
   float* dinv = LT + kDB * kDLD;   // [128] 1 / u_kk
-  __shared__ __align__(16) float t16[kDB][kDB];  // the step's 16 x 16 inverse of L, transposed
+  __shared__ __align__(16) float t16[kDB][kDB];  // the step's 16 x 16 L, transposed
   __shared__ __align__(16) float prow[2][2 * kDB];  // the pivot row of step A
   __shared__ int bad;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -260,7 +230,10 @@ __global__ void __launch_bounds__(kDThreads, 1)
         const float m = r > k ? c * pi : 0.f;
         mypiv = lane == k ? p : mypiv;
         myinv = lane == k ? pi : myinv;
-        if (lane < 16 && r > k) D[k] = m;
+        if (lane < 16 && r > k) {
+          D[k] = m;
+          t16[k][r] = m;
+        }
         const float last = __fmaf_rn(-m, v[0], a[0]);
 #pragma unroll
         for (int j = 0; j + 1 < kDB; ++j) a[j] = __fmaf_rn(-m, v[j + 1], a[j + 1]);
@@ -275,110 +248,93 @@ __global__ void __launch_bounds__(kDThreads, 1)
       } else {
         float* out = IL + (j0 + r) * kDLD + j0;
 #pragma unroll
-        for (int j = 0; j < kDB; ++j) {
-          out[j] = a[j];
-          t16[j][r] = a[j];
-        }
+        for (int j = 0; j < kDB; ++j) out[j] = a[j];
       }
     }
     __syncthreads();
     const int j1 = j0 + kDB;
-    if (j1 < kNB) {
-      // ---- B
-      if (tid < kNB) {
-        const int row = j1 + tid;
-        if (row < kNB) {
-          float* p = S + row * kDLD + j0;
-          float x[kDB];
-#pragma unroll
-          for (int q = 0; q < kDB; q += 4) {
-            const float4 t = *reinterpret_cast<const float4*>(p + q);
-            x[q] = t.x; x[q + 1] = t.y; x[q + 2] = t.z; x[q + 3] = t.w;
-          }
-#pragma unroll
-          for (int i = 0; i < kDB; ++i) {
-            x[i] *= dinv[j0 + i];
-            const float* u = S + (j0 + i) * kDLD + j0;
-#pragma unroll
-            for (int q = (i + 1) & ~3; q < kDB; q += 4) {
-              const float4 t = *reinterpret_cast<const float4*>(u + q);
-              const float tv[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-              for (int w = 0; w < 4; ++w)
-                if (q + w > i) x[q + w] = __fmaf_rn(-x[i], tv[w], x[q + w]);
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < kDB; q += 4)
-            *reinterpret_cast<float4*>(p + q) = make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]);
-#pragma unroll
-          for (int j = 0; j < kDB; ++j) LT[j * kDLD + row] = x[j];
-        }
-      } else if (tid < 3 * kNB) {
-        // two threads per column, eight of the sixteen rows each
-        const int q = tid - kNB, col = j1 + (q & (kNB - 1)), h = 8 * (q >> 7);
-        float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (col < kNB) {
-#pragma unroll
-          for (int k = 0; k < kDB; ++k) {
-            const float x = S[(j0 + k) * kDLD + col];
-            const float4 t0 = *reinterpret_cast<const float4*>(&t16[k][h]);
-            const float4 t1 = *reinterpret_cast<const float4*>(&t16[k][h + 4]);
-            y[0] = __fmaf_rn(t0.x, x, y[0]);
-            y[1] = __fmaf_rn(t0.y, x, y[1]);
-            y[2] = __fmaf_rn(t0.z, x, y[2]);
-            y[3] = __fmaf_rn(t0.w, x, y[3]);
-            y[4] = __fmaf_rn(t1.x, x, y[4]);
-            y[5] = __fmaf_rn(t1.y, x, y[5]);
-            y[6] = __fmaf_rn(t1.z, x, y[6]);
-            y[7] = __fmaf_rn(t1.w, x, y[7]);
-          }
-        }
-        asm volatile("barrier.sync 1, 256;" ::: "memory");  // both halves have read the column
-        if (col < kNB)
-#pragma unroll
-          for (int i = 0; i < 8; ++i) S[(j0 + h + i) * kDLD + col] = y[i];
-      }
-      __syncthreads();
-    }
-    // ---- C
-    if (warp == 15) {
-      // column `lane` of the inverse of the 16 x 16 block of U, from the last row up
-      const float* U = S + j0 * kDLD + j0;
+    // ---- B
+    if (tid < kNB) {
+      // x U = a; the rows of the lower identity come into play with their own column
+      const int row = tid;
+      float* p = (row >= j1 ? S : IU) + row * kDLD + j0;
       float x[kDB];
 #pragma unroll
-      for (int i = kDB - 1; i >= 0; --i) {
-        float t0 = i == r ? 1.f : 0.f, t1 = 0.f;
-#pragma unroll
-        for (int q = i & ~3; q < kDB; q += 4) {
-          const float4 t = *reinterpret_cast<const float4*>(U + i * kDLD + q);
-          if (q > i) t0 = __fmaf_rn(-t.x, x[q], t0);
-          if (q + 1 > i) t1 = __fmaf_rn(-t.y, x[q + 1], t1);
-          if (q + 2 > i) t0 = __fmaf_rn(-t.z, x[q + 2], t0);
-          if (q + 3 > i) t1 = __fmaf_rn(-t.w, x[q + 3], t1);
-        }
-        x[i] = (t0 + t1) * dinv[j0 + i];
+      for (int q = 0; q < kDB; q += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(p + q);
+        x[q] = t.x; x[q + 1] = t.y; x[q + 2] = t.z; x[q + 3] = t.w;
       }
-      if (lane < 16)
 #pragma unroll
-        for (int i = 0; i < kDB; ++i) IU[(j0 + i) * kDLD + j0 + r] = x[i];
-    } else if (warp >= 1 && j1 < kNB) {
-      const int nt = (kNB - j1) / 4;
-      for (int q = tid - 32; q < nt * nt; q += kDThreads - 64) {
-        const int ti = q / nt, tj = q - ti * nt;
-        if (ti < kDB / 4 && tj < kDB / 4) continue;  // warp 0's
-        const int i = j1 + 4 * ti, j = j1 + 4 * tj;
-        float* c = S + i * kDLD + j;
-        float4 o[4];
+      for (int q = 0; q < kDB; ++q)
+        if (row == j0 + q) x[q] = 1.f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) o[u] = *reinterpret_cast<float4*>(c + u * kDLD);
+      for (int i = 0; i < kDB; ++i) {
+        x[i] *= dinv[j0 + i];
+        const float* u = S + (j0 + i) * kDLD + j0;
+#pragma unroll
+        for (int q = (i + 1) & ~3; q < kDB; q += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(u + q);
+          const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+          for (int w = 0; w < 4; ++w)
+            if (q + w > i) x[q + w] = __fmaf_rn(-x[i], tv[w], x[q + w]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kDB; q += 4)
+        *reinterpret_cast<float4*>(p + q) = make_float4(x[q], x[q + 1], x[q + 2], x[q + 3]);
+#pragma unroll
+      for (int j = 0; j < kDB; ++j) LT[j * kDLD + row] = x[j];
+    } else if (tid < 2 * kNB) {
+      // L y = a, except for the block's own columns (step A)
+      const int col = tid - kNB;
+      if (col < j0 || col >= j1) {
+        float* p = (col < j0 ? IL : S) + j0 * kDLD + col;
+        float y[kDB];
+#pragma unroll
+        for (int i = 0; i < kDB; ++i) y[i] = p[i * kDLD];
+#pragma unroll
+        for (int i = 0; i + 1 < kDB; ++i)
+#pragma unroll
+          for (int q = (i + 1) & ~3; q < kDB; q += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(&t16[i][q]);
+            const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+              if (q + w > i) y[q + w] = __fmaf_rn(-tv[w], y[i], y[q + w]);
+          }
+#pragma unroll
+        for (int i = 1; i < kDB; ++i) p[i * kDLD] = y[i];
+      }
+    }
+    __syncthreads();
+    // ---- C: rows below the block in all columns (inv(L) left of j1, S from
+    // there on), the other rows (inv(U)) from column j1 on
+    if (warp >= 1 && j1 < kNB) {
+      const int nc = (kNB - j1) / 4, below = (kNB - j1) / 8 * (kNB / 4);
+      for (int q = tid - 32; q < below + j1 / 8 * nc; q += kDThreads - 32) {
+        int i, j;
+        if (q < below) {
+          i = j1 + 8 * (q / (kNB / 4));
+          j = 4 * (q % (kNB / 4));
+          if (i < j1 + kDB && j >= j1 && j < j1 + kDB) continue;  // warp 0's
+        } else {
+          i = 8 * ((q - below) / nc);
+          j = j1 + 4 * ((q - below) % nc);
+        }
+        const float* src = (j < j1 ? IL : S) + j0 * kDLD + j;
+        float* c = (i < j1 ? IU : j < j1 ? IL : S) + i * kDLD + j;
+        float4 o[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) o[u] = *reinterpret_cast<float4*>(c + u * kDLD);
 #pragma unroll 4
         for (int k = 0; k < kDB; ++k) {
-          const float4 l = *reinterpret_cast<const float4*>(LT + k * kDLD + i);
-          const float4 t = *reinterpret_cast<const float4*>(S + (j0 + k) * kDLD + j);
-          const float lv[4] = {l.x, l.y, l.z, l.w};
+          const float4 l0 = *reinterpret_cast<const float4*>(LT + k * kDLD + i);
+          const float4 l1 = *reinterpret_cast<const float4*>(LT + k * kDLD + i + 4);
+          const float4 t = *reinterpret_cast<const float4*>(src + k * kDLD);
+          const float lv[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+          for (int u = 0; u < 8; ++u) {
             o[u].x = __fmaf_rn(-lv[u], t.x, o[u].x);
             o[u].y = __fmaf_rn(-lv[u], t.y, o[u].y);
             o[u].z = __fmaf_rn(-lv[u], t.z, o[u].z);
@@ -386,7 +342,7 @@ __global__ void __launch_bounds__(kDThreads, 1)
           }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(c + u * kDLD) = o[u];
+        for (int u = 0; u < 8; ++u) *reinterpret_cast<float4*>(c + u * kDLD) = o[u];
       }
     }
   }
@@ -394,46 +350,6 @@ __global__ void __launch_bounds__(kDThreads, 1)
   if (bad) {
     if (tid == 0) dev_fail(err, WBEM_ERR_SINGULAR, 51, k0, 0);
     return;  // uniform
-  }
-  // ---- inverses by doubling; tiles of 4 x 4, half of the threads on L, half on
-  // U. The triangular factor of a product bounds its k by the tile's column
-  // or row: a warp takes tiles with the same bound fc, the factor U in the
-  // opposite order, so that short and long warps share a scheduler. Bounded by
-  // the column: columns fc .., rows fr + b / 4 u (consecutive lanes, consecutive
-  // rows); by the row: rows fc .., columns 4 fr ...
-#pragma unroll 1
-  for (int b = kDB; b < kNB; b *= 2) {
-    const int sd = b / 4, per = sd * sd, n = per * (kNB / (2 * b));  // tiles per block, per factor
-    const int w = tid < n ? 0 : 1, q = w == 0 ? tid : 2 * n - 1 - tid;
-    const bool on = q >= 0;
-    const int o = on ? 2 * b * (q / per) : 0;
-    const int fr = (on ? q % per : 0) % sd, fc = 4 * ((on ? q % per : 0) / sd);
-    // T_L = L21 IL11 in IU's lower block, T_U = IU11 U12 in IL's upper block
-    if (on) {
-      if (w == 0)
-        diag_tile(S + (o + b + fr) * kDLD + o, IL + o * kDLD + o + fc, IU + (o + b + fr) * kDLD + o + fc, sd,
-                  fc, b, 1.f);
-      else
-        diag_tile(IU + (o + fc) * kDLD + o, S + o * kDLD + o + b + 4 * fr, IL + (o + fc) * kDLD + o + b + 4 * fr,
-                  1, fc, b, 1.f);
-    }
-    __syncthreads();
-    if (on) {
-      if (w == 0)
-        diag_tile(IL + (o + b + fc) * kDLD + o + b, IU + (o + b) * kDLD + o + 4 * fr,
-                  IL + (o + b + fc) * kDLD + o + 4 * fr, 1, 0, fc + 4, -1.f);
-      else
-        diag_tile(IL + (o + fr) * kDLD + o + b, IU + (o + b) * kDLD + o + b + fc,
-                  IU + (o + fr) * kDLD + o + b + fc, sd, 0, fc + 4, -1.f);
-    }
-    __syncthreads();
-    if (2 * b == kNB) break;  // the last products are masked on the way out
-    if (on) {
-      float* t = w == 0 ? IU + (o + b + fc) * kDLD + o + 4 * fr : IL + (o + fc) * kDLD + o + b + 4 * fr;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(t + u * kDLD) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncthreads();
   }
   for (int idx = tid; idx < kNB * kNB / 4; idx += kDThreads) {
     const int rr = idx >> 5, cc = (idx & 31) * 4;
@@ -447,13 +363,11 @@ __global__ void __launch_bounds__(kDThreads, 1)
         for (int u = 0; cc + u < nb; ++u) ap[u] = e[u];
       }
     }
-    float4 x = *reinterpret_cast<const float4*>(IU + rr * kDLD + cc);
-    if (cc + 3 < rr) x = make_float4(0.f, 0.f, 0.f, 0.f);
-    reinterpret_cast<float4*>(uinv)[idx] = x;
+    reinterpret_cast<float4*>(uinv)[idx] = *reinterpret_cast<const float4*>(IU + rr * kDLD + cc);
   }
   // transposed: consecutive lanes read consecutive rows (4 of them share a bank)
   for (int idx = tid; idx < kNB * kNB; idx += kDThreads)
-    linvT[idx] = (idx & (kNB - 1)) >= (idx >> 7) ? IL[(idx & (kNB - 1)) * kDLD + (idx >> 7)] : 0.f;
+    linvT[idx] = IL[(idx & (kNB - 1)) * kDLD + (idx >> 7)];
 }
 
 // The inverses the chain does not read, once per factorisation: linv from
@@ -731,12 +645,13 @@ static cudaError_t run_panel_small(const PanelArgs& pa, const SplitOut& s1, cons
 // 128) per CTA, or subtracted from X; up to two products share a launch. X and
 // Y are given by the strides of their (y, z) and (y, k) elements, so a row
 // panel is computed transposed, and X may overlie Y: a CTA reads its Y first,
-// and no other CTA reads it. 16 CTAs per 128 x 128 block; each of four warps
-// takes a quarter of K (its rows of Z come straight into registers, 16 at a
-// time, so the loads' latency is paid once or twice), the partial sums meet in
-// shared memory (16 KB: fits beside a trailing-update CTA). One launch takes
-// 5.2 us; the 64 x 128 tiles of k_panel_small put such a block on two CTAs
-// and took 13.9 to 15.5 us.
+// and no other CTA reads it. 16 CTAs per 128 x 128 block; a thread holds one
+// column, whose entries of Z come straight into registers, 64 ahead of their
+// use, and eight rows (4 KB of shared memory: fits beside a trailing-update
+// CTA). A product's terms are added in ascending k, in one chain per entry, as
+// k_panel_small does for the rows below (see k_diag_block for why the order
+// counts). One launch takes 5.4 us; the 64 x 128 tiles of k_panel_small put
+// such a block on two CTAs and took 13.9 to 15.5 us.
 struct StripProd {
   const float* Y;
   const float* Z;  // Z(k, z) = Z[k * ldz + z]
@@ -747,8 +662,8 @@ struct StripProd {
   int ny, nz;      // valid y and z
   int sub;         // 1: X -= product, 0: X = product
 };
-constexpr int kStripY = 8, kStripZ = 128, kStripThreads = 128, kStripWarps = kStripThreads / 32;
-constexpr int kStripB = 16;  // rows of Z in registers at a time
+constexpr int kStripY = 8, kStripZ = 128, kStripThreads = kStripZ;
+constexpr int kStripB = 64;  // entries of Z in registers at a time
 
 __host__ __device__ inline int strip_ctas(const StripProd& p) {
   return ((p.ny + kStripY - 1) / kStripY) * ((p.nz + kStripZ - 1) / kStripZ);
@@ -756,33 +671,19 @@ __host__ __device__ inline int strip_ctas(const StripProd& p) {
 
 // n0: CTAs of product p0; the others take p1
 __global__ void __launch_bounds__(kStripThreads) k_strip(StripProd p0, StripProd p1, int n0) {
-  __shared__ __align__(16) float Ys[kNB][kStripY];  // then the last warp's partial sums
-  __shared__ __align__(16) float red[kStripWarps - 1][kStripY][kStripZ];
-  static_assert(kNB * kStripY == kStripY * kStripZ, "the partial sums fit in Ys");
+  __shared__ __align__(16) float Ys[kNB][kStripY];
+  static_assert(kNB % kStripB == 0 && kStripThreads == kNB, "loads of Z and Y");
   const bool first = (int)blockIdx.x < n0;
   const StripProd p = first ? p0 : p1;
   const int t = first ? blockIdx.x : blockIdx.x - n0;
   const int nty = (p.ny + kStripY - 1) / kStripY;
-  const int y0 = (t % nty) * kStripY, z0 = (t / nty) * kStripZ;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int z = z0 + 4 * lane, kw = warp * (kNB / kStripWarps);
-  const bool zfull = z + 3 < p.nz;
-  float4 zr[kStripB];
-  auto load = [&](int k0) {
+  const int y0 = (t % nty) * kStripY;
+  const int tid = threadIdx.x, z = (t / nty) * kStripZ + tid;
+  const bool on = z < p.nz;
+  const float* zp = p.Z + z;
+  float zr[kStripB];
 #pragma unroll
-    for (int k = 0; k < kStripB; ++k) {
-      const float* src = p.Z + (size_t)(k0 + k) * p.ldz + z;
-      if (zfull) {
-        zr[k] = __ldcg(reinterpret_cast<const float4*>(src));
-      } else {
-        zr[k].x = z < p.nz ? src[0] : 0.f;
-        zr[k].y = z + 1 < p.nz ? src[1] : 0.f;
-        zr[k].z = z + 2 < p.nz ? src[2] : 0.f;
-        zr[k].w = 0.f;
-      }
-    }
-  };
-  load(kw);
+  for (int k = 0; k < kStripB; ++k) zr[k] = on ? __ldcg(zp + (size_t)k * p.ldz) : 0.f;
   if (p.yk == 1) {  // rows of K floats
 #pragma unroll
     for (int u = 0; u < kStripY * kNB / 4 / kStripThreads; ++u) {
@@ -805,65 +706,38 @@ __global__ void __launch_bounds__(kStripThreads) k_strip(StripProd p0, StripProd
       for (int y = 0; y < kStripY; ++y) Ys[tid][y] = y0 + y < p.ny ? src[y] : 0.f;
     }
   }
+  float* x = p.X + (size_t)y0 * p.xy + (size_t)z * p.xz;
+  float old[kStripY];  // of a product that is subtracted: X apart from Y and Z
+#pragma unroll
+  for (int y = 0; y < kStripY; ++y) old[y] = p.sub && on && y0 + y < p.ny ? x[(size_t)y * p.xy] : 0.f;
   __syncthreads();
-  float acc[kStripY][4];
+  float acc[kStripY];
 #pragma unroll
-  for (int y = 0; y < kStripY; ++y)
+  for (int y = 0; y < kStripY; ++y) acc[y] = 0.f;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc[y][v] = 0.f;
-#pragma unroll
-  for (int kb = 0; kb < kNB / kStripWarps; kb += kStripB) {
+  for (int kb = 0; kb < kNB; kb += kStripB)
 #pragma unroll
     for (int k = 0; k < kStripB; ++k) {
-      const float4 a = *reinterpret_cast<const float4*>(&Ys[kw + kb + k][0]);
-      const float4 b = *reinterpret_cast<const float4*>(&Ys[kw + kb + k][4]);
-      const float4 w = zr[k];
+      const float4 a = *reinterpret_cast<const float4*>(&Ys[kb + k][0]);
+      const float4 b = *reinterpret_cast<const float4*>(&Ys[kb + k][4]);
+      const float w = zr[k];
+      // the next batch's entry as soon as this one is used
+      if (kb + kStripB < kNB) zr[k] = on ? __ldcg(zp + (size_t)(kb + kStripB + k) * p.ldz) : 0.f;
       const float ya[kStripY] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int y = 0; y < kStripY; ++y) {
-        acc[y][0] = __fmaf_rn(ya[y], w.x, acc[y][0]);
-        acc[y][1] = __fmaf_rn(ya[y], w.y, acc[y][1]);
-        acc[y][2] = __fmaf_rn(ya[y], w.z, acc[y][2]);
-        acc[y][3] = __fmaf_rn(ya[y], w.w, acc[y][3]);
-      }
-      // the next batch's row as soon as this one is used
-      if (kb + kStripB < kNB / kStripWarps) {
-        const float* src = p.Z + (size_t)(kw + kb + kStripB + k) * p.ldz + z;
-        if (zfull) {
-          zr[k] = __ldcg(reinterpret_cast<const float4*>(src));
-        } else {
-          zr[k].x = z < p.nz ? src[0] : 0.f;
-          zr[k].y = z + 1 < p.nz ? src[1] : 0.f;
-          zr[k].z = z + 2 < p.nz ? src[2] : 0.f;
-          zr[k].w = 0.f;
-        }
-      }
+      for (int y = 0; y < kStripY; ++y) acc[y] = __fmaf_rn(ya[y], w, acc[y]);
     }
-  }
-  __syncthreads();  // Ys is read
-  float(*mine)[kStripZ] = warp + 1 < kStripWarps ? red[warp] : reinterpret_cast<float(*)[kStripZ]>(&Ys[0][0]);
+  if (!on) return;
 #pragma unroll
   for (int y = 0; y < kStripY; ++y)
-    *reinterpret_cast<float4*>(&mine[y][4 * lane]) = make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
-  __syncthreads();
-  const float(*last)[kStripZ] = reinterpret_cast<const float(*)[kStripZ]>(&Ys[0][0]);
+    if (p.sub) acc[y] = old[y] - acc[y];
+  if (p.xy == 1 && y0 + kStripY <= p.ny) {  // 8 consecutive floats (rows of X: multiples of 32 floats)
+    reinterpret_cast<float4*>(x)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    reinterpret_cast<float4*>(x)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  } else {
 #pragma unroll
-  for (int u = 0; u < kStripY / kStripWarps; ++u) {
-    const int yl = warp * (kStripY / kStripWarps) + u, y = y0 + yl;
-    if (y >= p.ny) continue;
-    const float4 s0 = *reinterpret_cast<const float4*>(&red[0][yl][4 * lane]);
-    const float4 s1 = *reinterpret_cast<const float4*>(&red[1][yl][4 * lane]);
-    const float4 s2 = *reinterpret_cast<const float4*>(&red[2][yl][4 * lane]);
-    const float4 s3 = *reinterpret_cast<const float4*>(&last[yl][4 * lane]);
-    const float sum[4] = {(s0.x + s1.x) + (s2.x + s3.x), (s0.y + s1.y) + (s2.y + s3.y),
-                          (s0.z + s1.z) + (s2.z + s3.z), (s0.w + s1.w) + (s2.w + s3.w)};
-    float* x = p.X + (size_t)y * p.xy + (size_t)z * p.xz;
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-      if (z + v < p.nz) {
-        float* o = x + (size_t)v * p.xz;
-        *o = p.sub ? *o - sum[v] : sum[v];
-      }
+    for (int y = 0; y < kStripY; ++y)
+      if (y0 + y < p.ny) x[(size_t)y * p.xy] = acc[y];
   }
 }
 
@@ -1338,7 +1212,10 @@ static cudaError_t run_gemm(const GemmMaps& mp, const CUtensorMap& cmap, int cro
 // reading the factor does. An entry is therefore published together with the
 // sweep's number in one 64-bit word, and each of 128 threads polls the word of
 // the entry that it needs: one trip through L2 instead of fence, flag, poll and
-// load. Sums stay in registers until the diagonal block. A CTA has to take a
+// load. A row's running value stays in a register until the diagonal block;
+// the blocks are subtracted from it one by one, in the order of the sweep, and
+// a row of the diagonal block is four chains over every fourth input (the
+// orders are part of the result, see k_diag_block). A CTA has to take a
 // block in no longer than a link: it reads the next block's words before it
 // multiplies the last one, and asks for its tiles three blocks ahead in L2 and
 // one ahead in registers. Per sweep, with flags and shuffled sums per block
@@ -1411,7 +1288,7 @@ __global__ void __launch_bounds__(kTriThreads, 2)
   float* sInv = tsm;               // kNB x kNB: output r of input c at [c * kNB + r]
   float* acc = sInv + kNB * kNB;   // [kNB]
   float* v = acc + kNB;            // [2][kNB]: the block just seen, alternating
-  float* part = v + 2 * kNB;       // [8][kNB]
+  float* part = v + 2 * kNB;       // [4][kNB]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool fwd = (mode == 0 || mode == 2);
   const bool vec4 = (ld & 3) == 0;
@@ -1425,16 +1302,20 @@ __global__ void __launch_bounds__(kTriThreads, 2)
     const float4* Dk = reinterpret_cast<const float4*>(dinv + (size_t)k * kNB * kNB);
     for (int idx = tid; idx < kNB * kNB / 4; idx += kTriThreads)
       reinterpret_cast<float4*>(sInv)[idx] = Dk[idx];
-    if (tid < kNB) acc[tid] = (tid < nb) ? in[k0 + tid] : 0.f;
     const int jbeg = fwd ? 0 : nblk - 1, jend = k, jstep = fwd ? 1 : -1;
     float t[64];
     if (jbeg != jend) {
       const int j0 = jbeg * kNB;
       tri_load(t, mode, LU, ld, k0, nb, j0, min(kNB, N - j0), vec4);
     }
-    // modes 0/1: row warp * 16 + (lane >> 1) of the block (lane pairs hold the
-    // same sum); modes 2/3: column tid % 128, rows of one parity
-    float sum = 0.f;
+    // the running value: modes 0/1 of row warp * 16 + (lane >> 1) of the block
+    // (lane pairs hold the same), modes 2/3 of column tid (tid < 128)
+    const int mine = mode <= 1 ? warp * 16 + (lane >> 1) : tid;
+    float run = mine < nb ? in[k0 + mine] : 0.f;
+    // modes 2/3: the two halves of the last block's product (by parity of the row)
+    auto settle = [&](int half) {
+      if (tid < kNB) run -= part[half * 2 * kNB + tid] + part[half * 2 * kNB + kNB + tid];
+    };
     int buf = 0;
     // the word of the next block, read ahead of its turn: a CTA behind the
     // front of the sweep finds the entry in it and does not poll
@@ -1455,6 +1336,7 @@ __global__ void __launch_bounds__(kTriThreads, 2)
         return;
       }
       const float* vb = v + buf * kNB;
+      if (mode >= 2 && j != jbeg) settle(buf ^ 1);
       const int jn2 = j + jstep, j02 = jn2 * kNB;
       if (tid < kNB && jn2 != jend && j02 + tid < N)
         asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(ahead) : "l"(words + j02 + tid) : "memory");
@@ -1496,7 +1378,7 @@ __global__ void __launch_bounds__(kTriThreads, 2)
               s2[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
         }
-        sum += s2[0] + __shfl_xor_sync(0xffffffffu, s2[0], 1);
+        run -= s2[0] + __shfl_xor_sync(0xffffffffu, s2[0], 1);
       } else {
         // four independent partial sums (the dot product is on the chain)
         const int h = tid >> 7;
@@ -1509,43 +1391,41 @@ __global__ void __launch_bounds__(kTriThreads, 2)
           q3 = __fmaf_rn(t[i + 3], vb[h + 2 * i + 6], q3);
         }
         if (jn2 != jend) tri_load(t, mode, LU, ld, k0, nb, j02, min(kNB, N - j02), vec4);
-        sum += (q0 + q1) + (q2 + q3);
+        part[buf * 2 * kNB + tid] = (q0 + q1) + (q2 + q3);
       }
     }
-    __syncthreads();
     if (mode <= 1) {
-      if ((lane & 1) == 0) acc[warp * 16 + (lane >> 1)] -= sum;
+      if ((lane & 1) == 0) acc[mine] = run;
     } else {
-      part[tid] = sum;
       __syncthreads();
-      if (tid < kNB) acc[tid] -= part[tid] + part[kNB + tid];
+      if (jbeg != jend) settle(buf ^ 1);
+      if (tid < kNB) acc[tid] = run;
     }
     __syncthreads();
-    // diagonal block: warp w takes the inputs 16 w .. 16 w + 15, lane l the
-    // outputs 4 l .. 4 l + 3; lanes whose outputs the triangle leaves out of
-    // these inputs (inverses of L and U^T: outputs above them, of U and L^T:
-    // below) read nothing
+    // diagonal block: warp w takes the inputs w % 4, w % 4 + 4, ... and the
+    // outputs 64 (w / 4) + 2 lane, + 1; the half of the inputs that the
+    // triangle leaves out of all of its outputs is not read (inverses of L and
+    // U^T: inputs beyond the outputs, of U and L^T: inputs before them)
     {
-      float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int c0 = 16 * warp;
-      if (fwd ? 4 * lane + 3 >= c0 : 4 * lane <= c0 + 15) {
+      float2 y = make_float2(0.f, 0.f);
+      const int c = warp & 3, half = warp >> 2;
+      const float* m = sInv + c * kNB + 64 * half + 2 * lane;
+      auto chain = [&](int m0) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float a = acc[c0 + i];
-          const float4 m = reinterpret_cast<const float4*>(sInv + (c0 + i) * kNB)[lane];
-          y.x = __fmaf_rn(m.x, a, y.x);
-          y.y = __fmaf_rn(m.y, a, y.y);
-          y.z = __fmaf_rn(m.z, a, y.z);
-          y.w = __fmaf_rn(m.w, a, y.w);
+        for (int i = 0; i < kNB / 8; ++i) {
+          const float a = acc[4 * (m0 + i) + c];
+          const float2 e = *reinterpret_cast<const float2*>(m + 4 * (m0 + i) * kNB);
+          y.x = __fmaf_rn(e.x, a, y.x);
+          y.y = __fmaf_rn(e.y, a, y.y);
         }
-      }
-      reinterpret_cast<float4*>(part + warp * kNB)[lane] = y;
+      };
+      if (fwd || half == 0) chain(0);
+      if (!fwd || half == 1) chain(kNB / 8);
+      *reinterpret_cast<float2*>(part + c * kNB + 64 * half + 2 * lane) = y;
     }
     __syncthreads();
     if (tid < nb) {
-      float y = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) y += part[w * kNB + tid];
+      const float y = (part[tid] + part[kNB + tid]) + (part[2 * kNB + tid] + part[3 * kNB + tid]);
       const unsigned long long word = ((unsigned long long)epoch << 32) | __float_as_uint(y);
       asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(words + k0 + tid), "l"(word) : "memory");
       out[k0 + tid] = y;
@@ -1630,7 +1510,7 @@ static int tri_sweep(wbem_context* h, LuState& L, int mode, const float* in, flo
   const float* dinv = (mode == 0) ? L.linvT : (mode == 1) ? L.uinvT : (mode == 2) ? L.uinv : L.linv;
   unsigned long long* words = L.words;
   unsigned epoch = ++L.epoch;
-  const size_t smem = (size_t)(kNB * kNB + 11 * kNB) * sizeof(float);
+  const size_t smem = (size_t)(kNB * kNB + 7 * kNB) * sizeof(float);
   // per device: attribute and co-resident grid size on the first sweep there
   static std::atomic<int> grid_of[kMaxDev];
   int dev = 0;
@@ -1769,7 +1649,11 @@ int factor_mixed(wbem_context* h) {
     WB_CU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     WB_CU(cudaStreamCreateWithPriority(&L.s_panel, cudaStreamNonBlocking, hi));
     WB_CU(cudaStreamCreateWithPriority(&L.s_trail, cudaStreamNonBlocking, lo));
-    WB_CU(cudaStreamCreateWithPriority(&L.s_row, cudaStreamNonBlocking, hi < lo ? hi + 1 : hi));
+    // the row panel is needed last, and its launches hold CTA slots beside the
+    // bulk update: above it in priority they delayed both the chain and the
+    // update once a diagonal block took 30 us (32,768 dofs: factorisation 61.5
+    // ms, at the update's priority 57.6; 20,011: 18.9 and 18.8)
+    WB_CU(cudaStreamCreateWithPriority(&L.s_row, cudaStreamNonBlocking, lo));
     WB_CU(cudaStreamCreateWithPriority(&L.s_col2, cudaStreamNonBlocking, hi));
     for (cudaEvent_t* e : {&L.ev_fork, &L.ev_row, &L.ev_trail, &L.ev_join, &L.ev_next_rows, &L.ev_blk,
                            &L.ev_u12, &L.ev_inrow, &L.ev_col2[0], &L.ev_col2[1]})
@@ -1938,7 +1822,7 @@ int factor_mixed(wbem_context* h) {
       WB_CU(cudaEventRecord(L.ev_row, sp));
       WB_CU(cudaStreamWaitEvent(st, L.ev_row, 0));
       // a few SMs stay free for the next panel's diagonal blocks (one
-      // 200 KB CTA each); its panel kernels (13 and 16 KB CTAs) run beside this
+      // 200 KB CTA each); its panel kernels (13 and 4 KB CTAs) run beside this
       // update's CTAs on every SM. The next panel's rows [p1, p2) go first,
       // so that its row panel can start while the rows below are updated.
       const int spare = prof ? 0 : kLookaheadSMs;

@@ -550,25 +550,30 @@ __global__ void __cluster_dims__(kBJCtas, 1, 1) __launch_bounds__(kBJThreads, 4)
           key = (unsigned long long)__double_as_longlong(fabs(colv[lane]));
           rev = __brev((unsigned)pos);
         }
+        // one lane writes: once all rows of the CTA have been pivots every lane
+        // is in the ballot, and the candidate is none (key 0, no row)
         const unsigned top = bj_first(key, rev);
-        if (top >> lane & 1u) best = {key, pos, lane};
+        if (lane == __ffs(top) - 1) best = {key, pos, lane & (kBJRows - 1)};
       }
       __syncthreads();
       // the candidate row scaled by its pivot, 1 / pivot in the pivot's slot:
       // one warp per scheduler scales, 32 columns each
-      if (rl == best.row)
+      const bool have = best.key != 0;  // the same in the whole CTA
+      if (have && rl == best.row)
 #pragma unroll
         for (int m = 0; m < kBJPer; ++m) own[g + kBJGroups * m] = a[m];
-      if (tid == 0) pinv = 1.0 / colv[best.row];
+      if (have && tid == 0) pinv = 1.0 / colv[best.row];
       __syncthreads();
-      if (tid < kBJ) own[tid] = tid == k ? pinv : own[tid] * pinv;
+      if (have && tid < kBJ) own[tid] = tid == k ? pinv : own[tid] * pinv;
       __syncthreads();
       {
         const int dst = tid / 32;  // one warp per destination
-        double2* to = reinterpret_cast<double2*>(cl.map_shared_rank(&cand[par][rank][0], dst));
-        const double2* from = reinterpret_cast<const double2*>(own);
-        to[lane] = from[lane];
-        to[lane + 32] = from[lane + 32];
+        if (have) {
+          double2* to = reinterpret_cast<double2*>(cl.map_shared_rank(&cand[par][rank][0], dst));
+          const double2* from = reinterpret_cast<const double2*>(own);
+          to[lane] = from[lane];
+          to[lane + 32] = from[lane + 32];
+        }
         if (lane == 0) {
           BJCand* ci = cl.map_shared_rank(&cinfo[par][rank], dst);
           *ci = {best.key, best.pos, rank * kBJRows + best.row};

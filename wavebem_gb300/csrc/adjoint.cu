@@ -24,13 +24,6 @@
 #include "kernels.h"
 
 namespace wbem {
-cudaError_t upload_quadrature_force(const QuadTables& t);
-static __constant__ QuadTables c_qa;
-cudaError_t upload_quadrature_adjoint(const QuadTables& t) {
-  cudaError_t e = cudaMemcpyToSymbol(c_qa, &t, sizeof(QuadTables));
-  if (e != cudaSuccess) return e;
-  return upload_quadrature_force(t);
-}
 int ensure_vectors(wbem_context* h, int restart);
 int solve_assembled(wbem_context* h, const double* rhs, double* x, int transpose);
 
@@ -71,7 +64,7 @@ int hull_force_dev(wbem_context* h, const int* hull_cells, int n_hull, const dou
     h->hull_cap = n_hull + 1;
   }
   WB_CU(cudaMemcpyAsync(h->d_hull, hd.data(), sizeof(int4) * n_hull, cudaMemcpyHostToDevice, h->stream));
-  WB_CU(launch_hull_force(n_hull, h->d_hull, h->d_X, U, dir, d_phi, d_dphi, h->d_hull_part, h->stream));
+  WB_CU(launch_hull_force(n_hull, h->d_hull, h->quad, h->d_X, U, dir, d_phi, d_dphi, h->d_hull_part, h->stream));
   WB_CU(cudaMemcpyAsync(force, h->d_hull_part + n_hull, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   WB_CU(cudaStreamSynchronize(h->stream));
   return WBEM_OK;
@@ -108,16 +101,16 @@ constexpr int kAdjChunk = 8;
 constexpr int kPt = 12;
 
 // FP64 point data of regular point q of the panel with dofs d (layout above).
-__device__ __forceinline__ void adj_point(const double* __restrict__ X, int4 d, int q,
-                                          const double* __restrict__ phi,
+__device__ __forceinline__ void adj_point(const PanelRule& c_q, const double* __restrict__ X,
+                                          int4 d, int q, const double* __restrict__ phi,
                                           const double* __restrict__ dn, double* p) {
   const int id[4] = {d.x, d.y, d.z, d.w};
-  const double s = c_qa.gp[q][0], u = c_qa.gp[q][1], w = c_qa.gp[q][2] * kI4P;
+  const double s = c_q.gp[q][0], u = c_q.gp[q][1], w = c_q.gp[q][2] * kI4P;
   const double Ns[4] = {-(1 - u), (1 - u), -u, u};
   const double Nt[4] = {-(1 - s), -s, (1 - s), s};
   double x[3] = {0, 0, 0}, jx[3] = {0, 0, 0}, je[3] = {0, 0, 0}, fp = 0, fn = 0;
   for (int v = 0; v < 4; ++v) {
-    const double nv = c_qa.phi[q][v];
+    const double nv = c_q.phi[q][v];
     for (int e = 0; e < 3; ++e) {
       const double P = X[3 * (size_t)id[v] + e];
       x[e] += nv * P;
@@ -195,14 +188,15 @@ template <int Q1>
 __global__ void k_adj_points(int C, const double* __restrict__ X,
                              const int4* __restrict__ cell_dofs, const double* __restrict__ phi,
                              const double* __restrict__ dn, double* __restrict__ recd,
-                             float4* __restrict__ recf, double* __restrict__ pgeo) {
+                             float4* __restrict__ recf, double* __restrict__ pgeo,
+                             const __grid_constant__ PanelRule c_q) {
   constexpr int NQ = Q1 * Q1;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= C * NQ) return;
   const int cell = t / NQ, q = t - cell * NQ;
   const int4 d = cell_dofs[cell];
   double p[kPt];
-  adj_point(X, d, q, phi, dn, p);
+  adj_point(c_q, X, d, q, phi, dn, p);
   const double c0 = p[4] * p[8] - p[5] * p[7], c1 = p[5] * p[6] - p[3] * p[8],
                c2 = p[3] * p[7] - p[4] * p[6];
   const double rd[kPt] = {p[0], p[1], p[2], c0, c1, c2, p[10], p[11] * p[9], p[11] / p[9], 0.0, 0.0, 0.0};
@@ -303,7 +297,8 @@ __global__ void __launch_bounds__(128)
                const int4* __restrict__ cell_dofs, const double* __restrict__ recd,
                const double* __restrict__ pgeo, const double* __restrict__ lam,
                const double* __restrict__ phi, double* __restrict__ grow_part,
-               double* __restrict__ gcell_part, int cells_per_block) {
+               double* __restrict__ gcell_part, int cells_per_block,
+               const __grid_constant__ PanelRule c_q) {
   constexpr int NQ = Q1 * Q1, kRec = 10;  // record: x, c, w'phi, w'dn |c|, w'dn / |c|
   __shared__ __align__(16) double sp[kAdjChunk][NQ][kRec];
   __shared__ double wmom[4][kAdjChunk][24];
@@ -357,7 +352,7 @@ __global__ void __launch_bounds__(128)
         const double2 A = p2[0], B = p2[1], Cc = p2[2], E = p2[3];
         const double wnoj = sp[k][q][8];
         const double c[3] = {B.y, Cc.x, Cc.y};
-        const double gw = c_qa.gp[q][2];
+        const double gw = c_q.gp[q][2];
         double aR[3] = {0, 0, 0}, ac[3] = {0, 0, 0}, Ks = 0, Kc = 0;
 #pragma unroll
         for (int j = 0; j < kAdjRpt; ++j) {
@@ -385,7 +380,7 @@ __global__ void __launch_bounds__(128)
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-          const double nv = c_qa.phi[q][w];
+          const double nv = c_q.phi[q][w];
 #pragma unroll
           for (int e = 0; e < 3; ++e) {
             v[3 * w + e] = fma(nv, aR[e], v[3 * w + e]);
@@ -430,7 +425,8 @@ __global__ void __launch_bounds__(128, 4)
                      const float4* __restrict__ recf, const double* __restrict__ recd,
                      const double* __restrict__ pgeo, const double* __restrict__ lam,
                      const double* __restrict__ phi, double* __restrict__ grow_part,
-                     double* __restrict__ gcell_part, int cells_per_block) {
+                     double* __restrict__ gcell_part, int cells_per_block,
+                     const __grid_constant__ PanelRule c_q) {
   constexpr int NQ = Q1 * Q1;
   __shared__ __align__(16) float sp[kAdjChunk][NQ][12];
   __shared__ float wmom[4][kAdjChunk][24];
@@ -523,7 +519,7 @@ __global__ void __launch_bounds__(128, 4)
         const float4 B = *reinterpret_cast<const float4*>(p + 4);
         const float wnoj = p[8];
         const float c[3] = {A.w, B.x, B.y};
-        const float gw = c_qa.gpf[q][2];
+        const float gw = c_q.gpf[q][2];
         float aR[3] = {0.f, 0.f, 0.f}, ac[3] = {0.f, 0.f, 0.f}, Ks = 0.f, Kc = 0.f;
 #pragma unroll
         for (int j = 0; j < kAdjRpt; ++j) {
@@ -552,7 +548,7 @@ __global__ void __launch_bounds__(128, 4)
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
-          const float nv = c_qa.phif[q][w];
+          const float nv = c_q.phif[q][w];
 #pragma unroll
           for (int e = 0; e < 3; ++e) {
             v[3 * w + e] = fmaf(nv, aR[e], v[3 * w + e]);
@@ -617,7 +613,7 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll
             for (int i = 0; i < NPT; ++i)
               if (NQ % 16 == 0 || (lane & 15) + 16 * i < NQ)
-                adj_near_point(p[i], c_qa.gp[(lane & 15) + 16 * i][2], xi, li, lpw, aR[i], ac[i], g);
+                adj_near_point(p[i], c_q.gp[(lane & 15) + 16 * i][2], xi, li, lpw, aR[i], ac[i], g);
           }
           // g over the 16 points: component (lane >> 2) & 3 ends on lane & 15 = 0, 4, 8
           const bool h1 = lane & 8, h2 = lane & 4;
@@ -645,8 +641,8 @@ __global__ void __launch_bounds__(128, 4)
           for (int w = 0; w < 4; ++w)
 #pragma unroll
             for (int e = 0; e < 3; ++e) {
-              m64[3 * w + e] = fma(c_qa.phi[q][w], aR[i][e], m64[3 * w + e]);
-              m64[12 + 3 * w + e] = fma(c_qa.phi[q][w], ac[i][e], m64[12 + 3 * w + e]);
+              m64[3 * w + e] = fma(c_q.phi[q][w], aR[i][e], m64[3 * w + e]);
+              m64[12 + 3 * w + e] = fma(c_q.phi[q][w], ac[i][e], m64[12 + 3 * w + e]);
             }
       }
       double n3[3];
@@ -692,7 +688,8 @@ __global__ void __launch_bounds__(32 * kAdjSingWarps)
                    const int* __restrict__ sptr, const int* __restrict__ scell,
                    const int4* __restrict__ cell_dofs, const double* __restrict__ lam,
                    const double* __restrict__ phi, const double* __restrict__ dn,
-                   double* __restrict__ grow_sing, double* __restrict__ gpair) {
+                   const QuadTables* __restrict__ qt, double* __restrict__ grow_sing,
+                   double* __restrict__ gpair) {
   __shared__ double mom[kAdjSingWarps][24], edges[kAdjSingWarps][12], part[kAdjSingWarps][3];
   const int row = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const double xi[3] = {X[3 * (size_t)row], X[3 * (size_t)row + 1], X[3 * (size_t)row + 2]};
@@ -701,6 +698,7 @@ __global__ void __launch_bounds__(32 * kAdjSingWarps)
 #pragma unroll
   for (int k = 0; k < kMaxSet; ++k) set[k] = dnset[(size_t)row * kMaxSet + k];
   double grow = 0.0;  // lanes 0..2: component
+  const int nsp = qt->nsp;
   for (int e = sptr[row] + warp; e < sptr[row + 1]; e += kAdjSingWarps) {
     const int4 d = cell_dofs[scell[e]];
     const int id[4] = {d.x, d.y, d.z, d.w};
@@ -738,8 +736,8 @@ __global__ void __launch_bounds__(32 * kAdjSingWarps)
     double m[24];
 #pragma unroll
     for (int t = 0; t < 24; ++t) m[t] = 0.0;
-    for (int q = lane; q < c_qa.nsp; q += 32) {
-      const double s = c_qa.sp[v][q][0], u = c_qa.sp[v][q][1], w = c_qa.sp[v][q][2] * (kI4P * li);
+    for (int q = lane; q < nsp; q += 32) {
+      const double s = qt->sp[v][q][0], u = qt->sp[v][q][1], w = qt->sp[v][q][2] * (kI4P * li);
       const double N4[4] = {(1 - s) * (1 - u), s * (1 - u), (1 - s) * u, s * u};
       double R[3], jx[3], je[3];
 #pragma unroll
@@ -863,12 +861,12 @@ static cudaError_t launch_adj_tile_t(int N, int C, const double* X, const int* d
                                      const int4* cd, const double* lam, const double* phi,
                                      const double* dn, double* recd, double* pgeo,
                                      double* grow_part, double* gcell_part, int cpb,
-                                     cudaStream_t s) {
+                                     const PanelRule& rule, cudaStream_t s) {
   constexpr int NQ = Q1 * Q1;
-  k_adj_points<Q1><<<(C * NQ + 255) / 256, 256, 0, s>>>(C, X, cd, phi, dn, recd, nullptr, pgeo);
+  k_adj_points<Q1><<<(C * NQ + 255) / 256, 256, 0, s>>>(C, X, cd, phi, dn, recd, nullptr, pgeo, rule);
   dim3 grid((C + cpb - 1) / cpb, (N + kAdjRowsCta - 1) / kAdjRowsCta);
   k_adj_tile<Q1><<<grid, 128, 0, s>>>(N, C, X, dnset, cd, recd, pgeo, lam, phi, grow_part,
-                                      gcell_part, cpb);
+                                      gcell_part, cpb, rule);
   return cudaGetLastError();
 }
 
@@ -877,12 +875,13 @@ static cudaError_t launch_adj_mixed_t(int N, int C, const double* X, const int* 
                                       const int4* cd, const float4* geo, const double* lam,
                                       const double* phi, const double* dn, double* recd,
                                       float4* recf, double* pgeo, double* grow_part,
-                                      double* gcell_part, int cpb, cudaStream_t s) {
+                                      double* gcell_part, int cpb, const PanelRule& rule,
+                                      cudaStream_t s) {
   constexpr int NQ = Q1 * Q1;
-  k_adj_points<Q1><<<(C * NQ + 255) / 256, 256, 0, s>>>(C, X, cd, phi, dn, recd, recf, pgeo);
+  k_adj_points<Q1><<<(C * NQ + 255) / 256, 256, 0, s>>>(C, X, cd, phi, dn, recd, recf, pgeo, rule);
   dim3 grid((C + cpb - 1) / cpb, (N + kAdjRowsCta - 1) / kAdjRowsCta);
   k_adj_tile_mixed<Q1><<<grid, 128, 0, s>>>(N, C, X, dnset, cd, geo, recf, recd, pgeo, lam, phi,
-                                            grow_part, gcell_part, cpb);
+                                            grow_part, gcell_part, cpb, rule);
   return cudaGetLastError();
 }
 
@@ -974,7 +973,7 @@ static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const
     // fields and direct force derivatives
     k_fields<<<nb, bs, 0, h->stream>>>(N, h->d_mask, h->d_sol, h->d_b, phi, dn);
     if (hull_cells) {
-      WB_CU(launch_hull_force_grad(n_hull, hd, h->d_X, U, dir, phi, dn, d_ghull, d_gph, d_gpn, h->stream));
+      WB_CU(launch_hull_force_grad(n_hull, hd, h->quad, h->d_X, U, dir, phi, dn, d_ghull, d_gph, d_gpn, h->stream));
       k_hull_node_sum<<<nb, bs, 0, h->stream>>>(N, h->d_ncptr, h->d_ncent, d_hoc, d_gph, d_gpn, nph, npn);
     } else {
       std::vector<double> dj(2 * (size_t)N);
@@ -1003,24 +1002,24 @@ static int adjoint_run(wbem_context* h, const int* hull_cells, int n_hull, const
     if (mixed) {
       const int4* cd = h->d_cell_dofs;
       switch (q1) {
-        case 2: e = launch_adj_mixed_t<2>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        case 3: e = launch_adj_mixed_t<3>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        case 4: e = launch_adj_mixed_t<4>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        case 5: e = launch_adj_mixed_t<5>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        default: e = launch_adj_mixed_t<6>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->stream); break;
+        case 2: e = launch_adj_mixed_t<2>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        case 3: e = launch_adj_mixed_t<3>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        case 4: e = launch_adj_mixed_t<4>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        case 5: e = launch_adj_mixed_t<5>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        default: e = launch_adj_mixed_t<6>(N, C, h->d_X, h->d_dnset, cd, geo, lamu, phi, dn, recd, recf, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
       }
     } else {
       switch (q1) {
-        case 2: e = launch_adj_tile_t<2>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        case 3: e = launch_adj_tile_t<3>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        case 4: e = launch_adj_tile_t<4>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        case 5: e = launch_adj_tile_t<5>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
-        default: e = launch_adj_tile_t<6>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->stream); break;
+        case 2: e = launch_adj_tile_t<2>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        case 3: e = launch_adj_tile_t<3>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        case 4: e = launch_adj_tile_t<4>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        case 5: e = launch_adj_tile_t<5>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
+        default: e = launch_adj_tile_t<6>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, lamu, phi, dn, recd, pgeo, grow_part, gcell_part, cpb, h->quad, h->stream); break;
       }
     }
     WB_CU(e);
     k_adj_singular<<<N, 32 * kAdjSingWarps, 0, h->stream>>>(N, h->d_X, h->d_dnset, h->d_sptr, h->d_scell,
-                                                        h->d_cell_dofs, lamu, phi, dn, grow_sing, gpair);
+                                                        h->d_cell_dofs, lamu, phi, dn, h->d_quad, grow_sing, gpair);
     k_adj_reduce<<<(3 * N + bs - 1) / bs, bs, 0, h->stream>>>(N, C, n_cb, n_rb, grow_part, grow_sing, gcell_part, gpair,
                                            d_cpptr, d_cpidx, h->d_ncptr, h->d_ncent, d_hoc, d_ghull,
                                            d_out);

@@ -24,8 +24,6 @@
 
 namespace wbem {
 
-static __constant__ QuadTables c_q;
-
 constexpr double kInv4Pi = 0.07957747154594766788;  // 1 / (4 pi)
 
 __device__ __forceinline__ void q1_geometry(const double P[4][3], double xi, double eta,
@@ -46,7 +44,8 @@ __device__ __forceinline__ void q1_geometry(const double P[4][3], double xi, dou
 // Per-cell record: for each regular point q: {x, y, z, JxW/(4 pi), n_x JxW/(4 pi),
 // n_y JxW/(4 pi), n_z JxW/(4 pi), 0}.
 __global__ void k_cell_records_fp64(int C, const double* __restrict__ X,
-                                    const int4* __restrict__ cell_dofs, double* __restrict__ rec) {
+                                    const int4* __restrict__ cell_dofs, double* __restrict__ rec,
+                                    const __grid_constant__ PanelRule c_q) {
   const int nq = c_q.q1 * c_q.q1;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = gid / nq, q = gid % nq;
@@ -74,10 +73,10 @@ __global__ void k_cell_records_fp64(int C, const double* __restrict__ X,
 }
 
 cudaError_t launch_cell_records_fp64(int C, const double* X, const int4* cell_dofs, double* rec,
-                                     int q1, cudaStream_t s) {
-  const long total = (long)C * q1 * q1;
+                                     const PanelRule& rule, cudaStream_t s) {
+  const long total = (long)C * rule.q1 * rule.q1;
   const int bs = 128;
-  k_cell_records_fp64<<<(unsigned)((total + bs - 1) / bs), bs, 0, s>>>(C, X, cell_dofs, rec);
+  k_cell_records_fp64<<<(unsigned)((total + bs - 1) / bs), bs, 0, s>>>(C, X, cell_dofs, rec, rule);
   return cudaGetLastError();
 }
 
@@ -100,7 +99,8 @@ __global__ void __launch_bounds__(kF64Threads)
     k_tile_fp64(int N, const double* __restrict__ X, const int* __restrict__ dnset,
                 const int* __restrict__ tile_ptr, const int2* __restrict__ tile_ent,
                 const int4* __restrict__ cell_dofs, const double* __restrict__ rec,
-                double* __restrict__ Nm, double* __restrict__ Dm, DevErr* err) {
+                double* __restrict__ Nm, double* __restrict__ Dm, DevErr* err,
+                const __grid_constant__ PanelRule c_q) {
   constexpr int NQ = Q1 * Q1;
   constexpr int RECD = NQ * 8;  // doubles per panel record
   constexpr int RT = kRowsF64, CT = kColsPerTileF64, LDA = RT + 1;
@@ -303,11 +303,10 @@ struct FarTables {
   float2 wc;                                             // weight of the centre point
   float2 t[kMaxQ1], w[kMaxQ1], wt[kMaxQ1];               // node, weight, weight * node
 };
-static __constant__ FarTables c_far;
 
 constexpr size_t kFarHeader = 256;  // the scale, before the records
 
-cudaError_t upload_quadrature_fp64(const QuadTables& t) {
+static FarTables far_tables(const PanelRule& t) {
   const int n = t.q1;
   auto pair = [](double x) { return make_float2((float)x, (float)(x - (double)(float)x)); };
   FarTables f{};
@@ -325,8 +324,7 @@ cudaError_t upload_quadrature_fp64(const QuadTables& t) {
       f.wp[n - 1 - b] = pair(w);
     }
   }
-  const cudaError_t e = cudaMemcpyToSymbol(c_far, &f, sizeof(f));
-  return e != cudaSuccess ? e : cudaMemcpyToSymbol(c_q, &t, sizeof(QuadTables));
+  return f;
 }
 
 // lengths are scaled by the power of two that brings the mesh's largest
@@ -396,7 +394,8 @@ __global__ void k_mesh_scale(int n3, const double* __restrict__ X, double* __res
 template <int Q1>
 __global__ void __launch_bounds__(128)
     k_far_records(int C, const double* __restrict__ X, const int4* __restrict__ cell_dofs,
-                  const double* __restrict__ scale, FarRecord<Q1>* __restrict__ out) {
+                  const double* __restrict__ scale, FarRecord<Q1>* __restrict__ out,
+                  const __grid_constant__ PanelRule c_q) {
   constexpr int NQ = Q1 * Q1, G = NQ <= 16 ? 16 : 32, NC = FarRecord<Q1>::NC;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) / G, lane = threadIdx.x % G;
   if (c - (int)(threadIdx.x % 32) / G >= C) return;  // the whole warp
@@ -517,7 +516,8 @@ __global__ void __launch_bounds__(128)
 // the eight sums of a far pair: ln (N) and ld (D), R0 = centre - row
 template <int Q1, bool SECOND>
 __device__ __forceinline__ void far_pair(const FarRecord<Q1>& r, double Rx, double Ry, double Rz,
-                                         double p, float p1, double ln[4], double ld[4]) {
+                                         double p, float p1, const FarTables& c_far, double ln[4],
+                                         double ld[4]) {
   constexpr int NP = Q1 / 2, NC = FarRecord<Q1>::NC;
   // w = 1 / |R0| and its low part: a third-order step from the FP32 root
   float yf;
@@ -692,7 +692,8 @@ __global__ void __launch_bounds__(kFarThreads, 2)
                const int* __restrict__ dnset, const int* __restrict__ tile_ptr,
                const int2* __restrict__ tile_ent, const int4* __restrict__ cell_dofs,
                const FarRecord<Q1>* __restrict__ far, const double* __restrict__ rec,
-               double* __restrict__ Nm, double* __restrict__ Dm, DevErr* err) {
+               double* __restrict__ Nm, double* __restrict__ Dm, DevErr* err,
+               const __grid_constant__ PanelRule c_q, const __grid_constant__ FarTables c_far) {
   using Rec = FarRecord<Q1>;
   constexpr int NQ = Q1 * Q1;
   constexpr int RT = kRowsF64, CT = kColsPerTileF64, LDA = RT + 1;
@@ -807,8 +808,8 @@ __global__ void __launch_bounds__(kFarThreads, 2)
       // one form per warp: both, one after the other, would cost their sum
       const bool second = __any_sync(0xffffffffu, isfar && !(p1 > r.thr1));
       if (isfar) {
-        if (second) far_pair<Q1, true>(r, Rx, Ry, Rz, p, p1, ln, ld);
-        else far_pair<Q1, false>(r, Rx, Ry, Rz, p, p1, ln, ld);
+        if (second) far_pair<Q1, true>(r, Rx, Ry, Rz, p, p1, c_far, ln, ld);
+        else far_pair<Q1, false>(r, Rx, Ry, Rz, p, p1, c_far, ln, ld);
       }
       // the row's four panels mostly share no column (the tile's list is in
       // that order): then all add at once
@@ -894,7 +895,8 @@ template <int Q1>
 static cudaError_t launch_tile_fp64_t(int N, const double* X, const int* dnset, int n_tiles,
                                       const int* tile_ptr, const int2* tile_ent,
                                       const int4* cell_dofs, const double* rec, double* Nm,
-                                      double* Dm, DevErr* err, cudaStream_t s) {
+                                      double* Dm, DevErr* err, const PanelRule& rule,
+                                      cudaStream_t s) {
   constexpr int RECD = Q1 * Q1 * 8;
   const size_t smem = (size_t)2 * kChunk * RECD * 8 +
                       (size_t)2 * kColsPerTileF64 * (kRowsF64 + 1) * 8 +
@@ -904,7 +906,7 @@ static cudaError_t launch_tile_fp64_t(int N, const double* X, const int* dnset, 
   if (e != cudaSuccess) return e;
   dim3 grid(n_tiles, (N + kRowsF64 - 1) / kRowsF64);
   k_tile_fp64<Q1><<<grid, kF64Threads, smem, s>>>(N, X, dnset, tile_ptr, tile_ent, cell_dofs, rec,
-                                                   Nm, Dm, err);
+                                                   Nm, Dm, err, rule);
   return cudaGetLastError();
 }
 
@@ -912,7 +914,8 @@ template <int Q1>
 static cudaError_t launch_tile_far_t(int N, int C, const double* X, const int* dnset, int n_tiles,
                                      const int* tile_ptr, const int2* tile_ent,
                                      const int4* cell_dofs, const double* rec, void* far,
-                                     double* Nm, double* Dm, DevErr* err, cudaStream_t s) {
+                                     double* Nm, double* Dm, DevErr* err, const PanelRule& rule,
+                                     cudaStream_t s) {
   using Rec = FarRecord<Q1>;
   constexpr int G = Q1 * Q1 <= 16 ? 16 : 32, PB = 128 / G;
   const size_t smem = (size_t)2 * kFarChunk * sizeof(Rec) +
@@ -924,10 +927,10 @@ static cudaError_t launch_tile_far_t(int N, int C, const double* X, const int* d
   double* scale = static_cast<double*>(far);
   Rec* recs = reinterpret_cast<Rec*>(static_cast<char*>(far) + kFarHeader);
   k_mesh_scale<<<1, 1024, 0, s>>>(3 * N, X, scale);
-  k_far_records<Q1><<<(C + PB - 1) / PB, 128, 0, s>>>(C, X, cell_dofs, scale, recs);
+  k_far_records<Q1><<<(C + PB - 1) / PB, 128, 0, s>>>(C, X, cell_dofs, scale, recs, rule);
   const unsigned grid = (unsigned)n_tiles * ((N + kRowsF64 - 1) / kRowsF64);
   k_tile_far<Q1><<<grid, kFarThreads, smem, s>>>(N, n_tiles, X, scale, dnset, tile_ptr, tile_ent, cell_dofs,
-                                                 recs, rec, Nm, Dm, err);
+                                                 recs, rec, Nm, Dm, err, rule, far_tables(rule));
   return cudaGetLastError();
 }
 
@@ -945,17 +948,17 @@ size_t far_bytes(int q1, int C) {
   }
 }
 
-cudaError_t launch_tile_fp64(int N, int C, int q1, const double* X, const int* dnset, int n_tiles,
+cudaError_t launch_tile_fp64(int N, int C, const PanelRule& rule, const double* X, const int* dnset, int n_tiles,
                              const int* tile_ptr, const int2* tile_ent, const int4* cell_dofs,
                              const double* rec, void* far, double* Nm, double* Dm, DevErr* err,
                              cudaStream_t s) {
-  switch (q1) {
-    case 1: return launch_tile_fp64_t<1>(N, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, Nm, Dm, err, s);
-    case 2: return launch_tile_fp64_t<2>(N, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, Nm, Dm, err, s);
-    case 3: return launch_tile_far_t<3>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, s);
-    case 4: return launch_tile_far_t<4>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, s);
-    case 5: return launch_tile_far_t<5>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, s);
-    case 6: return launch_tile_far_t<6>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, s);
+  switch (rule.q1) {
+    case 1: return launch_tile_fp64_t<1>(N, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, Nm, Dm, err, rule, s);
+    case 2: return launch_tile_fp64_t<2>(N, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, Nm, Dm, err, rule, s);
+    case 3: return launch_tile_far_t<3>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, rule, s);
+    case 4: return launch_tile_far_t<4>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, rule, s);
+    case 5: return launch_tile_far_t<5>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, rule, s);
+    case 6: return launch_tile_far_t<6>(N, C, X, dnset, n_tiles, tile_ptr, tile_ent, cell_dofs, rec, far, Nm, Dm, err, rule, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -974,8 +977,8 @@ constexpr int kSingWarps = 4, kSingBatch = 32;  // panels whose sums are held at
 __global__ void __launch_bounds__(kSingWarps * 32)
     k_singular_fp64(int N, const double* __restrict__ X, const int* __restrict__ dnset,
                     const int* __restrict__ sptr, const int* __restrict__ scell,
-                    const int4* __restrict__ cell_dofs, double* __restrict__ Nm,
-                    double* __restrict__ Dm, DevErr* err) {
+                    const int4* __restrict__ cell_dofs, const QuadTables* __restrict__ qt,
+                    double* __restrict__ Nm, double* __restrict__ Dm, DevErr* err) {
   __shared__ double sums[kSingBatch][8];
   __shared__ int ids[kSingBatch][4];
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1002,7 +1005,7 @@ __global__ void __launch_bounds__(kSingWarps * 32)
         for (int k = 0; k < 4; ++k)
 #pragma unroll
           for (int c = 0; c < 3; ++c) P[k][c] = X[3 * (size_t)id[k] + c];
-        val = singular_panel(P, x, c_q.sp[v], c_q.nsp, lane);
+        val = singular_panel(P, x, qt->sp[v], qt->nsp, lane);
       }
       if ((lane & 17) == 0) sums[e][(lane >> 1) & 7] = val;
       if (lane < 4) ids[e][lane] = id[lane];
@@ -1017,9 +1020,9 @@ __global__ void __launch_bounds__(kSingWarps * 32)
 }
 
 cudaError_t launch_singular_fp64(int N, const double* X, const int* dnset, const int* sptr,
-                                 const int* scell, const int4* cell_dofs, double* Nm, double* Dm,
-                                 DevErr* err, cudaStream_t s) {
-  k_singular_fp64<<<N, kSingWarps * 32, 0, s>>>(N, X, dnset, sptr, scell, cell_dofs, Nm, Dm, err);
+                                 const int* scell, const int4* cell_dofs, const QuadTables* qt,
+                                 double* Nm, double* Dm, DevErr* err, cudaStream_t s) {
+  k_singular_fp64<<<N, kSingWarps * 32, 0, s>>>(N, X, dnset, sptr, scell, cell_dofs, qt, Nm, Dm, err);
   return cudaGetLastError();
 }
 

@@ -193,6 +193,7 @@ struct wbem_context {
   void* fma_state = nullptr;
   bool fma_geometry_stale = true;
   wbem::QuadTables quad{};  // the quadrature tables of the last set-up
+  wbem::QuadTables* d_quad = nullptr;  // and their device copy
 
   wbem::DevErr* d_err = nullptr;
   int launches = 0;

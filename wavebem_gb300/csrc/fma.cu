@@ -1668,7 +1668,7 @@ int assemble_fma(wbem_context* h, const QuadTables& qt) {
   }
   if (!h->d_alpha) WB_CHK(dev_alloc(h, &h->d_alpha, (size_t)N));
   EvTimer tm(h->stream);
-  WB_CU(launch_cell_records_fp64(C, h->d_X, h->d_cell_dofs, h->d_rec, qt.q1, h->stream));
+  WB_CU(launch_cell_records_fp64(C, h->d_X, h->d_cell_dofs, h->d_rec, qt, h->stream));
   h->stats.t_geometry_ms = tm.ms();
   const int npts = C * nq;
   k_fma_points<<<(npts + 255) / 256, 256, 0, h->stream>>>(npts, nq, F->d_leaf_pan, F->d_pos_leaf,

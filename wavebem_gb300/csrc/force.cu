@@ -13,12 +13,6 @@
 
 namespace wbem {
 
-static __constant__ QuadTables c_qf;
-
-cudaError_t upload_quadrature_force(const QuadTables& t) {
-  return cudaMemcpyToSymbol(c_qf, &t, sizeof(QuadTables));
-}
-
 // Per-point force integrand and its partial derivatives with respect to the
 // 4 panel vertices (12), the 4 nodal phi and the 4 nodal dphi/dn.
 // When grad == nullptr only the value is computed.
@@ -114,7 +108,7 @@ constexpr int kHullLanes = 16;
 __global__ void __launch_bounds__(128)
     k_hull_force(int nh, const int4* __restrict__ hd, const double* __restrict__ X, double U0, double U1,
                  double U2, int dir, const double* __restrict__ phi, const double* __restrict__ dphi,
-                 double* __restrict__ part) {
+                 double* __restrict__ part, const __grid_constant__ PanelRule c_q) {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) / kHullLanes, lane = threadIdx.x % kHullLanes;
   const int4 d = hd[min(c, nh - 1)];
   const int id[4] = {d.x, d.y, d.z, d.w};
@@ -128,10 +122,10 @@ __global__ void __launch_bounds__(128)
   }
   const double U[3] = {U0, U1, U2};
   double F = 0;
-  const int nq = c_qf.q1 * c_qf.q1;
+  const int nq = c_q.q1 * c_q.q1;
   for (int q = lane; q < nq; q += kHullLanes) {
     double v;
-    force_point(P, ph, pn, U, dir, c_qf.gp[q][0], c_qf.gp[q][1], c_qf.gp[q][2], &v, nullptr,
+    force_point(P, ph, pn, U, dir, c_q.gp[q][0], c_q.gp[q][1], c_q.gp[q][2], &v, nullptr,
                 nullptr, nullptr);
     F += v;
   }
@@ -153,12 +147,12 @@ __global__ void k_sum_serial(int n, const double* __restrict__ part, double* __r
   if (threadIdx.x == 0) out[0] = red[0];
 }
 
-cudaError_t launch_hull_force(int nh, const int4* hull_dofs, const double* X, const double* U,
-                              int dir, const double* phi, const double* dphi, double* part,
-                              cudaStream_t s) {
+cudaError_t launch_hull_force(int nh, const int4* hull_dofs, const PanelRule& rule, const double* X,
+                              const double* U, int dir, const double* phi, const double* dphi,
+                              double* part, cudaStream_t s) {
   if (nh > 0)
     k_hull_force<<<(nh * kHullLanes + 127) / 128, 128, 0, s>>>(nh, hull_dofs, X, U[0], U[1], U[2], dir,
-                                                               phi, dphi, part);
+                                                               phi, dphi, part, rule);
   k_sum_serial<<<1, 256, 0, s>>>(nh, part, part + nh);
   return cudaGetLastError();
 }
@@ -169,7 +163,8 @@ __global__ void __launch_bounds__(128)
     k_hull_force_grad(int nh, const int4* __restrict__ hd, const double* __restrict__ X, double U0,
                       double U1, double U2, int dir, const double* __restrict__ phi,
                       const double* __restrict__ dphi, double* __restrict__ gX,
-                      double* __restrict__ gph, double* __restrict__ gpn) {
+                      double* __restrict__ gph, double* __restrict__ gpn,
+                      const __grid_constant__ PanelRule c_q) {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) / kHullLanes, lane = threadIdx.x % kHullLanes;
   const int4 d = hd[min(c, nh - 1)];
   const int id[4] = {d.x, d.y, d.z, d.w};
@@ -183,10 +178,10 @@ __global__ void __launch_bounds__(128)
   }
   const double U[3] = {U0, U1, U2};
   double gP[4][3] = {}, g1[4] = {}, g2[4] = {};
-  const int nq = c_qf.q1 * c_qf.q1;
+  const int nq = c_q.q1 * c_q.q1;
   for (int q = lane; q < nq; q += kHullLanes) {
     double v;
-    force_point(P, ph, pn, U, dir, c_qf.gp[q][0], c_qf.gp[q][1], c_qf.gp[q][2], &v, gP, g1, g2);
+    force_point(P, ph, pn, U, dir, c_q.gp[q][0], c_q.gp[q][1], c_q.gp[q][2], &v, gP, g1, g2);
   }
   auto sum = [](double v) {
 #pragma unroll
@@ -210,13 +205,13 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-cudaError_t launch_hull_force_grad(int nh, const int4* hull_dofs, const double* X,
-                                   const double* U, int dir, const double* phi, const double* dphi,
-                                   double* gX_cell, double* gphi_cell, double* gdphi_cell,
-                                   cudaStream_t s) {
+cudaError_t launch_hull_force_grad(int nh, const int4* hull_dofs, const PanelRule& rule,
+                                   const double* X, const double* U, int dir, const double* phi,
+                                   const double* dphi, double* gX_cell, double* gphi_cell,
+                                   double* gdphi_cell, cudaStream_t s) {
   if (nh > 0)
     k_hull_force_grad<<<(nh * kHullLanes + 127) / 128, 128, 0, s>>>(
-        nh, hull_dofs, X, U[0], U[1], U[2], dir, phi, dphi, gX_cell, gphi_cell, gdphi_cell);
+        nh, hull_dofs, X, U[0], U[1], U[2], dir, phi, dphi, gX_cell, gphi_cell, gdphi_cell, rule);
   return cudaGetLastError();
 }
 

@@ -29,30 +29,33 @@ struct ChunkMeta {
   float4 geo;
 };
 
-// quadrature tables (constant memory, per translation unit that uses them)
-struct QuadTables {
+// A handle's quadrature rules. The kernels take the regular rule as a parameter
+// (__grid_constant__: constant memory that belongs to the launch) and the
+// singular rules from the handle's device copy of the tables, so that handles
+// with other rules, in this thread or another, do not meet in them.
+struct PanelRule {
   int q1;                            // regular order per direction
-  int nsp;                           // points of each vertex-singular rule
   double gp[kMaxQ1 * kMaxQ1][3];     // regular rule: xi, eta, w
   double phi[kMaxQ1 * kMaxQ1][4];    // shape values at the regular points
-  double sp[4][kMaxSingular][3];     // singular rules per vertex: xi, eta, w
   float gpf[kMaxQ1 * kMaxQ1][3];     // FP32 copies of gp / phi
   float phif[kMaxQ1 * kMaxQ1][4];
 };
-
-cudaError_t upload_quadrature(const QuadTables& t);
+struct QuadTables : PanelRule {
+  int nsp;                           // points of each vertex-singular rule
+  double sp[4][kMaxSingular][3];     // singular rules per vertex: xi, eta, w
+};
 
 // ---- assembly (FP64 plain form)
 cudaError_t launch_cell_records_fp64(int C, const double* X, const int4* cell_dofs, double* rec,
-                                     int q1, cudaStream_t s);
+                                     const PanelRule& rule, cudaStream_t s);
 size_t far_bytes(int q1, int C);  // scratch of launch_tile_fp64 (may be 0)
-cudaError_t launch_tile_fp64(int N, int C, int q1, const double* X, const int* dnset, int n_tiles,
+cudaError_t launch_tile_fp64(int N, int C, const PanelRule& rule, const double* X, const int* dnset, int n_tiles,
                              const int* tile_ptr, const int2* tile_ent, const int4* cell_dofs,
                              const double* rec, void* far, double* Nm, double* Dm, DevErr* err,
                              cudaStream_t s);
 cudaError_t launch_singular_fp64(int N, const double* X, const int* dnset, const int* sptr,
-                                 const int* scell, const int4* cell_dofs, double* Nm, double* Dm,
-                                 DevErr* err, cudaStream_t s);
+                                 const int* scell, const int4* cell_dofs, const QuadTables* qt,
+                                 double* Nm, double* Dm, DevErr* err, cudaStream_t s);
 cudaError_t launch_alpha_rowsum(int N, const double* Nm, double* alpha, cudaStream_t s);
 
 // ---- assembly (mixed form): A2 / B2 hold the selected (hi, lo) float pairs
@@ -134,12 +137,12 @@ cudaError_t launch_gather_rows(int N, int r0, int nr, const int* ip, const doubl
                                cudaStream_t s);
 
 // hull force and adjoint
-cudaError_t launch_hull_force(int nh, const int4* hull_dofs, const double* X, const double* U,
-                              int dir, const double* phi, const double* dphi, double* part,
-                              cudaStream_t s);
-cudaError_t launch_hull_force_grad(int nh, const int4* hull_dofs, const double* X,
-                                   const double* U, int dir, const double* phi, const double* dphi,
-                                   double* gX_cell, double* gphi_cell, double* gdphi_cell,
-                                   cudaStream_t s);
+cudaError_t launch_hull_force(int nh, const int4* hull_dofs, const PanelRule& rule, const double* X,
+                              const double* U, int dir, const double* phi, const double* dphi,
+                              double* part, cudaStream_t s);
+cudaError_t launch_hull_force_grad(int nh, const int4* hull_dofs, const PanelRule& rule,
+                                   const double* X, const double* U, int dir, const double* phi,
+                                   const double* dphi, double* gX_cell, double* gphi_cell,
+                                   double* gdphi_cell, cudaStream_t s);
 
 }  // namespace wbem

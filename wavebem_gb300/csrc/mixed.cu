@@ -24,11 +24,6 @@
 
 namespace wbem {
 
-static __constant__ QuadTables c_qm;
-cudaError_t upload_quadrature_mixed(const QuadTables& t) {
-  return cudaMemcpyToSymbol(c_qm, &t, sizeof(QuadTables));
-}
-
 constexpr double kInv4PiM = 0.07957747154594766788;
 
 // Panel record: 20 floats per pair of points (2 p, 2 p + 1), the nine values of
@@ -93,7 +88,8 @@ constexpr int kRecPoints = 36;  // most points of the mixed form's rule (order 6
 template <bool HALF>
 __global__ void __launch_bounds__(kRecWarps * 32)
     k_cell_records_mixed(int C, const double* __restrict__ X, const int4* __restrict__ cell_dofs,
-                         float* __restrict__ rec, float4* __restrict__ cellgeo, float ratio) {
+                         float* __restrict__ rec, float4* __restrict__ cellgeo, float ratio,
+                         const __grid_constant__ PanelRule c_q) {
   constexpr int W = HALF ? 16 : 32, kPts = HALF ? 16 : kRecPoints;
   // per panel and point: offset from the centre, cross product, its norm
   __shared__ double s_pt[kRecWarps * (32 / W)][7][kPts];
@@ -101,7 +97,7 @@ __global__ void __launch_bounds__(kRecWarps * 32)
   const int c0 = blockIdx.x * (kRecWarps * 32 / W) + slot;
   const int c = min(c0, C - 1);  // past the last panel: its work again, not written
   double(*pt)[kPts] = s_pt[slot];
-  const int nq = c_qm.q1 * c_qm.q1;
+  const int nq = c_q.q1 * c_q.q1;
   const int RF = mixed_rec_floats(nq);
   const int4 d = cell_dofs[c];
   const int id[4] = {d.x, d.y, d.z, d.w};
@@ -115,7 +111,7 @@ __global__ void __launch_bounds__(kRecWarps * 32)
   for (int e = 0; e < 3; ++e) cen[e] = 0.25 * (P[0][e] + P[1][e] + P[2][e] + P[3][e]);
   for (int q = lane; q < nq; q += W) {
     double x[3], cr[3];
-    q1_geo(P, c_qm.gp[q][0], c_qm.gp[q][1], x, cr);
+    q1_geo(P, c_q.gp[q][0], c_q.gp[q][1], x, cr);
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
       pt[e][q] = x[e] - cen[e];
@@ -129,8 +125,8 @@ __global__ void __launch_bounds__(kRecWarps * 32)
   if (lane < 7) {
     const double* a = lane < 3 ? pt[3 + lane] : pt[6];
     for (int q = 0; q < nq; ++q) {
-      const double w = c_qm.gp[q][2];
-      sum += lane < 3 ? a[q] * w : c_qm.phi[q][max(lane - 3, 0)] * (a[q] * w * kInv4PiM);
+      const double w = c_q.gp[q][2];
+      sum += lane < 3 ? a[q] * w : c_q.phi[q][max(lane - 3, 0)] * (a[q] * w * kInv4PiM);
     }
   }
   double nu[3], M[4];
@@ -159,7 +155,7 @@ __global__ void __launch_bounds__(kRecWarps * 32)
                          -(float)(n[1] - nu[1]),
                          -(float)(n[2] - nu[2]),
                          -(float)(del[0] * n[0] + del[1] * n[1] + del[2] * n[2]),
-                         (float)(det * c_qm.gp[q][2] * kInv4PiM),
+                         (float)(det * c_q.gp[q][2] * kInv4PiM),
                          0.f};
     float* rp = r + (q >> 1) * kPairFloats + (q & 1);
 #pragma unroll
@@ -236,7 +232,7 @@ __global__ void __launch_bounds__(kRowsPerTile)
                  const int4* __restrict__ cell_dofs, const float* __restrict__ rec,
                  const float4* __restrict__ cellgeo, float2* __restrict__ A2,
                  float2* __restrict__ B2, double* __restrict__ alpha_part, SysOut so,
-                 DevErr* err) {
+                 DevErr* err, const __grid_constant__ PanelRule c_q) {
   constexpr int NQ = Q1 * Q1;
   constexpr int RF = mixed_rec_floats(NQ);
   constexpr int RT = kRowsPerTile, CT = kColsPerTile, LDA = RT + 1;
@@ -416,13 +412,13 @@ __global__ void __launch_bounds__(kRowsPerTile)
         for (int h = 0; h < 2; ++h) {
           const int q = 2 * p + h;
           if (q >= NQ) break;
-          const float xa = c_qm.gpf[q][0];
+          const float xa = c_q.gpf[q][0];
           st = __fadd_rn(st, fs[h]);
           s1 = __fmaf_rn(fs[h], xa, s1);
           nt = __fadd_rn(nt, fn[h]);
           n1 = __fmaf_rn(fn[h], xa, n1);
           if ((q + 1) % Q1) continue;
-          const float eb = c_qm.gpf[q][1];
+          const float eb = c_q.gpf[q][1];
           const float s0 = st - s1, n0 = nt - n1;
           ls0 = __fmaf_rn(s0, 1.f - eb, ls0);
           ls1 = __fmaf_rn(s1, 1.f - eb, ls1);
@@ -491,7 +487,8 @@ static cudaError_t launch_tile_mixed_t(int N, const double* X, const int* dnset,
                                        const int* tile_ptr, const int2* tile_ent,
                                        const int4* cell_dofs, const float* rec,
                                        const float4* cellgeo, float2* A2, float2* B2,
-                                       double* alpha_part, SysOut so, DevErr* err, cudaStream_t s) {
+                                       double* alpha_part, SysOut so, DevErr* err,
+                                       const PanelRule& rule, cudaStream_t s) {
   constexpr int RF = mixed_rec_floats(Q1 * Q1);
   const size_t acc = (size_t)kColsPerTile * (kRowsPerTile + 1);
   const size_t smem = (size_t)2 * kChunkM * RF * 4 + 4 * acc * 4 + 16 +
@@ -501,7 +498,7 @@ static cudaError_t launch_tile_mixed_t(int N, const double* X, const int* dnset,
   if (e != cudaSuccess) return e;
   dim3 grid(n_tiles, (N + kRowsPerTile - 1) / kRowsPerTile);
   k_tile_mixed<Q1><<<grid, kRowsPerTile, smem, s>>>(N, X, dnset, tile_ptr, tile_ent, cell_dofs, rec,
-                                                    cellgeo, A2, B2, alpha_part, so, err);
+                                                    cellgeo, A2, B2, alpha_part, so, err, rule);
   return cudaGetLastError();
 }
 
@@ -660,7 +657,7 @@ __global__ void __launch_bounds__(256)
                  const double* __restrict__ rec64, int* __restrict__ item_cnt,
                  int* __restrict__ item_dof, double2* __restrict__ item_val,
                  double* __restrict__ alpha_near, const int* __restrict__ ncnt,
-                 const int* __restrict__ nlist, DevErr* err) {
+                 const int* __restrict__ nlist, DevErr* err, const __grid_constant__ PanelRule c_q) {
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= N) return;
@@ -669,7 +666,7 @@ __global__ void __launch_bounds__(256)
   int set[kMaxSet];
 #pragma unroll
   for (int k = 0; k < kMaxSet; ++k) set[k] = dnset[(size_t)row * kMaxSet + k];
-  const int nq = c_qm.q1 * c_qm.q1;
+  const int nq = c_q.q1 * c_q.q1;
   constexpr int W = HALF ? 16 : 32;
   const int q0 = lane & (W - 1), half = HALF ? lane >> 4 : 0;
   // the lane that holds component j of a panel's sums writes it once
@@ -678,7 +675,7 @@ __global__ void __launch_bounds__(256)
   double ph[4] = {0, 0, 0, 0};
   if (HALF && q0 < nq)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) ph[k] = c_qm.phi[q0][k];
+    for (int k = 0; k < 4; ++k) ph[k] = c_q.phi[q0][k];
   double asum = 0.0;
   int nitem = 0;
   double* vals = reinterpret_cast<double*>(item_val + (size_t)row * kItemCap);
@@ -719,8 +716,8 @@ __global__ void __launch_bounds__(256)
             v[k] = dq * ph[k];
             v[4 + k] = sq * ph[k];
           } else {
-            v[k] = fma(dq, c_qm.phi[q][k], v[k]);
-            v[4 + k] = fma(sq, c_qm.phi[q][k], v[4 + k]);
+            v[k] = fma(dq, c_q.phi[q][k], v[k]);
+            v[4 + k] = fma(sq, c_q.phi[q][k], v[4 + k]);
           }
         }
       }
@@ -758,9 +755,9 @@ constexpr int kSingWarpsM = 4;
 __global__ void __launch_bounds__(kSingWarpsM * 32)
     k_singular_mixed(int N, const double* __restrict__ X, const int* __restrict__ dnset,
                      const int* __restrict__ sptr, const int* __restrict__ scell,
-                     const int4* __restrict__ cell_dofs, int* __restrict__ item_cnt,
-                     int* __restrict__ item_dof, double2* __restrict__ item_val,
-                     double* __restrict__ alpha_sing, DevErr* err) {
+                     const int4* __restrict__ cell_dofs, const QuadTables* __restrict__ qt,
+                     int* __restrict__ item_cnt, int* __restrict__ item_dof,
+                     double2* __restrict__ item_val, double* __restrict__ alpha_sing, DevErr* err) {
   __shared__ double s_alpha[kSingWarpsM];
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double x[3] = {X[3 * (size_t)row], X[3 * (size_t)row + 1], X[3 * (size_t)row + 2]};
@@ -788,7 +785,7 @@ __global__ void __launch_bounds__(kSingWarpsM * 32)
       for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int c = 0; c < 3; ++c) P[k][c] = X[3 * (size_t)id[k] + c];
-      s = singular_panel(P, x, c_qm.sp[v], c_qm.nsp, lane);
+      s = singular_panel(P, x, qt->sp[v], qt->nsp, lane);
     }
     if ((lane & 17) == 0) {
       const int it = 4 * e + (j & 3);
@@ -877,14 +874,14 @@ int assemble_mixed(wbem_context* h) {
   CHKM(dev_alloc(h, &h->d_rec, (size_t)C * nq * 8));
   h->rec_cells = (size_t)C * nq;
   EvTimer tm(h->stream);
-  CUM(launch_cell_records_fp64(C, h->d_X, h->d_cell_dofs, h->d_rec, q1, h->stream));
+  CUM(launch_cell_records_fp64(C, h->d_X, h->d_cell_dofs, h->d_rec, h->quad, h->stream));
   float4* geo_w = reinterpret_cast<float4*>(h->d_cellgeo);
   if (nq <= 16)
     k_cell_records_mixed<true><<<(C + 2 * kRecWarps - 1) / (2 * kRecWarps), kRecWarps * 32, 0, h->stream>>>(
-        C, h->d_X, h->d_cell_dofs, h->d_rec32, geo_w, (float)o.near_field_ratio);
+        C, h->d_X, h->d_cell_dofs, h->d_rec32, geo_w, (float)o.near_field_ratio, h->quad);
   else
     k_cell_records_mixed<false><<<(C + kRecWarps - 1) / kRecWarps, kRecWarps * 32, 0, h->stream>>>(
-        C, h->d_X, h->d_cell_dofs, h->d_rec32, geo_w, (float)o.near_field_ratio);
+        C, h->d_X, h->d_cell_dofs, h->d_rec32, geo_w, (float)o.near_field_ratio, h->quad);
   CUM(cudaGetLastError());
   h->stats.t_geometry_ms = tm.ms();
   const float4* geo = reinterpret_cast<const float4*>(h->d_cellgeo);
@@ -936,26 +933,26 @@ int assemble_mixed(wbem_context* h) {
     if (nq <= 16)
       k_near_mixed<true><<<nwb, 256, 0, ax>>>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, geo, h->d_rec,
                                               h->d_item_cnt, h->d_item_dof, h->d_item_val,
-                                              h->d_alpha_near, h->d_near_cnt, h->d_near_cells, h->d_err);
+                                              h->d_alpha_near, h->d_near_cnt, h->d_near_cells, h->d_err, h->quad);
     else
       k_near_mixed<false><<<nwb, 256, 0, ax>>>(N, C, h->d_X, h->d_dnset, h->d_cell_dofs, geo, h->d_rec,
                                                h->d_item_cnt, h->d_item_dof, h->d_item_val,
                                                h->d_alpha_near, h->d_near_cnt, h->d_near_cells,
-                                               h->d_err);
+                                               h->d_err, h->quad);
     CUM(cudaGetLastError());
     k_singular_mixed<<<N, kSingWarpsM * 32, 0, ax>>>(N, h->d_X, h->d_dnset, h->d_sptr, h->d_scell,
-                                                     h->d_cell_dofs, h->d_item_cnt, h->d_item_dof,
+                                                     h->d_cell_dofs, h->d_quad, h->d_item_cnt, h->d_item_dof,
                                                      h->d_item_val, h->d_alpha_sing, h->d_err);
     CUM(cudaGetLastError());
     CUM(cudaEventRecord(h->ev_aux_join, ax));
   }
   cudaError_t e;
   switch (q1) {
-    case 2: e = launch_tile_mixed_t<2>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->stream); break;
-    case 3: e = launch_tile_mixed_t<3>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->stream); break;
-    case 4: e = launch_tile_mixed_t<4>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->stream); break;
-    case 5: e = launch_tile_mixed_t<5>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->stream); break;
-    default: e = launch_tile_mixed_t<6>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->stream); break;
+    case 2: e = launch_tile_mixed_t<2>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->quad, h->stream); break;
+    case 3: e = launch_tile_mixed_t<3>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->quad, h->stream); break;
+    case 4: e = launch_tile_mixed_t<4>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->quad, h->stream); break;
+    case 5: e = launch_tile_mixed_t<5>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->quad, h->stream); break;
+    default: e = launch_tile_mixed_t<6>(N, h->d_X, h->d_dnset, h->n_tiles, h->d_tile_ptr, h->d_tile_ent, h->d_cell_dofs, h->d_rec32, geo, h->d_A2, h->d_B2, h->d_alpha_part, so, h->d_err, h->quad, h->stream); break;
   }
   CUM(e);
   h->stats.t_assemble_ms = tm.ms();

@@ -22,9 +22,6 @@
 using namespace wbem;
 
 namespace wbem {
-cudaError_t upload_quadrature_fp64(const QuadTables& t);
-cudaError_t upload_quadrature_mixed(const QuadTables& t);
-cudaError_t upload_quadrature_adjoint(const QuadTables& t);
 int solve_mixed(wbem_context* h, const double* d_rhs, double* d_x, int transpose);
 void free_lu(wbem_context* h);
 int assemble_mixed(wbem_context* h);
@@ -80,7 +77,8 @@ static int build_quadrature(wbem_context* h, int q1, int sorder) {
   if (q1 < 1 || q1 > kMaxQ1) return fail(h, WBEM_ERR_ARG, "quadrature_order must be in [1,8]");
   if (sorder < 1 || 2 * sorder * sorder > kMaxSingular)
     return fail(h, WBEM_ERR_ARG, "singular_quadrature_order must be in [1,8]");
-  QuadTables t{};
+  QuadTables t;
+  std::memset(&t, 0, sizeof t);  // padding too: compared as bytes below
   t.q1 = q1;
   std::vector<double> x, w;
   quad::gauss_legendre01(q1, x, w);
@@ -116,10 +114,15 @@ static int build_quadrature(wbem_context* h, int q1, int sorder) {
       t.sp[v][k][2] = pw[k];
     }
   }
-  CU(upload_quadrature_fp64(t));
-  CU(upload_quadrature_mixed(t));
-  CU(upload_quadrature_adjoint(t));
-  h->quad = t;
+  // the device copy changes with the rule alone
+  if (!h->d_quad) {
+    CHK(dev_alloc(h, &h->d_quad, (size_t)1));
+  } else if (std::memcmp(&t, &h->quad, sizeof t) == 0) {
+    return WBEM_OK;
+  }
+  h->quad.q1 = 0;  // no tables, should the copy fail
+  CU(copy_sync(h, h->d_quad, &t, sizeof t, cudaMemcpyHostToDevice));
+  std::memcpy(&h->quad, &t, sizeof t);
   return WBEM_OK;
 }
 
@@ -918,6 +921,7 @@ int wbem_destroy(wbem_handle h) {
   cudaSetDevice(h->device);
   release_mesh_buffers(h);
   if (h->d_err) cudaFree(h->d_err);
+  if (h->d_quad) cudaFree(h->d_quad);
   if (h->aux_stream) cudaStreamDestroy(h->aux_stream);
   if (h->ev_aux_fork) cudaEventDestroy(h->ev_aux_fork);
   if (h->ev_aux_join) cudaEventDestroy(h->ev_aux_join);
@@ -1105,7 +1109,7 @@ int wbem_assemble(wbem_handle h, const wbem_options* opt) {
       CHK(dev_alloc(h, &h->d_rec, (size_t)h->C * nq * 8));
       h->rec_cells = (size_t)h->C * nq;
     }
-    CU(launch_cell_records_fp64(h->C, h->d_X, h->d_cell_dofs, h->d_rec, o.quadrature_order, h->stream));
+    CU(launch_cell_records_fp64(h->C, h->d_X, h->d_cell_dofs, h->d_rec, h->quad, h->stream));
     h->stats.t_geometry_ms = tm.ms();
     const size_t fb = far_bytes(o.quadrature_order, h->C);
     if (fb > h->far_size) {
@@ -1113,11 +1117,11 @@ int wbem_assemble(wbem_handle h, const wbem_options* opt) {
       CHK(dev_alloc(h, &h->d_far, fb));
       h->far_size = fb;
     }
-    CU(launch_tile_fp64(N, h->C, o.quadrature_order, h->d_X, h->d_dnset, h->n_tiles64,
+    CU(launch_tile_fp64(N, h->C, h->quad, h->d_X, h->d_dnset, h->n_tiles64,
                         h->d_tile_ptr64, h->d_tile_ent64, h->d_cell_dofs, h->d_rec, h->d_far,
                         h->d_N, h->d_D, h->d_err, h->stream));
     h->stats.t_assemble_ms = tm.ms();
-    CU(launch_singular_fp64(N, h->d_X, h->d_dnset, h->d_sptr, h->d_scell, h->d_cell_dofs, h->d_N,
+    CU(launch_singular_fp64(N, h->d_X, h->d_dnset, h->d_sptr, h->d_scell, h->d_cell_dofs, h->d_quad, h->d_N,
                             h->d_D, h->d_err, h->stream));
     h->stats.t_singular_ms = tm.ms();
     CU(launch_alpha_rowsum(N, h->d_N, h->d_alpha, h->stream));

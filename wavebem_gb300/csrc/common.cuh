@@ -111,16 +111,19 @@ __device__ __forceinline__ bool flag_wait_bounded(const unsigned* flag, unsigned
 
 // Barrier of all CTAs of a cooperative launch: the counter has reached target
 // (the launch's arrivals so far) in every CTA. A bounded wait; `where` names
-// the barrier in the error word.
-__device__ __forceinline__ void grid_barrier(unsigned* ctr, unsigned target, int where, DevErr* err) {
+// the barrier in the error word. False (in the whole CTA) if it gave up: the
+// kernel ends then.
+__device__ __forceinline__ bool grid_barrier(unsigned* ctr, unsigned target, int where, DevErr* err) {
+  bool ok = true;
   __syncthreads();
   if (threadIdx.x == 0) {
     // release: this CTA's writes (ordered before by the CTA barrier) are seen
     // by whoever acquires the count
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
-    if (!flag_wait_bounded(ctr, target, err)) dev_fail(err, WBEM_ERR_TIMEOUT, where, blockIdx.x, (int)target);
+    ok = flag_wait_bounded(ctr, target, err);
+    if (!ok) dev_fail(err, WBEM_ERR_TIMEOUT, where, blockIdx.x, (int)target);
   }
-  __syncthreads();
+  return !__syncthreads_or(!ok);
 }
 
 // 1-D bulk copy global -> shared (TMA engine), completion counted on `bar`.

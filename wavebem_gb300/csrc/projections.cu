@@ -198,13 +198,14 @@ __global__ void __launch_bounds__(kProjThreads)
   unsigned target = 0;
   int slot = 0;  // the sums of successive barriers use part in turn
   // totals over all CTAs of the component's two per-thread sums
+  // (false: the barrier gave up, and the kernel ends)
   auto total2 = [&](double a, double b, double* ta, double* tb) {
     proj_warp_sum2(a, b, lane);
     double* pp = part + ((size_t)slot * 6 + 2 * d) * G;
     slot ^= 1;
     if (lane < 2) pp[(size_t)lane * G + g] = lane ? b : a;
     target += (unsigned)G;
-    grid_barrier(ctr, target, 62, err);
+    if (!grid_barrier(ctr, target, 62, err)) return false;
     a = b = 0.0;
     for (int q = lane; q < G; q += 32) {
       a += __ldcg(pp + q);
@@ -213,6 +214,7 @@ __global__ void __launch_bounds__(kProjThreads)
     proj_warp_sum2(a, b, lane);
     *ta = a;
     *tb = b;
+    return true;
   };
   // the lane's row in the ONE form
   const int row = i0 + lane;
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__(kProjThreads)
       s1 = fma(b, v.zp[od + i].x, s1);
     }
   }
-  total2(s0, s1, &bn2, &rz);
+  if (!total2(s0, s1, &bn2, &rz)) return;
   const double bn = sqrt(bn2);
   bool done = !(bn > 0.0);  // of this component
   double beta = 0.0;
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(kProjThreads)
       }
     }
     double tp, unused;
-    total2(pap, 0.0, &tp, &unused);
+    if (!total2(pap, 0.0, &tp, &unused)) return;
     const double alpha = done ? 0.0 : rz / tp;
     double rn = 0.0, rz2 = 0.0;
     if (ONE) {
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(kProjThreads)
       }
     }
     double trn, trz;
-    total2(rn, rz2, &trn, &trz);
+    if (!total2(rn, rz2, &trn, &trz)) return;
     // not a number ends the component too (the caller sees it in x)
     done = done || !(sqrt(trn) >= 1e-15 * bn);
     beta = done ? 0.0 : trz / rz;

@@ -767,6 +767,10 @@ __global__ void __launch_bounds__(kOrthoThreads)
   const int G = gridDim.x, b = blockIdx.x;
   const int per = (N + G - 1) / G;
   const int i0 = min(N, b * per), i1 = min(N, i0 + per);
+  // not a number as the norm: the solver stops, and finds the error word
+  auto give_up = [&]() {
+    if (b == 0 && tid == 0) out[k] = __longlong_as_double(0x7ff8000000000000ll);
+  };
   double nrm = 0.0;
   for (int pass = 0; pass < 2; ++pass) {
     double* pp = part + (size_t)pass * kOrthoMaxK * G;
@@ -784,7 +788,7 @@ __global__ void __launch_bounds__(kOrthoThreads)
       }
       if (lane == 0) pp[(size_t)j * G + b] = s;
     }
-    grid_barrier(ctr, base + (unsigned)(pass + 1) * G, 61, err);
+    if (!grid_barrier(ctr, base + (unsigned)(pass + 1) * G, 61, err)) return give_up();
     if (ORDERED) {
       // a thread per vector adds the CTAs' parts in ascending order
       for (int j = tid; j < k; j += kOrthoThreads) {
@@ -837,7 +841,7 @@ __global__ void __launch_bounds__(kOrthoThreads)
   unsigned target = base + 3u * G;
   if (ORDERED) {
     // the norm's rows: 256 b + t + 256 G m, of other CTAs' chunks too
-    grid_barrier(ctr, target, 61, err);
+    if (!grid_barrier(ctr, target, 61, err)) return give_up();
     target += G;
     if (warp == 0) {
       const double s = tree256_dot(w, w, 256 * b, N, 256 * G, lane);
@@ -854,7 +858,7 @@ __global__ void __launch_bounds__(kOrthoThreads)
       pn[b] = s;
     }
   }
-  grid_barrier(ctr, target, 61, err);
+  if (!grid_barrier(ctr, target, 61, err)) return give_up();
   const double hn = sqrt(warp_total<ORDERED>(pn, G, lane));
   if (b == 0 && tid == 0) out[k] = hn;
   const double inv = 1.0 / hn;

@@ -42,6 +42,11 @@ int wbem_test_lu_factors(struct wbem_context* h, float* A_host, float* LU_host, 
  * WBEM_SOLVER_LU. Returns a wbem.h status. */
 int wbem_test_lu_apply(struct wbem_context* h, const double* v, double* z, int transpose);
 
+/* Writes `code` (a wbem.h status) into the handle's device error word, as a
+ * kernel whose bounded wait gave up does, for tests of what the calls report
+ * and that the word does not outlive the call that reports it. */
+int wbem_test_device_error(struct wbem_context* h, int code);
+
 /* Kernel profiling. With profiling on, the LU factorisation runs on the
  * handle's stream alone (no look-ahead overlap) and every launch of the
  * kernel classes below is bracketed by CUDA events on that stream, so the

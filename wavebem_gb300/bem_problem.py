@@ -105,6 +105,7 @@ def load_library(path: str = LIB_PATH):
     L.wbem_get_stats.argtypes = [H, C.POINTER(Stats)]
     L.wbem_test_lu_factors.argtypes = [H, C.c_void_p, C.c_void_p, C.c_void_p]
     L.wbem_test_lu_apply.argtypes = [H, dp, dp, C.c_int]
+    L.wbem_test_device_error.argtypes = [H, C.c_int]
     _lib = L
     return L
 

@@ -570,6 +570,7 @@ int gmres(wbem_context* h, const double* rhs, double* x, int restart, int max_st
       ++it;
       for (int j = 0; j <= k; ++j) H[(size_t)j * restart + k] = hv[j];
       const double hn = hv[k + 1];
+      if (!std::isfinite(hn)) return fail(h, WBEM_ERR_NONFINITE, "GMRES: non-finite residual");
       H[(size_t)(k + 1) * restart + k] = hn;
       for (int j = 0; j < k; ++j) {
         double a = H[(size_t)j * restart + k], b = H[(size_t)(j + 1) * restart + k];
@@ -712,8 +713,10 @@ int gmres_ir(wbem_context* h, const double* rhs, double* x, int transpose) {
     double res = 0;
     const int st = gmres(h, r, d, h->opt.gmres_restart, budget, std::max(eta * rnorm, 0.5 * target),
                          op32, prec, &it, &res);
-    // an inner solve that stops at its step budget still gives a correction
+    // an inner solve that stops at its step budget still gives a correction,
+    // unless it stopped for a wait that gave up
     if (st != WBEM_OK && st != WBEM_ERR_NOCONV) return st;
+    if (st == WBEM_ERR_NOCONV) CHK(check_device_error(h, "GMRES-IR"));
     total += it;
     ++outer;
     CU(launch_axpby(N, 1.0, d, 1.0, x, h->stream));
@@ -757,9 +760,7 @@ int resolved_solver(const wbem_context* h) {
   }
 }
 
-// Solve A x = rhs (transpose: A^T x = rhs) with the solver of the current
-// assembly, preparing its preconditioner once per assembly.
-int solve_assembled(wbem_context* h, const double* rhs, double* x, int transpose) {
+static int prepare_and_solve(wbem_context* h, const double* rhs, double* x, int transpose) {
   const int solver = resolved_solver(h);
   if (solver < 0) return fail(h, WBEM_ERR_ARG, "solver option does not apply to this precision");
   if (!h->factors_valid || h->factors_kind != solver) {
@@ -786,6 +787,23 @@ int solve_assembled(wbem_context* h, const double* rhs, double* x, int transpose
   if (solver == WBEM_SOLVER_GMRES) return gmres_fp64(h, rhs, x, transpose);
   if (solver == WBEM_SOLVER_LU) return solve_mixed(h, rhs, x, transpose);
   return gmres_ir(h, rhs, x, transpose);
+}
+
+// Solve A x = rhs (transpose: A^T x = rhs) with the solver of the current
+// assembly, preparing its preconditioner once per assembly. A solve that fails
+// reports the device's error word first, where it is set (a wait that gave up
+// shows in the solver as a residual that is not a number or does not fall),
+// and leaves it cleared and no work beside the handle's stream behind.
+int solve_assembled(wbem_context* h, const double* rhs, double* x, int transpose) {
+  const int st = prepare_and_solve(h, rhs, x, transpose);
+  if (st == WBEM_OK) return st;
+  const std::string what = h->err;
+  if (h->rhs_pending) {
+    h->rhs_pending = false;
+    CU(cudaStreamWaitEvent(h->stream, h->ev_rhs, 0));
+  }
+  CHK(check_device_error(h, "solve"));
+  return fail(h, st, what);
 }
 
 }  // namespace wbem
@@ -1410,6 +1428,14 @@ int wbem_adjoint(wbem_handle h, const double* dJ_dphi, const double* dJ_ddn, dou
   if (!h->have_solution) return fail(h, WBEM_ERR_STATE, "wbem_adjoint: solve first");
   cudaSetDevice(h->device);
   return adjoint_objective(h, dJ_dphi, dJ_ddn, dJ_dX, dJ_drhs);
+}
+
+int wbem_test_device_error(wbem_handle h, int code) {
+  if (!h) return WBEM_ERR_ARG;
+  cudaSetDevice(h->device);
+  const DevErr e{code, 0, 0, 0};
+  CU(copy_sync(h, h->d_err, &e, sizeof e, cudaMemcpyHostToDevice));
+  return WBEM_OK;
 }
 
 int wbem_set_profiling(wbem_handle h, int on) {

@@ -29,6 +29,20 @@ struct ChunkMeta {
   float4 geo;
 };
 
+// A cooperative launch by n CTAs, or by as many as the context holds at once:
+// where it has fewer SMs to use than the device (a partition, a limited
+// client), n is halved until the runtime accepts it. For kernels that run with
+// any number of CTAs; n is the number that was launched.
+template <typename Launch>
+inline cudaError_t launch_coresident(int& n, Launch launch) {
+  for (;;) {
+    const cudaError_t e = launch(n);
+    if (e != cudaErrorCooperativeLaunchTooLarge || n <= 1) return e;
+    cudaGetLastError();
+    n = (n + 1) / 2;
+  }
+}
+
 // A handle's quadrature rules. The kernels take the regular rule as a parameter
 // (__grid_constant__: constant memory that belongs to the launch) and the
 // singular rules from the handle's device copy of the tables, so that handles

@@ -1528,15 +1528,17 @@ static int tri_sweep(wbem_context* h, LuState& L, int mode, const float* in, flo
   }
   // more block rows than co-resident CTAs: each CTA takes block rows
   // blockIdx.x, blockIdx.x + grid, ... in sweep order (no size limit)
-  const int grid = std::min(nblk, cap);
+  int grid = std::min(nblk, cap);
   const float* LU = h->d_lu;
   DevErr* err = h->d_err;
   const int ld = L.ld;
   void* args[] = {(void*)&N, (void*)&ld, (void*)&nblk, (void*)&mode, (void*)&LU, (void*)&dinv,
                   (void*)&in, (void*)&out, (void*)&words, (void*)&epoch, (void*)&err};
   if (h->profiling) h->prof_trsv.begin(h->stream);
-  WB_CU(cudaLaunchCooperativeKernel((const void*)k_trsv_wave, dim3(grid), dim3(kTriThreads), args,
-                                    smem, h->stream));
+  WB_CU(launch_coresident(grid, [&](int n) {
+    return cudaLaunchCooperativeKernel((const void*)k_trsv_wave, dim3(n), dim3(kTriThreads), args, smem,
+                                       h->stream);
+  }));
   if (h->profiling) h->prof_trsv.end(h->stream, 2.0 * (double)N * N);
   return WBEM_OK;
 }

@@ -400,9 +400,12 @@ int project_field(wbem_context* h, int kind, const double* in, std::vector<doubl
   int max_it = 10 * N + 100;
   void* args[] = {(void*)&N, (void*)&max_it, (void*)&h->d_ncptr, (void*)&pv, (void*)&P->part, (void*)&P->ctr,
                   (void*)&h->d_err};
-  const bool one = (N + P->ctas - 1) / P->ctas <= kProjRows;
-  WB_CU(cudaLaunchCooperativeKernel(one ? (const void*)k_proj_pcg<true> : (const void*)k_proj_pcg<false>,
-                                    dim3(P->ctas), dim3(kProjThreads), args, 0, h->stream));
+  int ctas = P->ctas;
+  WB_CU(launch_coresident(ctas, [&](int n) {
+    const bool one = (N + n - 1) / n <= kProjRows;
+    return cudaLaunchCooperativeKernel(one ? (const void*)k_proj_pcg<true> : (const void*)k_proj_pcg<false>,
+                                       dim3(n), dim3(kProjThreads), args, 0, h->stream);
+  }));
   std::vector<double> xi(n3);
   WB_CU(cudaMemcpyAsync(xi.data(), pv.x, sizeof(double) * n3, cudaMemcpyDeviceToHost, h->stream));
   WB_CHK(check_device_error(h, "L2 projection"));

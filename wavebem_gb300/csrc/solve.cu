@@ -765,28 +765,34 @@ __global__ void __launch_bounds__(kOrthoThreads)
   constexpr int kWarps = kOrthoThreads / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = gridDim.x, b = blockIdx.x;
-  const int per = (N + G - 1) / G;
-  const int i0 = min(N, b * per), i1 = min(N, i0 + per);
+  // ordered: always kRedBlocks chunks of rows, however many CTAs share them
+  const int CH = ORDERED ? kRedBlocks : G;
+  const int per = (N + CH - 1) / CH;
+  auto begin = [&](int c) { return min(N, c * per); };
+  auto end = [&](int c) { return min(N, begin(c) + per); };
   // not a number as the norm: the solver stops, and finds the error word
   auto give_up = [&]() {
     if (b == 0 && tid == 0) out[k] = __longlong_as_double(0x7ff8000000000000ll);
   };
   double nrm = 0.0;
   for (int pass = 0; pass < 2; ++pass) {
-    double* pp = part + (size_t)pass * kOrthoMaxK * G;
+    double* pp = part + (size_t)pass * kOrthoMaxK * CH;
     // this CTA's part of every dot product: a warp per basis vector
-    for (int j = warp; j < k; j += kWarps) {
-      const double* vj = V + (size_t)j * N;
-      double s = 0.0;
-      if (ORDERED) {
-        s = tree256_dot(vj, w, i0, i1, 256, lane);
-      } else {
+    for (int c = b; c < CH; c += G) {
+      const int i0 = begin(c), i1 = end(c);
+      for (int j = warp; j < k; j += kWarps) {
+        const double* vj = V + (size_t)j * N;
+        double s = 0.0;
+        if (ORDERED) {
+          s = tree256_dot(vj, w, i0, i1, 256, lane);
+        } else {
 #pragma unroll 4
-        for (int i = i0 + lane; i < i1; i += 32) s = fma(vj[i], w[i], s);
+          for (int i = i0 + lane; i < i1; i += 32) s = fma(vj[i], w[i], s);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+          for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        }
+        if (lane == 0) pp[(size_t)j * CH + c] = s;
       }
-      if (lane == 0) pp[(size_t)j * G + b] = s;
     }
     if (!grid_barrier(ctr, base + (unsigned)(pass + 1) * G, 61, err)) return give_up();
     if (ORDERED) {
@@ -794,13 +800,13 @@ __global__ void __launch_bounds__(kOrthoThreads)
       for (int j = tid; j < k; j += kOrthoThreads) {
         double s = 0.0;
 #pragma unroll 8
-        for (int g = 0; g < G; ++g) s += __ldcg(pp + (size_t)j * G + g);
+        for (int g = 0; g < CH; ++g) s += __ldcg(pp + (size_t)j * CH + g);
         hs[j] = s;
         if (b == 0) out[j] = pass == 0 ? s : out[j] + s;
       }
     } else {
       for (int j = warp; j < k; j += kWarps) {
-        const double s = warp_total<false>(pp + (size_t)j * G, G, lane);
+        const double s = warp_total<false>(pp + (size_t)j * CH, CH, lane);
         if (lane == 0) {
           hs[j] = s;
           if (b == 0) out[j] = pass == 0 ? s : out[j] + s;
@@ -810,15 +816,17 @@ __global__ void __launch_bounds__(kOrthoThreads)
     __syncthreads();
     // w -= V h on this CTA's rows
     if (ORDERED) {
-      for (int i = i0 + tid; i < i1; i += kOrthoThreads) {
-        double s = 0.0;
+      for (int c = b; c < CH; c += G)
+        for (int i = begin(c) + tid; i < end(c); i += kOrthoThreads) {
+          double s = 0.0;
 #pragma unroll 8
-        for (int j = 0; j < k; ++j) s = fma(hs[j], V[(size_t)j * N + i], s);
-        w[i] -= s;
-      }
+          for (int j = 0; j < k; ++j) s = fma(hs[j], V[(size_t)j * N + i], s);
+          w[i] -= s;
+        }
       __syncthreads();
     } else {
       // 64 rows at a time, the vectors over 4 groups
+      const int i0 = begin(b), i1 = end(b);
       const int r = tid & (kOrthoRows - 1), q = tid / kOrthoRows;
       for (int c0 = i0; c0 < i1; c0 += kOrthoRows) {
         const int i = c0 + r;
@@ -837,15 +845,15 @@ __global__ void __launch_bounds__(kOrthoThreads)
       }
     }
   }
-  double* pn = part + (size_t)2 * kOrthoMaxK * G;
+  double* pn = part + (size_t)2 * kOrthoMaxK * CH;
   unsigned target = base + 3u * G;
   if (ORDERED) {
-    // the norm's rows: 256 b + t + 256 G m, of other CTAs' chunks too
+    // the norm's rows: 256 c + t + 256 CH m, of other CTAs' chunks too
     if (!grid_barrier(ctr, target, 61, err)) return give_up();
     target += G;
-    if (warp == 0) {
-      const double s = tree256_dot(w, w, 256 * b, N, 256 * G, lane);
-      if (lane == 0) pn[b] = s;
+    for (int c = b + warp * G; c < CH; c += kWarps * G) {
+      const double s = tree256_dot(w, w, 256 * c, N, 256 * CH, lane);
+      if (lane == 0) pn[c] = s;
     }
   } else {
 #pragma unroll
@@ -859,11 +867,12 @@ __global__ void __launch_bounds__(kOrthoThreads)
     }
   }
   if (!grid_barrier(ctr, target, 61, err)) return give_up();
-  const double hn = sqrt(warp_total<ORDERED>(pn, G, lane));
+  const double hn = sqrt(warp_total<ORDERED>(pn, CH, lane));
   if (b == 0 && tid == 0) out[k] = hn;
   const double inv = 1.0 / hn;
   if (hn > 0.0)
-    for (int i = i0 + tid; i < i1; i += kOrthoThreads) v[i] = inv * w[i];
+    for (int c = b; c < CH; c += G)
+      for (int i = begin(c) + tid; i < end(c); i += kOrthoThreads) v[i] = inv * w[i];
 }
 
 // The same step for small N by one cluster of 16 CTAs: the parts meet in
@@ -1006,11 +1015,14 @@ cudaError_t launch_ortho(int N, int k, const double* V, double* w, double* v, do
     return cudaLaunchKernelEx(&c, k_ortho_cluster, N, k, V, w, v, out);
   }
   unsigned base = *epoch;
-  *epoch += (ordered ? 4u : 3u) * (unsigned)n_ctas;
   void* args[] = {(void*)&N, (void*)&k, (void*)&V, (void*)&w, (void*)&v, (void*)&part,
                   (void*)&out, (void*)&ctr, (void*)&base, (void*)&err};
   const void* f = ordered ? (const void*)k_ortho<true> : (const void*)k_ortho<false>;
-  return cudaLaunchCooperativeKernel(f, dim3(n_ctas), dim3(kOrthoThreads), args, 0, s);
+  const cudaError_t e = launch_coresident(n_ctas, [&](int n) {
+    return cudaLaunchCooperativeKernel(f, dim3(n), dim3(kOrthoThreads), args, 0, s);
+  });
+  *epoch += (ordered ? 4u : 3u) * (unsigned)n_ctas;
+  return e;
 }
 
 __global__ void k_axpy_basis(int N, int k, const double* __restrict__ V, const double* __restrict__ h,

@@ -24,6 +24,12 @@ int wbem_test_gemm_bf16x3(int M, int Nc, int K, const float* dA, const float* dB
  * arguments, conditions and synchronisation as wbem_test_gemm_bf16x3. */
 int wbem_test_gemm_tf32(int M, int Nc, int K, const float* dA, const float* dB, float* dC);
 
+/* y = S x, S FP32 (N x N, row-major, leading dimension ld >= N, a multiple of
+ * 4), x and y FP64, all device pointers: the inner operator of the refinement
+ * solver. Runs on the legacy default stream and synchronizes. Returns a wbem.h
+ * status. */
+int wbem_test_matvec_s32(int N, int ld, const float* dS, const double* dx, double* dy);
+
 /* The mixed-precision system matrix and its LU factors, for factor tests.
  * After wbem_assemble (WBEM_PREC_MIXED) and wbem_set_bc: forms the FP32
  * system matrix S (the constrained operator with alpha on its diagonal, rows

@@ -112,7 +112,8 @@ cudaError_t launch_set_rows(int nrows, const int* crow, const double* val, doubl
                             cudaStream_t s);
 
 // block-Jacobi (FP64)
-cudaError_t launch_matvec_s32(int N, int ld, const float* S, const double* x, double* y,
+// xf: N floats of scratch, 16-byte aligned, that no other stream uses meanwhile
+cudaError_t launch_matvec_s32(int N, int ld, const float* S, const double* x, float* xf, double* y,
                               cudaStream_t s);
 cudaError_t launch_matvec_s32_t(int N, int ld, const float* S, const double* x, double* y,
                                 double* part, cudaStream_t s);

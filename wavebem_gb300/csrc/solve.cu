@@ -12,6 +12,7 @@
 #include <stdint.h>
 #include <algorithm>
 #include <atomic>
+#include "dfloat.cuh"
 #include "kernels.h"
 #include "../../include/wbem.h"
 
@@ -192,32 +193,40 @@ cudaError_t launch_matvec_mixed(int N, int mode, const float2* P, const uint8_t*
 // y = S x for the FP32 system matrix S (row-major, leading dimension ld, the
 // constrained operator with alpha on its diagonal): the inner operator of the
 // refinement solver. A CTA takes 8 rows, a thread four columns (16 bytes) of
-// each per step; products and sums in FP32, at most kMvFlush terms per FP32
-// partial sum (as pairs of floats beyond, FP64 across the threads), so the
-// operator is S to about 1e-6 relative, at 4 bytes of HBM traffic per entry.
-// HBM-bound: 317 us (5.1 TB/s) at N = 20,011 with a warp per row, now 271 us.
+// each per step; products and sums in FP32, kMvFlush terms per FP32 sum and
+// FP64 beyond, so the operator is S to about 1e-6 relative, at 4 bytes of HBM
+// traffic per entry. Four such sums are added without rounding error in FP32
+// before they go to FP64, whose pipe would hold up the stream otherwise; for
+// the same reason x is rounded to FP32 once, by k_round_x.
+// HBM-bound: 317 us (5.1 TB/s) at N = 20,011 with a warp per row, now 255 us.
 constexpr int kMvRows32 = 8;
-constexpr int kMvFlush = 64;
+constexpr int kMvFlush = 16;
+
+__global__ void k_round_x(int N, const double* __restrict__ x, float* __restrict__ xf) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < N) xf[i] = (float)x[i];
+}
 
 __global__ void __launch_bounds__(kMvThreads, 2)
-    k_matvec_s32(int N, int ld, const float* __restrict__ S, const double* __restrict__ x,
+    k_matvec_s32(int N, int ld, const float* __restrict__ S, const float* __restrict__ xf,
                  double* __restrict__ y) {
   constexpr int R = kMvRows32;
   const int row0 = blockIdx.x * R, tid = threadIdx.x;
   const float* row[R];
-  df acc[R];
+  double acc[R];
   float a[R][4];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     row[r] = S + (size_t)min(row0 + r, N - 1) * ld;
-    acc[r] = {0.f, 0.f};
+    acc[r] = 0.0;
     a[r][0] = a[r][1] = a[r][2] = a[r][3] = 0.f;
   }
   auto flush = [&]() {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const df u = two_sum(a[r][0], a[r][1]), w = two_sum(a[r][2], a[r][3]);
-      acc[r] = df_add(acc[r], df_add(u, w));
+      const df u = two_sum(a[r][0], a[r][1]), w = two_sum(a[r][2], a[r][3]), t = two_sum(u.hi, w.hi);
+      acc[r] += (double)t.hi;
+      acc[r] += widen(t.lo + (u.lo + w.lo));
       a[r][0] = a[r][1] = a[r][2] = a[r][3] = 0.f;
     }
   };
@@ -227,14 +236,13 @@ __global__ void __launch_bounds__(kMvThreads, 2)
     float4 v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = __ldcs(reinterpret_cast<const float4*>(row[r] + j));
-    // x may be a basis vector of odd length N: 8-byte aligned only
-    const float f0 = (float)x[j], f1 = (float)x[j + 1], f2 = (float)x[j + 2], f3 = (float)x[j + 3];
+    const float4 f = *reinterpret_cast<const float4*>(xf + j);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      a[r][0] = __fmaf_rn(v[r].x, f0, a[r][0]);
-      a[r][1] = __fmaf_rn(v[r].y, f1, a[r][1]);
-      a[r][2] = __fmaf_rn(v[r].z, f2, a[r][2]);
-      a[r][3] = __fmaf_rn(v[r].w, f3, a[r][3]);
+      a[r][0] = __fmaf_rn(v[r].x, f.x, a[r][0]);
+      a[r][1] = __fmaf_rn(v[r].y, f.y, a[r][1]);
+      a[r][2] = __fmaf_rn(v[r].z, f.z, a[r][2]);
+      a[r][3] = __fmaf_rn(v[r].w, f.w, a[r][3]);
     }
     if (++n == kMvFlush) {
       flush();
@@ -243,20 +251,18 @@ __global__ void __launch_bounds__(kMvThreads, 2)
   }
   flush();
   if (nq + tid < N) {  // the last one to three columns
-    const float f = (float)x[nq + tid];
+    const float f = xf[nq + tid];
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = df_add(acc[r], two_prod(row[r][nq + tid], f));
+    for (int r = 0; r < R; ++r) acc[r] += (double)row[r][nq + tid] * (double)f;
   }
-  double v[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) v[r] = df_to_double(acc[r]);
-  const double s = cta_rows_sum<R>(v);
+  const double s = cta_rows_sum<R>(acc);
   if (tid < R && row0 + tid < N) y[row0 + tid] = s;
 }
 
-cudaError_t launch_matvec_s32(int N, int ld, const float* S, const double* x, double* y,
+cudaError_t launch_matvec_s32(int N, int ld, const float* S, const double* x, float* xf, double* y,
                               cudaStream_t s) {
-  k_matvec_s32<<<(N + kMvRows32 - 1) / kMvRows32, kMvThreads, 0, s>>>(N, ld, S, x, y);
+  k_round_x<<<(N + 255) / 256, 256, 0, s>>>(N, x, xf);
+  k_matvec_s32<<<(N + kMvRows32 - 1) / kMvRows32, kMvThreads, 0, s>>>(N, ld, S, xf, y);
   return cudaGetLastError();
 }
 

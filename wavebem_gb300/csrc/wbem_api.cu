@@ -683,8 +683,8 @@ int gmres_ir(wbem_context* h, const double* rhs, double* x, int transpose) {
     if (transpose)
       CU(launch_matvec_s32_t(N, ld, h->d_lu, a, b, h->d_part + 256 * 128, h->stream));
     else
-      CU(launch_matvec_s32(N, ld, h->d_lu, a, b, h->stream));
-    h->launches += transpose ? 2 : 1;
+      CU(launch_matvec_s32(N, ld, h->d_lu, a, reinterpret_cast<float*>(h->d_xs), b, h->stream));
+    h->launches += 2;
     return WBEM_OK;
   };
   auto prec = [&](const double* a, double* b) -> int {
@@ -1428,6 +1428,16 @@ int wbem_adjoint(wbem_handle h, const double* dJ_dphi, const double* dJ_ddn, dou
   if (!h->have_solution) return fail(h, WBEM_ERR_STATE, "wbem_adjoint: solve first");
   cudaSetDevice(h->device);
   return adjoint_objective(h, dJ_dphi, dJ_ddn, dJ_dX, dJ_drhs);
+}
+
+int wbem_test_matvec_s32(int N, int ld, const float* dS, const double* dx, double* dy) {
+  if (N < 1 || ld < N || (ld & 3) || !dS || !dx || !dy) return WBEM_ERR_ARG;
+  float* xf = nullptr;
+  if (cudaMalloc(&xf, sizeof(float) * N) != cudaSuccess) return WBEM_ERR_NOMEM;
+  cudaError_t e = launch_matvec_s32(N, ld, dS, dx, xf, dy, nullptr);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  cudaFree(xf);
+  return e == cudaSuccess ? WBEM_OK : WBEM_ERR_CUDA;
 }
 
 int wbem_test_device_error(wbem_handle h, int code) {

@@ -1013,7 +1013,10 @@ __global__ void __launch_bounds__(kSingWarps * 32)
     __syncthreads();
     if (tid < 8) {
       double* M = (tid < 4 ? Nm : Dm) + (size_t)row * N;
-      for (int e = 0; e < n; ++e) M[ids[e][tid & 3]] += sums[e][tid];
+      for (int e = 0; e < n; ++e) {
+        M[ids[e][tid & 3]] += sums[e][tid];
+        __syncwarp(0xffu);  // the next panel's shared vertex may be another thread's
+      }
     }
     __syncthreads();
   }

@@ -109,7 +109,11 @@ __global__ void __launch_bounds__(kProjWarps * 32)
 // Vectors of the solve, planar (component d of node i at d N + i): right-hand
 // side b gathered from the panels (rhs) or given (in b), r = b, zp = (r / diag,
 // p = 0), x = 0. The mass matrix by rows: the rcnt[i] entries (rcol, rval) of
-// node i from 4 ncptr[i] on.
+// node i from 4 ncptr[i] on; a node of many panels keeps the entries of a column
+// apart (merging them is a search per entry, by one thread).
+constexpr int kProjRow = 16;    // entries of a row held in shared memory
+constexpr int kProjMerge = 64;  // panels of a node whose entries are merged
+
 struct ProjVectors {
   double *b, *dinv, *r, *x, *p, *ap;
   double2* zp;
@@ -126,6 +130,7 @@ __global__ void k_proj_init(int N, const int* __restrict__ ncptr, const int* __r
   int* col = v.rcol + 4 * (size_t)ncptr[i];
   double* val = v.rval + 4 * (size_t)ncptr[i];
   int n = 0;
+  const bool merge = ncptr[i + 1] - ncptr[i] <= kProjMerge;
   for (int e = ncptr[i]; e < ncptr[i + 1]; ++e) {
     const int c = ncent[e] >> 2, k = ncent[e] & 3;
     const double* row = mass + 16 * (size_t)c + 4 * k;
@@ -133,7 +138,7 @@ __global__ void k_proj_init(int N, const int* __restrict__ ncptr, const int* __r
     const int id[4] = {q.x, q.y, q.z, q.w};
     m += row[k];
     for (int u = 0; u < 4; ++u) {
-      int t = 0;
+      int t = merge ? 0 : n;
       while (t < n && col[t] != id[u]) ++t;
       if (t < n) {
         val[t] += row[u];
@@ -180,7 +185,6 @@ __device__ __forceinline__ void proj_warp_sum2(double& a, double& b, int lane) {
 // Bound by the barriers' latency and the FP64 chain between them: 0.39 ms for
 // the three components at N = 2,000 (41 iterations), where the host's three
 // solves, one after the other, took 2.3 ms.
-constexpr int kProjRow = 16;
 constexpr int kProjRows = 32;
 constexpr int kProjThreads = 3 * kProjRows;
 

@@ -334,7 +334,9 @@ static int build_topology(wbem_context* h) {
   tile_lists(tstart64, tptr64, tent64);
   // order of an FP64 tile's panels: groups of four that share no column where
   // that can be had (k_tile_far adds such a group's entries at once). The
-  // members are looked for a quarter of the list apart.
+  // members are looked for a quarter of the list apart, among kSeek panels (a
+  // tile of thousands has a vertex that most of them share).
+  constexpr int kSeek = 1024;
   std::vector<int2> in;
   std::vector<char> used;
   for (int t = 0; t < h->n_tiles64; ++t) {
@@ -345,7 +347,8 @@ static int build_topology(wbem_context* h) {
     std::fill(taken, taken + 256, -1);
     for (int k = 0; k < n; ++k) {
       int pick = -1, any = -1, i = (k % 4 * quarter + k / 4) % n;
-      for (int tries = 0; tries < n && pick < 0; ++tries, i = i + 1 < n ? i + 1 : 0) {
+      for (int tries = 0; tries < n && pick < 0 && (tries < kSeek || any < 0);
+           ++tries, i = i + 1 < n ? i + 1 : 0) {
         if (used[i]) continue;
         any = i;
         bool free = true;

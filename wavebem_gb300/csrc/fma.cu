@@ -1132,7 +1132,6 @@ struct FmaState {
   double* d_blocks = nullptr;    // near-field diagonal blocks of the system
   double* d_a = nullptr;         // product inputs (N each)
   double* d_b = nullptr;
-  QuadTables* d_qt = nullptr;
   FmaConst cst{};                // expansion constants, a parameter of every kernel
   std::vector<void*> owned;
 };
@@ -1504,8 +1503,6 @@ static int fma_build(wbem_context* h, FmaState* F, const QuadTables& qt) {
   WB_CHK(fma_alloc(h, F, &F->d_blocks, (size_t)nb * kBJ * kBJ));
   WB_CHK(fma_alloc(h, F, &F->d_a, (size_t)N));
   WB_CHK(fma_alloc(h, F, &F->d_b, (size_t)N));
-  std::vector<QuadTables> qv(1, qt);
-  WB_CHK(fma_upload(h, F, &F->d_qt, qv));
   // constants
   FmaConst& fc = F->cst;
   fc = FmaConst{};
@@ -1681,7 +1678,7 @@ int assemble_fma(wbem_context* h, const QuadTables& qt) {
     k_fma_close_val<<<(unsigned)((cnt + 127) / 128), 128, 0, h->stream>>>(
         (long long)cnt, F->d_plist + off, F->d_pair_row, F->d_pair_pan, h->d_X, h->d_dnset,
         h->d_cell_dofs, h->d_rec, F->d_tgt_leaf, F->d_pan_pos, F->d_pos_leaf, F->lev[F->L].d_cen,
-        F->d_xloc, F->d_ppos, F->d_close_val, F->d_qt, F->cst);
+        F->d_xloc, F->d_ppos, F->d_close_val, h->d_quad, F->cst);
     WB_CU(cudaGetLastError());
     h->launches++;
   }

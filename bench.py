@@ -263,16 +263,16 @@ def run_reference(args, rank, world):
 # move O(N^2) bytes per launch, so a launch at N dofs is scaled by
 # (N / 8192)^2.
 NCU_TRAFFIC = {
-    "k_tile_mixed": 17.5424e6 + 1314.548e6,
-    "k_matvec_mixed": 537.038080e6 + 3.272192e6,
-    "k_trsv_wave": 136.424192e6 + 3.058176e6,
+    "k_tile_mixed": 19.637504e6 + 1314.780928e6,
+    "k_matvec_mixed": 537.101568e6 + 2.960384e6,
+    "k_trsv_wave": 136.495360e6 + 2.752256e6,
 }
 
 
 # Warp instructions of one far-field assembly launch at N = 8,192 (ncu
 # smsp__inst_executed.sum); they scale with the (row, panel) pairs, i.e. with
 # N^2 on the same family of meshes.
-NCU_TILE_INSTR = 2949815885.0
+NCU_TILE_INSTR = 2161757708.0
 
 # DRAM bytes of a trailing-update launch over its algorithmic C traffic
 # (8 bytes per element of C, read and written once): 2.205 GB against

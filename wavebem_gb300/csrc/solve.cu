@@ -111,6 +111,10 @@ cudaError_t launch_matvec_fp64(int N, int mode, const double* Nm, const double* 
 // per step where N is even. HBM-bound: 285 us (4.0 TB/s) at N = 12,000 with a
 // warp per row, now 182 us (6.3 TB/s); 1.55 ms at N = 32,768, now 1.21 ms.
 constexpr int kMvRowsM = 4;
+// Up to this size every CTA splits x itself (SPLIT): its few columns cost less
+// than the launch. A vmult and a compute_rhs on host arrays, us, this way / with
+// k_split_x: 600 dofs 82.5 / 86, 1,500 86 / 89, 2,000 112 / 95.
+constexpr int kMvSplitCols = 1500;
 
 __global__ void k_split_x(int N, const double* __restrict__ x, float2* __restrict__ xs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -125,7 +129,7 @@ __device__ __forceinline__ void pair_fma(df& acc, float ah, float al, float xh, 
   acc = df_add(acc, p);
 }
 
-template <bool EVEN>
+template <bool EVEN, bool SPLIT>
 __global__ void __launch_bounds__(kMvThreads)
     k_matvec_mixed(int N, int mode, const float2* __restrict__ P, const uint8_t* __restrict__ mask,
                    const double* __restrict__ alpha, const float2* __restrict__ xs,
@@ -138,13 +142,24 @@ __global__ void __launch_bounds__(kMvThreads)
   df acc[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) acc[r] = {0.f, 0.f};
+  auto x_pair = [&](int j) {
+    if (!SPLIT) return xs[j];
+    const df v = df_from_double(x[j]);
+    return make_float2(v.hi, v.lo);
+  };
   if (EVEN) {
 #pragma unroll 2
     for (int j = 2 * tid; j < N; j += 2 * kMvThreads) {
       float4 a[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) a[r] = __ldcs(reinterpret_cast<const float4*>(row[r] + j));
-      const float4 xv = *reinterpret_cast<const float4*>(xs + j);
+      float4 xv;
+      if (SPLIT) {
+        const float2 u = x_pair(j), v = x_pair(j + 1);
+        xv = make_float4(u.x, u.y, v.x, v.y);
+      } else {
+        xv = *reinterpret_cast<const float4*>(xs + j);
+      }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         pair_fma(acc[r], a[r].x, a[r].y, xv.x, xv.y);
@@ -157,7 +172,7 @@ __global__ void __launch_bounds__(kMvThreads)
       float2 a[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) a[r] = __ldcs(row[r] + j);
-      const float2 xv = xs[j];
+      const float2 xv = x_pair(j);
 #pragma unroll
       for (int r = 0; r < R; ++r) pair_fma(acc[r], a[r].x, a[r].y, xv.x, xv.y);
     }
@@ -181,12 +196,19 @@ __global__ void __launch_bounds__(kMvThreads)
 cudaError_t launch_matvec_mixed(int N, int mode, const float2* P, const uint8_t* mask,
                                 const double* alpha, const double* x, float2* xs, double* y,
                                 cudaStream_t s) {
-  k_split_x<<<(N + 255) / 256, 256, 0, s>>>(N, x, xs);
   const int g = (N + kMvRowsM - 1) / kMvRowsM;
+  if (N <= kMvSplitCols) {
+    if (N & 1)
+      k_matvec_mixed<false, true><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, nullptr, x, y);
+    else
+      k_matvec_mixed<true, true><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, nullptr, x, y);
+    return cudaGetLastError();
+  }
+  k_split_x<<<(N + 255) / 256, 256, 0, s>>>(N, x, xs);
   if (N & 1)
-    k_matvec_mixed<false><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, xs, x, y);
+    k_matvec_mixed<false, false><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, xs, x, y);
   else
-    k_matvec_mixed<true><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, xs, x, y);
+    k_matvec_mixed<true, false><<<g, kMvThreads, 0, s>>>(N, mode, P, mask, alpha, xs, x, y);
   return cudaGetLastError();
 }
 

@@ -343,6 +343,10 @@ __global__ void __launch_bounds__(128)
         lk[j] = u ? l[j] : 0.0;
         lpk[j] = u ? lp[j] : 0.0;
       }
+      if (!__any_sync(0xffffffffu, use)) {  // no row, no multiplier, or singular pairs alone
+        if (lane < 24) wmom[warp][k][lane] = 0.0;
+        continue;
+      }
       double v[24];
 #pragma unroll
       for (int i = 0; i < 24; ++i) v[i] = 0.0;

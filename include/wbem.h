@@ -44,7 +44,12 @@ extern "C" {
 #define WBEM_ERR_TIMEOUT 8    /* a bounded device wait gave up */
 
 /* precision forms */
-#define WBEM_PREC_FP64 0  /* plain: FP64 everywhere */
+#define WBEM_PREC_FP64 0  /* plain: FP64 storage, products and solver. Panels beyond six of their
+                             radii, with rules of 3 to 6 points per direction: FP64 centre terms
+                             and a remainder of relative size radius / distance (its square up to
+                             32 radii) summed over the points in pairs of FP32 numbers (48 bits),
+                             which leaves the entries as far from exact sums as FP64 point by
+                             point does; everything else in FP64 */
 #define WBEM_PREC_MIXED 1 /* FP32 far field (double-float panel base + FP32 quadrature deltas),
                              FP64 singular/near field and alpha; (hi, lo) FP32 storage;
                              FP32 LU (TF32 tensor-core updates) or FP32 inner GMRES,

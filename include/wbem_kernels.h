@@ -65,7 +65,7 @@ typedef struct {
   int gemm_launches;
   double diag_ms;       /* k_diag_block: 128 x 128 diagonal LU + triangle inverses */
   int diag_launches;
-  double panel_ms;      /* k_panel_gemm + k_rowpanel_update (FP32 SIMT panels) */
+  double panel_ms;      /* k_strip + k_panel_small (FP32 SIMT panels) */
   int panel_launches;
   double matvec_ms;     /* system mat-vecs of the refinement (k_matvec_mixed) */
   double matvec_bytes;  /*   matrix bytes they stream: 8 N^2 per launch */
@@ -84,11 +84,12 @@ int wbem_get_kernel_profile(struct wbem_context* h, wbem_kernel_profile* p);
 int wbem_set_stream(struct wbem_context* h, void* cuda_stream);
 
 /* Hull force from device-resident fields without touching the allocator.
- * No counterpart in the reference. For callers that must not allocate device
- * memory: a time loop that evaluates the force after every Newton iteration
- * on its own stream (allocating and freeing device memory synchronises the
- * whole device) or that runs with device memory owned by another framework's
- * caching allocator. Same integral as wbem_hull_force, but hull_cells
+ * No counterpart in the reference. For callers whose fields are on the device
+ * already and that must neither wait nor allocate device memory: a time loop
+ * that evaluates the force after every Newton iteration on its own stream, or
+ * one that runs with device memory owned by another framework's caching
+ * allocator (wbem_hull_force copies its fields, grows buffers of the handle with
+ * the number of panels and waits for its result). Same integral as wbem_hull_force, but hull_cells
  * (n_hull panel indices, caller numbering), phi and dphi_dn (caller order) and
  * force (one double) are DEVICE pointers; U is a host array of 3 doubles.
  * The work is queued on `stream` (NULL: the handle's stream) and the call

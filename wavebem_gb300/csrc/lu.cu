@@ -13,7 +13,7 @@
 //
 // Step k (block size kNB = 128), inside outer panels of kNB2 = 512 columns:
 //   1. k_diag_block: LU of A_kk (one CTA, shared memory), plus the inverses of
-//      its unit-lower and upper factors;
+//      its unit-lower and upper factors, all by one elimination;
 //   2. L_ik = A_ik inv(U_kk) and U_kj = inv(L_kk) A_kj (FP32 SIMT), then the
 //      panel's own trailing update A_ij -= L_ik U_kj (FP32, K = 128): for the
 //      next block's 128 rows (the strip the next diagonal block needs) by
@@ -1219,7 +1219,7 @@ static cudaError_t run_gemm(const GemmMaps& mp, const CUtensorMap& cmap, int cro
 // block in no longer than a link: it reads the next block's words before it
 // multiplies the last one, and asks for its tiles three blocks ahead in L2 and
 // one ahead in registers. Per sweep, with flags and shuffled sums per block
-// before: 151 us (268) at 12,000 dofs, 473 us (930) at 32,768. (Tiles staged
+// before: 147 us (268) at 12,000 dofs, 470 us (930) at 32,768. (Tiles staged
 // two deep in shared memory: 161 to 180 us and 647 us with cp.async, whose
 // copies pass through the same pipe twice; 390 us and 1.49 ms with a bulk copy
 // per tile row.)

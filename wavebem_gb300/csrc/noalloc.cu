@@ -1,13 +1,13 @@
 // Hull force on device-resident fields, without any device allocation.
 //
-// wbem_hull_force allocates a small buffer for its per-panel partial sums on
-// every call and frees it again. Freeing device memory synchronises the whole
-// device, and allocating goes around whatever memory pool the caller runs
-// with. A time-stepping caller that evaluates the force after every Newton
-// iteration, on a stream of its own and with device memory handed out by
-// another framework's caching allocator, cannot afford either. This variant
-// takes device pointers only and keeps its partial sums in a fixed array in
-// the library's own device memory, so it never calls the allocator.
+// wbem_hull_force takes host fields, waits for its result and grows device
+// buffers of the handle with the number of panels; growing synchronises the
+// whole device and goes around whatever memory pool the caller runs with. A
+// time-stepping caller that evaluates the force after every Newton iteration,
+// on a stream of its own and with device memory handed out by another
+// framework's caching allocator, cannot afford these. This variant takes
+// device pointers only and keeps its partial sums in a fixed array in the
+// library's own device memory, so it never calls the allocator.
 #include <cuda_runtime.h>
 #include <atomic>
 #include <cmath>

@@ -1,7 +1,6 @@
 // Host construction of the library's quadrature rules (plain C++, no CUDA):
 // the Gauss-Legendre rule on [0, 1] and the vertex-singular rule of the unit
-// square. build_quadrature (wbem_api.cu) turns them into the constant-memory
-// tables; tests/quadrature_check.cpp prints them for the CPU comparison with
+// square. build_quadrature (wbem_api.cu) turns them into the handle's tables; tests/quadrature_check.cpp prints them for the CPU comparison with
 // the oracle's rules.
 #pragma once
 #include <cmath>
